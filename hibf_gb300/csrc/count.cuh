@@ -145,6 +145,14 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
+            if (u > 0 && base + static_cast<uint64_t>(u * 32) >= n)
+            {
+                // a call of the early exit often ends within a pass: no hashing for values that are not there
+#pragma unroll
+                for (int i = 0; i < H; ++i)
+                    off[u][i] = 0;
+                continue;
+            }
             uint64_t const idx = base + static_cast<uint64_t>(u * 32 + lane);
             uint64_t const v = idx < n ? __ldcg(vals + idx) : 0u;
             if (stage && idx < n)

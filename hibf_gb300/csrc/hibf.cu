@@ -1561,8 +1561,10 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "too many technical bins in total");
                 // per-bin descriptors
                 std::vector<uint2> descs(off[n_ibfs]);
+                std::vector<uint32_t> max_seg(n_ibfs, 0);
                 for (uint64_t k = 0; k < n_ibfs; ++k)
                 {
+                    uint64_t head = 0; // first bin of the summation segment
                     for (uint64_t b = 0; b < bins[k]; ++b)
                     {
                         uint64_t const i = off[k] + b;
@@ -1600,7 +1602,12 @@ extern "C"
                             if (prev_merged || prev_end)
                                 flags |= F_HEAD;
                         }
-                        descs[i] = make_uint2(id, flags);
+                        if (flags & F_HEAD)
+                            head = b;
+                        uint32_t const dist = static_cast<uint32_t>(b - head);
+                        if (flags & (F_MERGED | F_RUN_END))
+                            max_seg[k] = std::max(max_seg[k], dist + 1u);
+                        descs[i] = make_uint2(id, flags | dist << kDistShift);
                     }
                 }
                 // depth of the hierarchy (longest merged-bin path from the root); a cycle makes it unbounded
@@ -1682,6 +1689,7 @@ extern "C"
                         nd.hash_funs = static_cast<uint32_t>(hash_funs[k]);
                         nd.desc_offset = static_cast<uint32_t>(off[k]);
                         nd.lpv_log2 = lanes_per_value_log2(bw);
+                        nd.max_seg = max_seg[k];
                         uint32_t const need = bw > 32 ? static_cast<uint32_t>(64 * bw) : (64u << nd.lpv_log2);
                         cpw = std::max(cpw, need);
                         h->nodes.push_back(nd);

@@ -23,7 +23,7 @@ struct alignas(16) dev_node
     uint32_t hash_funs;
     uint32_t desc_offset;
     uint32_t lpv_log2;
-    uint32_t pad;
+    uint32_t max_seg; // bins of the widest summation segment that ends in a report or a descent
 };
 
 

@@ -35,6 +35,7 @@ constexpr uint32_t F_MERGED = 1u;
 constexpr uint32_t F_DELETED = 2u;
 constexpr uint32_t F_RUN_END = 4u;
 constexpr uint32_t F_HEAD = 8u;
+constexpr uint32_t kDistShift = 4; // the flags word's other bits: the bin's distance from its segment's first bin
 
 constexpr unsigned long long kEmpty = ~0ull;
 // stats words: tasks, value visits the reference's traversal implies, value visits executed
@@ -234,6 +235,24 @@ __device__ inline bool wait_arrival(query_params const & p, uint64_t q)
     }
 }
 
+// Sum of bin b's summation segment up to and including b, for 32 bins of which this lane holds one: c = the bin's
+// count, dist = its distance from the segment's first bin (desc.y >> kDistShift), carry = the sum of the segment that
+// is open where the 32 bins begin.  A warp-wide prefix sum and the prefix in front of the segment's first bin.
+__device__ __forceinline__ uint32_t segment_sum(uint32_t c, uint32_t dist, uint32_t carry, int lane)
+{
+    uint32_t s = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        uint32_t const y = __shfl_up_sync(kFullMask, s, o);
+        if (lane >= o)
+            s += y;
+    }
+    uint32_t const l = static_cast<uint32_t>(lane);
+    uint32_t const before = __shfl_sync(kFullMask, s, dist < l ? static_cast<int>(l - dist - 1u) : 0);
+    return dist < l ? s - before : (dist > l ? s + carry : s);
+}
+
 // The state of a task after counting all but `remaining` of its values, from each summation segment's sum so far x
 // and its number of bins w (every bin of a segment adds its count, and a value adds at most one to every bin, so the
 // final sum lies in [x, top] with top = x + w * remaining):
@@ -245,24 +264,90 @@ __device__ inline bool wait_arrival(query_params const & p, uint64_t q)
 // A sum that could exceed the counter range is never decided (its wrapped value is not bounded).  Either early state
 // gives the same outcome as counting every value.
 //
-// `next` (if given) receives how many more values must be counted before the state can change at all (top falls by
-// at most w and x grows by at most w per value): an open segment passes for good no sooner than after
-// ceil((t - x) / w) values (and ceil((top - mask) / w) for a sum that could wrap), and turns unreachable no sooner
-// than after ceil((top - t + 1) / w); a task turns hopeless only once every reachable segment can be unreachable, and
-// (membership) decided once every open segment can be settled.  kNever: no later change is possible (a segment that
-// reached the threshold keeps a bulk count open).
+// `next` receives after how many more values the next check is due (kNever: none, a bulk count with a segment that
+// reached the threshold stays open): the farthest of the open segments' distances to being settled, each projected
+// from the share of its values that hit so far, to pass or to fail, whichever is nearer.
+//
+// Every warp runs this a few times per task, between a few dozen loads, so its instructions count: at 8,192 user bins
+// a level below the root (whose rows L2 holds) spent 8,400 instructions per task of 734 counted values, three
+// quarters of them in checks.  Hence 32-bit sums (the caller takes the 64-bit form, segment_state, for tasks whose
+// sums could pass 2^31), no scan where every segment is one bin, float divisions, and a projected distance: the
+// distance at which the outcome could change at the earliest took 4.7 checks per task, the projected one takes 1.9
+// for 1% more values (8,192 bins, simulated over 400 queries).
 constexpr int kOpen = 0;
 constexpr int kHopeless = 1;
 constexpr int kDecided = 2;
 constexpr unsigned int kNever = 0xFFFFFFFFu;
+constexpr uint64_t kNarrowSums = 1ull << 31; // tasks with n * (bins of the widest segment) below this use 32-bit sums
+
+__device__ __forceinline__ int task_state(query_params const & p, dev_node const & nd, uint32_t const * counts,
+                                          uint32_t done, uint32_t remaining, uint64_t thr, int lane,
+                                          unsigned int & next)
+{
+    uint2 const * __restrict__ d = p.descs + nd.desc_offset;
+    uint32_t const mask = static_cast<uint32_t>(min(p.count_mask, uint64_t{0xFFFFFFFFu}));
+    uint32_t const t = static_cast<uint32_t>(min(thr, uint64_t{0xFFFFFFFFu}));
+    float const fdone = static_cast<float>(done);
+    bool reach = false, open = false, never = false;
+    float far = 0.0f;
+    uint32_t carry = 0;
+    for (uint32_t c = 0; c < nd.bins; c += 32)
+    {
+        uint32_t const b = c + lane;
+        bool const valid = b < nd.bins;
+        uint32_t const f = valid ? __ldg(&d[b].y) : 0u;
+        uint32_t x = valid ? counts[b] : 0u;
+        bool const ends = (f & (F_RUN_END | F_MERGED)) != 0;
+        uint32_t w = 1;
+        if (nd.max_seg > 1)
+        {
+            x = segment_sum(x, f >> kDistShift, carry, lane);
+            carry = __shfl_sync(kFullMask, ends ? 0u : x, 31);
+            w = (f >> kDistShift) + 1u;
+        }
+        uint32_t const top = x + w * remaining;
+        bool const reachable = ends && (top >= t || top > mask);
+        bool const passed = x >= t && top <= mask;
+        reach = reach || reachable;
+        if (reachable && !p.decide && x >= t)
+            never = true; // a reached segment stays reachable: the bulk count never turns hopeless
+        if (reachable && !passed)
+        {
+            open = true;
+            // misses still needed to fail, hits still needed to pass, and this segment's rates of both so far
+            float const miss = fmaxf(static_cast<float>(w * done - x), 0.5f);
+            float const hit = fmaxf(static_cast<float>(x), 0.5f);
+            float const wrap = top > mask ? static_cast<float>(top - mask) : 0.0f;
+            float const fail = fmaxf(top >= t ? static_cast<float>(top - t + 1u) : 0.0f, wrap);
+            float k = __fdividef(fail * fdone, miss);
+            if (p.decide)
+                k = fminf(k, fmaxf(x < t ? __fdividef(static_cast<float>(t - x) * fdone, hit) : 0.0f,
+                                   __fdividef(wrap * fdone, miss)));
+            far = fmaxf(far, k);
+        }
+    }
+    bool const any_reach = __any_sync(kFullMask, reach);
+    bool const any_open = __any_sync(kFullMask, open);
+    next = static_cast<unsigned int>(
+        fminf(__uint_as_float(__reduce_max_sync(kFullMask, __float_as_uint(far))), 2.0e9f)) + 1u;
+    if (__any_sync(kFullMask, never))
+        next = kNever;
+    if (!any_reach)
+        return kHopeless;
+    return p.decide && !any_open ? kDecided : kOpen;
+}
 
 __device__ __forceinline__ unsigned long long ceil_div(unsigned long long a, unsigned long long w)
 {
     return (a + w - 1u) / w;
 }
 
-__device__ inline int segment_state(query_params const & p, dev_node const & nd, uint32_t const * counts,
-                                    uint64_t remaining, uint64_t thr, int lane, unsigned int * next = nullptr)
+// task_state with 64-bit sums, for the tasks that need them (n * widest segment of 2^31 or more) and for a threshold
+// of 0 before anything is counted.  `next` is the earliest distance at which the state can change at all (top falls
+// by at most w and x grows by at most w per value).  Not inlined: it is hardly ever taken, and its registers would
+// weigh on the counting code.
+static __device__ __noinline__ int segment_state(query_params const & p, dev_node const & nd, uint32_t const * counts,
+                                                 uint64_t remaining, uint64_t thr, int lane, unsigned int & next)
 {
     uint2 const * d = p.descs + nd.desc_offset;
     unsigned long long carry = 0, carry_w = 0;
@@ -313,34 +398,26 @@ __device__ inline int segment_state(query_params const & p, dev_node const & nd,
         bool const cut = (lastf & (F_MERGED | F_RUN_END)) != 0;
         carry = cut ? 0ull : lastx;
         carry_w = cut ? 0ull : lastw;
-        if (next)
+        if (reachable)
         {
-            if (reachable)
+            unsigned long long const unreach = ceil_div(top >= thr ? top - thr + 1u : top - mask, w);
+            unsigned long long k = 0;
+            if (p.decide)
             {
-                unsigned long long const unreach = ceil_div(top >= thr ? top - thr + 1u : top - mask, w);
-                unsigned long long k = 0;
-                if (p.decide)
-                {
-                    if (!passed)
-                        k = min(unreach, max(x < thr ? ceil_div(thr - x, w) : 0ull,
-                                             top > mask ? ceil_div(top - mask, w) : 0ull));
-                }
-                else if (x >= thr)
-                    never = true; // a reached segment stays reachable: the bulk count never turns hopeless
-                else
-                    k = unreach;
-                wait = max(wait, static_cast<unsigned int>(min(k, 0xFFFFFFFEull)));
+                if (!passed)
+                    k = min(unreach, max(x < thr ? ceil_div(thr - x, w) : 0ull,
+                                         top > mask ? ceil_div(top - mask, w) : 0ull));
             }
+            else if (x >= thr)
+                never = true; // a reached segment stays reachable: the bulk count never turns hopeless
+            else
+                k = unreach;
+            wait = max(wait, static_cast<unsigned int>(min(k, 0xFFFFFFFEull)));
         }
-        else if (any_reachable && !p.decide)
-            return kOpen; // only hopelessness is of interest: one reachable segment settles it
     }
-    if (next)
-    {
-        bool const nv = __any_sync(kFullMask, never);
-        unsigned int const wmax = __reduce_max_sync(kFullMask, wait);
-        *next = nv ? kNever : max(wmax, 1u);
-    }
+    bool const nv = __any_sync(kFullMask, never);
+    unsigned int const wmax = __reduce_max_sync(kFullMask, wait);
+    next = nv ? kNever : max(wmax, 1u);
     if (!any_reachable)
         return kHopeless;
     if (!p.decide)
@@ -378,17 +455,107 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
     }
 }
 
-// The bin scan of a counted task: report user bins and queue child IBFs whose summation segment reaches the
-// threshold, then retire the task (one warp; `counts` = the task's per-bin counts).
-__device__ inline void emit_task(query_params const & p, dev_node const & nd, uint32_t const * counts, uint64_t q,
-                                 uint32_t depth, uint64_t n, uint64_t done, uint64_t thr, int lane,
-                                 unsigned long long & n_tasks, unsigned long long & n_visits,
-                                 unsigned long long & n_executed)
+// Reports and descents of 32 bins of a counted task: this lane's bin `ds` ends its segment with `sum` (already reduced
+// to the counter range).  `level`: the launch answers one level, so nobody reads the children before it ends.
+__device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsigned long long sum, bool pass,
+                                          uint64_t q, uint32_t depth, int lane)
+{
+    unsigned const lt_mask = (1u << lane) - 1u;
+    uint64_t const gq = q + p.q_base;
+    bool const emit_ub = (ds.y & F_RUN_END) && pass;
+    bool const emit_child = (ds.y & F_MERGED) && pass;
+    unsigned const rb = __ballot_sync(kFullMask, emit_ub);
+    if (rb)
+    {
+        unsigned const nr = __popc(rb);
+        unsigned long long base = 0;
+        if (lane == 0)
+        {
+            base = atomicAdd(p.ctrl + C_NREC, static_cast<unsigned long long>(nr));
+            atomicAdd(p.qcount + gq, nr);
+            if (base + nr > p.rec_cap)
+                atomicOr(p.ctrl + C_ERROR, E_OVERFLOW_REC);
+        }
+        base = __shfl_sync(kFullMask, base, 0);
+        if (emit_ub)
+        {
+            unsigned long long const r = base + __popc(rb & lt_mask);
+            if (r < p.rec_cap)
+            {
+                p.rec_q[r] = static_cast<uint32_t>(gq);
+                p.rec_ub[r] = ds.x;
+                p.rec_cnt[r] = sum;
+            }
+        }
+    }
+    unsigned const cb = __ballot_sync(kFullMask, emit_child);
+    if (cb)
+    {
+        unsigned const nc = __popc(cb);
+        if (depth + 1u > p.max_depth)
+        {
+            if (lane == 0)
+                atomicOr(p.ctrl + C_ERROR, E_CYCLE);
+        }
+        else
+        {
+            unsigned long long base = 0;
+            if (lane == 0)
+            {
+                if (!p.level)
+                    atomicAdd(p.ctrl + C_PENDING, static_cast<unsigned long long>(nc));
+                base = atomicAdd(p.ctrl + C_TAIL, static_cast<unsigned long long>(nc));
+            }
+            base = __shfl_sync(kFullMask, base, 0);
+            if (emit_child)
+            {
+                unsigned long long const s = base + __popc(cb & lt_mask);
+                if (s < p.task_cap)
+                {
+                    if (p.level)
+                        p.tasks[s] = make_task(q, depth + 1u, ds.x);
+                    else
+                        atomicExch(p.tasks + s, make_task(q, depth + 1u, ds.x));
+                }
+                else
+                {
+                    atomicOr(p.ctrl + C_ERROR, E_OVERFLOW_TASK);
+                    if (!p.level)
+                        atomicAdd(p.ctrl + C_PENDING, ~0ull); // this child will never run
+                }
+                if (!p.level)
+                    __threadfence();
+            }
+        }
+    }
+}
+
+// A finished task leaves the count of unfinished ones (the level schedule keeps none: its launches end by themselves)
+// and enters the work counters.
+__device__ __forceinline__ void retire_task(query_params const & p, uint64_t q, uint64_t n, uint64_t done, int lane,
+                                            unsigned long long & n_tasks, unsigned long long & n_visits,
+                                            unsigned long long & n_executed)
+{
+    if (lane != 0)
+        return;
+    if (p.qwork)
+        atomicAdd(p.qwork + q + p.q_base, static_cast<unsigned long long>(done));
+    if (!p.level)
+    {
+        __threadfence();
+        atomicAdd(p.ctrl + C_PENDING, ~0ull);
+    }
+    ++n_tasks;
+    n_visits += n;
+    n_executed += done;
+}
+
+// The bin scan of a counted task with 64-bit sums (see segment_state).
+static __device__ __noinline__ void emit_bins_wide(query_params const & p, dev_node const & nd, uint32_t const * counts,
+                                                   uint64_t q, uint32_t depth, uint64_t thr, int lane)
 {
     uint2 const * d = p.descs + nd.desc_offset;
     unsigned long long carry = 0;
-    unsigned const lt_mask = (1u << lane) - 1u;
-    uint64_t const gq = q + p.q_base;
     for (uint32_t c = 0; c < nd.bins; c += 32)
     {
         uint32_t const b = c + lane;
@@ -410,86 +577,47 @@ __device__ inline void emit_task(query_params const & p, dev_node const & nd, ui
                 f = f || fy;
             }
         }
-        uint64_t const sum = x & p.count_mask;
-        bool const pass = sum >= thr;
-        bool const emit_ub = valid && (ds.y & F_RUN_END) && pass;
-        bool const emit_child = valid && (ds.y & F_MERGED) && pass;
-
-        unsigned const rb = __ballot_sync(kFullMask, emit_ub);
-        if (rb)
-        {
-            unsigned const nr = __popc(rb);
-            unsigned long long base = 0;
-            if (lane == 0)
-            {
-                base = atomicAdd(p.ctrl + C_NREC, static_cast<unsigned long long>(nr));
-                atomicAdd(p.qcount + gq, nr);
-                if (base + nr > p.rec_cap)
-                    atomicOr(p.ctrl + C_ERROR, E_OVERFLOW_REC);
-            }
-            base = __shfl_sync(kFullMask, base, 0);
-            if (emit_ub)
-            {
-                unsigned long long const r = base + __popc(rb & lt_mask);
-                if (r < p.rec_cap)
-                {
-                    p.rec_q[r] = static_cast<uint32_t>(gq);
-                    p.rec_ub[r] = ds.x;
-                    p.rec_cnt[r] = sum;
-                }
-            }
-        }
-        unsigned const cb = __ballot_sync(kFullMask, emit_child);
-        if (cb)
-        {
-            unsigned const nc = __popc(cb);
-            if (depth + 1u > p.max_depth)
-            {
-                if (lane == 0)
-                    atomicOr(p.ctrl + C_ERROR, E_CYCLE);
-            }
-            else
-            {
-                unsigned long long base = 0;
-                if (lane == 0)
-                {
-                    atomicAdd(p.ctrl + C_PENDING, static_cast<unsigned long long>(nc));
-                    base = atomicAdd(p.ctrl + C_TAIL, static_cast<unsigned long long>(nc));
-                }
-                base = __shfl_sync(kFullMask, base, 0);
-                if (emit_child)
-                {
-                    unsigned long long const s = base + __popc(cb & lt_mask);
-                    if (s < p.task_cap)
-                    {
-                        atomicExch(p.tasks + s, make_task(q, depth + 1u, ds.x));
-                    }
-                    else
-                    {
-                        atomicOr(p.ctrl + C_ERROR, E_OVERFLOW_TASK);
-                        atomicAdd(p.ctrl + C_PENDING, ~0ull); // this child will never run
-                    }
-                    __threadfence();
-                }
-            }
-        }
+        unsigned long long const sum = x & p.count_mask;
+        emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane);
         unsigned long long const lastx = __shfl_sync(kFullMask, x, 31);
         uint32_t const lastf = __shfl_sync(kFullMask, ds.y, 31);
         carry = (lastf & (F_MERGED | F_RUN_END)) ? 0ull : lastx;
     }
-    __syncwarp();
-    if (lane == 0)
-    {
-        if (p.qwork)
-            atomicAdd(p.qwork + q + p.q_base, static_cast<unsigned long long>(done));
-        __threadfence();
-        atomicAdd(p.ctrl + C_PENDING, ~0ull); // this task retires
-        ++n_tasks;
-        n_visits += n;
-        n_executed += done;
-    }
 }
 
+// The bin scan of a counted task: report user bins and queue child IBFs whose summation segment reaches the
+// threshold, then retire the task (one warp; `counts` = the task's per-bin counts).
+__device__ __forceinline__ void emit_task(query_params const & p, dev_node const & nd, uint32_t const * counts,
+                                          uint64_t q, uint32_t depth, uint64_t n, uint64_t done, uint64_t thr,
+                                          int lane, unsigned long long & n_tasks, unsigned long long & n_visits,
+                                          unsigned long long & n_executed)
+{
+    if (n * nd.max_seg < kNarrowSums)
+    {
+        uint2 const * __restrict__ d = p.descs + nd.desc_offset;
+        uint32_t carry = 0;
+        for (uint32_t c = 0; c < nd.bins; c += 32)
+        {
+            uint32_t const b = c + lane;
+            bool const valid = b < nd.bins;
+            uint2 const ds = valid ? __ldg(d + b) : make_uint2(0u, 0u);
+            uint32_t x = valid ? counts[b] : 0u;
+            if (nd.max_seg > 1)
+            {
+                x = segment_sum(x, ds.y >> kDistShift, carry, lane);
+                carry = __shfl_sync(kFullMask, (ds.y & (F_MERGED | F_RUN_END)) ? 0u : x, 31);
+            }
+            unsigned long long const sum = x & p.count_mask;
+            emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane);
+        }
+    }
+    else
+    {
+        emit_bins_wide(p, nd, counts, q, depth, thr, lane);
+    }
+    __syncwarp();
+    retire_task(p, q, n, done, lane, n_tasks, n_visits, n_executed);
+}
 
 template <int H, int V>
 __device__ void process_task(query_params const & p, unsigned long long task, uint32_t * counts, int lane,
@@ -538,8 +666,16 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
     bool const stage_root = p.stage && depth == 0;
     uint64_t const staged = p.stage && depth > 0 ? p.staged[q] : 0u;
     bool const adaptive = p.ee_stages == kEarlyExitAdaptive && n >= p.ee_min;
+    uint64_t const most = n * nd.max_seg; // no segment's sum passes this
+    bool const narrow = most < kNarrowSums;
     unsigned int next = kNever;
-    int state = segment_state(p, nd, counts, n, thr, lane, adaptive ? &next : nullptr);
+    int state = kOpen;
+    if (!narrow || thr == 0)
+        state = segment_state(p, nd, counts, n, thr, lane, next);
+    else if (most < thr && most <= p.count_mask)
+        state = kHopeless;
+    else // nothing counted yet: a one-bin segment can fail after n - thr + 1 values and pass after thr
+        next = static_cast<unsigned int>(thr > n ? 1u : (p.decide ? min(n - thr + 1u, thr) : n - thr + 1u));
     uint32_t const stages = !adaptive && state == kOpen && n >= p.ee_min ? p.ee_stages : 0u;
     uint32_t s = 0;
 #pragma unroll 1
@@ -548,9 +684,13 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         uint64_t stop = n; // the next checkpoint past `done` (checkpoints are below 100%, so below n), else the end
         if (adaptive)
         {
-            // the earliest position where the outcome can change, at least ee_step values on
+            // where the outcome is expected to be settled, at least ee_step values on and at a whole warp of values
+            // from the task's first (a pass then has no idle lanes); a rest of less than that is counted at once
             if (next != kNever)
-                stop = min(n, done + static_cast<uint64_t>(max(next, p.ee_step)));
+            {
+                uint64_t const at = (done + static_cast<uint64_t>(max(next, p.ee_step)) + 31u) / 32u * 32u;
+                stop = at + 32u < n ? at : n;
+            }
         }
         else
         {
@@ -577,7 +717,9 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         if (done < n)
         {
             __syncwarp();
-            state = segment_state(p, nd, counts, n - done, thr, lane, adaptive ? &next : nullptr);
+            state = narrow ? task_state(p, nd, counts, static_cast<uint32_t>(done), static_cast<uint32_t>(n - done), thr,
+                                        lane, next)
+                           : segment_state(p, nd, counts, n - done, thr, lane, next);
         }
     }
     __syncwarp();
@@ -585,16 +727,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         p.staged[q] = static_cast<uint32_t>(done); // read by the next level's launch
     if (state == kHopeless)
     {
-        if (lane == 0)
-        {
-            if (p.qwork)
-                atomicAdd(p.qwork + q + p.q_base, static_cast<unsigned long long>(done));
-            __threadfence();
-            atomicAdd(p.ctrl + C_PENDING, ~0ull); // retires without results or children
-            ++n_tasks;
-            n_visits += n;
-            n_executed += done;
-        }
+        retire_task(p, q, n, done, lane, n_tasks, n_visits, n_executed); // without results or children
         return;
     }
 
@@ -608,7 +741,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
 #    define HIBF_QUERY_MIN_BLOCKS 2
 #endif
 template <int H, int V>
-__global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(query_params p)
+__global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
     int const lane = threadIdx.x & 31;
@@ -828,7 +961,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(query_para
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
 template <int H>
-__global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(query_params p)
+__global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
     __shared__ unsigned long long s_task;
@@ -943,7 +1076,7 @@ constexpr int kCostFeatures = 6;
 using features_kernel_t = void (*)(query_params, uint32_t, float *);
 
 template <int H>
-__global__ void __launch_bounds__(256) k_query_features(query_params p, uint32_t probe, float * __restrict__ out)
+__global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_params const p, uint32_t probe, float * __restrict__ out)
 {
     extern __shared__ uint32_t s_counts[];
     int const lane = threadIdx.x & 31;
