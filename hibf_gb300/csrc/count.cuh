@@ -139,6 +139,14 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
             P[e][k] = 0;
     int acc = 0;
 
+    // values of the next pass are loaded while this pass's rows are on their way
+    uint64_t nv[U];
+#pragma unroll
+    for (int u = 0; u < U; ++u)
+    {
+        uint64_t const idx = static_cast<uint64_t>(u * 32 + lane);
+        nv[u] = idx < n ? __ldcg(vals + idx) : 0u;
+    }
     for (uint64_t base = 0; base < n; base += BLOCK)
     {
         uint64_t off[U][H];
@@ -154,12 +162,18 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
                 continue;
             }
             uint64_t const idx = base + static_cast<uint64_t>(u * 32 + lane);
-            uint64_t const v = idx < n ? __ldcg(vals + idx) : 0u;
+            uint64_t const v = nv[u];
             if (stage && idx < n)
                 stage[idx] = v;
 #pragma unroll
             for (int i = 0; i < H; ++i)
                 off[u][i] = hash_row(v, c_hash_seeds[i], rp.hash_shift, rp.bin_size) * rp.row_words;
+        }
+#pragma unroll
+        for (int u = 0; u < U; ++u)
+        {
+            uint64_t const idx = base + static_cast<uint64_t>(BLOCK + u * 32 + lane);
+            nv[u] = idx < n ? __ldcg(vals + idx) : 0u;
         }
         // one group: GS masks per lane (GS sub-steps of LPV-lane groups), their H * W loads issued together
         auto group = [&](int s)
