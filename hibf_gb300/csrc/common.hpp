@@ -86,15 +86,6 @@ inline uint64_t padded_row_words(uint64_t bin_words)
     return (bin_words + 3) / 4 * 4;
 }
 
-// Lanes per value for a row of bin_words words: the next power of two, capped at a warp.
-inline uint32_t lanes_per_value_log2(uint64_t bin_words)
-{
-    uint32_t l = 0;
-    while ((1ull << l) < bin_words && l < 5)
-        ++l;
-    return l;
-}
-
 inline void require_device()
 {
     int n = 0;

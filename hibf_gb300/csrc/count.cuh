@@ -27,9 +27,11 @@ struct row_params
 };
 
 // `added` (warp-uniform) masks went into the planes since the last flush, so planes k with 2^k > added are zero and
-// are not transposed.  Lane j of an LPV-lane group holds word W * j (+ the caller's offset of `out`) of its rows.
-template <int LPV, int K, bool ATOMIC, int W = 1>
-__device__ __forceinline__ void planes_flush_to(uint64_t (&P)[K], uint32_t * out, int lane, int added)
+// are not transposed.  Lane j of an LPV-lane group holds word W * j (+ the caller's offset of `out`) of its rows.  Full
+// warps (LPV = 32) write the counters of the row's `words` words only: a wide row's counters end with its last word.
+template <int LPV, int K, int W = 1>
+__device__ __forceinline__ void planes_flush_to(uint64_t (&P)[K], uint32_t * out, int lane, int added,
+                                                uint32_t words)
 {
     int const kmax = 32 - __clz(added);
     uint32_t lo[K], hi[K];
@@ -51,6 +53,8 @@ __device__ __forceinline__ void planes_flush_to(uint64_t (&P)[K], uint32_t * out
 #pragma unroll
     for (int j = 0; j < LPV; ++j)
     {
+        if (LPV == 32 && static_cast<uint32_t>(W * j) >= words)
+            break;
         uint32_t gm = 0;
 #pragma unroll
         for (int g = 0; g < 32 / LPV; ++g)
@@ -62,18 +66,8 @@ __device__ __forceinline__ void planes_flush_to(uint64_t (&P)[K], uint32_t * out
             cl += static_cast<uint32_t>(__popc(lo[k] & gm)) << k;
             ch += static_cast<uint32_t>(__popc(hi[k] & gm)) << k;
         }
-        if constexpr (ATOMIC)
-        {
-            if (cl)
-                atomicAdd(out + 64 * W * j + lane, cl);
-            if (ch)
-                atomicAdd(out + 64 * W * j + 32 + lane, ch);
-        }
-        else
-        {
-            out[64 * W * j + lane] += cl;
-            out[64 * W * j + 32 + lane] += ch;
-        }
+        out[64 * W * j + lane] += cl;
+        out[64 * W * j + 32 + lane] += ch;
     }
 }
 
@@ -107,15 +101,14 @@ __device__ __forceinline__ void load_row_words(uint64_t const * p, uint64_t (&w)
 // engine while the kernel runs, and a task reads them only after their chunk's arrival counter (query.cuh), so the
 // loads must not come from a non-coherent cache.  Each task reads its values once, so L1 gives them nothing.
 //
-// One warp counts vals[0, n) into counts[0, 64 * LPV * W) with H hash functions.  ATOMIC: counters shared with other
-// warps.  A row is read by LPV lanes, each loading W consecutive words (W = 2: one 16-byte load; the row stride
-// must then be even).  Each lane hashes U values per pass and keeps their H row offsets; the row words of
+// One warp counts vals[0, n) into counts[0, 64 * LPV * W) with H hash functions.  A row is read by LPV lanes, each
+// loading W consecutive words (W = 2: one 16-byte load; the row stride must then be even).  Each lane hashes U values per pass and keeps their H row offsets; the row words of
 // GS = 4 * UM masks per lane are loaded together, so GS * H * W loads per lane are in flight.  K planes count up to
 // 2^K - 1 masks between flushes.
 //
 // stage (optional): every value read is also stored at stage[i], so that later reads of the same values (the lower
 // levels of an in-place host batch) come from device memory instead of the host link.
-template <int LPV, int H, int K, bool ATOMIC, int UM = 1, int W = 1, bool EF = false>
+template <int LPV, int H, int K, int UM = 1, int W = 1, bool EF = false>
 __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const * __restrict__ vals, uint64_t n,
                                            uint32_t * counts, int lane, uint64_t * __restrict__ stage = nullptr)
 {
@@ -224,7 +217,7 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
                 {
 #pragma unroll
                     for (int e = 0; e < W; ++e)
-                        planes_flush_to<LPV, K, ATOMIC, W>(P[e], counts + 64 * e, lane, acc);
+                        planes_flush_to<LPV, K, W>(P[e], counts + 64 * e, lane, acc, rp.bin_words);
                     acc = 0;
                 }
             }
@@ -244,107 +237,43 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
     {
 #pragma unroll
         for (int e = 0; e < W; ++e)
-            planes_flush_to<LPV, K, ATOMIC, W>(P[e], counts + 64 * e, lane, acc);
+            planes_flush_to<LPV, K, W>(P[e], counts + 64 * e, lane, acc, rp.bin_words);
     }
 }
 
-// Rows wider than a warp (bin_words > 32): lanes stride over the words, set bits are added one by one.
-__device__ __forceinline__ void warp_count_wide(row_params const & rp, uint64_t const * __restrict__ vals, uint64_t n,
-                                                uint32_t * counts, int lane, uint64_t * __restrict__ stage = nullptr)
-{
-    for (uint64_t i = 0; i < n; ++i)
-    {
-        uint64_t const v = __ldcg(vals + i);
-        if (stage && lane == 0)
-            stage[i] = v;
-        uint64_t off[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            off[k] = (static_cast<uint32_t>(k) < rp.hash_funs)
-                       ? hash_row(v, c_hash_seeds[k], rp.hash_shift, rp.bin_size) * rp.row_words
-                       : 0u;
-        for (uint32_t wi = lane; wi < rp.bin_words; wi += 32)
-        {
-            uint64_t x = ~0ull;
-#pragma unroll
-            for (int k = 0; k < 5; ++k)
-                if (static_cast<uint32_t>(k) < rp.hash_funs)
-                    x &= __ldg(rp.words + off[k] + wi);
-            while (x)
-            {
-                int const b = __ffsll(static_cast<long long>(x)) - 1;
-                x &= x - 1;
-                atomicAdd(counts + 64 * wi + b, 1u);
-            }
-        }
-    }
-}
-
-template <int H, bool ATOMIC, bool EF = false>
+template <int H, bool EF = false>
 __device__ __forceinline__ void warp_count_lpv(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
                                                uint64_t n, uint32_t * counts, int lane, uint64_t * stage = nullptr)
 {
     switch (lpv_log2)
     {
     case 0:
-        warp_count<1, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<1, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 1:
-        warp_count<2, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<2, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 2:
-        warp_count<4, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<4, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 3:
-        warp_count<8, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<8, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 4:
-        warp_count<16, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<16, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     default:
-        warp_count<32, H, 7, ATOMIC, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<32, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
     }
 }
 
-// Dispatch on lanes-per-value for a compile-time hash function count (rows wider than a warp use the generic loop).
-template <int H, bool ATOMIC>
-__device__ __forceinline__ void warp_count_h(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
-                                             uint64_t n, uint32_t * counts, int lane, uint64_t * stage = nullptr)
+// Rows wider than a warp (more than kSlabWords words) are counted in slabs of kSlabWords words, one word per lane.
+__device__ __forceinline__ row_params row_slab(row_params const & rp, uint32_t first_word)
 {
-    if (rp.bin_words > 32)
-        warp_count_wide(rp, vals, n, counts, lane, stage);
-    else
-        warp_count_lpv<H, ATOMIC>(rp, lpv_log2, vals, n, counts, lane, stage);
-}
-
-// Dispatch on the node's hash function count and lanes-per-value (log2).  K = 7 planes: flush every 124 masks per
-// lane.
-template <bool ATOMIC>
-__device__ __forceinline__ void warp_count_any(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
-                                               uint64_t n, uint32_t * counts, int lane)
-{
-    if (rp.bin_words > 32)
-    {
-        warp_count_wide(rp, vals, n, counts, lane);
-        return;
-    }
-    switch (rp.hash_funs)
-    {
-    case 1:
-        warp_count_lpv<1, ATOMIC>(rp, lpv_log2, vals, n, counts, lane);
-        break;
-    case 2:
-        warp_count_lpv<2, ATOMIC>(rp, lpv_log2, vals, n, counts, lane);
-        break;
-    case 3:
-        warp_count_lpv<3, ATOMIC>(rp, lpv_log2, vals, n, counts, lane);
-        break;
-    case 4:
-        warp_count_lpv<4, ATOMIC>(rp, lpv_log2, vals, n, counts, lane);
-        break;
-    default:
-        warp_count_lpv<5, ATOMIC>(rp, lpv_log2, vals, n, counts, lane);
-    }
+    row_params sp = rp;
+    sp.words += first_word;
+    sp.bin_words = min(kSlabWords, rp.bin_words - first_word);
+    return sp;
 }
 
 } // namespace hibf_gb300

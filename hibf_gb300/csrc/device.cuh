@@ -15,6 +15,23 @@ namespace hibf_gb300
 {
 
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
+constexpr uint32_t kSlabWords = 32; // words of a row that a warp reads at once, one per lane
+
+// Lanes per value (log2) for a row, or the last slab of a row, of `words` 64-bit words (1 to kSlabWords).
+__host__ __device__ constexpr uint32_t lanes_log2(uint32_t words)
+{
+    uint32_t l = 0;
+    while ((1u << l) < words && l < 5u)
+        ++l;
+    return l;
+}
+
+// Counters the counting loop writes for rows of `words` words: 64 per lane of a row that one warp reads at once, 64 per
+// word of a wider one.
+__host__ __device__ constexpr uint32_t row_counters(uint32_t words)
+{
+    return words > kSlabWords ? 64u * words : 64u << lanes_log2(words);
+}
 
 // The multiplicative hashing seeds of include/hibf/interleaved_bloom_filter.hpp:172-176.  A filter's bit positions
 // are defined by them, so bit-exact parity requires the same five constants.

@@ -1688,10 +1688,9 @@ extern "C"
                         nd.hash_shift = static_cast<uint32_t>(__builtin_clzll(bin_sizes[k]));
                         nd.hash_funs = static_cast<uint32_t>(hash_funs[k]);
                         nd.desc_offset = static_cast<uint32_t>(off[k]);
-                        nd.lpv_log2 = lanes_per_value_log2(bw);
+                        nd.lpv_log2 = lanes_log2(static_cast<uint32_t>(std::min<uint64_t>(bw, kSlabWords)));
                         nd.max_seg = max_seg[k];
-                        uint32_t const need = bw > 32 ? static_cast<uint32_t>(64 * bw) : (64u << nd.lpv_log2);
-                        cpw = std::max(cpw, need);
+                        cpw = std::max(cpw, row_counters(static_cast<uint32_t>(bw)));
                         h->nodes.push_back(nd);
                         h->stores.push_back(std::move(st));
                     }

@@ -196,49 +196,18 @@ __global__ void k_widen(uint64_t * __restrict__ dst, uint32_t dst_row_words, uin
     }
 }
 
-// bulk_contains (src/interleaved_bloom_filter.cpp:204-291) for many values: out[v * bin_words + j] = AND of word j
-// of the h rows.  LPV lanes per value, one row word per lane per pass (strided when the row is wider than a warp).
-template <int LPV>
-__global__ void k_bulk_contains(row_params rp, uint64_t const * __restrict__ values, uint64_t n,
-                                uint64_t * __restrict__ out)
-{
-    constexpr int G = 32 / LPV;
-    int const lane = threadIdx.x & 31;
-    int const g = lane / LPV;
-    int const j = lane % LPV;
-    uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
-    uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
-    for (uint64_t base = warp * G; base < n; base += nwarps * G)
-    {
-        uint64_t const i = base + g;
-        if (i >= n)
-            continue;
-        uint64_t const v = values[i];
-        uint64_t off[5];
-#pragma unroll
-        for (int k = 0; k < 5; ++k)
-            off[k] = (static_cast<uint32_t>(k) < rp.hash_funs)
-                       ? hash_row(v, c_hash_seeds[k], rp.hash_shift, rp.bin_size) * rp.row_words
-                       : 0u;
-        for (uint32_t w = j; w < rp.bin_words; w += LPV)
-        {
-            uint64_t x = ~0ull;
-#pragma unroll
-            for (int k = 0; k < 5; ++k)
-                if (static_cast<uint32_t>(k) < rp.hash_funs)
-                    x &= __ldg(rp.words + off[k] + w);
-            out[i * rp.bin_words + w] = x;
-        }
-    }
-}
-
-// bulk_contains for rows of up to 32 words with H hash functions: the same work mapping as the counting loop
-// (count.cuh) -- LPV lanes per row, lanes hash U values each, the H row words of four sub-steps are loaded together
-// (4 * H loads per lane in flight) -- and each lane stores its word of the AND.
+// bulk_contains (src/interleaved_bloom_filter.cpp:204-291) for many values with H hash functions: out[v * bin_words + j]
+// = AND of word j of the h rows.  The same work mapping as the counting loop (count.cuh) -- LPV lanes per row, lanes
+// hash U values each, the H row words of four sub-steps are loaded together (4 * H loads per lane in flight) -- and
+// each lane stores its word of the AND.  The grid's second dimension is the slab of a row wider than a warp, from
+// word `first_slab` on.
 template <int LPV, int H>
-__global__ void __launch_bounds__(256) k_bulk_contains_h(row_params rp, uint64_t const * __restrict__ values,
-                                                         uint64_t n, uint64_t * __restrict__ out)
+__global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_t first_slab,
+                                                         uint64_t const * __restrict__ values, uint64_t n,
+                                                         uint64_t * __restrict__ out)
 {
+    uint32_t const w0 = (first_slab + blockIdx.y) * kSlabWords;
+    row_params const rp = row_slab(row, w0);
     constexpr int G = 32 / LPV;
     constexpr int U = LPV >= 4 ? 1 : 4 / LPV;
     constexpr int STEPS = U * LPV;
@@ -247,8 +216,9 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params rp, uint64_t
     int const g = lane / LPV;
     int const j = lane % LPV;
     bool const wj = static_cast<uint32_t>(j) < rp.bin_words;
-    uint64_t const bw = rp.bin_words;
+    uint64_t const bw = row.bin_words;
     uint64_t const * __restrict__ words = rp.words + j;
+    out += w0;
     uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
     uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     for (uint64_t base = warp * BLOCK; base < n; base += nwarps * BLOCK)
@@ -301,68 +271,70 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params rp, uint64_t
 }
 
 template <int H>
-void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint64_t const * d_values, uint64_t n,
-                       uint64_t * d_out, unsigned grid, cudaStream_t s)
+void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint32_t first_slab, uint32_t slabs,
+                       uint64_t const * d_values, uint64_t n, uint64_t * d_out, unsigned grid_x, cudaStream_t s)
 {
+    dim3 const grid(grid_x, slabs);
     switch (lpv_log2)
     {
     case 0:
-        k_bulk_contains_h<1, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<1, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 1:
-        k_bulk_contains_h<2, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<2, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 2:
-        k_bulk_contains_h<4, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<4, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 3:
-        k_bulk_contains_h<8, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<8, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 4:
-        k_bulk_contains_h<16, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<16, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     default:
-        k_bulk_contains_h<32, H><<<grid, 256, 0, s>>>(rp, d_values, n, d_out);
+        k_bulk_contains_h<32, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
     }
 }
 
-// bulk_count over n values into one counting vector: every warp counts a contiguous chunk into the block's shared
-// counters, the block adds them to 64-bit global totals.
+// bulk_count over n values into one counting vector: every warp counts a contiguous chunk into shared counters of its
+// own (planes_flush_to, no shared-memory atomics), the block adds them up and to the 64-bit global totals.
 // Four blocks per SM (64 registers, some spilled for h >= 3) measured faster than two blocks without spills (1.53 vs
-// 2.16 ms for 2^24 values on 1,024 bins, h = 3): more warps keep more row loads in flight.  PRIVATE: every warp
-// flushes into counters of its own (no shared-memory atomics), summed by the block at the end; otherwise the block's
-// warps share one set of counters.
-template <int H, bool PRIVATE>
+// 2.16 ms for 2^24 values on 1,024 bins, h = 3): more warps keep more row loads in flight.
+// The grid's second dimension is the slab of a row wider than a warp: a block counts 32 words of every row, a warp one
+// whole 256-byte piece per value and hash function.  (Rows wider than a warp were counted one value at a time, every
+// set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms, now 0.219.)
+template <int H>
 __global__ void __launch_bounds__(256, 4)
-    k_bulk_count(row_params rp, uint32_t lpv_log2, uint64_t const * __restrict__ values, uint64_t n, uint64_t chunk,
-                 unsigned long long * __restrict__ totals, uint32_t n_counters)
+    k_bulk_count(row_params row, uint64_t const * __restrict__ values, uint64_t n, uint64_t chunk,
+                 unsigned long long * __restrict__ totals)
 {
     extern __shared__ uint32_t s_counts[];
+    uint32_t const w0 = blockIdx.y * kSlabWords;
+    row_params const rp = row_slab(row, w0);
+    uint32_t const lpv_log2 = lanes_log2(rp.bin_words);
+    uint32_t const n_counters = 64u << lpv_log2;
     int const nwarps_block = blockDim.x >> 5;
-    uint32_t const n_smem = PRIVATE ? n_counters * nwarps_block : n_counters;
-    for (uint32_t i = threadIdx.x; i < n_smem; i += blockDim.x)
+    for (uint32_t i = threadIdx.x; i < n_counters * nwarps_block; i += blockDim.x)
         s_counts[i] = 0;
     __syncthreads();
     int const lane = threadIdx.x & 31;
-    uint32_t * counts = PRIVATE ? s_counts + (threadIdx.x >> 5) * n_counters : s_counts;
+    uint32_t * counts = s_counts + (threadIdx.x >> 5) * n_counters;
     uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
     uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     for (uint64_t start = warp * chunk; start < n; start += nwarps * chunk)
     {
         uint64_t const len = (n - start) < chunk ? (n - start) : chunk;
-        if (PRIVATE && rp.bin_words <= 32)
-            warp_count_lpv<H, false, true>(rp, lpv_log2, values + start, len, counts, lane);
-        else
-            warp_count_h<H, true>(rp, lpv_log2, values + start, len, counts, lane);
+        warp_count_lpv<H, true>(rp, lpv_log2, values + start, len, counts, lane);
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n_counters; i += blockDim.x)
     {
         uint64_t sum = 0;
-        for (int w = 0; w < (PRIVATE ? nwarps_block : 1); ++w)
+        for (int w = 0; w < nwarps_block; ++w)
             sum += s_counts[w * n_counters + i];
         if (sum)
-            atomicAdd(totals + i, static_cast<unsigned long long>(sum));
+            atomicAdd(totals + 64u * w0 + i, static_cast<unsigned long long>(sum));
     }
 }
 
@@ -390,26 +362,22 @@ __global__ void k_store_counts(unsigned long long const * __restrict__ totals, u
     }
 }
 
-using bulk_count_kernel_t = void (*)(row_params, uint32_t, uint64_t const *, uint64_t, uint64_t,
-                                     unsigned long long *, uint32_t);
+using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *);
 
-// Warp-private counters when eight sets fit in 96 KiB of shared memory (up to 3,072 technical bins).
-constexpr uint32_t kPrivateCountersMax = 3072;
-
-bulk_count_kernel_t bulk_count_kernel(uint64_t h, bool priv)
+bulk_count_kernel_t bulk_count_kernel(uint64_t h)
 {
     switch (h)
     {
     case 1:
-        return priv ? k_bulk_count<1, true> : k_bulk_count<1, false>;
+        return k_bulk_count<1>;
     case 2:
-        return priv ? k_bulk_count<2, true> : k_bulk_count<2, false>;
+        return k_bulk_count<2>;
     case 3:
-        return priv ? k_bulk_count<3, true> : k_bulk_count<3, false>;
+        return k_bulk_count<3>;
     case 4:
-        return priv ? k_bulk_count<4, true> : k_bulk_count<4, false>;
+        return k_bulk_count<4>;
     default:
-        return priv ? k_bulk_count<5, true> : k_bulk_count<5, false>;
+        return k_bulk_count<5>;
     }
 }
 
@@ -464,9 +432,10 @@ struct hibf_gpu_ibf
         return row_params{store.as<uint64_t>(), bin_size, static_cast<uint32_t>(row_words),
                           static_cast<uint32_t>(bin_words), shift, static_cast<uint32_t>(hash_funs)};
     }
-    uint32_t lpv_log2() const
+    // slabs of a row: kSlabWords words each, the last one what is left
+    uint32_t slabs() const
     {
-        return lanes_per_value_log2(bin_words);
+        return static_cast<uint32_t>((bin_words + kSlabWords - 1) / kSlabWords);
     }
     uint64_t technical_bins() const
     {
@@ -558,7 +527,7 @@ void launch_emplace(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const 
 // Per-bin counters bulk_count accumulates for filter f (a multiple of 64, at least its technical bins).
 uint64_t count_counters(hibf_gpu_ibf const * f)
 {
-    return 64u * (f->bin_words <= 32 ? (1u << f->lpv_log2()) : f->bin_words);
+    return row_counters(static_cast<uint32_t>(f->bin_words));
 }
 
 // bulk_count of n device values into d_out.  `totals` is device scratch for count_counters(f) 64-bit totals; null
@@ -576,20 +545,25 @@ void launch_count(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, int w
     if (n)
     {
         unsigned const block = 256;
-        // one contiguous chunk per warp of a full wave (4 blocks of 8 warps per SM), at least 512 values: fewer,
-        // larger chunks left SMs idle on small calls (128 blocks for 2^21 values with fixed 2,048-value chunks)
-        uint64_t const wave = static_cast<uint64_t>(sm_count()) * 4u * 8u;
-        uint64_t const chunk = std::max<uint64_t>(512, ((n + wave - 1) / wave + 127) / 128 * 128);
+        // One contiguous chunk per warp of a full wave, over all slabs: 4 blocks of 8 warps per SM, or the 3 whose 64
+        // KiB of counters fit where a slab is 32 words.  Rows of up to 1,024 bins take at least 512 values per chunk:
+        // fewer, larger chunks left SMs idle on small calls (128 blocks for 2^21 values with fixed 2,048-value
+        // chunks); wide rows make a chunk of 64 values 32 KiB or more of row bytes, worth a warp.
+        uint32_t const slabs = f->slabs();
+        bool const full_slabs = f->bin_words > kSlabWords / 2;
+        uint64_t const blocks = std::max<uint64_t>(1, static_cast<uint64_t>(sm_count()) * (full_slabs ? 3u : 4u) / slabs);
+        uint64_t const wave = blocks * 8u;
+        uint64_t const round = full_slabs ? 32 : 128;
+        uint64_t const chunk =
+            std::max<uint64_t>(full_slabs ? 64 : 512, ((n + wave - 1) / wave + round - 1) / round * round);
         uint64_t const warps = (n + chunk - 1) / chunk;
-        unsigned const grid = static_cast<unsigned>(
-            std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, static_cast<uint64_t>(sm_count()) * 4u)));
-        bool const priv = nc <= kPrivateCountersMax;
-        size_t const smem = nc * sizeof(uint32_t) * (priv ? block / 32 : 1);
+        unsigned const grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, blocks)));
+        size_t const smem = (64u << lanes_log2(static_cast<uint32_t>(std::min<uint64_t>(f->bin_words, kSlabWords)))) *
+                            sizeof(uint32_t) * (block / 32);
+        bulk_count_kernel_t const kernel = bulk_count_kernel(f->hash_funs);
         if (smem > 48 * 1024)
-            HG_CUDA(cudaFuncSetAttribute(bulk_count_kernel(f->hash_funs, priv),
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        bulk_count_kernel(f->hash_funs, priv)<<<grid, block, smem, s>>>(f->rp(), f->lpv_log2(), d_values, n, chunk,
-                                                                        totals, static_cast<uint32_t>(nc));
+            HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        kernel<<<dim3(grid, slabs), block, smem, s>>>(f->rp(), d_values, n, chunk, totals);
         HG_CUDA(cudaGetLastError());
     }
     k_store_counts<<<grid_for(f->bins, 256), 256, 0, s>>>(totals, f->bins, width, d_out);
@@ -600,36 +574,37 @@ void launch_contains(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, ui
 {
     if (n == 0)
         return;
-    unsigned const block = 256;
-    uint32_t const l = f->lpv_log2();
     row_params const rp = f->rp();
-    if (f->bin_words > 32)
+    // all full slabs in one launch, a narrower last slab in one of its own (its lanes per row differ)
+    uint32_t const full = static_cast<uint32_t>(f->bin_words / kSlabWords);
+    uint32_t const rest = static_cast<uint32_t>(f->bin_words % kSlabWords);
+    unsigned const grid = grid_for(n, 256);
+    auto launch = [&](uint32_t lpv_log2, uint32_t first, uint32_t slabs)
     {
-        // rows wider than a warp: lanes stride over the words
-        k_bulk_contains<32><<<grid_for(n << 5, block), block, 0, s>>>(rp, d_values, n, d_out);
-    }
-    else
-    {
-        unsigned const grid = grid_for(n, block);
         switch (f->hash_funs)
         {
         case 1:
-            launch_contains_h<1>(rp, l, d_values, n, d_out, grid, s);
+            launch_contains_h<1>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 2:
-            launch_contains_h<2>(rp, l, d_values, n, d_out, grid, s);
+            launch_contains_h<2>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 3:
-            launch_contains_h<3>(rp, l, d_values, n, d_out, grid, s);
+            launch_contains_h<3>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 4:
-            launch_contains_h<4>(rp, l, d_values, n, d_out, grid, s);
+            launch_contains_h<4>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         default:
-            launch_contains_h<5>(rp, l, d_values, n, d_out, grid, s);
+            launch_contains_h<5>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
         }
-    }
-    HG_CUDA(cudaGetLastError());
+        HG_CUDA(cudaGetLastError());
+    };
+    constexpr uint32_t kMaxGridY = 65535;
+    for (uint32_t first = 0; first < full; first += kMaxGridY)
+        launch(5, first, std::min(kMaxGridY, full - first));
+    if (rest)
+        launch(lanes_log2(rest), full, 1);
 }
 
 int width_ok(int width)

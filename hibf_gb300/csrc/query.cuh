@@ -435,23 +435,33 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
     switch (lpv_log2)
     {
     case 0:
-        warp_count<1, H, Q::K, false, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+        warp_count<1, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
         break;
     case 1:
         if constexpr (Q::W == 2)
-            warp_count<1, H, Q::K, false, Q::UM, 2>(rp, vals, n, counts, lane, stage);
+            warp_count<1, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
         else
-            warp_count<2, H, Q::K, false, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+            warp_count<2, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
         break;
     case 2:
         if constexpr (Q::W == 2)
-            warp_count<2, H, Q::K, false, Q::UM, 2>(rp, vals, n, counts, lane, stage);
+            warp_count<2, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
         else
-            warp_count<4, H, Q::K, false, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+            warp_count<4, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+        break;
+    case 3:
+        if constexpr (V == 0)
+            warp_count<8, H, Q::K>(rp, vals, n, counts, lane, stage);
+        break;
+    case 4:
+        if constexpr (V == 0)
+            warp_count<16, H, Q::K>(rp, vals, n, counts, lane, stage);
         break;
     default:
         if constexpr (V == 0)
-            warp_count_h<H, false>(rp, lpv_log2, vals, n, counts, lane, stage);
+#pragma unroll 1
+            for (uint32_t w0 = 0; w0 < rp.bin_words; w0 += kSlabWords) // one slab unless the row is wider than a warp
+                warp_count<32, H, Q::K>(row_slab(rp, w0), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
     }
 }
 
@@ -652,7 +662,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         }
         return;
     }
-    uint32_t const ncount = nd.bin_words > 32 ? 64u * nd.bin_words : (64u << nd.lpv_log2);
+    uint32_t const ncount = row_counters(nd.bin_words);
     for (uint32_t i = lane; i < ncount; i += 32)
         counts[i] = 0;
     __syncwarp();
@@ -1034,7 +1044,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
         dev_node const nd = p.nodes[static_cast<uint32_t>(task) & kNodeMask];
         uint64_t const b0 = p.qoff[q];
         uint64_t const n = p.qoff[q + 1] - b0;
-        uint32_t const ncount = nd.bin_words > 32 ? 64u * nd.bin_words : (64u << nd.lpv_log2);
+        uint32_t const ncount = row_counters(nd.bin_words);
         for (uint32_t i = lane; i < ncount; i += 32)
             counts[i] = 0;
         __syncwarp();
@@ -1085,7 +1095,7 @@ __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_
     uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     dev_node const nd = p.nodes[0];
     row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift, nd.hash_funs};
-    uint32_t const ncount = nd.bin_words > 32 ? 64u * nd.bin_words : (64u << nd.lpv_log2);
+    uint32_t const ncount = row_counters(nd.bin_words);
     uint2 const * d = p.descs + nd.desc_offset;
     for (uint64_t q = warp; q < p.n_queries; q += nwarps)
     {
