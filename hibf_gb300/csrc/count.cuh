@@ -6,7 +6,7 @@
 // Work mapping.  A row of bin_words 64-bit words is read by LPV = next_pow2(bin_words) lanes (capped at 32), lane
 // j of a group reading word j, so a row is one coalesced access of ceil(bytes/32) sectors.  Each lane first hashes
 // a different value (32 values per warp per pass), then the groups take turns on those values, receiving the row
-// offsets by shuffle.  Each lane accumulates its word's 64 bins in K bit-sliced planes (planes_add4) and flushes
+// indices (of type R) by shuffle.  Each lane accumulates its word's 64 bins in K bit-sliced planes (planes_add4) and flushes
 // them through a warp transpose into 32-bit counters in shared memory before they can overflow (2^K - 1 masks).
 // Counts are exact; the caller reduces them modulo the counter width, which equals the reference's wraparound.
 #pragma once
@@ -102,13 +102,13 @@ __device__ __forceinline__ void load_row_words(uint64_t const * p, uint64_t (&w)
 // loads must not come from a non-coherent cache.  Each task reads its values once, so L1 gives them nothing.
 //
 // One warp counts vals[0, n) into counts[0, 64 * LPV * W) with H hash functions.  A row is read by LPV lanes, each
-// loading W consecutive words (W = 2: one 16-byte load; the row stride must then be even).  Each lane hashes U values per pass and keeps their H row offsets; the row words of
+// loading W consecutive words (W = 2: one 16-byte load; the row stride must then be even).  Each lane hashes U values per pass and keeps their H row indices; the row words of
 // GS = 4 * UM masks per lane are loaded together, so GS * H * W loads per lane are in flight.  K planes count up to
 // 2^K - 1 masks between flushes.
 //
 // stage (optional): every value read is also stored at stage[i], so that later reads of the same values (the lower
 // levels of an in-place host batch) come from device memory instead of the host link.
-template <int LPV, int H, int K, int UM = 1, int W = 1, bool EF = false>
+template <typename R, int LPV, int H, int K, int UM = 1, int W = 1, bool EF = false>
 __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const * __restrict__ vals, uint64_t n,
                                            uint32_t * counts, int lane, uint64_t * __restrict__ stage = nullptr)
 {
@@ -142,7 +142,7 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
     }
     for (uint64_t base = 0; base < n; base += BLOCK)
     {
-        uint64_t off[U][H];
+        R row[U][H];
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
@@ -151,7 +151,7 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
                 // a call of the early exit often ends within a pass: no hashing for values that are not there
 #pragma unroll
                 for (int i = 0; i < H; ++i)
-                    off[u][i] = 0;
+                    row[u][i] = 0;
                 continue;
             }
             uint64_t const idx = base + static_cast<uint64_t>(u * 32 + lane);
@@ -160,7 +160,7 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
                 stage[idx] = v;
 #pragma unroll
             for (int i = 0; i < H; ++i)
-                off[u][i] = hash_row(v, c_hash_seeds[i], rp.hash_shift, rp.bin_size) * rp.row_words;
+                row[u][i] = hash_row_as<R>(v, c_hash_seeds[i], rp.hash_shift, rp.bin_size);
         }
 #pragma unroll
         for (int u = 0; u < U; ++u)
@@ -183,11 +183,11 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
 #pragma unroll
                 for (int i = 0; i < H; ++i)
                 {
-                    uint64_t o = off[u][i];
+                    R r = row[u][i];
                     if constexpr (LPV > 1)
-                        o = __shfl_sync(kFullMask, o, src);
+                        r = __shfl_sync(kFullMask, r, src);
                     if (ok[t])
-                        load_row_words<W, EF>(words + o, w[t][i]);
+                        load_row_words<W, EF>(words + static_cast<uint64_t>(r) * rp.row_words, w[t][i]);
                     else
 #pragma unroll
                         for (int e = 0; e < W; ++e)
@@ -241,29 +241,29 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
     }
 }
 
-template <int H, bool EF = false>
+template <typename R, int H, bool EF = false>
 __device__ __forceinline__ void warp_count_lpv(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
                                                uint64_t n, uint32_t * counts, int lane, uint64_t * stage = nullptr)
 {
     switch (lpv_log2)
     {
     case 0:
-        warp_count<1, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 1, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 1:
-        warp_count<2, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 2, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 2:
-        warp_count<4, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 4, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 3:
-        warp_count<8, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 8, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     case 4:
-        warp_count<16, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 16, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
         break;
     default:
-        warp_count<32, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 32, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
     }
 }
 

@@ -35,12 +35,26 @@ namespace
 {
 
 
-__global__ void k_init_ctrl(unsigned long long * ctrl, unsigned long long * stats, uint64_t n_queries)
+// One launch readies a batch's workspace: the control and work counters (n_ctrl words, all 0 but the count of
+// unfinished tasks), the queries' result counts, the work queue's empty-slot marks and the levels' histograms.  (A kernel
+// and three or four memsets took about 3 us each of a batch that answers 100 queries in 40.)
+__global__ void k_begin(unsigned long long * __restrict__ ctrl, uint32_t n_ctrl, unsigned long long pending,
+                        unsigned int * __restrict__ qcount, uint64_t nq, unsigned long long * __restrict__ tasks,
+                        uint64_t n_marks, unsigned int * __restrict__ hist, uint64_t n_hist)
 {
-    if (threadIdx.x < C_WORDS)
-        ctrl[threadIdx.x] = threadIdx.x == C_PENDING ? n_queries : 0ull;
-    if (threadIdx.x < kStats)
-        stats[threadIdx.x] = 0;
+    uint64_t const first = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    if (first < n_ctrl)
+        ctrl[first] = first == C_PENDING ? pending : 0ull;
+    for (uint64_t i = first; i < nq; i += stride)
+        qcount[i] = 0;
+    for (uint64_t i = first; i < n_hist; i += stride)
+        hist[i] = 0;
+    ulonglong2 * const pairs = reinterpret_cast<ulonglong2 *>(tasks); // cudaMalloc'ed: aligned
+    for (uint64_t i = first; i < n_marks / 2; i += stride)
+        pairs[i] = make_ulonglong2(kEmpty, kEmpty);
+    if (first == 0 && (n_marks & 1u))
+        tasks[n_marks - 1] = kEmpty;
 }
 
 // ---- level schedule: the tasks one level appended (tasks[0, ctrl[C_TAIL])), grouped by IBF for the next level ----
@@ -144,6 +158,9 @@ __global__ void k_level_scatter(unsigned long long const * __restrict__ tasks, u
 }
 
 // ---- exclusive scan of the per-query result counts -> result offsets (n + 1 entries) ----
+// Up to kOneBlockScan queries one block scans them in one launch (four per thread and turn); more take three launches
+// over all SMs.  One block needs about 0.7 us per 4,096 queries, the three launches 10 us before they scale.
+constexpr uint64_t kOneBlockScan = 65536;
 constexpr int kScanBlock = 1024;
 
 __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long x, int lane)
@@ -156,6 +173,53 @@ __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long 
             x += y;
     }
     return x;
+}
+
+__global__ void __launch_bounds__(kScanBlock) k_scan_one_block(unsigned int const * __restrict__ in, uint64_t n,
+                                                              unsigned long long * __restrict__ out)
+{
+    __shared__ unsigned long long warp_sums[32];
+    int const lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    unsigned long long carry = 0;
+    for (uint64_t base = 0; base < n; base += 4u * kScanBlock)
+    {
+        uint64_t const i = base + 4u * threadIdx.x;
+        uint4 v = make_uint4(0u, 0u, 0u, 0u);
+        if (i + 4 <= n)
+        {
+            v = *reinterpret_cast<uint4 const *>(in + i);
+        }
+        else
+        {
+            if (i < n)
+                v.x = in[i];
+            if (i + 1 < n)
+                v.y = in[i + 1];
+            if (i + 2 < n)
+                v.z = in[i + 2];
+        }
+        unsigned long long const mine = static_cast<unsigned long long>(v.x) + v.y + v.z + v.w;
+        unsigned long long x = warp_incl_scan(mine, lane);
+        if (lane == 31)
+            warp_sums[w] = x;
+        __syncthreads();
+        if (w == 0)
+            warp_sums[lane] = warp_incl_scan(warp_sums[lane], lane);
+        __syncthreads();
+        x += carry + (w > 0 ? warp_sums[w - 1] : 0ull) - mine;
+        carry += warp_sums[31];
+        if (i < n)
+            out[i] = x;
+        if (i + 1 < n)
+            out[i + 1] = x + v.x;
+        if (i + 2 < n)
+            out[i + 2] = x + v.x + v.y;
+        if (i + 3 < n)
+            out[i + 3] = x + v.x + v.y + v.z;
+        __syncthreads(); // warp_sums is rewritten
+    }
+    if (threadIdx.x == 0)
+        out[n] = carry;
 }
 
 __global__ void __launch_bounds__(kScanBlock) k_scan_local(unsigned int const * __restrict__ in, uint64_t n,
@@ -227,11 +291,11 @@ __global__ void k_scan_add(unsigned long long * out, uint64_t n, unsigned long l
         out[n] = sums[nb];
 }
 
-// ---- scatter records into per-query segments ----
+// ---- scatter records into per-query segments (each query's count runs down to 0 as its records find their places) ----
 __global__ void k_scatter(unsigned long long const * __restrict__ ctrl, uint32_t const * __restrict__ rec_q,
                           uint32_t const * __restrict__ rec_ub, unsigned long long const * __restrict__ rec_cnt,
                           uint64_t rec_cap, unsigned long long const * __restrict__ roff,
-                          unsigned int * __restrict__ cursor, uint64_t * __restrict__ out_ids,
+                          unsigned int * __restrict__ qcount, uint64_t * __restrict__ out_ids,
                           uint64_t * __restrict__ out_cnt)
 {
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
@@ -243,47 +307,30 @@ __global__ void k_scatter(unsigned long long const * __restrict__ ctrl, uint32_t
          r += static_cast<uint64_t>(gridDim.x) * blockDim.x)
     {
         uint32_t const q = rec_q[r];
-        uint64_t const pos = roff[q] + atomicAdd(cursor + q, 1u);
+        uint64_t const pos = roff[q] + (atomicSub(qcount + q, 1u) - 1u);
         out_ids[pos] = rec_ub[r];
         out_cnt[pos] = rec_cnt[r];
     }
 }
 
-// ---- sort every query's segment by user bin id ----
-constexpr uint32_t kSmallSegment = 32;
+// ---- sort every query's segment by user bin id, and its counts to the counter width ----
 constexpr uint32_t kSmemSegment = 2048;
 
-__global__ void k_sort_small(unsigned long long const * __restrict__ roff, uint64_t nq, uint64_t * ids,
-                             uint64_t * cnt, uint32_t * large, unsigned long long * ctrl)
+__device__ __forceinline__ void store_count(void * out, int width, uint64_t i, uint64_t v)
 {
-    if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
-        return;
-    for (uint64_t q = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; q < nq;
-         q += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+    switch (width)
     {
-        uint64_t const b = roff[q], e = roff[q + 1];
-        uint64_t const len = e - b;
-        if (len <= 1)
-            continue;
-        if (len > kSmallSegment)
-        {
-            unsigned long long const slot = atomicAdd(ctrl + C_NLARGE, 1ull);
-            large[slot] = static_cast<uint32_t>(q);
-            continue;
-        }
-        for (uint64_t i = b + 1; i < e; ++i)
-        {
-            uint64_t const ki = ids[i], ci = cnt[i];
-            uint64_t jx = i;
-            while (jx > b && ids[jx - 1] > ki)
-            {
-                ids[jx] = ids[jx - 1];
-                cnt[jx] = cnt[jx - 1];
-                --jx;
-            }
-            ids[jx] = ki;
-            cnt[jx] = ci;
-        }
+    case 1:
+        static_cast<uint8_t *>(out)[i] = static_cast<uint8_t>(v);
+        break;
+    case 2:
+        static_cast<uint16_t *>(out)[i] = static_cast<uint16_t>(v);
+        break;
+    case 4:
+        static_cast<uint32_t *>(out)[i] = static_cast<uint32_t>(v);
+        break;
+    default:
+        static_cast<uint64_t *>(out)[i] = v;
     }
 }
 
@@ -306,90 +353,111 @@ __device__ __forceinline__ void cmp_asc(uint64_t * kid, uint64_t * kcn, uint64_t
     }
 }
 
-__global__ void k_sort_large(unsigned long long const * __restrict__ roff, uint32_t const * __restrict__ large,
-                             unsigned long long const * __restrict__ ctrl, uint64_t * ids, uint64_t * cnt)
+// A warp takes `per` queries a turn (at most 32, one per lane): it sorts their segments of 2 to 32 results one after
+// the other by rank, one result per lane; the block then takes the longer ones of its warps together.  narrow (count
+// mode, width < 8): the counts in their width.  One launch for what were three (short segments, long ones, counts),
+// each about 3 us of a small batch.
+__global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * __restrict__ roff, uint64_t nq,
+                                                       uint32_t per, unsigned long long const * __restrict__ ctrl,
+                                                       uint64_t * ids, uint64_t * cnt, int width, void * narrow)
 {
     __shared__ uint64_t s_ids[kSmemSegment];
     __shared__ uint64_t s_cnt[kSmemSegment];
+    __shared__ uint32_t s_long[256]; // the turn's long segments, as offsets from its first query
+    __shared__ uint32_t s_n_long;
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
         return;
-    unsigned long long const nl = ctrl[C_NLARGE];
-    for (unsigned long long li = blockIdx.x; li < nl; li += gridDim.x)
+    int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    uint64_t const turn = 8ull * per;
+    for (uint64_t base = blockIdx.x * turn; base < nq; base += gridDim.x * turn)
     {
-        uint32_t const q = large[li];
-        uint64_t const b = roff[q];
-        uint64_t const len = roff[q + 1] - b;
-        uint64_t P = 1;
-        while (P < len)
-            P <<= 1;
-        bool const in_smem = len <= kSmemSegment;
-        uint64_t * kid = in_smem ? s_ids : ids + b;
-        uint64_t * kcn = in_smem ? s_cnt : cnt + b;
-        if (in_smem)
+        if (threadIdx.x == 0)
+            s_n_long = 0;
+        __syncthreads();
+        uint32_t const k = warp * per + lane;
+        bool const has = static_cast<uint32_t>(lane) < per && base + k < nq;
+        uint64_t const b = has ? roff[base + k] : 0u;
+        uint64_t const len = has ? roff[base + k + 1] - b : 0u;
+        if (len > 32)
+            s_long[atomicAdd(&s_n_long, 1u)] = k;
+        else if (len == 1 && narrow)
+            store_count(narrow, width, b, cnt[b]);
+        for (unsigned todo = __ballot_sync(kFullMask, len > 1 && len <= 32); todo; todo &= todo - 1)
         {
-            for (uint64_t i = threadIdx.x; i < len; i += blockDim.x)
+            int const src = __ffs(todo) - 1;
+            uint64_t const sb = __shfl_sync(kFullMask, b, src);
+            int const n = static_cast<int>(__shfl_sync(kFullMask, len, src));
+            uint64_t const id = lane < n ? ids[sb + lane] : ~0ull;
+            uint64_t const c = lane < n ? cnt[sb + lane] : 0u;
+            uint32_t rank = 0;
+            for (int j = 0; j < n; ++j)
             {
-                s_ids[i] = ids[b + i];
-                s_cnt[i] = cnt[b + i];
+                uint64_t const other = __shfl_sync(kFullMask, id, j);
+                rank += other < id || (other == id && j < lane);
+            }
+            __syncwarp();
+            if (lane < n)
+            {
+                ids[sb + rank] = id;
+                cnt[sb + rank] = c;
+                if (narrow)
+                    store_count(narrow, width, sb + rank, c);
             }
         }
         __syncthreads();
-        for (uint64_t k = 2; k <= P; k <<= 1)
+        for (uint32_t l = 0; l < s_n_long; ++l)
         {
-            for (uint64_t i = threadIdx.x; i < P; i += blockDim.x)
+            uint64_t const lb = roff[base + s_long[l]];
+            uint64_t const llen = roff[base + s_long[l] + 1] - lb;
+            uint64_t P = 1;
+            while (P < llen)
+                P <<= 1;
+            bool const in_smem = llen <= kSmemSegment;
+            uint64_t * kid = in_smem ? s_ids : ids + lb;
+            uint64_t * kcn = in_smem ? s_cnt : cnt + lb;
+            if (in_smem)
             {
-                uint64_t const l = i ^ (k - 1);
-                if (l > i && i < len)
-                    cmp_asc(kid, kcn, i, l, len);
+                for (uint64_t i = threadIdx.x; i < llen; i += blockDim.x)
+                {
+                    s_ids[i] = ids[lb + i];
+                    s_cnt[i] = cnt[lb + i];
+                }
             }
             __syncthreads();
-            for (uint64_t jj = k >> 2; jj > 0; jj >>= 1)
+            for (uint64_t kk = 2; kk <= P; kk <<= 1)
             {
                 for (uint64_t i = threadIdx.x; i < P; i += blockDim.x)
                 {
-                    uint64_t const l = i ^ jj;
-                    if (l > i && i < len)
-                        cmp_asc(kid, kcn, i, l, len);
+                    uint64_t const m = i ^ (kk - 1);
+                    if (m > i && i < llen)
+                        cmp_asc(kid, kcn, i, m, llen);
                 }
                 __syncthreads();
+                for (uint64_t jj = kk >> 2; jj > 0; jj >>= 1)
+                {
+                    for (uint64_t i = threadIdx.x; i < P; i += blockDim.x)
+                    {
+                        uint64_t const m = i ^ jj;
+                        if (m > i && i < llen)
+                            cmp_asc(kid, kcn, i, m, llen);
+                    }
+                    __syncthreads();
+                }
             }
-        }
-        if (in_smem)
-        {
-            for (uint64_t i = threadIdx.x; i < len; i += blockDim.x)
+            for (uint64_t i = threadIdx.x; i < llen; i += blockDim.x)
             {
-                ids[b + i] = s_ids[i];
-                cnt[b + i] = s_cnt[i];
+                uint64_t const c = kcn[i];
+                if (in_smem)
+                {
+                    ids[lb + i] = s_ids[i];
+                    cnt[lb + i] = c;
+                }
+                if (narrow)
+                    store_count(narrow, width, lb + i, c);
             }
+            __syncthreads();
         }
-        __syncthreads();
-    }
-}
-
-__global__ void k_narrow(unsigned long long const * __restrict__ roff, uint64_t nq, uint64_t const * __restrict__ in,
-                         int width, void * out, unsigned long long const * __restrict__ ctrl)
-{
-    if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
-        return;
-    uint64_t const n = roff[nq];
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-    {
-        uint64_t const v = in[i];
-        switch (width)
-        {
-        case 1:
-            static_cast<uint8_t *>(out)[i] = static_cast<uint8_t>(v);
-            break;
-        case 2:
-            static_cast<uint16_t *>(out)[i] = static_cast<uint16_t>(v);
-            break;
-        case 4:
-            static_cast<uint32_t *>(out)[i] = static_cast<uint32_t>(v);
-            break;
-        default:
-            static_cast<uint64_t *>(out)[i] = v;
-        }
+        __syncthreads(); // s_n_long and s_long are rewritten
     }
 }
 
@@ -447,13 +515,12 @@ struct hibf_gpu_agent
     unsigned long long * qwork{};          // executed value visits per query (device; null = not recorded)
     uint64_t qwork_n{};                    // its length: batches may have at most this many queries
     // device workspace
-    dbuf ctrl, stats, tasks, rec_q, rec_ub, rec_cnt, qcount, cursor, roff, bsum, out_ids, out_cnt, out_cntw, large;
+    // ctrl: the control words, the work counters and (level schedule) each level's work counters, read back together
+    dbuf ctrl, tasks, rec_q, rec_ub, rec_cnt, qcount, roff, bsum, out_ids, out_cnt, out_cntw;
     // level schedule: a level's tasks grouped by IBF, the per-IBF histogram / cursors, the level's task count; an
     // event after each level of the last batch (timing)
     dbuf lvl_tasks, lvl_hist, lvl_count;
     // level schedule: each level's tasks, value visits and executed value visits (kStats words per level)
-    dbuf lvl_stats;
-    hbuf h_lvl_stats;
     std::vector<uint64_t> last_level_stats;
     std::vector<cudaEvent_t> ev_lvl;
     uint32_t last_levels{};
@@ -480,7 +547,7 @@ struct hibf_gpu_agent
     cudaEvent_t tl_t0{}, tl_done{};
     std::vector<cudaEvent_t> tl_chunk;
     uint32_t tl_n{};
-    hbuf h_roff, h_ids, h_cnt, h_ctrl, h_stats;
+    hbuf h_roff, h_ids, h_cnt, h_ctrl;
     std::vector<uint64_t> single_ids;
     std::vector<uint8_t> dense;
     std::vector<uint64_t> thr_tmp, qoff_tmp;
@@ -489,15 +556,19 @@ struct hibf_gpu_agent
 namespace
 {
 
+// Words of the control buffer: the control words, the batch's work counters, the work counters of every level.
+uint32_t ctrl_words(hibf_gpu_hibf const * h)
+{
+    return C_WORDS + kStats * (2u + h->max_depth);
+}
+
 void ensure_capacity(hibf_gpu_agent * a, uint64_t nq, uint64_t tasks, uint64_t results)
 {
     if (nq > a->cap_queries)
     {
         a->qcount.ensure(nq * 4);
-        a->cursor.ensure(nq * 4);
         a->roff.ensure((nq + 1) * 8);
         a->bsum.ensure(((nq + kScanBlock - 1) / kScanBlock + 1) * 8);
-        a->large.ensure(nq * 4);
         a->cap_queries = nq;
     }
     if (tasks > a->cap_tasks)
@@ -508,10 +579,8 @@ void ensure_capacity(hibf_gpu_agent * a, uint64_t nq, uint64_t tasks, uint64_t r
     if (a->tune.schedule == HIBF_GPU_SCHEDULE_LEVELS) // no-ops once large enough
     {
         a->lvl_tasks.ensure(a->cap_tasks * 8);
-        a->lvl_hist.ensure(a->h->n_ibfs * 4);
+        a->lvl_hist.ensure(std::max<uint64_t>(a->h->max_depth, 1) * a->h->n_ibfs * 4); // one per level below the root
         a->lvl_count.ensure(8);
-        a->lvl_stats.ensure((a->h->max_depth + 1) * kStats * 8);
-        a->h_lvl_stats.ensure((a->h->max_depth + 1) * kStats * 8);
     }
     if (results > a->cap_results)
     {
@@ -549,7 +618,7 @@ query_params base_params(hibf_gpu_agent * a, uint64_t const * d_values, uint64_t
     p.rec_cnt = a->rec_cnt.as<unsigned long long>();
     p.rec_cap = a->cap_results;
     p.qcount = a->qcount.as<unsigned int>();
-    p.stats = a->stats.as<unsigned long long>();
+    p.stats = a->ctrl.as<unsigned long long>() + C_WORDS;
     p.wait_limit_ns = 10ull * 1000 * 1000 * 1000;
     p.self_init = 0;
     p.ee_first = a->tune.early_exit_first;
@@ -573,6 +642,20 @@ uint64_t mask_for(int mode, int width)
     return w >= 8 ? ~0ull : ((1ull << (8 * w)) - 1u);
 }
 
+// The kernels of a hierarchy: its hash function count and the width of its row indices.
+query_kernel_t query_kernel(hibf_gpu_hibf const * h, int variant)
+{
+    return query_kernels_of(h->hash_count).variant(variant, h->wide_rows);
+}
+query_kernel_t query_block_kernel(hibf_gpu_hibf const * h)
+{
+    return query_kernels_of(h->hash_count).block(h->wide_rows);
+}
+features_kernel_t features_kernel(hibf_gpu_hibf const * h)
+{
+    return query_kernels_of(h->hash_count).features(h->wide_rows);
+}
+
 size_t query_smem(hibf_gpu_hibf const * h)
 {
     return static_cast<size_t>(8) * h->counters_per_warp * sizeof(uint32_t);
@@ -581,39 +664,51 @@ size_t query_smem(hibf_gpu_hibf const * h)
 void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
 {
     cudaStream_t s = a->stream;
-    uint64_t const nb = (nq + kScanBlock - 1) / kScanBlock;
-    if (nq)
+    if (nq <= kOneBlockScan)
     {
+        k_scan_one_block<<<1, kScanBlock, 0, s>>>(a->qcount.as<unsigned int>(), nq, a->roff.as<unsigned long long>());
+        HG_CUDA(cudaGetLastError());
+    }
+    else
+    {
+        uint64_t const nb = (nq + kScanBlock - 1) / kScanBlock;
         k_scan_local<<<static_cast<unsigned>(nb), kScanBlock, 0, s>>>(
             a->qcount.as<unsigned int>(), nq, a->roff.as<unsigned long long>(), a->bsum.as<unsigned long long>());
         HG_CUDA(cudaGetLastError());
+        k_scan_sums<<<1, kScanBlock, 0, s>>>(a->bsum.as<unsigned long long>(), nb);
+        HG_CUDA(cudaGetLastError());
+        k_scan_add<<<static_cast<unsigned>((nq + 255) / 256), 256, 0, s>>>(a->roff.as<unsigned long long>(), nq,
+                                                                          a->bsum.as<unsigned long long>(), nb);
+        HG_CUDA(cudaGetLastError());
     }
-    k_scan_sums<<<1, kScanBlock, 0, s>>>(a->bsum.as<unsigned long long>(), nb);
-    HG_CUDA(cudaGetLastError());
-    k_scan_add<<<static_cast<unsigned>(std::max<uint64_t>(1, (nq + 255) / 256)), 256, 0, s>>>(
-        a->roff.as<unsigned long long>(), nq, a->bsum.as<unsigned long long>(), nb);
-    HG_CUDA(cudaGetLastError());
-    HG_CUDA(cudaMemsetAsync(a->cursor.p, 0, std::max<uint64_t>(nq, 1) * 4, s));
+    if (!nq)
+        return;
     k_scatter<<<grid_cap(a->cap_results, 256, 8), 256, 0, s>>>(
         a->ctrl.as<unsigned long long>(), a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(),
         a->rec_cnt.as<unsigned long long>(), a->cap_results, a->roff.as<unsigned long long>(),
-        a->cursor.as<unsigned int>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
+        a->qcount.as<unsigned int>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
     HG_CUDA(cudaGetLastError());
-    k_sort_small<<<grid_cap(nq, 256, 8), 256, 0, s>>>(a->roff.as<unsigned long long>(), nq, a->out_ids.as<uint64_t>(),
-                                                     a->out_cnt.as<uint64_t>(), a->large.as<uint32_t>(),
-                                                     a->ctrl.as<unsigned long long>());
+    bool const narrow = mode == HIBF_GPU_QUERY_COUNT && width != 8;
+    // few queries: one per warp; from a full wave of warps on, up to 32 per warp (most have no result or one)
+    unsigned const sort_grid = grid_cap(nq, 8, 6);
+    uint32_t const per =
+        static_cast<uint32_t>(std::min<uint64_t>(32, (nq + 8ull * sort_grid - 1) / (8ull * sort_grid)));
+    k_sort_segments<<<sort_grid, 256, 0, s>>>(a->roff.as<unsigned long long>(), nq, per,
+                                              a->ctrl.as<unsigned long long>(), a->out_ids.as<uint64_t>(),
+                                              a->out_cnt.as<uint64_t>(), width, narrow ? a->out_cntw.p : nullptr);
     HG_CUDA(cudaGetLastError());
-    k_sort_large<<<static_cast<unsigned>(sm_count()), 256, 0, s>>>(
-        a->roff.as<unsigned long long>(), a->large.as<uint32_t>(), a->ctrl.as<unsigned long long>(),
-        a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
+}
+
+// Readies the workspace for a batch of nq queries (k_begin): `marks` empty-slot marks, `levels` histograms.
+void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t marks, uint64_t levels)
+{
+    uint64_t const n_hist = levels * a->h->n_ibfs;
+    uint64_t const most = std::max({static_cast<uint64_t>(ctrl_words(a->h)), nq, marks / 2, n_hist});
+    k_begin<<<grid_cap(most, 256, 8), 256, 0, a->stream>>>(a->ctrl.as<unsigned long long>(), ctrl_words(a->h), pending,
+                                                          a->qcount.as<unsigned int>(), nq,
+                                                          a->tasks.as<unsigned long long>(), marks,
+                                                          a->lvl_hist.as<unsigned int>(), n_hist);
     HG_CUDA(cudaGetLastError());
-    if (mode == HIBF_GPU_QUERY_COUNT && width != 8)
-    {
-        k_narrow<<<grid_cap(a->cap_results, 256, 8), 256, 0, s>>>(a->roff.as<unsigned long long>(), nq,
-                                                                 a->out_cnt.as<uint64_t>(), width, a->out_cntw.p,
-                                                                 a->ctrl.as<unsigned long long>());
-        HG_CUDA(cudaGetLastError());
-    }
 }
 
 // One persistent launch over all queries plus compaction.  Asynchronous.
@@ -631,16 +726,15 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
     hibf_gpu_hibf * h = a->h;
     check_order_and_work(a, nq, false);
     cudaStream_t s = a->stream;
-    k_init_ctrl<<<1, 32, 0, s>>>(a->ctrl.as<unsigned long long>(), a->stats.as<unsigned long long>(), nq);
-    HG_CUDA(cudaGetLastError());
     // One decision for the whole batch.  The queue (persistent or block kernel) waits on empty-slot marks in the
     // task array, so every batch it runs starts from a fully marked array; the level schedule reads only the slots
     // a finished launch wrote.
     bool const blk = nq <= a->tune.block_queries;
     bool const levels = !blk && a->tune.schedule == HIBF_GPU_SCHEDULE_LEVELS && !a->force_queue;
-    if (!levels)
-        HG_CUDA(cudaMemsetAsync(a->tasks.p, 0xFF, a->cap_tasks * 8, s)); // the queue's empty-slot marks
-    HG_CUDA(cudaMemsetAsync(a->qcount.p, 0, std::max<uint64_t>(nq, 1) * 4, s));
+    if (levels && (!a->lvl_tasks.p || a->lvl_tasks.bytes < a->cap_tasks * 8 || !a->lvl_hist.p ||
+                   a->lvl_hist.bytes < h->max_depth * h->n_ibfs * 4 || !a->lvl_count.p))
+        fail(HIBF_GPU_ERR_LOGIC, "level schedule buffers missing (set the tuning through set_tuning)");
+    launch_begin(a, nq, nq, levels ? 0 : a->cap_tasks, levels ? h->max_depth : 0);
     if (a->qwork && nq)
         HG_CUDA(cudaMemsetAsync(a->qwork, 0, nq * 8, s));
     a->last_levels = 0;
@@ -666,14 +760,8 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
             p.stage = a->stage_values;
             p.staged = a->stage_counts;
             // one launch per level: the roots, then each level's appended tasks grouped by IBF
-            uint64_t const stats_bytes = (h->max_depth + 1) * kStats * 8;
-            if (!a->lvl_tasks.p || a->lvl_tasks.bytes < a->cap_tasks * 8 || !a->lvl_hist.p ||
-                a->lvl_hist.bytes < h->n_ibfs * 4 || !a->lvl_count.p || a->lvl_stats.bytes < stats_bytes ||
-                a->h_lvl_stats.bytes < stats_bytes)
-                fail(HIBF_GPU_ERR_LOGIC, "level schedule buffers missing (set the tuning through set_tuning)");
             // each level counts its work into its own kStats words; read_status sums them
-            HG_CUDA(cudaMemsetAsync(a->lvl_stats.p, 0, stats_bytes, s));
-            unsigned long long * const lvl_stats = a->lvl_stats.as<unsigned long long>();
+            unsigned long long * const lvl_stats = a->ctrl.as<unsigned long long>() + C_WORDS + kStats;
             while (a->ev_lvl.size() <= h->max_depth)
             {
                 cudaEvent_t e{};
@@ -688,7 +776,7 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
             unsigned const grid_child = static_cast<unsigned>(sm_count()) * static_cast<unsigned>(child_per_sm);
             p.level = 1;
             p.stats = lvl_stats;
-            query_kernel(h->hash_count, a->variant)<<<grid_full, 256, query_smem(h), s>>>(p);
+            query_kernel(h, a->variant)<<<grid_full, 256, query_smem(h), s>>>(p);
             HG_CUDA(cudaGetLastError());
             HG_CUDA(cudaEventRecordWithFlags(a->ev_lvl[0], s, rec_flags));
             uint32_t const n_ibfs = static_cast<uint32_t>(h->n_ibfs);
@@ -696,24 +784,22 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
             unsigned const sort_grid = static_cast<unsigned>(sm_count()) * 4u;
             for (uint32_t d = 1; d <= h->max_depth; ++d)
             {
-                HG_CUDA(cudaMemsetAsync(a->lvl_hist.p, 0, n_ibfs * 4u, s));
+                unsigned int * const hist = a->lvl_hist.as<unsigned int>() + static_cast<uint64_t>(d - 1u) * n_ibfs;
                 k_level_hist<<<sort_grid, 256, use_smem ? n_ibfs * 4u : 0u, s>>>(
-                    a->tasks.as<unsigned long long>(), a->ctrl.as<unsigned long long>(), a->cap_tasks,
-                    a->lvl_hist.as<unsigned int>(), n_ibfs, use_smem);
+                    a->tasks.as<unsigned long long>(), a->ctrl.as<unsigned long long>(), a->cap_tasks, hist,
+                    n_ibfs, use_smem);
                 HG_CUDA(cudaGetLastError());
-                k_level_scan<<<1, 1024, 0, s>>>(a->lvl_hist.as<unsigned int>(), n_ibfs,
-                                                a->ctrl.as<unsigned long long>(), a->cap_tasks,
+                k_level_scan<<<1, 1024, 0, s>>>(hist, n_ibfs, a->ctrl.as<unsigned long long>(), a->cap_tasks,
                                                 a->lvl_count.as<unsigned long long>());
                 HG_CUDA(cudaGetLastError());
                 k_level_scatter<<<sort_grid, 256, 0, s>>>(a->tasks.as<unsigned long long>(),
-                                                          a->lvl_count.as<unsigned long long>(),
-                                                          a->lvl_hist.as<unsigned int>(),
+                                                          a->lvl_count.as<unsigned long long>(), hist,
                                                           a->lvl_tasks.as<unsigned long long>(), n_ibfs);
                 HG_CUDA(cudaGetLastError());
                 p.in_tasks = a->lvl_tasks.as<unsigned long long>();
                 p.in_count = a->lvl_count.as<unsigned long long>();
                 p.stats = lvl_stats + d * kStats;
-                query_kernel(h->hash_count, child_variant)<<<grid_child, 256, query_smem(h), s>>>(p);
+                query_kernel(h, child_variant)<<<grid_child, 256, query_smem(h), s>>>(p);
                 HG_CUDA(cudaGetLastError());
                 HG_CUDA(cudaEventRecordWithFlags(a->ev_lvl[d], s, rec_flags));
             }
@@ -721,7 +807,7 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
         }
         else
         {
-            (blk ? query_block_kernel(h->hash_count) : query_kernel(h->hash_count, a->variant))<<<grid, 256,
+            (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256,
                                                                                                query_smem(h), s>>>(p);
             HG_CUDA(cudaGetLastError());
         }
@@ -737,9 +823,8 @@ void launch_plain(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
     hibf_gpu_hibf * h = a->h;
     check_order_and_work(a, nq, true);
     cudaStream_t s = a->stream;
-    k_init_ctrl<<<1, 32, 0, s>>>(a->ctrl.as<unsigned long long>(), a->stats.as<unsigned long long>(), 0);
-    HG_CUDA(cudaGetLastError());
-    HG_CUDA(cudaMemsetAsync(a->qcount.p, 0, std::max<uint64_t>(nq, 1) * 4, s));
+    launch_begin(a, 0, nq, 0, 0);
+    a->last_levels = 0;
     if (a->qwork && nq)
         HG_CUDA(cudaMemsetAsync(a->qwork, 0, nq * 8, s));
     uint64_t const mask = mask_for(mode, width);
@@ -753,7 +838,7 @@ void launch_plain(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
         p.self_init = 1;
         HG_CUDA(cudaMemsetAsync(a->tasks.p, 0xFF, std::min<uint64_t>(a->cap_tasks, 64u * h->n_ibfs + 64u) * 8, s));
         p.task_cap = std::min<uint64_t>(a->cap_tasks, 64u * h->n_ibfs + 64u);
-        (a->tune.block_queries ? query_block_kernel(h->hash_count) : query_kernel(h->hash_count, a->variant))<<<
+        (a->tune.block_queries ? query_block_kernel(h) : query_kernel(h, a->variant))<<<
             1, 256, query_smem(h), s>>>(p);
         HG_CUDA(cudaGetLastError());
     }
@@ -762,22 +847,19 @@ void launch_plain(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
 
 int read_status(hibf_gpu_agent * a)
 {
-    HG_CUDA(cudaMemcpyAsync(a->h_ctrl.p, a->ctrl.p, C_WORDS * 8, cudaMemcpyDeviceToHost, a->stream));
-    HG_CUDA(cudaMemcpyAsync(a->h_stats.p, a->stats.p, kStats * 8, cudaMemcpyDeviceToHost, a->stream));
     uint32_t const levels = a->last_levels;
-    if (levels)
-        HG_CUDA(cudaMemcpyAsync(a->h_lvl_stats.p, a->lvl_stats.p, levels * kStats * 8, cudaMemcpyDeviceToHost,
-                                a->stream));
+    HG_CUDA(cudaMemcpyAsync(a->h_ctrl.p, a->ctrl.p, (C_WORDS + kStats * (1u + levels)) * 8, cudaMemcpyDeviceToHost,
+                            a->stream));
     HG_CUDA(cudaStreamSynchronize(a->stream));
     unsigned long long const * c = a->h_ctrl.as<unsigned long long>();
-    unsigned long long const * st = a->h_stats.as<unsigned long long>();
+    unsigned long long const * st = c + C_WORDS;
     a->last_tasks = st[0];
     a->last_visits = st[1];
     a->last_executed = st[2];
     a->last_level_stats.clear();
     if (levels)
     {
-        unsigned long long const * ls = a->h_lvl_stats.as<unsigned long long>();
+        unsigned long long const * ls = st + kStats;
         a->last_level_stats.assign(ls, ls + levels * kStats);
         for (uint32_t d = 0; d < levels; ++d)
         {
@@ -1003,6 +1085,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     uint64_t tasks = std::max<uint64_t>(a->cap_tasks, nq * 4 + 1024);
     uint64_t results = std::max<uint64_t>(a->cap_results, nq * 4 + 1024);
     ensure_capacity(a, std::max<uint64_t>(nq, 1), tasks, results); // allocations synchronise: before any copy
+    a->h_roff.ensure((nq + 1) * 8);
     uint32_t const n_tl = streamed ? static_cast<uint32_t>(qb.size() - 1) : 1u;
     if (!a->tl_t0)
     {
@@ -1096,7 +1179,8 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
             launch_batch(a, mode, d_values, a->in_qoff.as<uint64_t>(), a->in_thr.as<uint64_t>(), nq, width);
         if (streamed && attempt == 0)
             HG_CUDA(cudaStreamWaitEvent(a->stream, a->ev_copied, 0)); // later work on the stream follows the copies
-        int const st = read_status(a);
+        HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
+        int const st = read_status(a); // waits for the offsets too
         if (st == HIBF_GPU_OK)
             break;
         unsigned long long const * c = a->h_ctrl.as<unsigned long long>();
@@ -1112,9 +1196,6 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         if (c[C_ERROR] & E_OVERFLOW_REC)
             results = std::max<uint64_t>(results * 4, c[C_NREC] + 1024);
     }
-    a->h_roff.ensure((nq + 1) * 8);
-    HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
-    HG_CUDA(cudaStreamSynchronize(a->stream));
     uint64_t const nr = a->h_roff.as<uint64_t>()[nq];
     a->h_ids.ensure(nr * 8);
     a->h_cnt.ensure(nr * 8);
@@ -1451,7 +1532,7 @@ extern "C"
                 uint64_t const want = (n_queries + 7) / 8;
                 unsigned const grid = static_cast<unsigned>(
                     std::max<uint64_t>(1, std::min<uint64_t>(want, static_cast<uint64_t>(sm_count()) * 8u)));
-                features_kernel(a->h->hash_count)<<<grid, 256, query_smem(a->h), a->stream>>>(p, probe, d_features);
+                features_kernel(a->h)<<<grid, 256, query_smem(a->h), a->stream>>>(p, probe, d_features);
                 HG_CUDA(cudaGetLastError());
             });
     }
@@ -1671,6 +1752,7 @@ extern "C"
                         uint64_t const rw = padded_row_words(bw);
                         h->bins.push_back(bins[k]);
                         h->bin_size.push_back(bin_sizes[k]);
+                        h->wide_rows = h->wide_rows || bin_sizes[k] > UINT32_MAX;
                         h->hash_funs.push_back(hash_funs[k]);
                         h->bin_words.push_back(bw);
                         h->row_words.push_back(rw);
@@ -1707,13 +1789,13 @@ extern "C"
                     HG_CUDA(cudaStreamSynchronize(h->stream));
                     size_t const smem = query_smem(h);
                     for (int v = 0; v < kQueryVariants; ++v)
-                        HG_CUDA(cudaFuncSetAttribute(query_kernel(h->hash_count, v),
+                        HG_CUDA(cudaFuncSetAttribute(query_kernel(h, v),
                                                      cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                      static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
-                    HG_CUDA(cudaFuncSetAttribute(features_kernel(h->hash_count),
+                    HG_CUDA(cudaFuncSetAttribute(features_kernel(h),
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
-                    HG_CUDA(cudaFuncSetAttribute(query_block_kernel(h->hash_count),
+                    HG_CUDA(cudaFuncSetAttribute(query_block_kernel(h),
                                                  cudaFuncAttributeMaxDynamicSharedMemorySize,
                                                  static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
                 }
@@ -2120,20 +2202,18 @@ extern "C"
                     a->stream = a->own;
                     HG_CUDA(cudaEventCreate(&a->ev_k0));
                     HG_CUDA(cudaEventCreate(&a->ev_k1));
-                    a->ctrl.ensure(C_WORDS * 8);
-                    a->stats.ensure(kStats * 8);
-                    a->h_ctrl.ensure(C_WORDS * 8);
-                    a->h_stats.ensure(kStats * 8);
+                    a->ctrl.ensure(ctrl_words(h) * 8);
+                    a->h_ctrl.ensure(ctrl_words(h) * 8);
                     for (int v = 0; v < kQueryVariants; ++v)
                     {
                         int nb = 0;
-                        HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, query_kernel(h->hash_count, v), 256,
+                        HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, query_kernel(h, v), 256,
                                                                               query_smem(h)));
                         a->max_blocks[v] = std::max(1, nb);
                     }
                     {
                         int nb = 0;
-                        HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, query_block_kernel(h->hash_count),
+                        HG_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, query_block_kernel(h),
                                                                               256, query_smem(h)));
                         a->max_blocks_blk = std::max(1, nb);
                     }
@@ -2354,13 +2434,12 @@ extern "C"
                 if (n_queries > a->cap_queries)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "more queries than the agent's last batch can hold");
                 check_mode(mode, width, nullptr, 0);
-                int const st = read_status(a);
-                if (st != HIBF_GPU_OK)
-                    fail(st, "device-side failure in the last batch");
                 a->h_roff.ensure((n_queries + 1) * 8);
                 HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (n_queries + 1) * 8, cudaMemcpyDeviceToHost,
                                         a->stream));
-                HG_CUDA(cudaStreamSynchronize(a->stream));
+                int const st = read_status(a); // waits for the offsets too
+                if (st != HIBF_GPU_OK)
+                    fail(st, "device-side failure in the last batch");
                 uint64_t const nr = a->h_roff.as<uint64_t>()[n_queries];
                 a->h_ids.ensure(nr * 8);
                 a->h_cnt.ensure(nr * 8);
@@ -2573,13 +2652,12 @@ extern "C"
                 a->in_thr.ensure(8);
                 HG_CUDA(cudaMemsetAsync(a->in_qoff.p, 0, 16, s));
                 // no query, but one task announced that nobody will ever push: every worker's wait must expire
-                k_init_ctrl<<<1, 32, 0, s>>>(a->ctrl.as<unsigned long long>(), a->stats.as<unsigned long long>(), 1);
-                HG_CUDA(cudaGetLastError());
-                HG_CUDA(cudaMemsetAsync(a->tasks.p, 0xFF, a->cap_tasks * 8, s));
+                launch_begin(a, 1, 1, a->cap_tasks, 0);
+                a->last_levels = 0;
                 query_params p = base_params(a, a->in_values.as<uint64_t>(), a->in_qoff.as<uint64_t>(),
                                              a->in_thr.as<uint64_t>(), 0, 0xFFFFu);
                 p.wait_limit_ns = static_cast<uint64_t>(limit_ms * 1e6);
-                query_kernel(a->h->hash_count, a->variant)<<<1, 256, query_smem(a->h), s>>>(p);
+                query_kernel(a->h, a->variant)<<<1, 256, query_smem(a->h), s>>>(p);
                 HG_CUDA(cudaGetLastError());
                 int const st = read_status(a);
                 if (st != HIBF_GPU_ERR_TIMEOUT)

@@ -61,6 +61,7 @@ struct hibf_gpu_hibf
     uint32_t max_depth{};
     uint32_t hash_count{}; // number of hash functions, the same for every IBF
     uint32_t counters_per_warp{};
+    bool wide_rows{}; // an IBF has 2^32 rows or more: the kernels take 64-bit row indices
     uint64_t total_bytes{};
     std::vector<hibf_gb300::dev_node> nodes;           // host copy
     std::vector<std::unique_ptr<hibf_gb300::dbuf>> stores;

@@ -201,7 +201,7 @@ __global__ void k_widen(uint64_t * __restrict__ dst, uint32_t dst_row_words, uin
 // hash U values each, the H row words of four sub-steps are loaded together (4 * H loads per lane in flight) -- and
 // each lane stores its word of the AND.  The grid's second dimension is the slab of a row wider than a warp, from
 // word `first_slab` on.
-template <int LPV, int H>
+template <int LPV, int H, typename R>
 __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_t first_slab,
                                                          uint64_t const * __restrict__ values, uint64_t n,
                                                          uint64_t * __restrict__ out)
@@ -223,7 +223,7 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
     uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     for (uint64_t base = warp * BLOCK; base < n; base += nwarps * BLOCK)
     {
-        uint64_t off[U][H];
+        R row_of[U][H];
 #pragma unroll
         for (int u = 0; u < U; ++u)
         {
@@ -231,7 +231,7 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
             uint64_t const v = idx < n ? values[idx] : 0u;
 #pragma unroll
             for (int i = 0; i < H; ++i)
-                off[u][i] = hash_row(v, c_hash_seeds[i], rp.hash_shift, rp.bin_size) * rp.row_words;
+                row_of[u][i] = hash_row_as<R>(v, c_hash_seeds[i], rp.hash_shift, rp.bin_size);
         }
 #pragma unroll 1
         for (int s = 0; s < STEPS; s += 4)
@@ -250,10 +250,10 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
 #pragma unroll
                 for (int i = 0; i < H; ++i)
                 {
-                    uint64_t o = off[u][i];
+                    R r = row_of[u][i];
                     if constexpr (LPV > 1)
-                        o = __shfl_sync(kFullMask, o, src);
-                    w[t][i] = ok[t] ? ldg_evict_first(words + o) : 0ull;
+                        r = __shfl_sync(kFullMask, r, src);
+                    w[t][i] = ok[t] ? ldg_evict_first(words + static_cast<uint64_t>(r) * rp.row_words) : 0ull;
                 }
             }
 #pragma unroll
@@ -270,7 +270,7 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
     }
 }
 
-template <int H>
+template <int H, typename R>
 void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint32_t first_slab, uint32_t slabs,
                        uint64_t const * d_values, uint64_t n, uint64_t * d_out, unsigned grid_x, cudaStream_t s)
 {
@@ -278,22 +278,22 @@ void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint32_t first_
     switch (lpv_log2)
     {
     case 0:
-        k_bulk_contains_h<1, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<1, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 1:
-        k_bulk_contains_h<2, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<2, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 2:
-        k_bulk_contains_h<4, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<4, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 3:
-        k_bulk_contains_h<8, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<8, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     case 4:
-        k_bulk_contains_h<16, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<16, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
         break;
     default:
-        k_bulk_contains_h<32, H><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        k_bulk_contains_h<32, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
     }
 }
 
@@ -304,7 +304,7 @@ void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint32_t first_
 // The grid's second dimension is the slab of a row wider than a warp: a block counts 32 words of every row, a warp one
 // whole 256-byte piece per value and hash function.  (Rows wider than a warp were counted one value at a time, every
 // set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms, now 0.219.)
-template <int H>
+template <int H, typename R>
 __global__ void __launch_bounds__(256, 4)
     k_bulk_count(row_params row, uint64_t const * __restrict__ values, uint64_t n, uint64_t chunk,
                  unsigned long long * __restrict__ totals)
@@ -325,7 +325,7 @@ __global__ void __launch_bounds__(256, 4)
     for (uint64_t start = warp * chunk; start < n; start += nwarps * chunk)
     {
         uint64_t const len = (n - start) < chunk ? (n - start) : chunk;
-        warp_count_lpv<H, true>(rp, lpv_log2, values + start, len, counts, lane);
+        warp_count_lpv<R, H, true>(rp, lpv_log2, values + start, len, counts, lane);
     }
     __syncthreads();
     for (uint32_t i = threadIdx.x; i < n_counters; i += blockDim.x)
@@ -364,20 +364,21 @@ __global__ void k_store_counts(unsigned long long const * __restrict__ totals, u
 
 using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *);
 
+template <typename R>
 bulk_count_kernel_t bulk_count_kernel(uint64_t h)
 {
     switch (h)
     {
     case 1:
-        return k_bulk_count<1>;
+        return k_bulk_count<1, R>;
     case 2:
-        return k_bulk_count<2>;
+        return k_bulk_count<2, R>;
     case 3:
-        return k_bulk_count<3>;
+        return k_bulk_count<3, R>;
     case 4:
-        return k_bulk_count<4>;
+        return k_bulk_count<4, R>;
     default:
-        return k_bulk_count<5>;
+        return k_bulk_count<5, R>;
     }
 }
 
@@ -431,6 +432,10 @@ struct hibf_gpu_ibf
     {
         return row_params{store.as<uint64_t>(), bin_size, static_cast<uint32_t>(row_words),
                           static_cast<uint32_t>(bin_words), shift, static_cast<uint32_t>(hash_funs)};
+    }
+    bool wide_rows() const // the kernels take 64-bit row indices
+    {
+        return bin_size > UINT32_MAX;
     }
     // slabs of a row: kSlabWords words each, the last one what is left
     uint32_t slabs() const
@@ -560,7 +565,8 @@ void launch_count(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, int w
         unsigned const grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, blocks)));
         size_t const smem = (64u << lanes_log2(static_cast<uint32_t>(std::min<uint64_t>(f->bin_words, kSlabWords)))) *
                             sizeof(uint32_t) * (block / 32);
-        bulk_count_kernel_t const kernel = bulk_count_kernel(f->hash_funs);
+        bulk_count_kernel_t const kernel = f->wide_rows() ? bulk_count_kernel<uint64_t>(f->hash_funs)
+                                                          : bulk_count_kernel<uint32_t>(f->hash_funs);
         if (smem > 48 * 1024)
             HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         kernel<<<dim3(grid, slabs), block, smem, s>>>(f->rp(), d_values, n, chunk, totals);
@@ -579,26 +585,34 @@ void launch_contains(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, ui
     uint32_t const full = static_cast<uint32_t>(f->bin_words / kSlabWords);
     uint32_t const rest = static_cast<uint32_t>(f->bin_words % kSlabWords);
     unsigned const grid = grid_for(n, 256);
-    auto launch = [&](uint32_t lpv_log2, uint32_t first, uint32_t slabs)
+    auto launch_h = [&](auto row_index, uint32_t lpv_log2, uint32_t first, uint32_t slabs)
     {
+        using R = decltype(row_index);
         switch (f->hash_funs)
         {
         case 1:
-            launch_contains_h<1>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
+            launch_contains_h<1, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 2:
-            launch_contains_h<2>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
+            launch_contains_h<2, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 3:
-            launch_contains_h<3>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
+            launch_contains_h<3, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         case 4:
-            launch_contains_h<4>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
+            launch_contains_h<4, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
             break;
         default:
-            launch_contains_h<5>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
+            launch_contains_h<5, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
         }
         HG_CUDA(cudaGetLastError());
+    };
+    auto launch = [&](uint32_t lpv_log2, uint32_t first, uint32_t slabs)
+    {
+        if (f->wide_rows())
+            launch_h(uint64_t{}, lpv_log2, first, slabs);
+        else
+            launch_h(uint32_t{}, lpv_log2, first, slabs);
     };
     constexpr uint32_t kMaxGridY = 65535;
     for (uint32_t first = 0; first < full; first += kMaxGridY)

@@ -51,7 +51,6 @@ enum : int
     C_PENDING = 2,
     C_NREC = 3,
     C_ERROR = 4,
-    C_NLARGE = 5,
     C_CHILD = 6, // streamed inputs: claims of child slots (roots and children are then claimed separately)
     C_WORDS = 8
 };
@@ -427,7 +426,7 @@ static __device__ __noinline__ int segment_state(query_params const & p, dev_nod
 
 // Counting with variant V.  Variant 0 handles every row width; the tuned variants only rows of up to 4 words (the
 // host offers them only for such hierarchies, and process_task refuses wider rows).
-template <int H, int V>
+template <int H, int V, typename R>
 __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
                                               uint64_t n, uint32_t * counts, int lane, uint64_t * stage)
 {
@@ -435,33 +434,33 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
     switch (lpv_log2)
     {
     case 0:
-        warp_count<1, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+        warp_count<R, 1, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
         break;
     case 1:
         if constexpr (Q::W == 2)
-            warp_count<1, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 1, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
         else
-            warp_count<2, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 2, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
         break;
     case 2:
         if constexpr (Q::W == 2)
-            warp_count<2, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 2, H, Q::K, Q::UM, 2>(rp, vals, n, counts, lane, stage);
         else
-            warp_count<4, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 4, H, Q::K, Q::UM, 1>(rp, vals, n, counts, lane, stage);
         break;
     case 3:
         if constexpr (V == 0)
-            warp_count<8, H, Q::K>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 8, H, Q::K>(rp, vals, n, counts, lane, stage);
         break;
     case 4:
         if constexpr (V == 0)
-            warp_count<16, H, Q::K>(rp, vals, n, counts, lane, stage);
+            warp_count<R, 16, H, Q::K>(rp, vals, n, counts, lane, stage);
         break;
     default:
         if constexpr (V == 0)
 #pragma unroll 1
             for (uint32_t w0 = 0; w0 < rp.bin_words; w0 += kSlabWords) // one slab unless the row is wider than a warp
-                warp_count<32, H, Q::K>(row_slab(rp, w0), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
+                warp_count<R, 32, H, Q::K>(row_slab(rp, w0), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
     }
 }
 
@@ -513,10 +512,15 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
             if (lane == 0)
             {
                 if (!p.level)
+                {
+                    // counted before any of them can be seen, run and retired
                     atomicAdd(p.ctrl + C_PENDING, static_cast<unsigned long long>(nc));
+                    __threadfence();
+                }
                 base = atomicAdd(p.ctrl + C_TAIL, static_cast<unsigned long long>(nc));
             }
             base = __shfl_sync(kFullMask, base, 0);
+            __syncwarp();
             if (emit_child)
             {
                 unsigned long long const s = base + __popc(cb & lt_mask);
@@ -533,15 +537,15 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
                     if (!p.level)
                         atomicAdd(p.ctrl + C_PENDING, ~0ull); // this child will never run
                 }
-                if (!p.level)
-                    __threadfence();
             }
         }
     }
 }
 
 // A finished task leaves the count of unfinished ones (the level schedule keeps none: its launches end by themselves)
-// and enters the work counters.
+// and enters the work counters.  No fence: a waiting worker learns of a child from its slot alone (one atomic word),
+// the task's children were counted by this same thread, and records are read by later launches only.  (A fence per
+// task was the second largest stall of a batch of 10,000 short queries.)
 __device__ __forceinline__ void retire_task(query_params const & p, uint64_t q, uint64_t n, uint64_t done, int lane,
                                             unsigned long long & n_tasks, unsigned long long & n_visits,
                                             unsigned long long & n_executed)
@@ -551,10 +555,7 @@ __device__ __forceinline__ void retire_task(query_params const & p, uint64_t q, 
     if (p.qwork)
         atomicAdd(p.qwork + q + p.q_base, static_cast<unsigned long long>(done));
     if (!p.level)
-    {
-        __threadfence();
         atomicAdd(p.ctrl + C_PENDING, ~0ull);
-    }
     ++n_tasks;
     n_visits += n;
     n_executed += done;
@@ -629,7 +630,7 @@ __device__ __forceinline__ void emit_task(query_params const & p, dev_node const
     retire_task(p, q, n, done, lane, n_tasks, n_visits, n_executed);
 }
 
-template <int H, int V>
+template <int H, int V, typename R>
 __device__ void process_task(query_params const & p, unsigned long long task, uint32_t * counts, int lane,
                              unsigned long long & n_tasks, unsigned long long & n_visits,
                              unsigned long long & n_executed)
@@ -720,7 +721,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         {
             bool const from_stage = done < staged;
             uint64_t const end = from_stage ? min(stop, staged) : stop;
-            count_variant<H, V>(rp, nd.lpv_log2, (from_stage ? p.stage : p.values) + b0 + done, end - done, counts,
+            count_variant<H, V, R>(rp, nd.lpv_log2, (from_stage ? p.stage : p.values) + b0 + done, end - done, counts,
                                 lane, stage_root ? p.stage + b0 + done : nullptr);
             done = end;
         }
@@ -750,7 +751,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
 #ifndef HIBF_QUERY_MIN_BLOCKS
 #    define HIBF_QUERY_MIN_BLOCKS 2
 #endif
-template <int H, int V>
+template <int H, int V, typename R>
 __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
@@ -816,7 +817,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
                     break; // E_TIMEOUT is set
                 task = make_task(q, 0u, 0u);
             }
-            process_task<H, V>(p, task, counts, lane, n_tasks, n_visits, n_executed);
+            process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed);
         }
     }
     for (; !p.level;)
@@ -954,7 +955,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
                     break;
             }
         }
-        process_task<H, V>(p, task, counts, lane, n_tasks, n_visits, n_executed);
+        process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed);
     }
     if (lane == 0 && n_tasks)
     {
@@ -970,7 +971,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
 // grandchild of its slowest query bounds it).  No early exit: a slice's counts do not bound the task's.
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
-template <int H>
+template <int H, typename R>
 __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
@@ -1053,7 +1054,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
         uint64_t const lo = min(n, static_cast<uint64_t>(warp) * per);
         uint64_t const hi = min(n, lo + per);
         if (hi > lo)
-            count_variant<H, 0>(rp, nd.lpv_log2, p.values + b0 + lo, hi - lo, counts, lane, nullptr);
+            count_variant<H, 0, R>(rp, nd.lpv_log2, p.values + b0 + lo, hi - lo, counts, lane, nullptr);
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < ncount; i += blockDim.x)
         {
@@ -1085,7 +1086,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
 constexpr int kCostFeatures = 6;
 using features_kernel_t = void (*)(query_params, uint32_t, float *);
 
-template <int H>
+template <int H, typename R>
 __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_params const p, uint32_t probe, float * __restrict__ out)
 {
     extern __shared__ uint32_t s_counts[];
@@ -1106,7 +1107,7 @@ __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_
             counts[i] = 0;
         __syncwarp();
         if (m)
-            count_variant<H, 0>(rp, nd.lpv_log2, p.values + b0, m, counts, lane, nullptr);
+            count_variant<H, 0, R>(rp, nd.lpv_log2, p.values + b0, m, counts, lane, nullptr);
         __syncwarp();
         double const rate = n ? static_cast<double>(p.thr[q]) / static_cast<double>(n) : 0.0;
         unsigned long long const need = static_cast<unsigned long long>(ceil(rate * static_cast<double>(m)));
@@ -1164,100 +1165,76 @@ __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_
     }
 }
 
-// The kernel of variant v (0 <= v < kQueryVariants; H > 3 has the default variant only).
+// The kernel of variant v (0 <= v < kQueryVariants; H > 3 has the default variant only).  `wide`: some IBF has 2^32 rows
+// or more, so row indices are 64 bits wide (the default variant only; a schedule does not change results).
 template <int H>
-query_kernel_t query_kernel_variant(int v)
+query_kernel_t query_kernel_variant(int v, bool wide)
 {
+    if (wide)
+        return k_query<H, 0, uint64_t>;
     if constexpr (H > 3)
     {
         (void)v;
-        return k_query<H, 0>;
+        return k_query<H, 0, uint32_t>;
     }
     else
     {
         switch (v)
         {
         case 1:
-            return k_query<H, 1>;
+            return k_query<H, 1, uint32_t>;
         case 2:
-            return k_query<H, 2>;
+            return k_query<H, 2, uint32_t>;
         case 3:
-            return k_query<H, 3>;
+            return k_query<H, 3, uint32_t>;
         case 4:
-            return k_query<H, 4>;
+            return k_query<H, 4, uint32_t>;
         case 5:
-            return k_query<H, 5>;
+            return k_query<H, 5, uint32_t>;
         default:
-            return k_query<H, 0>;
+            return k_query<H, 0, uint32_t>;
         }
     }
 }
 
-// Defined in query_h1.cu .. query_h5.cu.
-query_kernel_t query_kernel_h1(int v);
-query_kernel_t query_kernel_h2(int v);
-query_kernel_t query_kernel_h3(int v);
-query_kernel_t query_kernel_h4(int v);
-query_kernel_t query_kernel_h5(int v);
-query_kernel_t query_block_kernel_h1();
-query_kernel_t query_block_kernel_h2();
-query_kernel_t query_block_kernel_h3();
-query_kernel_t query_block_kernel_h4();
-query_kernel_t query_block_kernel_h5();
-features_kernel_t features_kernel_h1();
-features_kernel_t features_kernel_h2();
-features_kernel_t features_kernel_h3();
-features_kernel_t features_kernel_h4();
-features_kernel_t features_kernel_h5();
-
-inline query_kernel_t query_block_kernel(uint32_t h)
+// The three query kernels of one hash function count, defined in query_h1.cu .. query_h5.cu.
+struct query_kernels
 {
-    switch (h)
-    {
-    case 1:
-        return query_block_kernel_h1();
-    case 2:
-        return query_block_kernel_h2();
-    case 3:
-        return query_block_kernel_h3();
-    case 4:
-        return query_block_kernel_h4();
-    default:
-        return query_block_kernel_h5();
-    }
+    query_kernel_t (*variant)(int v, bool wide);
+    query_kernel_t (*block)(bool wide);
+    features_kernel_t (*features)(bool wide);
+};
+
+template <int H>
+constexpr query_kernels make_query_kernels()
+{
+    return query_kernels{query_kernel_variant<H>,
+                         [](bool wide) -> query_kernel_t
+                         { return wide ? k_query_blk<H, uint64_t> : k_query_blk<H, uint32_t>; },
+                         [](bool wide) -> features_kernel_t
+                         { return wide ? k_query_features<H, uint64_t> : k_query_features<H, uint32_t>; }};
 }
 
-inline features_kernel_t features_kernel(uint32_t h)
-{
-    switch (h)
-    {
-    case 1:
-        return features_kernel_h1();
-    case 2:
-        return features_kernel_h2();
-    case 3:
-        return features_kernel_h3();
-    case 4:
-        return features_kernel_h4();
-    default:
-        return features_kernel_h5();
-    }
-}
+extern query_kernels const query_kernels_h1;
+extern query_kernels const query_kernels_h2;
+extern query_kernels const query_kernels_h3;
+extern query_kernels const query_kernels_h4;
+extern query_kernels const query_kernels_h5;
 
-inline query_kernel_t query_kernel(uint32_t h, int v)
+inline query_kernels const & query_kernels_of(uint32_t h)
 {
     switch (h)
     {
     case 1:
-        return query_kernel_h1(v);
+        return query_kernels_h1;
     case 2:
-        return query_kernel_h2(v);
+        return query_kernels_h2;
     case 3:
-        return query_kernel_h3(v);
+        return query_kernels_h3;
     case 4:
-        return query_kernel_h4(v);
+        return query_kernels_h4;
     default:
-        return query_kernel_h5(v);
+        return query_kernels_h5;
     }
 }
 

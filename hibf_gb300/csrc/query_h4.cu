@@ -1,20 +1,9 @@
-// query_h4.cu -- the HIBF query kernels for hierarchies with 4 hash function(s): every tuning variant and the
-// learned scheduler's feature kernel.
-// One translation unit per hash function count keeps the instantiations compiling in parallel.
+// query_h4.cu -- the query kernels for 4 hash functions (see query.cuh).
 #include "query.cuh"
 
 namespace hibf_gb300
 {
-query_kernel_t query_kernel_h4(int v)
-{
-    return query_kernel_variant<4>(v);
-}
-query_kernel_t query_block_kernel_h4()
-{
-    return k_query_blk<4>;
-}
-features_kernel_t features_kernel_h4()
-{
-    return k_query_features<4>;
-}
+
+query_kernels const query_kernels_h4 = make_query_kernels<4>();
+
 } // namespace hibf_gb300

@@ -1,20 +1,9 @@
-// query_h5.cu -- the HIBF query kernels for hierarchies with 5 hash function(s): every tuning variant and the
-// learned scheduler's feature kernel.
-// One translation unit per hash function count keeps the instantiations compiling in parallel.
+// query_h5.cu -- the query kernels for 5 hash functions (see query.cuh).
 #include "query.cuh"
 
 namespace hibf_gb300
 {
-query_kernel_t query_kernel_h5(int v)
-{
-    return query_kernel_variant<5>(v);
-}
-query_kernel_t query_block_kernel_h5()
-{
-    return k_query_blk<5>;
-}
-features_kernel_t features_kernel_h5()
-{
-    return k_query_features<5>;
-}
+
+query_kernels const query_kernels_h5 = make_query_kernels<5>();
+
 } // namespace hibf_gb300
