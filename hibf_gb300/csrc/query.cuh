@@ -465,14 +465,15 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
 }
 
 // Reports and descents of 32 bins of a counted task: this lane's bin `ds` ends its segment with `sum` (already reduced
-// to the counter range).  `level`: the launch answers one level, so nobody reads the children before it ends.
+// to the counter range).  In the level schedule nobody reads the children before the launch ends.  `keep` (optional, in
+// shared memory, kEmpty before the task): the task's first child goes there instead of into the queue.
 __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsigned long long sum, bool pass,
-                                          uint64_t q, uint32_t depth, int lane)
+                                          uint64_t q, uint32_t depth, int lane, unsigned long long * keep)
 {
     unsigned const lt_mask = (1u << lane) - 1u;
     uint64_t const gq = q + p.q_base;
     bool const emit_ub = (ds.y & F_RUN_END) && pass;
-    bool const emit_child = (ds.y & F_MERGED) && pass;
+    bool emit_child = (ds.y & F_MERGED) && pass;
     unsigned const rb = __ballot_sync(kFullMask, emit_ub);
     if (rb)
     {
@@ -497,7 +498,19 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
             }
         }
     }
-    unsigned const cb = __ballot_sync(kFullMask, emit_child);
+    unsigned cb = __ballot_sync(kFullMask, emit_child);
+    if (cb && keep && depth < p.max_depth && *keep == kEmpty)
+    {
+        int const first = __ffs(cb) - 1;
+        __syncwarp(); // every lane has read *keep
+        if (lane == 0)
+            atomicAdd(p.ctrl + C_PENDING, 1ull);
+        if (lane == first)
+            *keep = make_task(q, depth + 1u, ds.x);
+        __syncwarp();
+        cb &= cb - 1;
+        emit_child = emit_child && lane != first;
+    }
     if (cb)
     {
         unsigned const nc = __popc(cb);
@@ -563,7 +576,8 @@ __device__ __forceinline__ void retire_task(query_params const & p, uint64_t q, 
 
 // The bin scan of a counted task with 64-bit sums (see segment_state).
 static __device__ __noinline__ void emit_bins_wide(query_params const & p, dev_node const & nd, uint32_t const * counts,
-                                                   uint64_t q, uint32_t depth, uint64_t thr, int lane)
+                                                   uint64_t q, uint32_t depth, uint64_t thr, int lane,
+                                            unsigned long long * keep)
 {
     uint2 const * d = p.descs + nd.desc_offset;
     unsigned long long carry = 0;
@@ -589,7 +603,7 @@ static __device__ __noinline__ void emit_bins_wide(query_params const & p, dev_n
             }
         }
         unsigned long long const sum = x & p.count_mask;
-        emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane);
+        emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane, keep);
         unsigned long long const lastx = __shfl_sync(kFullMask, x, 31);
         uint32_t const lastf = __shfl_sync(kFullMask, ds.y, 31);
         carry = (lastf & (F_MERGED | F_RUN_END)) ? 0ull : lastx;
@@ -601,7 +615,7 @@ static __device__ __noinline__ void emit_bins_wide(query_params const & p, dev_n
 __device__ __forceinline__ void emit_task(query_params const & p, dev_node const & nd, uint32_t const * counts,
                                           uint64_t q, uint32_t depth, uint64_t n, uint64_t done, uint64_t thr,
                                           int lane, unsigned long long & n_tasks, unsigned long long & n_visits,
-                                          unsigned long long & n_executed)
+                                          unsigned long long & n_executed, unsigned long long * keep = nullptr)
 {
     if (n * nd.max_seg < kNarrowSums)
     {
@@ -619,12 +633,12 @@ __device__ __forceinline__ void emit_task(query_params const & p, dev_node const
                 carry = __shfl_sync(kFullMask, (ds.y & (F_MERGED | F_RUN_END)) ? 0u : x, 31);
             }
             unsigned long long const sum = x & p.count_mask;
-            emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane);
+            emit_bins(p, ds, sum, valid && sum >= thr, q, depth, lane, keep);
         }
     }
     else
     {
-        emit_bins_wide(p, nd, counts, q, depth, thr, lane);
+        emit_bins_wide(p, nd, counts, q, depth, thr, lane, keep);
     }
     __syncwarp();
     retire_task(p, q, n, done, lane, n_tasks, n_visits, n_executed);
@@ -633,7 +647,7 @@ __device__ __forceinline__ void emit_task(query_params const & p, dev_node const
 template <int H, int V, typename R>
 __device__ void process_task(query_params const & p, unsigned long long task, uint32_t * counts, int lane,
                              unsigned long long & n_tasks, unsigned long long & n_visits,
-                             unsigned long long & n_executed)
+                             unsigned long long & n_executed, unsigned long long * keep)
 {
     uint64_t const q = task >> 32;
     uint32_t const depth = static_cast<uint32_t>(task >> kNodeBits) & 63u;
@@ -742,7 +756,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
         return;
     }
 
-    emit_task(p, nd, counts, q, depth, n, done, thr, lane, n_tasks, n_visits, n_executed);
+    emit_task(p, nd, counts, q, depth, n, done, thr, lane, n_tasks, n_visits, n_executed, keep);
 }
 
 // H = the hierarchy's hash function count (one value for all IBFs, as in the reference's build).
@@ -774,12 +788,12 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
     // instead of piling up behind the last chunk; a warp whose claimed root (`held`) has not arrived yet runs queued
     // children meanwhile.
     // The streamed-mode state of each warp lives in shared memory, off the registers of the counting code.
-    __shared__ unsigned long long s_held[8], s_held_since[8];
+    __shared__ unsigned long long s_held[8], s_held_since[8], s_keep[8];
     __shared__ unsigned int s_held_need[8], s_backoff[8], s_polls[8];
     int const w = threadIdx.x >> 5;
     if (lane == 0)
     {
-        s_held[w] = kEmpty;
+        s_held[w] = s_keep[w] = kEmpty;
         s_held_since[w] = 0;
         s_held_need[w] = s_backoff[w] = s_polls[w] = 0;
     }
@@ -817,12 +831,25 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
                     break; // E_TIMEOUT is set
                 task = make_task(q, 0u, 0u);
             }
-            process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed);
+            process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed, nullptr);
         }
     }
+    // With a claim order (longest query first) a worker goes on with the first child of its task instead of queueing it
+    // behind the roots: a query's work then runs in one piece, in the order given, and the batch ends with the shortest
+    // queries.  (Children behind all roots ended it with the descents of long ones: 20,000 queries of 8,192 user bins at
+    // a hundredth of their size, 0.242 ms in the learned order against 0.249 in query order.)
+    bool const chain = p.order && !p.arrived;
     for (; !p.level;)
     {
         unsigned long long task = kEmpty;
+        if (chain)
+        {
+            task = s_keep[w];
+            __syncwarp();
+            if (lane == 0)
+                s_keep[w] = kEmpty;
+            __syncwarp();
+        }
         unsigned long long held = s_held[w];
         if (held != kEmpty)
         {
@@ -955,7 +982,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
                     break;
             }
         }
-        process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed);
+        process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed, chain ? s_keep + w : nullptr);
     }
     if (lane == 0 && n_tasks)
     {
