@@ -461,6 +461,118 @@ __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const 
     }
 }
 
+// ---- a small host batch: everything after its query kernel in one block ----
+constexpr uint64_t kSmallBatch = 1024;      // queries
+constexpr uint32_t kSmallRecords = 2048;    // results; more take the general passes
+constexpr uint64_t kPackValues = 8192;      // values that travel with the offsets and thresholds in one copy
+// words of the host buffer k_finish_small writes: control words and counters, whether it could, offsets, ids, counts
+constexpr uint32_t kSmallOk = C_WORDS + kStats;
+constexpr uint32_t kSmallOffsets = 16;
+constexpr uint32_t kSmallIds = kSmallOffsets + kSmallBatch + 2;
+constexpr uint32_t kSmallCounts = kSmallIds + kSmallRecords;
+constexpr uint32_t kSmallWords = kSmallCounts + kSmallRecords;
+
+// Offsets, placement, order and counter width of up to kSmallRecords results of up to kSmallBatch queries, in shared
+// memory, written to the agent's device buffers and straight to page-locked host memory, so that no copy follows.  It
+// leaves the workspace as the next batch wants it (control words, counts and used task slots reset), so that nothing
+// precedes the next query kernel.  Bound by latency: one block, a handful of dependent steps, about 4 us, for seven
+// launches and three copies before (17 us of kernels alone).
+__global__ void __launch_bounds__(1024) k_finish_small(unsigned long long * ctrl, unsigned int * qcount, uint32_t nq,
+                                                       unsigned long long * tasks, uint64_t task_cap,
+                                                       uint32_t const * __restrict__ rec_q,
+                                                       uint32_t const * __restrict__ rec_ub,
+                                                       unsigned long long const * __restrict__ rec_cnt,
+                                                       unsigned long long * __restrict__ roff,
+                                                       uint64_t * __restrict__ out_ids, uint64_t * __restrict__ out_cnt,
+                                                       int width, void * narrow, bool counts,
+                                                       unsigned long long * __restrict__ host)
+{
+    __shared__ uint32_t s_off[kSmallBatch + 1], s_left[kSmallBatch], s_warp[32];
+    __shared__ uint32_t s_id[kSmallRecords];
+    __shared__ unsigned long long s_cnt[kSmallRecords];
+    __shared__ uint16_t s_q[kSmallRecords];
+    uint32_t const t = threadIdx.x;
+    int const lane = t & 31, w = t >> 5;
+    unsigned long long const n_all = ctrl[C_NREC];
+    bool const ok = n_all <= kSmallRecords && ctrl[C_ERROR] == 0;
+    uint64_t const tail = ctrl[C_TAIL];
+    uint32_t const n = ok ? static_cast<uint32_t>(n_all) : 0u;
+    uint32_t const c = ok && t < nq ? qcount[t] : 0u;
+    uint32_t x = c;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1)
+    {
+        uint32_t const y = __shfl_up_sync(kFullMask, x, o);
+        if (lane >= o)
+            x += y;
+    }
+    if (lane == 31)
+        s_warp[w] = x;
+    __syncthreads();
+    if (w == 0)
+    {
+        uint32_t z = s_warp[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1)
+        {
+            uint32_t const y = __shfl_up_sync(kFullMask, z, o);
+            if (lane >= o)
+                z += y;
+        }
+        s_warp[lane] = z;
+    }
+    __syncthreads();
+    x += w ? s_warp[w - 1] : 0u;
+    s_off[t + 1] = x;
+    if (t == 0)
+        s_off[0] = 0;
+    s_left[t] = c;
+    __syncthreads();
+    for (uint32_t r = t; r < n; r += blockDim.x)
+    {
+        uint32_t const q = rec_q[r];
+        uint32_t const pos = s_off[q] + (atomicSub(s_left + q, 1u) - 1u);
+        s_id[pos] = rec_ub[r];
+        s_cnt[pos] = rec_cnt[r];
+        s_q[pos] = static_cast<uint16_t>(q);
+    }
+    __syncthreads();
+    for (uint32_t i = t; i < n; i += blockDim.x)
+    {
+        uint32_t const id = s_id[i], b = s_off[s_q[i]], e = s_off[s_q[i] + 1u];
+        uint32_t at = b; // this result's rank among its query's
+        for (uint32_t j = b; j < e; ++j)
+            at += s_id[j] < id || (s_id[j] == id && j < i);
+        out_ids[at] = id;
+        out_cnt[at] = s_cnt[i];
+        host[kSmallIds + at] = id;
+        if (counts)
+            store_count(host + kSmallCounts, width, at, s_cnt[i]);
+        if (narrow)
+            store_count(narrow, width, at, s_cnt[i]);
+    }
+    if (ok)
+    {
+        for (uint32_t q = t; q <= nq; q += blockDim.x)
+        {
+            roff[q] = s_off[q];
+            host[kSmallOffsets + q] = s_off[q];
+        }
+        if (t < nq)
+            qcount[t] = 0;
+        for (uint64_t i = t; i < min(tail, task_cap); i += blockDim.x)
+            tasks[i] = kEmpty;
+    }
+    if (t < C_WORDS + kStats)
+    {
+        host[t] = ctrl[t];
+        if (ok)
+            ctrl[t] = 0; // every thread has read the control words it needs (barriers above)
+    }
+    if (t == 0)
+        host[kSmallOk] = ok;
+}
+
 // emplace into an IBF (same as the single-level kernel, repeated here to keep the translation units independent).
 __global__ void k_hibf_emplace(uint64_t * __restrict__ words, uint64_t bin_size, uint32_t row_words, uint32_t shift,
                                uint32_t h, uint64_t const * __restrict__ values, uint64_t const * __restrict__ bins,
@@ -548,6 +660,14 @@ struct hibf_gpu_agent
     std::vector<cudaEvent_t> tl_chunk;
     uint32_t tl_n{};
     hbuf h_roff, h_ids, h_cnt, h_ctrl;
+    // small host batches: inputs packed for one copy, results and control words written by k_finish_small
+    hbuf h_pack, h_small;
+    dbuf d_pack;
+    bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: the next one needs no k_begin
+    // the last host batch's results: in h_small, or in h_roff / h_ids / h_cnt
+    uint64_t const * res_off{};
+    uint64_t const * res_ids{};
+    void const * res_cnt{};
     std::vector<uint64_t> single_ids;
     std::vector<uint8_t> dense;
     std::vector<uint64_t> thr_tmp, qoff_tmp;
@@ -567,12 +687,14 @@ void ensure_capacity(hibf_gpu_agent * a, uint64_t nq, uint64_t tasks, uint64_t r
     if (nq > a->cap_queries)
     {
         a->qcount.ensure(nq * 4);
+        a->clean = false;
         a->roff.ensure((nq + 1) * 8);
         a->bsum.ensure(((nq + kScanBlock - 1) / kScanBlock + 1) * 8);
         a->cap_queries = nq;
     }
     if (tasks > a->cap_tasks)
     {
+        a->clean = false;
         a->tasks.ensure(tasks * 8);
         a->cap_tasks = tasks;
     }
@@ -702,6 +824,7 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
 // Readies the workspace for a batch of nq queries (k_begin): `marks` empty-slot marks, `levels` histograms.
 void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t marks, uint64_t levels)
 {
+    a->clean = false;
     uint64_t const n_hist = levels * a->h->n_ibfs;
     uint64_t const most = std::max({static_cast<uint64_t>(ctrl_words(a->h)), nq, marks / 2, n_hist});
     k_begin<<<grid_cap(most, 256, 8), 256, 0, a->stream>>>(a->ctrl.as<unsigned long long>(), ctrl_words(a->h), pending,
@@ -845,8 +968,31 @@ void launch_plain(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
     launch_postprocess(a, nq, mode, width);
 }
 
+// The status of a batch whose kernels set these error bits.
+int status_of(unsigned long long e)
+{
+    if (e & E_TIMEOUT)
+        return HIBF_GPU_ERR_TIMEOUT;
+    if (e & E_CYCLE)
+        return HIBF_GPU_ERR_CYCLE;
+    if (e & E_VARIANT)
+        return HIBF_GPU_ERR_LOGIC;
+    if (e & E_ORDER)
+        return HIBF_GPU_ERR_INVALID_ARG;
+    if (e & E_TASK)
+        return HIBF_GPU_ERR_LOGIC;
+    if (e & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
+        return HIBF_GPU_ERR_OVERFLOW;
+    return HIBF_GPU_OK;
+}
+
 int read_status(hibf_gpu_agent * a)
 {
+    if (a->clean) // the last batch was a small one that succeeded: its counters are read, the device's reset
+    {
+        HG_CUDA(cudaStreamSynchronize(a->stream));
+        return HIBF_GPU_OK;
+    }
     uint32_t const levels = a->last_levels;
     HG_CUDA(cudaMemcpyAsync(a->h_ctrl.p, a->ctrl.p, (C_WORDS + kStats * (1u + levels)) * 8, cudaMemcpyDeviceToHost,
                             a->stream));
@@ -868,20 +1014,7 @@ int read_status(hibf_gpu_agent * a)
             a->last_executed += ls[d * kStats + 2];
         }
     }
-    unsigned long long const e = c[C_ERROR];
-    if (e & E_TIMEOUT)
-        return HIBF_GPU_ERR_TIMEOUT;
-    if (e & E_CYCLE)
-        return HIBF_GPU_ERR_CYCLE;
-    if (e & E_VARIANT)
-        return HIBF_GPU_ERR_LOGIC;
-    if (e & E_ORDER)
-        return HIBF_GPU_ERR_INVALID_ARG;
-    if (e & E_TASK)
-        return HIBF_GPU_ERR_LOGIC;
-    if (e & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
-        return HIBF_GPU_ERR_OVERFLOW;
-    return HIBF_GPU_OK;
+    return status_of(c[C_ERROR]);
 }
 
 // Runs ok(lo, hi) over [0, n) and returns whether every piece held: one piece below 2^17 entries, else up to eight
@@ -1031,6 +1164,133 @@ std::vector<uint64_t> const & traversal_rank(hibf_gpu_hibf * h)
     return h->trav_rank;
 }
 
+// Events of a host batch's timeline (hibf_gpu_agent_last_timeline) for n copies of values.
+void ensure_timeline(hibf_gpu_agent * a, uint32_t n)
+{
+    if (!a->tl_t0)
+    {
+        HG_CUDA(cudaEventCreate(&a->tl_t0));
+        HG_CUDA(cudaEventCreate(&a->tl_done));
+    }
+    while (a->tl_chunk.size() < n)
+    {
+        cudaEvent_t e{};
+        HG_CUDA(cudaEventCreate(&e));
+        a->tl_chunk.push_back(e);
+    }
+}
+
+// A host batch of at most kSmallBatch queries that runs a task per block (or is one plain query): one copy in (two when
+// the values do not fit the packed buffer), the query kernel, k_finish_small, one wait.  kRerun: not a small batch, or a
+// capacity was exceeded (now larger) or an error occurred: the general path starts over; kCounted: more results than
+// k_finish_small takes, they wait in the workspace for the general passes.  One plain query of 250 values on 8,192 user
+// bins took 105 us through the general path: three waits, a dozen launches, memsets and copies.
+enum class small_result
+{
+    kRerun,
+    kCounted,
+    kDone
+};
+small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t const * qoff, uint64_t nq,
+                         uint64_t const * thr, int width, bool plain, uint64_t const * in_place)
+{
+    if (nq == 0 || nq > kSmallBatch || (!plain && nq > a->tune.block_queries) || a->order || a->qwork)
+        return small_result::kRerun;
+    hibf_gpu_hibf * h = a->h;
+    cudaStream_t s = a->stream;
+    uint64_t const nv = qoff[nq];
+    if (!in_place && nv * 8 >= kStreamMinBytes)
+        return small_result::kRerun; // streamed: the kernel runs beside the copy
+    bool const pack = !in_place && nv <= kPackValues;
+    uint64_t const words = 2 * nq + 1 + (pack ? nv : 0);
+    ensure_capacity(a, nq, std::max<uint64_t>(a->cap_tasks, nq * 4 + 1024),
+                    std::max<uint64_t>(a->cap_results, nq * 4 + 1024));
+    a->h_pack.ensure((2 * kSmallBatch + 1 + kPackValues) * 8);
+    a->d_pack.ensure((2 * kSmallBatch + 1 + kPackValues) * 8);
+    a->h_small.ensure(kSmallWords * 8);
+    if (!pack && !in_place)
+        a->in_values.ensure(nv * 8);
+    ensure_timeline(a, 1);
+    uint64_t * const hp = a->h_pack.as<uint64_t>();
+    std::memcpy(hp, qoff, (nq + 1) * 8);
+    std::memcpy(hp + nq + 1, thr, nq * 8);
+    if (pack && nv)
+        std::memcpy(hp + 2 * nq + 1, values, nv * 8);
+    a->tl_n = 0;
+    HG_CUDA(cudaEventRecord(a->tl_t0, s));
+    if (!a->clean)
+        launch_begin(a, 0, a->cap_queries, a->cap_tasks, 0);
+    a->clean = false; // until k_finish_small has run
+    HG_CUDA(cudaMemcpyAsync(a->d_pack.p, hp, words * 8, cudaMemcpyHostToDevice, s));
+    if (!pack && !in_place)
+        HG_CUDA(cudaMemcpyAsync(a->in_values.p, values, nv * 8, cudaMemcpyHostToDevice, s));
+    HG_CUDA(cudaEventRecord(a->tl_chunk[0], s));
+    a->tl_n = 1;
+    uint64_t const * const dp = a->d_pack.as<uint64_t>();
+    uint64_t const * const dv = in_place ? in_place : pack ? dp + 2 * nq + 1 : a->in_values.as<uint64_t>();
+    query_params p = base_params(a, dv, dp, dp + nq + 1, nq, mask_for(mode, width));
+    p.decide = mode == HIBF_GPU_QUERY_MEMBERSHIP;
+    p.pending_bias = nq;
+    bool const blk = !plain || a->tune.block_queries != 0;
+    int const fit = blk ? a->max_blocks_blk : a->max_blocks[a->variant];
+    int const per_sm = a->tune.blocks_per_sm ? std::min<int>(fit, static_cast<int>(a->tune.blocks_per_sm)) : fit;
+    unsigned const grid =
+        static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(sm_count()) * per_sm, blk ? nq : 1));
+    HG_CUDA(cudaEventRecord(a->ev_k0, s));
+    (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256, query_smem(h), s>>>(p);
+    HG_CUDA(cudaGetLastError());
+    HG_CUDA(cudaEventRecord(a->ev_k1, s));
+    bool const counts = mode == HIBF_GPU_QUERY_COUNT;
+    unsigned long long * const host = a->h_small.as<unsigned long long>();
+    k_finish_small<<<1, 1024, 0, s>>>(
+        a->ctrl.as<unsigned long long>(), a->qcount.as<unsigned int>(), static_cast<uint32_t>(nq),
+        a->tasks.as<unsigned long long>(), a->cap_tasks, a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(),
+        a->rec_cnt.as<unsigned long long>(), a->roff.as<unsigned long long>(), a->out_ids.as<uint64_t>(),
+        a->out_cnt.as<uint64_t>(), width, counts && width != 8 ? a->out_cntw.p : nullptr, counts, host);
+    HG_CUDA(cudaGetLastError());
+    HG_CUDA(cudaEventRecord(a->tl_done, s));
+    HG_CUDA(cudaStreamSynchronize(s));
+    a->last_levels = 0;
+    if (!host[kSmallOk])
+    {
+        if (host[C_ERROR] == 0)
+            return small_result::kCounted;
+        ensure_capacity(a, nq, host[C_ERROR] & E_OVERFLOW_TASK ? a->cap_tasks * 4 : a->cap_tasks,
+                        host[C_ERROR] & E_OVERFLOW_REC ? std::max<uint64_t>(a->cap_results * 4, host[C_NREC] + 1024)
+                                                       : a->cap_results);
+        return small_result::kRerun;
+    }
+    a->clean = true;
+    a->last_level_stats.clear();
+    a->last_tasks = host[C_WORDS];
+    a->last_visits = host[C_WORDS + 1];
+    a->last_executed = host[C_WORDS + 2];
+    a->res_off = a->h_small.as<uint64_t>() + kSmallOffsets;
+    a->res_ids = a->h_small.as<uint64_t>() + kSmallIds;
+    a->res_cnt = a->h_small.as<uint64_t>() + kSmallCounts;
+    return small_result::kDone;
+}
+
+// The results of a finished batch, whose offsets are in h_roff, into the agent's page-locked buffers.
+void fetch_host_results(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
+{
+    uint64_t const nr = a->h_roff.as<uint64_t>()[nq];
+    a->h_ids.ensure(nr * 8);
+    a->h_cnt.ensure(nr * 8);
+    if (nr)
+    {
+        HG_CUDA(cudaMemcpyAsync(a->h_ids.p, a->out_ids.p, nr * 8, cudaMemcpyDeviceToHost, a->stream));
+        if (mode == HIBF_GPU_QUERY_COUNT)
+            HG_CUDA(cudaMemcpyAsync(a->h_cnt.p, width == 8 ? a->out_cnt.p : a->out_cntw.p, nr * width,
+                                    cudaMemcpyDeviceToHost, a->stream));
+    }
+    HG_CUDA(cudaEventRecord(a->tl_done, a->stream));
+    HG_CUDA(cudaStreamSynchronize(a->stream));
+    a->res_off = a->h_roff.as<uint64_t>();
+    a->res_ids = a->h_ids.as<uint64_t>();
+    a->res_cnt = a->h_cnt.p;
+}
+
 void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t const * qoff, uint64_t nq,
                 uint64_t const * thr, int width, bool plain)
 {
@@ -1049,6 +1309,21 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         cudaGetLastError(); // pageable memory: the queries above fail, and the values are copied
     }
     a->last_in_place = in_place != nullptr;
+    a->last_chunks = 0;
+    small_result const small = small_batch(a, mode, values, qoff, nq, thr, width, plain, in_place);
+    if (small == small_result::kDone)
+        return;
+    if (small == small_result::kCounted)
+    {
+        a->h_roff.ensure((nq + 1) * 8);
+        launch_postprocess(a, nq, mode, width);
+        HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
+        int const st = read_status(a);
+        if (st != HIBF_GPU_OK)
+            fail(st, "device-side failure in the last batch");
+        fetch_host_results(a, nq, mode, width);
+        return;
+    }
     a->in_values.ensure(nv * 8); // the copy's destination, or where an in-place batch's roots stage the values
     if (in_place)
         a->staged.ensure(std::max<uint64_t>(nq, 1) * 4);
@@ -1087,17 +1362,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     ensure_capacity(a, std::max<uint64_t>(nq, 1), tasks, results); // allocations synchronise: before any copy
     a->h_roff.ensure((nq + 1) * 8);
     uint32_t const n_tl = streamed ? static_cast<uint32_t>(qb.size() - 1) : 1u;
-    if (!a->tl_t0)
-    {
-        HG_CUDA(cudaEventCreate(&a->tl_t0));
-        HG_CUDA(cudaEventCreate(&a->tl_done));
-    }
-    while (a->tl_chunk.size() < n_tl)
-    {
-        cudaEvent_t e{};
-        HG_CUDA(cudaEventCreate(&e));
-        a->tl_chunk.push_back(e);
-    }
+    ensure_timeline(a, n_tl);
     a->tl_n = 0;
     HG_CUDA(cudaEventRecord(a->tl_t0, a->stream));
     HG_CUDA(cudaMemcpyAsync(a->in_qoff.p, qoff, (nq + 1) * 8, cudaMemcpyHostToDevice, a->stream));
@@ -1196,18 +1461,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         if (c[C_ERROR] & E_OVERFLOW_REC)
             results = std::max<uint64_t>(results * 4, c[C_NREC] + 1024);
     }
-    uint64_t const nr = a->h_roff.as<uint64_t>()[nq];
-    a->h_ids.ensure(nr * 8);
-    a->h_cnt.ensure(nr * 8);
-    if (nr)
-    {
-        HG_CUDA(cudaMemcpyAsync(a->h_ids.p, a->out_ids.p, nr * 8, cudaMemcpyDeviceToHost, a->stream));
-        if (mode == HIBF_GPU_QUERY_COUNT)
-            HG_CUDA(cudaMemcpyAsync(a->h_cnt.p, width == 8 ? a->out_cnt.p : a->out_cntw.p, nr * width,
-                                    cudaMemcpyDeviceToHost, a->stream));
-    }
-    HG_CUDA(cudaEventRecord(a->tl_done, a->stream));
-    HG_CUDA(cudaStreamSynchronize(a->stream));
+    fetch_host_results(a, nq, mode, width);
 }
 
 // Whether the tuned kernel variants apply: at most 3 hash functions and rows of at most 4 words.
@@ -2302,8 +2556,8 @@ extern "C"
                 uint64_t const qoff[2] = {0, n};
                 uint64_t const thr = threshold;
                 host_batch(a, HIBF_GPU_QUERY_MEMBERSHIP, values, qoff, 1, &thr, 2, true);
-                uint64_t const nr = a->h_roff.as<uint64_t>()[1];
-                a->single_ids.assign(a->h_ids.as<uint64_t>(), a->h_ids.as<uint64_t>() + nr);
+                uint64_t const nr = a->res_off[1];
+                a->single_ids.assign(a->res_ids, a->res_ids + nr);
                 *ids = a->single_ids.data();
                 *n_ids = nr;
             });
@@ -2320,8 +2574,8 @@ extern "C"
                 uint64_t const qoff[2] = {0, n};
                 uint64_t const thr = threshold;
                 host_batch(a, HIBF_GPU_QUERY_MEMBERSHIP, values, qoff, 1, &thr, 2, true);
-                uint64_t const nr = a->h_roff.as<uint64_t>()[1];
-                a->single_ids.assign(a->h_ids.as<uint64_t>(), a->h_ids.as<uint64_t>() + nr);
+                uint64_t const nr = a->res_off[1];
+                a->single_ids.assign(a->res_ids, a->res_ids + nr);
                 std::vector<uint64_t> const & rank = traversal_rank(a->h);
                 std::sort(a->single_ids.begin(), a->single_ids.end(),
                           [&](uint64_t x, uint64_t y) { return rank[x] < rank[y]; });
@@ -2340,10 +2594,10 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
                 uint64_t const qoff[2] = {0, n};
                 host_batch(a, HIBF_GPU_QUERY_COUNT, values, qoff, 1, &threshold, width, true);
-                uint64_t const nr = a->h_roff.as<uint64_t>()[1];
+                uint64_t const nr = a->res_off[1];
                 a->dense.assign(a->h->n_user_bins * static_cast<size_t>(width), 0);
-                uint8_t const * src = a->h_cnt.as<uint8_t>();
-                uint64_t const * ids = a->h_ids.as<uint64_t>();
+                uint8_t const * src = static_cast<uint8_t const *>(a->res_cnt);
+                uint64_t const * ids = a->res_ids;
                 for (uint64_t i = 0; i < nr; ++i)
                     std::memcpy(a->dense.data() + ids[i] * width, src + i * width, width);
                 *counts = a->dense.data();
@@ -2365,10 +2619,10 @@ extern "C"
                 if (n_queries && query_offsets[n_queries] && !values)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null values");
                 host_batch(a, mode, values, query_offsets, n_queries, thresholds, width, false);
-                *result_offsets = a->h_roff.as<uint64_t>();
-                *result_ids = a->h_ids.as<uint64_t>();
+                *result_offsets = a->res_off;
+                *result_ids = a->res_ids;
                 if (result_counts)
-                    *result_counts = mode == HIBF_GPU_QUERY_COUNT ? a->h_cnt.p : nullptr;
+                    *result_counts = mode == HIBF_GPU_QUERY_COUNT ? a->res_cnt : nullptr;
             });
     }
 
@@ -2506,6 +2760,7 @@ extern "C"
             {
                 if (!a || !a->graph)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "no captured batch");
+                a->clean = false;
                 HG_CUDA(cudaGraphLaunch(a->graph, a->stream));
             });
     }

@@ -102,6 +102,9 @@ struct query_params
     unsigned int * qcount;
     unsigned long long * stats;
     uint64_t wait_limit_ns;
+    // the count of unfinished tasks is ctrl[C_PENDING] + pending_bias: the queries, for a launch that finds its control
+    // words at 0
+    uint64_t pending_bias;
     int self_init; // single-block launch that resets its own control words first
     // early exit: after counting first + s * step percent of a task's values (s < stages), stop when no segment can
     // reach the threshold any more; tasks shorter than ee_min values are counted in one stage
@@ -164,7 +167,7 @@ __device__ inline unsigned long long wait_for_task(query_params const & p, unsig
         unsigned long long v = *t;
         if (v != kEmpty)
             return v;
-        if (*pending == 0ull)
+        if (*pending + p.pending_bias == 0ull)
         {
             __threadfence();
             return *t; // still empty: nothing is queued or running, the batch is done

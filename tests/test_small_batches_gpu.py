@@ -1,0 +1,118 @@
+"""Small host batches (one copy in, the query kernel, one finishing block) against the general passes: at the edges of
+the query and result counts where the path changes, and in any order of small, large, device, replayed and failed
+batches on one agent, whose workspace the small ones leave ready for the next."""
+
+import numpy as np
+import pytest
+
+import hibf_gb300 as hg
+from hibf_gb300 import _native as N
+from tests import golden_io as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def case():
+    d = G.hibf_case("synth600")
+    t = G.tables(d)
+    H = hg.hierarchical_interleaved_bloom_filter.from_tables(t["n_user_bins"], t["bins"], t["bin_size"], t["hash_funs"],
+                                                             t["next_ibf"], t["user_bin"], words=t["words"])
+    return d, H
+
+
+def _batch(d, nq, seed, zero=()):
+    """nq queries sampled from the stored ones; queries in `zero` report every user bin (threshold 0)."""
+    rng = np.random.default_rng(seed)
+    qv, qo = d["q_values"], d["q_offsets"].astype(np.int64)
+    pick = rng.integers(0, qo.size - 1, nq)
+    vals = np.concatenate([qv[qo[i]:qo[i + 1]] for i in pick])
+    off = np.concatenate([[0], np.cumsum(qo[pick + 1] - qo[pick])]).astype(np.uint64)
+    thr = np.asarray(d["mem_t"])[pick].astype(np.uint64)
+    thr[list(zero)] = 0
+    return vals, off, thr
+
+
+def _general(H, b, mode=N.QUERY_MEMBERSHIP, width=2):
+    """The same batch through the warp-per-task kernel and the general passes."""
+    a = H.membership_agent()
+    a.tuning = dict(a.tuning, block_queries=0)
+    r = a.query_batch(*b, mode=mode, width=width)
+    return r, a.last_work()
+
+
+def _same(x, y):
+    for i, (p, q) in enumerate(zip(x, y)):
+        assert (p is None) == (q is None)
+        if p is not None:
+            np.testing.assert_array_equal(p, q, err_msg=f"result {i}")
+
+
+@pytest.mark.parametrize("nq,zero", [(1, ()), (1, (0,)), (3, (0, 1, 2)), (4, (0, 1, 2, 3)), (31, ()), (33, (5,)),
+                                     (1023, (7, 900)), (1024, (0, 1023)), (1025, (0,))])
+def test_small_batches_equal_general_ones(gpu_lib, case, nq, zero):
+    """600 user bins: 3 threshold-0 queries give 1,800 results, 4 give 2,400 (more than the finishing block takes)."""
+    d, H = case
+    b = _batch(d, nq, nq, zero)
+    want, work = _general(H, b)
+    a = H.membership_agent()
+    for _ in range(3):
+        _same(a.query_batch(*b), want)
+        assert a.last_work() == work
+        a.status()
+    offs, ids, _ = a.fetch_results(nq)
+    _same((offs, ids), want[:2])
+    for width in (1, 2, 4, 8):
+        c = (b[0], b[1], np.maximum(b[2] // np.uint64(2), 1))
+        want_c, _ = _general(H, c, N.QUERY_COUNT, width)
+        _same(H.counting_agent(width).query_batch(*c), want_c)
+
+
+def test_one_agent_any_order_of_batches(gpu_lib, case):
+    import torch
+
+    d, H = case
+    small, many, large = _batch(d, 50, 1), _batch(d, 40, 2, range(20)), _batch(d, 3000, 3)
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in large]
+    torch.cuda.synchronize()
+    nq = large[1].size - 1
+    want = {k: _general(H, b) for k, b in (("small", small), ("many", many), ("large", large))}
+    a = H.membership_agent()
+    a.reserve(nq, large[0].size, nq * 16, nq * 64)
+    a.capture_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), nq, dev[2].data_ptr())
+
+    def check(k, got):
+        _same(got[:2], want[k][0][:2])
+        assert a.last_work() == want[k][1]
+
+    def device():
+        a.query_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), nq, dev[2].data_ptr())
+        return a.fetch_results(nq)
+
+    def replayed():
+        a.replay()
+        return a.fetch_results(nq)
+
+    steps = {"s": lambda: check("small", a.query_batch(*small)), "m": lambda: check("many", a.query_batch(*many)),
+             "l": lambda: check("large", a.query_batch(*large)), "d": lambda: check("large", device()),
+             "r": lambda: check("large", replayed())}
+    for step in "ssmsslsdsrsmmsrrsdmls":
+        steps[step]()
+    v, o = small[0][:int(small[1][1])], int(small[2][0])
+    single = a.membership_for(v, o)
+    with pytest.raises(hg.InvalidArgument):
+        a.query_batch(small[0], small[1], small[2] + np.uint64(1 << 16))
+    np.testing.assert_array_equal(a.membership_for(v, o), single)
+    steps["s"]()
+
+
+def test_small_batch_outgrows_its_capacity(gpu_lib, case):
+    """A fresh agent holds 4,096 results; 12 threshold-0 queries have 7,200: the batch grows it and starts over."""
+    d, H = case
+    b = _batch(d, 12, 5, range(12))
+    a = H.membership_agent()
+    want, _ = _general(H, b)
+    for _ in range(2):
+        _same(a.query_batch(*b), want)
+    s = _batch(d, 9, 6)
+    _same(a.query_batch(*s), _general(H, s)[0])
