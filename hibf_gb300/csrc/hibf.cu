@@ -465,8 +465,11 @@ __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const 
 constexpr uint64_t kSmallBatch = 1024;      // queries
 constexpr uint32_t kSmallRecords = 2048;    // results; more take the general passes
 constexpr uint64_t kPackValues = 8192;      // values that travel with the offsets and thresholds in one copy
-// words of the host buffer k_finish_small writes: control words and counters, whether it could, offsets, ids, counts
+// words of the host buffer k_finish_small writes: control words and counters, whether it could, when it began and ended
+// (the GPU's clock, ns), offsets, ids, counts
 constexpr uint32_t kSmallOk = C_WORDS + kStats;
+constexpr uint32_t kSmallBegan = kSmallOk + 1;
+constexpr uint32_t kSmallEnded = kSmallOk + 2;
 constexpr uint32_t kSmallOffsets = 16;
 constexpr uint32_t kSmallIds = kSmallOffsets + kSmallBatch + 2;
 constexpr uint32_t kSmallCounts = kSmallIds + kSmallRecords;
@@ -493,6 +496,8 @@ __global__ void __launch_bounds__(1024) k_finish_small(unsigned long long * ctrl
     __shared__ uint16_t s_q[kSmallRecords];
     uint32_t const t = threadIdx.x;
     int const lane = t & 31, w = t >> 5;
+    if (t == 0)
+        host[kSmallBegan] = globaltimer_ns();
     unsigned long long const n_all = ctrl[C_NREC];
     bool const ok = n_all <= kSmallRecords && ctrl[C_ERROR] == 0;
     uint64_t const tail = ctrl[C_TAIL];
@@ -570,7 +575,10 @@ __global__ void __launch_bounds__(1024) k_finish_small(unsigned long long * ctrl
             ctrl[t] = 0; // every thread has read the control words it needs (barriers above)
     }
     if (t == 0)
+    {
         host[kSmallOk] = ok;
+        host[kSmallEnded] = globaltimer_ns();
+    }
 }
 
 // emplace into an IBF (same as the single-level kernel, repeated here to keep the translation units independent).
@@ -663,6 +671,10 @@ struct hibf_gpu_agent
     // small host batches: inputs packed for one copy, results and control words written by k_finish_small
     hbuf h_pack, h_small;
     dbuf d_pack;
+    // the last batch was a small one: its kernel's start and end and its results' time, by the GPU's clock (ns); such
+    // batches record no events (each costs the stream about 1.8 us)
+    bool stamped{};
+    uint64_t stamps[3]{};
     bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: the next one needs no k_begin
     // the last host batch's results: in h_small, or in h_roff / h_ids / h_cnt
     uint64_t const * res_off{};
@@ -825,6 +837,7 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
 void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t marks, uint64_t levels)
 {
     a->clean = false;
+    a->stamped = false;
     uint64_t const n_hist = levels * a->h->n_ibfs;
     uint64_t const most = std::max({static_cast<uint64_t>(ctrl_words(a->h)), nq, marks / 2, n_hist});
     k_begin<<<grid_cap(most, 256, 8), 256, 0, a->stream>>>(a->ctrl.as<unsigned long long>(), ctrl_words(a->h), pending,
@@ -1202,44 +1215,45 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
     if (!in_place && nv * 8 >= kStreamMinBytes)
         return small_result::kRerun; // streamed: the kernel runs beside the copy
     bool const pack = !in_place && nv <= kPackValues;
-    uint64_t const words = 2 * nq + 1 + (pack ? nv : 0);
     ensure_capacity(a, nq, std::max<uint64_t>(a->cap_tasks, nq * 4 + 1024),
                     std::max<uint64_t>(a->cap_results, nq * 4 + 1024));
+    bool const blk = !plain || a->tune.block_queries != 0;
+    // Few values travel in the packed buffer, which the kernel reads in place: its roots leave the values on the device
+    // for the other tasks, as with a caller's page-locked values.  Others are copied first.
     a->h_pack.ensure((2 * kSmallBatch + 1 + kPackValues) * 8);
-    a->d_pack.ensure((2 * kSmallBatch + 1 + kPackValues) * 8);
     a->h_small.ensure(kSmallWords * 8);
-    if (!pack && !in_place)
-        a->in_values.ensure(nv * 8);
-    ensure_timeline(a, 1);
+    a->in_values.ensure(std::max(nv, kPackValues) * 8);
     uint64_t * const hp = a->h_pack.as<uint64_t>();
     std::memcpy(hp, qoff, (nq + 1) * 8);
     std::memcpy(hp + nq + 1, thr, nq * 8);
     if (pack && nv)
         std::memcpy(hp + 2 * nq + 1, values, nv * 8);
-    a->tl_n = 0;
-    HG_CUDA(cudaEventRecord(a->tl_t0, s));
     if (!a->clean)
         launch_begin(a, 0, a->cap_queries, a->cap_tasks, 0);
     a->clean = false; // until k_finish_small has run
-    HG_CUDA(cudaMemcpyAsync(a->d_pack.p, hp, words * 8, cudaMemcpyHostToDevice, s));
-    if (!pack && !in_place)
-        HG_CUDA(cudaMemcpyAsync(a->in_values.p, values, nv * 8, cudaMemcpyHostToDevice, s));
-    HG_CUDA(cudaEventRecord(a->tl_chunk[0], s));
     a->tl_n = 1;
-    uint64_t const * const dp = a->d_pack.as<uint64_t>();
-    uint64_t const * const dv = in_place ? in_place : pack ? dp + 2 * nq + 1 : a->in_values.as<uint64_t>();
-    query_params p = base_params(a, dv, dp, dp + nq + 1, nq, mask_for(mode, width));
+    uint64_t const * inputs = hp;
+    uint64_t const * dv = in_place ? in_place : hp + 2 * nq + 1;
+    if (!pack && !in_place)
+    {
+        a->d_pack.ensure((2 * kSmallBatch + 1) * 8);
+        HG_CUDA(cudaMemcpyAsync(a->d_pack.p, hp, (2 * nq + 1) * 8, cudaMemcpyHostToDevice, s));
+        HG_CUDA(cudaMemcpyAsync(a->in_values.p, values, nv * 8, cudaMemcpyHostToDevice, s));
+        inputs = a->d_pack.as<uint64_t>();
+        dv = a->in_values.as<uint64_t>();
+    }
+    query_params p = base_params(a, dv, inputs, inputs + nq + 1, nq, mask_for(mode, width));
     p.decide = mode == HIBF_GPU_QUERY_MEMBERSHIP;
     p.pending_bias = nq;
-    bool const blk = !plain || a->tune.block_queries != 0;
+    p.stamp = 1;
+    if (blk && (pack || in_place))
+        p.stage = a->in_values.as<uint64_t>();
     int const fit = blk ? a->max_blocks_blk : a->max_blocks[a->variant];
     int const per_sm = a->tune.blocks_per_sm ? std::min<int>(fit, static_cast<int>(a->tune.blocks_per_sm)) : fit;
     unsigned const grid =
         static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(sm_count()) * per_sm, blk ? nq : 1));
-    HG_CUDA(cudaEventRecord(a->ev_k0, s));
     (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256, query_smem(h), s>>>(p);
     HG_CUDA(cudaGetLastError());
-    HG_CUDA(cudaEventRecord(a->ev_k1, s));
     bool const counts = mode == HIBF_GPU_QUERY_COUNT;
     unsigned long long * const host = a->h_small.as<unsigned long long>();
     k_finish_small<<<1, 1024, 0, s>>>(
@@ -1248,9 +1262,12 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
         a->rec_cnt.as<unsigned long long>(), a->roff.as<unsigned long long>(), a->out_ids.as<uint64_t>(),
         a->out_cnt.as<uint64_t>(), width, counts && width != 8 ? a->out_cntw.p : nullptr, counts, host);
     HG_CUDA(cudaGetLastError());
-    HG_CUDA(cudaEventRecord(a->tl_done, s));
     HG_CUDA(cudaStreamSynchronize(s));
     a->last_levels = 0;
+    a->stamped = true;
+    a->stamps[0] = host[C_STAMP];
+    a->stamps[1] = host[kSmallBegan];
+    a->stamps[2] = host[kSmallEnded];
     if (!host[kSmallOk])
     {
         if (host[C_ERROR] == 0)
@@ -1316,6 +1333,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     if (small == small_result::kCounted)
     {
         a->h_roff.ensure((nq + 1) * 8);
+        ensure_timeline(a, 1);
         launch_postprocess(a, nq, mode, width);
         HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
         int const st = read_status(a);
@@ -2761,6 +2779,7 @@ extern "C"
                 if (!a || !a->graph)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "no captured batch");
                 a->clean = false;
+                a->stamped = false;
                 HG_CUDA(cudaGraphLaunch(a->graph, a->stream));
             });
     }
@@ -2772,6 +2791,11 @@ extern "C"
             {
                 if (!a || !ms)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
+                if (a->stamped)
+                {
+                    *ms = static_cast<float>(static_cast<double>(a->stamps[1] - a->stamps[0]) * 1e-6);
+                    return;
+                }
                 HG_CUDA(cudaEventSynchronize(a->ev_k1));
                 HG_CUDA(cudaEventElapsedTime(ms, a->ev_k0, a->ev_k1));
             });
@@ -2862,9 +2886,16 @@ extern "C"
             {
                 if (!a || !n || (cap && !out_ms))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
-                if (!a->tl_t0 || a->tl_n == 0)
+                if (a->tl_n == 0 || (!a->stamped && !a->tl_t0))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "the agent has not answered a host batch");
                 *n = a->tl_n + 3;
+                if (a->stamped) // a small batch: from its kernel's start, before which its inputs were in place
+                {
+                    double const t[4] = {0.0, 0.0, static_cast<double>(a->stamps[1] - a->stamps[0]) * 1e-6,
+                                         static_cast<double>(a->stamps[2] - a->stamps[0]) * 1e-6};
+                    std::copy_n(t, std::min<uint32_t>(cap, 4), out_ms);
+                    return;
+                }
                 auto since = [&](cudaEvent_t e)
                 {
                     float ms = 0;

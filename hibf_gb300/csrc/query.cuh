@@ -51,6 +51,7 @@ enum : int
     C_PENDING = 2,
     C_NREC = 3,
     C_ERROR = 4,
+    C_STAMP = 5, // when the query kernel began (query_params::stamp), on the GPU's clock
     C_CHILD = 6, // streamed inputs: claims of child slots (roots and children are then claimed separately)
     C_WORDS = 8
 };
@@ -105,6 +106,7 @@ struct query_params
     // the count of unfinished tasks is ctrl[C_PENDING] + pending_bias: the queries, for a launch that finds its control
     // words at 0
     uint64_t pending_bias;
+    int stamp;     // the kernel notes its start in ctrl[C_STAMP]
     int self_init; // single-block launch that resets its own control words first
     // early exit: after counting first + s * step percent of a task's values (s < stages), stop when no segment can
     // reach the threshold any more; tasks shorter than ee_min values are counted in one stage
@@ -134,7 +136,8 @@ struct query_params
     unsigned long long const * in_count;
     // in-place host batches under the level schedule: `values` is the host's memory; root tasks store every value
     // they read at stage[same position] and how many they read (from the query's first value) at staged[query], and
-    // the lower levels read that prefix from stage and only the rest from the host.  Null otherwise.
+    // the lower levels read that prefix from stage and only the rest from the host.  k_query_blk's roots read all their
+    // values, so it needs no counts.  Null otherwise.
     uint64_t * stage;
     uint32_t * staged;
 };
@@ -528,11 +531,7 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
             if (lane == 0)
             {
                 if (!p.level)
-                {
-                    // counted before any of them can be seen, run and retired
                     atomicAdd(p.ctrl + C_PENDING, static_cast<unsigned long long>(nc));
-                    __threadfence();
-                }
                 base = atomicAdd(p.ctrl + C_TAIL, static_cast<unsigned long long>(nc));
             }
             base = __shfl_sync(kFullMask, base, 0);
@@ -543,9 +542,16 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
                 if (s < p.task_cap)
                 {
                     if (p.level)
+                    {
                         p.tasks[s] = make_task(q, depth + 1u, ds.x);
+                    }
                     else
+                    {
+                        // the children are counted, and the values a root staged for them written, before any of them
+                        // can be seen, run and retired
+                        __threadfence();
                         atomicExch(p.tasks + s, make_task(q, depth + 1u, ds.x));
+                    }
                 }
                 else
                 {
@@ -559,8 +565,8 @@ __device__ __forceinline__ void emit_bins(query_params const & p, uint2 ds, unsi
 }
 
 // A finished task leaves the count of unfinished ones (the level schedule keeps none: its launches end by themselves)
-// and enters the work counters.  No fence: a waiting worker learns of a child from its slot alone (one atomic word),
-// the task's children were counted by this same thread, and records are read by later launches only.  (A fence per
+// and enters the work counters.  No fence: a waiting worker learns of a child from its slot (emit_bins), the task's
+// children were counted by this same thread, and records are read by later launches only.  (A fence per
 // task was the second largest stall of a batch of 10,000 short queries.)
 __device__ __forceinline__ void retire_task(query_params const & p, uint64_t q, uint64_t n, uint64_t done, int lane,
                                             unsigned long long & n_tasks, unsigned long long & n_visits,
@@ -691,8 +697,8 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
     uint64_t done = 0;
     // in-place host batch under the level schedule: a root stages what it reads; a lower level reads the staged prefix
     // [0, staged) from device memory and the rest from the host
-    bool const stage_root = p.stage && depth == 0;
-    uint64_t const staged = p.stage && depth > 0 ? p.staged[q] : 0u;
+    bool const stage_root = p.staged && depth == 0;
+    uint64_t const staged = p.staged && depth > 0 ? p.staged[q] : 0u;
     bool const adaptive = p.ee_stages == kEarlyExitAdaptive && n >= p.ee_min;
     uint64_t const most = n * nd.max_seg; // no segment's sum passes this
     bool const narrow = most < kNarrowSums;
@@ -774,6 +780,8 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
     extern __shared__ uint32_t s_counts[];
     int const lane = threadIdx.x & 31;
     uint32_t * counts = s_counts + (threadIdx.x >> 5) * p.counters_per_warp;
+    if (p.stamp && blockIdx.x == 0 && threadIdx.x == 0)
+        p.ctrl[C_STAMP] = globaltimer_ns();
     if (p.self_init)
     {
         if (threadIdx.x == 0)
@@ -999,54 +1007,77 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
 // its own shared counters, the block adds the eight count arrays, warp 0 scans and emits.  A task then takes about an
 // eighth of the time, which shortens a batch whose tasks are fewer than the GPU's warps (the chain root -> child ->
 // grandchild of its slowest query bounds it).  No early exit: a slice's counts do not bound the task's.
+//
+// A task is a chain of dependent accesses (claim, task, IBF, values, rows, bin tables, results), about 10 us of which
+// little is work, so the chain is kept short: the block goes on with its task's first child (no queue, no claim, the
+// query's bounds at hand), the bin tables are on their way while the values are counted, and a block on its own looks at
+// the count of unfinished tasks before it claims a slot nobody will fill.  p.stage (optional): the values are the
+// host's memory; roots store what they read there, at the same positions, and the other tasks read it.
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
 template <int H, typename R>
 __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
-    __shared__ unsigned long long s_task;
+    __shared__ unsigned long long s_task, s_keep;
     int const lane = threadIdx.x & 31;
     int const warp = threadIdx.x >> 5;
     int const nwarps = blockDim.x >> 5;
     uint32_t * counts = s_counts + warp * p.counters_per_warp;
-    if (p.self_init)
+    if (threadIdx.x == 0)
     {
-        if (threadIdx.x == 0)
+        s_keep = kEmpty;
+        if (p.stamp && blockIdx.x == 0)
+            p.ctrl[C_STAMP] = globaltimer_ns();
+        if (p.self_init)
         {
             p.ctrl[C_HEAD] = 0;
             p.ctrl[C_TAIL] = 0;
             p.ctrl[C_PENDING] = p.n_queries;
             __threadfence();
         }
-        __syncthreads();
     }
+    __syncthreads();
     unsigned long long n_tasks = 0, n_visits = 0, n_executed = 0;
+    uint64_t q = ~0ull, b0 = 0, n = 0, thr = 0; // the query at hand
+    uint64_t claims = 0;                        // thread 0 of a block on its own
     for (;;)
     {
         if (threadIdx.x == 0)
         {
-            unsigned long long const idx = atomicAdd(p.ctrl + C_HEAD, 1ull);
-            unsigned long long task;
-            if (idx < p.n_queries)
+            unsigned long long task = s_keep;
+            s_keep = kEmpty;
+            if (task == kEmpty && gridDim.x == 1 && claims >= p.n_queries &&
+                *static_cast<volatile unsigned long long *>(p.ctrl + C_PENDING) + p.pending_bias == 0ull)
             {
-                uint64_t const q = p.order ? p.order[idx] : idx;
-                if (q >= p.n_queries)
+                // this block's own count: nothing is queued (it would be counted) and nobody else runs
+            }
+            else if (task == kEmpty)
+            {
+                unsigned long long const idx = atomicAdd(p.ctrl + C_HEAD, 1ull);
+                ++claims;
+                if (idx < p.n_queries)
                 {
-                    atomicOr(p.ctrl + C_ERROR, E_ORDER);
-                    __threadfence();
-                    atomicAdd(p.ctrl + C_PENDING, ~0ull);
-                    task = kSkipTask;
+                    uint64_t const root = p.order ? p.order[idx] : idx;
+                    if (root >= p.n_queries)
+                    {
+                        atomicOr(p.ctrl + C_ERROR, E_ORDER);
+                        __threadfence();
+                        atomicAdd(p.ctrl + C_PENDING, ~0ull);
+                        task = kSkipTask;
+                    }
+                    else
+                    {
+                        task = !p.arrived || wait_arrival(p, root) ? make_task(root, 0u, 0u) : kEmpty;
+                    }
                 }
                 else
                 {
-                    task = !p.arrived || wait_arrival(p, q) ? make_task(q, 0u, 0u) : kEmpty;
+                    unsigned long long const slot = idx - p.n_queries;
+                    task = slot >= p.task_cap ? kEmpty : wait_for_task(p, slot);
+                    if (p.stage)
+                        __threadfence(); // another block's root staged the values this task reads
                 }
-            }
-            else
-            {
-                unsigned long long const slot = idx - p.n_queries;
-                task = slot >= p.task_cap ? kEmpty : wait_for_task(p, slot);
             }
             s_task = task;
         }
@@ -1059,9 +1090,8 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
             __syncthreads();
             continue;
         }
-        uint64_t const q = task >> 32;
         uint32_t const depth = static_cast<uint32_t>(task >> kNodeBits) & 63u;
-        if (q >= p.n_queries || (static_cast<uint32_t>(task) & kNodeMask) >= p.n_nodes)
+        if ((task >> 32) >= p.n_queries || (static_cast<uint32_t>(task) & kNodeMask) >= p.n_nodes)
         {
             if (threadIdx.x == 0)
             {
@@ -1073,18 +1103,27 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
             continue;
         }
         dev_node const nd = p.nodes[static_cast<uint32_t>(task) & kNodeMask];
-        uint64_t const b0 = p.qoff[q];
-        uint64_t const n = p.qoff[q + 1] - b0;
+        if ((task >> 32) != q)
+        {
+            q = task >> 32;
+            b0 = p.qoff[q];
+            n = p.qoff[q + 1] - b0;
+            thr = p.thr[q];
+        }
         uint32_t const ncount = row_counters(nd.bin_words);
         for (uint32_t i = lane; i < ncount; i += 32)
             counts[i] = 0;
+        if (warp == nwarps - 1) // one 128-byte line of the bin table per lane and turn
+            for (uint32_t i = 16u * lane; i < nd.bins; i += 512u)
+                asm volatile("prefetch.global.L1 [%0];" ::"l"(p.descs + nd.desc_offset + i));
         __syncwarp();
         row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift, nd.hash_funs};
         uint64_t const per = (n + nwarps - 1) / nwarps;
         uint64_t const lo = min(n, static_cast<uint64_t>(warp) * per);
         uint64_t const hi = min(n, lo + per);
         if (hi > lo)
-            count_variant<H, 0, R>(rp, nd.lpv_log2, p.values + b0 + lo, hi - lo, counts, lane, nullptr);
+            count_variant<H, 0, R>(rp, nd.lpv_log2, (depth && p.stage ? p.stage : p.values) + b0 + lo, hi - lo, counts,
+                                   lane, !depth && p.stage ? p.stage + b0 + lo : nullptr);
         __syncthreads();
         for (uint32_t i = threadIdx.x; i < ncount; i += blockDim.x)
         {
@@ -1095,8 +1134,8 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid
         }
         __syncthreads();
         if (warp == 0)
-            emit_task(p, nd, s_counts, q, depth, n, n, p.thr[q], lane, n_tasks, n_visits, n_executed);
-        __syncthreads(); // the counters and s_task are reused by the next task
+            emit_task(p, nd, s_counts, q, depth, n, n, thr, lane, n_tasks, n_visits, n_executed, &s_keep);
+        __syncthreads(); // the counters, s_task and s_keep are used by the next task
     }
     if (threadIdx.x == 0 && n_tasks)
     {
