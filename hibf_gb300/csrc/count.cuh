@@ -241,38 +241,13 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
     }
 }
 
-template <typename R, int H, bool EF = false>
-__device__ __forceinline__ void warp_count_lpv(row_params const & rp, uint32_t lpv_log2, uint64_t const * vals,
-                                               uint64_t n, uint32_t * counts, int lane, uint64_t * stage = nullptr)
-{
-    switch (lpv_log2)
-    {
-    case 0:
-        warp_count<R, 1, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-        break;
-    case 1:
-        warp_count<R, 2, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-        break;
-    case 2:
-        warp_count<R, 4, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-        break;
-    case 3:
-        warp_count<R, 8, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-        break;
-    case 4:
-        warp_count<R, 16, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-        break;
-    default:
-        warp_count<R, 32, H, 7, 1, 1, EF>(rp, vals, n, counts, lane, stage);
-    }
-}
-
-// Rows wider than a warp (more than kSlabWords words) are counted in slabs of kSlabWords words, one word per lane.
-__device__ __forceinline__ row_params row_slab(row_params const & rp, uint32_t first_word)
+// Rows wider than a warp (more than kSlabWords words) are counted in slabs of as many words as lanes read them; the last
+// slab may have fewer.
+__device__ __forceinline__ row_params row_slab(row_params const & rp, uint32_t first_word, uint32_t slab_words)
 {
     row_params sp = rp;
     sp.words += first_word;
-    sp.bin_words = min(kSlabWords, rp.bin_words - first_word);
+    sp.bin_words = min(slab_words, rp.bin_words - first_word);
     return sp;
 }
 

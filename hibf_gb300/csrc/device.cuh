@@ -89,6 +89,25 @@ __device__ __forceinline__ uint64_t globaltimer_ns()
     return t;
 }
 
+// Counter i of an array of `width`-byte counters: v modulo the width (the reference's counting_vector wraps).
+__device__ __forceinline__ void store_count(void * out, int width, uint64_t i, uint64_t v)
+{
+    switch (width)
+    {
+    case 1:
+        static_cast<uint8_t *>(out)[i] = static_cast<uint8_t>(v);
+        break;
+    case 2:
+        static_cast<uint16_t *>(out)[i] = static_cast<uint16_t>(v);
+        break;
+    case 4:
+        static_cast<uint32_t *>(out)[i] = static_cast<uint32_t>(v);
+        break;
+    default:
+        static_cast<uint64_t *>(out)[i] = v;
+    }
+}
+
 // ---------------------------------------------------------------------------------------------------------------
 // Bit-sliced ("vertical") counters.  P[k] holds bit k of 64 independent counters, one per bin of a 64-bit row word.
 // Adding four 0/1 masks costs a carry-save tree (full adder + three half adders) plus a ripple through the planes:

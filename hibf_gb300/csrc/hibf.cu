@@ -316,24 +316,6 @@ __global__ void k_scatter(unsigned long long const * __restrict__ ctrl, uint32_t
 // ---- sort every query's segment by user bin id, and its counts to the counter width ----
 constexpr uint32_t kSmemSegment = 2048;
 
-__device__ __forceinline__ void store_count(void * out, int width, uint64_t i, uint64_t v)
-{
-    switch (width)
-    {
-    case 1:
-        static_cast<uint8_t *>(out)[i] = static_cast<uint8_t>(v);
-        break;
-    case 2:
-        static_cast<uint16_t *>(out)[i] = static_cast<uint16_t>(v);
-        break;
-    case 4:
-        static_cast<uint32_t *>(out)[i] = static_cast<uint32_t>(v);
-        break;
-    default:
-        static_cast<uint64_t *>(out)[i] = v;
-    }
-}
-
 // Bitonic sort of one segment with only ascending comparators (the "flip" form: the first exchange of every merge
 // pairs i with its mirror in the block, the rest are half-cleaners).  Positions >= len are virtual +infinity and,
 // being the larger element of every comparator they take part in, never move, so any length works.  The segment is

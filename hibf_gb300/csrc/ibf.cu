@@ -199,15 +199,14 @@ __global__ void k_widen(uint64_t * __restrict__ dst, uint32_t dst_row_words, uin
 // bulk_contains (src/interleaved_bloom_filter.cpp:204-291) for many values with H hash functions: out[v * bin_words + j]
 // = AND of word j of the h rows.  The same work mapping as the counting loop (count.cuh) -- LPV lanes per row, lanes
 // hash U values each, the H row words of four sub-steps are loaded together (4 * H loads per lane in flight) -- and
-// each lane stores its word of the AND.  The grid's second dimension is the slab of a row wider than a warp, from
-// word `first_slab` on.
+// each lane stores its word of the AND.  The grid's first dimension is the slab (LPV words) of a row wider than a warp, so
+// that blocks which start together read the pieces of the same rows.
 template <int LPV, int H, typename R>
-__global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_t first_slab,
-                                                         uint64_t const * __restrict__ values, uint64_t n,
-                                                         uint64_t * __restrict__ out)
+__global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint64_t const * __restrict__ values,
+                                                         uint64_t n, uint64_t * __restrict__ out)
 {
-    uint32_t const w0 = (first_slab + blockIdx.y) * kSlabWords;
-    row_params const rp = row_slab(row, w0);
+    uint32_t const w0 = blockIdx.x * LPV;
+    row_params const rp = row_slab(row, w0, LPV);
     constexpr int G = 32 / LPV;
     constexpr int U = LPV >= 4 ? 1 : 4 / LPV;
     constexpr int STEPS = U * LPV;
@@ -219,8 +218,8 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
     uint64_t const bw = row.bin_words;
     uint64_t const * __restrict__ words = rp.words + j;
     out += w0;
-    uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
-    uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+    uint64_t const warp = (blockIdx.y * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
+    uint64_t const nwarps = (static_cast<uint64_t>(gridDim.y) * blockDim.x) >> 5;
     for (uint64_t base = warp * BLOCK; base < n; base += nwarps * BLOCK)
     {
         R row_of[U][H];
@@ -270,115 +269,172 @@ __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint32_
     }
 }
 
+using contains_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t *);
+
 template <int H, typename R>
-void launch_contains_h(row_params const & rp, uint32_t lpv_log2, uint32_t first_slab, uint32_t slabs,
-                       uint64_t const * d_values, uint64_t n, uint64_t * d_out, unsigned grid_x, cudaStream_t s)
+contains_kernel_t contains_kernel_h(uint32_t lpv_log2)
 {
-    dim3 const grid(grid_x, slabs);
     switch (lpv_log2)
     {
     case 0:
-        k_bulk_contains_h<1, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
-        break;
+        return k_bulk_contains_h<1, H, R>;
     case 1:
-        k_bulk_contains_h<2, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
-        break;
+        return k_bulk_contains_h<2, H, R>;
     case 2:
-        k_bulk_contains_h<4, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
-        break;
+        return k_bulk_contains_h<4, H, R>;
     case 3:
-        k_bulk_contains_h<8, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
-        break;
+        return k_bulk_contains_h<8, H, R>;
     case 4:
-        k_bulk_contains_h<16, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
-        break;
+        return k_bulk_contains_h<16, H, R>;
     default:
-        k_bulk_contains_h<32, H, R><<<grid, 256, 0, s>>>(rp, first_slab, d_values, n, d_out);
+        return k_bulk_contains_h<32, H, R>;
     }
+}
+
+template <typename R>
+contains_kernel_t contains_kernel(uint64_t h, uint32_t lpv_log2)
+{
+    switch (h)
+    {
+    case 1:
+        return contains_kernel_h<1, R>(lpv_log2);
+    case 2:
+        return contains_kernel_h<2, R>(lpv_log2);
+    case 3:
+        return contains_kernel_h<3, R>(lpv_log2);
+    case 4:
+        return contains_kernel_h<4, R>(lpv_log2);
+    default:
+        return contains_kernel_h<5, R>(lpv_log2);
+    }
+}
+
+// The end of a counting block: the sum of its warps' counters, in the caller's width.  A block on its own in its slab
+// writes its sums, else the slab's last block (by ticket) writes the totals, and with `reset` leaves totals and ticket at
+// 0 for the next call.  (Clearing before and a storing kernel after cost a read of 250 values on 64 bins 5 of its 36
+// us.)
+__device__ __forceinline__ void finish_counts(uint32_t const * s_counts, uint32_t n_counters, uint32_t w0,
+                                              uint32_t slab_words, unsigned long long * totals, unsigned int * ticket,
+                                              bool reset, uint64_t bins, int width, void * out)
+{
+    int const nwarps_block = blockDim.x >> 5;
+    uint64_t const bin0 = 64ull * w0;
+    for (uint32_t i = threadIdx.x; i < n_counters; i += blockDim.x)
+    {
+        uint64_t sum = 0;
+        for (int w = 0; w < nwarps_block; ++w)
+            sum += s_counts[w * n_counters + i];
+        if (gridDim.y == 1)
+        {
+            if (bin0 + i < bins)
+                store_count(out, width, bin0 + i, sum);
+        }
+        else if (sum)
+        {
+            atomicAdd(totals + bin0 + i, static_cast<unsigned long long>(sum));
+        }
+    }
+    if (gridDim.y == 1)
+        return;
+    __shared__ bool s_last;
+    __threadfence(); // this thread's additions before the block's ticket
+    __syncthreads();
+    if (threadIdx.x == 0)
+        s_last = atomicAdd(ticket, 1u) == gridDim.y - 1u;
+    __syncthreads();
+    if (!s_last)
+        return;
+    __threadfence();
+    for (uint32_t i = threadIdx.x; i < n_counters; i += blockDim.x)
+    {
+        if (bin0 + i < bins)
+            store_count(out, width, bin0 + i, __ldcg(totals + bin0 + i));
+        if (reset && i < 64u * slab_words)
+            totals[bin0 + i] = 0;
+    }
+    if (reset && threadIdx.x == 0)
+        *ticket = 0;
 }
 
 // bulk_count over n values into one counting vector: every warp counts a contiguous chunk into shared counters of its
 // own (planes_flush_to, no shared-memory atomics), the block adds them up and to the 64-bit global totals.
-// Four blocks per SM (64 registers, some spilled for h >= 3) measured faster than two blocks without spills (1.53 vs
-// 2.16 ms for 2^24 values on 1,024 bins, h = 3): more warps keep more row loads in flight.
-// The grid's second dimension is the slab of a row wider than a warp: a block counts 32 words of every row, a warp one
-// whole 256-byte piece per value and hash function.  (Rows wider than a warp were counted one value at a time, every
-// set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms, now 0.219.)
-template <int H, typename R>
-__global__ void __launch_bounds__(256, 4)
+// Four blocks per SM (64 registers) measured faster than two (1.53 vs 2.16 ms for 2^24 values on 1,024 bins, h = 3): more
+// warps keep more row loads in flight.  For h of 4 and 5, whose rows fill more registers, three blocks: a million values
+// on 64 bins, h = 5, took 70 us with four, which spill.
+// The grid's first dimension is the slab of a row wider than a warp: a block counts LPV words of every row, a warp one
+// piece of 128 or 256 bytes per value and hash function.  (Rows wider than a warp were counted one value
+// at a time, every set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms, now
+// 0.21.)  One kernel per row width: with all six in one the loop spilled 156 bytes per thread at h = 3.
+constexpr unsigned count_blocks_per_sm(int h)
+{
+    return h <= 3 ? 4 : 3;
+}
+
+template <int LPV, int H, typename R>
+__global__ void __launch_bounds__(256, count_blocks_per_sm(H))
     k_bulk_count(row_params row, uint64_t const * __restrict__ values, uint64_t n, uint64_t chunk,
-                 unsigned long long * __restrict__ totals)
+                 unsigned long long * totals, unsigned int * tickets, bool reset, uint64_t bins, int width,
+                 void * __restrict__ out)
 {
     extern __shared__ uint32_t s_counts[];
-    uint32_t const w0 = blockIdx.y * kSlabWords;
-    row_params const rp = row_slab(row, w0);
-    uint32_t const lpv_log2 = lanes_log2(rp.bin_words);
-    uint32_t const n_counters = 64u << lpv_log2;
+    uint32_t const w0 = blockIdx.x * LPV;
+    row_params const rp = row_slab(row, w0, LPV);
+    constexpr uint32_t n_counters = 64u * LPV;
     int const nwarps_block = blockDim.x >> 5;
     for (uint32_t i = threadIdx.x; i < n_counters * nwarps_block; i += blockDim.x)
         s_counts[i] = 0;
     __syncthreads();
     int const lane = threadIdx.x & 31;
     uint32_t * counts = s_counts + (threadIdx.x >> 5) * n_counters;
-    uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
-    uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
+    uint64_t const warp = (blockIdx.y * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
+    uint64_t const nwarps = (static_cast<uint64_t>(gridDim.y) * blockDim.x) >> 5;
     for (uint64_t start = warp * chunk; start < n; start += nwarps * chunk)
     {
         uint64_t const len = (n - start) < chunk ? (n - start) : chunk;
-        warp_count_lpv<R, H, true>(rp, lpv_log2, values + start, len, counts, lane);
+        warp_count<R, LPV, H, 7, 1, 1, true>(rp, values + start, len, counts, lane);
     }
     __syncthreads();
-    for (uint32_t i = threadIdx.x; i < n_counters; i += blockDim.x)
-    {
-        uint64_t sum = 0;
-        for (int w = 0; w < nwarps_block; ++w)
-            sum += s_counts[w * n_counters + i];
-        if (sum)
-            atomicAdd(totals + 64u * w0 + i, static_cast<unsigned long long>(sum));
-    }
+    finish_counts(s_counts, n_counters, w0, rp.bin_words, totals, tickets + blockIdx.x, reset, bins, width, out);
 }
 
-// Reduce exact totals modulo the counter width (the reference's counting_vector wraps).
-__global__ void k_store_counts(unsigned long long const * __restrict__ totals, uint64_t bins, int width, void * out)
+using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *, unsigned int *,
+                                     bool, uint64_t, int, void *);
+
+template <int H, typename R>
+bulk_count_kernel_t bulk_count_kernel_h(uint32_t lpv_log2)
 {
-    for (uint64_t b = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; b < bins;
-         b += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+    switch (lpv_log2)
     {
-        uint64_t const t = totals[b];
-        switch (width)
-        {
-        case 1:
-            static_cast<uint8_t *>(out)[b] = static_cast<uint8_t>(t);
-            break;
-        case 2:
-            static_cast<uint16_t *>(out)[b] = static_cast<uint16_t>(t);
-            break;
-        case 4:
-            static_cast<uint32_t *>(out)[b] = static_cast<uint32_t>(t);
-            break;
-        default:
-            static_cast<uint64_t *>(out)[b] = t;
-        }
+    case 0:
+        return k_bulk_count<1, H, R>;
+    case 1:
+        return k_bulk_count<2, H, R>;
+    case 2:
+        return k_bulk_count<4, H, R>;
+    case 3:
+        return k_bulk_count<8, H, R>;
+    case 4:
+        return k_bulk_count<16, H, R>;
+    default:
+        return k_bulk_count<32, H, R>;
     }
 }
-
-using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *);
 
 template <typename R>
-bulk_count_kernel_t bulk_count_kernel(uint64_t h)
+bulk_count_kernel_t bulk_count_kernel(uint64_t h, uint32_t lpv_log2)
 {
     switch (h)
     {
     case 1:
-        return k_bulk_count<1, R>;
+        return bulk_count_kernel_h<1, R>(lpv_log2);
     case 2:
-        return k_bulk_count<2, R>;
+        return bulk_count_kernel_h<2, R>(lpv_log2);
     case 3:
-        return k_bulk_count<3, R>;
+        return bulk_count_kernel_h<3, R>(lpv_log2);
     case 4:
-        return k_bulk_count<4, R>;
+        return bulk_count_kernel_h<4, R>(lpv_log2);
     default:
-        return k_bulk_count<5, R>;
+        return bulk_count_kernel_h<5, R>(lpv_log2);
     }
 }
 
@@ -420,7 +476,9 @@ struct hibf_gpu_ibf
     bool track_occupancy{};
     dbuf store;     // bin_size * row_words words
     dbuf occupancy; // technical_bins counters
-    dbuf totals;    // technical_bins 64-bit totals (bulk_count scratch)
+    dbuf totals;    // technical_bins 64-bit totals and a ticket per slab (bulk_count scratch, cleared by each call)
+    dbuf host_totals; // the same for host-pointer calls, one at a time: left at 0 by each call
+    hbuf h_in, h_out; // small host-pointer calls: values the kernels read in place, results they write
     dbuf io;        // staging for host-pointer calls
     dbuf io2;
     dbuf flag; // device int: an emplace saw a bin index out of range
@@ -437,10 +495,29 @@ struct hibf_gpu_ibf
     {
         return bin_size > UINT32_MAX;
     }
-    // slabs of a row: kSlabWords words each, the last one what is left
-    uint32_t slabs() const
+    // Lanes (log2) that read a row, or a slab of a row, for n values.  Rows of up to 16 words are read whole.  Wider ones
+    // are counted in slabs of 16 words: with 32, whose counters leave room for three blocks per SM, 8,192 bins (h = 1, a
+    // million values) took 421 us against 336, 3,000 values 24 against 18.  Only long calls on rows of 17 to 31 words
+    // take one slab of 32 (1,500 bins, h = 4, 300,000 values: 64 us against 71).
+    uint32_t count_lanes_log2(uint64_t n) const
     {
-        return static_cast<uint32_t>((bin_words + kSlabWords - 1) / kSlabWords);
+        if (bin_words <= 16)
+            return lanes_log2(static_cast<uint32_t>(bin_words));
+        return bin_words < kSlabWords && n > (1u << 17) ? 5 : 4;
+    }
+    // bulk_contains keeps no counters, so long calls read slabs of 32 words where those leave at most half a slab idle at
+    // the row's end (2,048 bins, h = 2, a million values: 119 us against 123 with slabs of 16; 3,000 values 10.3 against
+    // 8.4; 2,500 bins, 40 words, 238 us with slabs of 16 and 251 with 32).
+    uint32_t contains_lanes_log2(uint64_t n) const
+    {
+        if (bin_words <= 16)
+            return lanes_log2(static_cast<uint32_t>(bin_words));
+        uint64_t const rest = bin_words % kSlabWords;
+        return n > (1u << 16) && (rest == 0 || rest > kSlabWords / 2) ? 5 : 4;
+    }
+    uint32_t slabs(uint32_t lanes_log2) const
+    {
+        return static_cast<uint32_t>((bin_words + (1u << lanes_log2) - 1) >> lanes_log2);
     }
     uint64_t technical_bins() const
     {
@@ -535,44 +612,55 @@ uint64_t count_counters(hibf_gpu_ibf const * f)
     return row_counters(static_cast<uint32_t>(f->bin_words));
 }
 
-// bulk_count of n device values into d_out.  `totals` is device scratch for count_counters(f) 64-bit totals; null
-// means the filter's own buffer (grown on demand, the only allocation here).
-void launch_count(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, int width, void * d_out, cudaStream_t s,
-                  unsigned long long * totals = nullptr)
+// Bytes of bulk_count's scratch for filter f: its totals and a ticket per slab (of 16 words, the narrowest).
+uint64_t count_scratch_bytes(hibf_gpu_ibf const * f)
 {
-    uint64_t const nc = count_counters(f);
+    return count_counters(f) * sizeof(unsigned long long) + f->slabs(4) * sizeof(unsigned int);
+}
+
+// bulk_count of n values into `out` (device memory, or mapped host memory).  `totals` is device scratch of
+// count_scratch_bytes(f); null means the filter's own buffer (grown on demand, the only allocation here).  `reset`: it
+// is at 0 and is left at 0.
+void launch_count(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int width, void * out, cudaStream_t s,
+                  unsigned long long * totals = nullptr, bool reset = false)
+{
+    if (!n)
+    {
+        HG_CUDA(cudaMemsetAsync(out, 0, f->bins * static_cast<uint64_t>(width), s));
+        return;
+    }
+    unsigned const block = 256;
+    // One contiguous chunk per warp of a full wave, over all slabs: as many blocks of 8 warps per SM as the kernel is
+    // built for, or the 3 whose 64 KiB of counters fit where a slab is 32 words.  A chunk is at least 32 values, one per
+    // lane: a call of 250 values then runs on eight warps of one block instead of one warp, one of 10,000 on 40 SMs
+    // (with chunks of 512: 1,000 bins, h = 3, 10,000 values 92 us, now 18).  From 128 values on, narrow rows round it to
+    // whole passes of four values per lane.
+    uint32_t const lanes = f->count_lanes_log2(n);
+    uint32_t const slabs = f->slabs(lanes);
+    bool const full_slabs = lanes == 5;
+    uint64_t const per_sm = full_slabs ? 3u : count_blocks_per_sm(static_cast<int>(f->hash_funs));
+    uint64_t const blocks = std::max<uint64_t>(1, static_cast<uint64_t>(sm_count()) * per_sm / slabs);
+    uint64_t const wave = blocks * 8u;
+    uint64_t const even = (n + wave - 1) / wave;
+    uint64_t const round = full_slabs || even <= 96 ? 32 : 128;
+    uint64_t const chunk = (even + round - 1) / round * round;
+    uint64_t const warps = (n + chunk - 1) / chunk;
+    unsigned const grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, blocks)));
     if (!totals)
     {
-        f->totals.ensure(nc * sizeof(unsigned long long));
+        f->totals.ensure(count_scratch_bytes(f));
         totals = f->totals.as<unsigned long long>();
     }
-    HG_CUDA(cudaMemsetAsync(totals, 0, nc * sizeof(unsigned long long), s));
-    if (n)
-    {
-        unsigned const block = 256;
-        // One contiguous chunk per warp of a full wave, over all slabs: 4 blocks of 8 warps per SM, or the 3 whose 64
-        // KiB of counters fit where a slab is 32 words.  Rows of up to 1,024 bins take at least 512 values per chunk:
-        // fewer, larger chunks left SMs idle on small calls (128 blocks for 2^21 values with fixed 2,048-value
-        // chunks); wide rows make a chunk of 64 values 32 KiB or more of row bytes, worth a warp.
-        uint32_t const slabs = f->slabs();
-        bool const full_slabs = f->bin_words > kSlabWords / 2;
-        uint64_t const blocks = std::max<uint64_t>(1, static_cast<uint64_t>(sm_count()) * (full_slabs ? 3u : 4u) / slabs);
-        uint64_t const wave = blocks * 8u;
-        uint64_t const round = full_slabs ? 32 : 128;
-        uint64_t const chunk =
-            std::max<uint64_t>(full_slabs ? 64 : 512, ((n + wave - 1) / wave + round - 1) / round * round);
-        uint64_t const warps = (n + chunk - 1) / chunk;
-        unsigned const grid = static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((warps + 7) / 8, blocks)));
-        size_t const smem = (64u << lanes_log2(static_cast<uint32_t>(std::min<uint64_t>(f->bin_words, kSlabWords)))) *
-                            sizeof(uint32_t) * (block / 32);
-        bulk_count_kernel_t const kernel = f->wide_rows() ? bulk_count_kernel<uint64_t>(f->hash_funs)
-                                                          : bulk_count_kernel<uint32_t>(f->hash_funs);
-        if (smem > 48 * 1024)
-            HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kernel<<<dim3(grid, slabs), block, smem, s>>>(f->rp(), d_values, n, chunk, totals);
-        HG_CUDA(cudaGetLastError());
-    }
-    k_store_counts<<<grid_for(f->bins, 256), 256, 0, s>>>(totals, f->bins, width, d_out);
+    if (grid > 1 && !reset)
+        HG_CUDA(cudaMemsetAsync(totals, 0, count_scratch_bytes(f), s));
+    size_t const smem = (64u << lanes) * sizeof(uint32_t) * (block / 32);
+    bulk_count_kernel_t const kernel = f->wide_rows() ? bulk_count_kernel<uint64_t>(f->hash_funs, lanes)
+                                                      : bulk_count_kernel<uint32_t>(f->hash_funs, lanes);
+    if (smem > 48 * 1024)
+        HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+    kernel<<<dim3(slabs, grid), block, smem, s>>>(f->rp(), values, n, chunk, totals,
+                                                  reinterpret_cast<unsigned int *>(totals + count_counters(f)), reset,
+                                                  f->bins, width, out);
     HG_CUDA(cudaGetLastError());
 }
 
@@ -580,45 +668,47 @@ void launch_contains(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, ui
 {
     if (n == 0)
         return;
-    row_params const rp = f->rp();
-    // all full slabs in one launch, a narrower last slab in one of its own (its lanes per row differ)
-    uint32_t const full = static_cast<uint32_t>(f->bin_words / kSlabWords);
-    uint32_t const rest = static_cast<uint32_t>(f->bin_words % kSlabWords);
-    unsigned const grid = grid_for(n, 256);
-    auto launch_h = [&](auto row_index, uint32_t lpv_log2, uint32_t first, uint32_t slabs)
+    uint32_t const lanes = f->contains_lanes_log2(n);
+    contains_kernel_t const kernel = f->wide_rows() ? contains_kernel<uint64_t>(f->hash_funs, lanes)
+                                                    : contains_kernel<uint32_t>(f->hash_funs, lanes);
+    kernel<<<dim3(f->slabs(lanes), grid_for(n, 256)), 256, 0, s>>>(f->rp(), d_values, n, d_out);
+    HG_CUDA(cudaGetLastError());
+}
+
+constexpr uint64_t kSmallBytes = 64u << 10; // host-pointer calls of up to this many bytes in and out need no copies
+
+// bulk_count of host values, finished on return: the counts in page-locked memory of the filter, valid until its next
+// host-pointer call (the caller holds f->mu).  Few values are read in place by the kernel, others are copied; the kernel
+// writes the counts to the host.
+void const * count_host(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int width)
+{
+    if (!f->host_totals.p || f->host_totals.bytes < count_scratch_bytes(f))
     {
-        using R = decltype(row_index);
-        switch (f->hash_funs)
-        {
-        case 1:
-            launch_contains_h<1, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
-            break;
-        case 2:
-            launch_contains_h<2, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
-            break;
-        case 3:
-            launch_contains_h<3, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
-            break;
-        case 4:
-            launch_contains_h<4, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
-            break;
-        default:
-            launch_contains_h<5, R>(rp, lpv_log2, first, slabs, d_values, n, d_out, grid, s);
-        }
-        HG_CUDA(cudaGetLastError());
-    };
-    auto launch = [&](uint32_t lpv_log2, uint32_t first, uint32_t slabs)
+        f->host_totals.ensure(count_scratch_bytes(f));
+        HG_CUDA(cudaMemsetAsync(f->host_totals.p, 0, f->host_totals.bytes, f->stream));
+    }
+    f->h_out.ensure(std::max<uint64_t>(f->bins * static_cast<uint64_t>(width), kSmallBytes));
+    if (!n)
     {
-        if (f->wide_rows())
-            launch_h(uint64_t{}, lpv_log2, first, slabs);
-        else
-            launch_h(uint32_t{}, lpv_log2, first, slabs);
-    };
-    constexpr uint32_t kMaxGridY = 65535;
-    for (uint32_t first = 0; first < full; first += kMaxGridY)
-        launch(5, first, std::min(kMaxGridY, full - first));
-    if (rest)
-        launch(lanes_log2(rest), full, 1);
+        std::memset(f->h_out.p, 0, f->bins * static_cast<uint64_t>(width));
+        return f->h_out.p;
+    }
+    uint64_t const * in = nullptr;
+    if (n * 8 <= kSmallBytes)
+    {
+        f->h_in.ensure(kSmallBytes);
+        std::memcpy(f->h_in.p, values, n * 8);
+        in = f->h_in.as<uint64_t>();
+    }
+    else
+    {
+        f->io.ensure(n * 8);
+        HG_CUDA(cudaMemcpyAsync(f->io.p, values, n * 8, cudaMemcpyHostToDevice, f->stream));
+        in = f->io.as<uint64_t>();
+    }
+    launch_count(f, in, n, width, f->h_out.p, f->stream, f->host_totals.as<unsigned long long>(), true);
+    HG_CUDA(cudaStreamSynchronize(f->stream));
+    return f->h_out.p;
 }
 
 int width_ok(int width)
@@ -631,7 +721,9 @@ int width_ok(int width)
 // instead of a cudaMalloc'd buffer.  Every device that loads the library holds it (128 KiB) until the process exits.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr uint64_t kNoAllocMaxCounters = HIBF_GPU_NOALLOC_MAX_BINS;
-static __device__ __align__(256) unsigned long long g_noalloc_totals[kNoAllocMaxCounters];
+// (and a 32-bit ticket per slab of at least 16 words)
+constexpr uint64_t kNoAllocTickets = kNoAllocMaxCounters / (64u * 16u);
+static __device__ __align__(256) unsigned long long g_noalloc_totals[kNoAllocMaxCounters + (kNoAllocTickets + 1) / 2];
 
 // Device address of g_noalloc_totals per device.  In host code the array's name is only a host-side stand-in, so
 // the address is looked up once per device (cudaGetSymbolAddress, with that device current) and cached.
@@ -977,6 +1069,16 @@ extern "C"
                 if (n == 0)
                     return;
                 std::lock_guard<std::mutex> lk(f->mu);
+                if (n * 8 <= kSmallBytes && n * f->bin_words * 8 <= kSmallBytes)
+                {
+                    f->h_in.ensure(kSmallBytes);
+                    f->h_out.ensure(kSmallBytes);
+                    std::memcpy(f->h_in.p, values, n * 8);
+                    launch_contains(f, f->h_in.as<uint64_t>(), n, f->h_out.as<uint64_t>(), f->stream);
+                    HG_CUDA(cudaStreamSynchronize(f->stream));
+                    std::memcpy(out, f->h_out.p, n * f->bin_words * 8);
+                    return;
+                }
                 f->io.ensure(n * 8);
                 f->io2.ensure(n * f->bin_words * 8);
                 HG_CUDA(cudaMemcpyAsync(f->io.p, values, n * 8, cudaMemcpyHostToDevice, f->stream));
@@ -1010,13 +1112,7 @@ extern "C"
                 if (!width_ok(width))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "width must be 1, 2, 4 or 8");
                 std::lock_guard<std::mutex> lk(f->mu);
-                f->io.ensure(n * 8);
-                f->io2.ensure(f->bins * 8);
-                if (n)
-                    HG_CUDA(cudaMemcpyAsync(f->io.p, values, n * 8, cudaMemcpyHostToDevice, f->stream));
-                launch_count(f, f->io.as<uint64_t>(), n, width, f->io2.p, f->stream);
-                HG_CUDA(cudaMemcpyAsync(out, f->io2.p, f->bins * width, cudaMemcpyDeviceToHost, f->stream));
-                HG_CUDA(cudaStreamSynchronize(f->stream));
+                std::memcpy(out, count_host(f, values, n, width), f->bins * static_cast<uint64_t>(width));
             });
     }
 
@@ -1028,10 +1124,8 @@ extern "C"
             {
                 if (!f || (n && !values) || !out_ids || !n_out)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
-                std::vector<uint16_t> counts(f->bins);
-                int const st = hibf_gpu_ibf_bulk_count(f, values, n, 2, counts.data());
-                if (st != HIBF_GPU_OK)
-                    fail(st, g_last_error);
+                std::lock_guard<std::mutex> lk(f->mu);
+                uint16_t const * const counts = static_cast<uint16_t const *>(count_host(f, values, n, 2));
                 uint64_t m = 0;
                 for (uint64_t b = 0; b < f->bins; ++b)
                     if (counts[b] >= threshold)

@@ -466,7 +466,7 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
         if constexpr (V == 0)
 #pragma unroll 1
             for (uint32_t w0 = 0; w0 < rp.bin_words; w0 += kSlabWords) // one slab unless the row is wider than a warp
-                warp_count<R, 32, H, Q::K>(row_slab(rp, w0), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
+                warp_count<R, 32, H, Q::K>(row_slab(rp, w0, kSlabWords), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
     }
 }
 
