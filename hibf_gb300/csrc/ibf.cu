@@ -10,8 +10,6 @@
 #include <string>
 #include <vector>
 
-#include <cub/cub.cuh>
-
 #include "../../include/hibf_gb300_synthetic.h"
 #include "archive.hpp"
 #include "common.hpp"
@@ -85,78 +83,124 @@ __global__ void k_synth_emplace(uint64_t * __restrict__ words, uint64_t bin_size
 // ---------------------------------------------------------------------------------------------------------------
 // Exact occupancy.  The reference counts a value for its bin when one of its bits was not set yet, inserting one value
 // after the other (src/interleaved_bloom_filter.cpp:119-140).  With concurrent atomicOr that depends on timing, so an
-// IBF that tracks occupancy inserts in chunks: every (value, hash) position of the chunk becomes a key row * tb + bin,
-// a stable sort groups equal positions in insertion order, and a value counts when it is the first of the chunk at a
-// position that was unset before the chunk.  Then the bits are set.
+// IBF that tracks occupancy inserts in chunks, in two passes.  The first enters every position (row * tb + bin) that is
+// still unset into a hash table and lowers the position's entry to the chunk's first value there; the second counts a
+// value that is first at one of its positions and sets its bits.  Both are bound by random accesses that L2 serves (the
+// table of a chunk is at most 100 MB): 530,624 values with h = 2 take 41 us; sorting the positions took 14 launches, 260
+// us, and as much again in allocations.
 // ---------------------------------------------------------------------------------------------------------------
-constexpr uint64_t kNoPosition = ~0ull;
+constexpr unsigned long long kFreeEntry = ~0ull;
+constexpr uint32_t kIsSet = ~0u; // the entry of a position whose bit was set before the chunk, or of no position
 
+// Value i of the chunk and its bin: from the arrays, or (SYNTH) value `first + i` of the generated bin `bin`.
 template <bool SYNTH>
-__global__ void k_occ_keys(uint64_t const * __restrict__ words, uint64_t bin_size, uint32_t row_words, uint32_t shift,
-                           uint32_t h, uint64_t const * __restrict__ values, uint64_t const * __restrict__ bins,
-                           uint64_t seed, uint64_t vpb, uint64_t first, uint64_t n, uint64_t bin, uint64_t n_bins,
-                           uint64_t tb, unsigned long long * __restrict__ keys, unsigned long long * __restrict__ ids,
-                           uint8_t * __restrict__ was_set, uint64_t * __restrict__ gen_values)
+__device__ __forceinline__ uint64_t occ_value(uint64_t const * values, uint64_t const * bins, uint64_t seed,
+                                              uint64_t vpb, uint64_t first, uint64_t i, uint64_t bin, uint64_t & b)
+{
+    b = !SYNTH && bins ? bins[i] : bin;
+    if constexpr (SYNTH)
+        return hg_ibf_bin_value(seed, vpb, bin, first + i);
+    else
+        return values[i];
+}
+
+// The table has mask + 1 slots (a power of two, at least 1.5 per position, so that a free one is always found): keys and
+// the lowest value index per key.  entries[i * h + k]: the slot of value i's position k.
+template <bool SYNTH>
+__global__ void k_occ_enter(uint64_t const * __restrict__ words, uint64_t bin_size, uint32_t row_words, uint32_t shift,
+                            uint32_t h, uint64_t const * __restrict__ values, uint64_t const * __restrict__ bins,
+                            uint64_t seed, uint64_t vpb, uint64_t first, uint64_t n, uint64_t bin, uint64_t n_bins,
+                            uint64_t tb, unsigned long long * keys, unsigned int * lowest, uint32_t mask,
+                            uint32_t * __restrict__ entries)
 {
     uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
     {
-        uint64_t v, b;
-        if constexpr (SYNTH)
-        {
-            b = bin;
-            v = hg_ibf_bin_value(seed, vpb, bin, first + i);
-            gen_values[i] = v;
-        }
-        else
-        {
-            v = values[i];
-            b = bins ? bins[i] : bin;
-        }
+        uint64_t b;
+        uint64_t const v = occ_value<SYNTH>(values, bins, seed, vpb, first, i, bin, b);
         for (uint32_t k = 0; k < h; ++k)
         {
-            uint64_t const idx = i * h + k;
-            ids[idx] = idx;
-            if (b >= n_bins)
+            uint32_t entry = kIsSet;
+            if (b < n_bins)
             {
-                keys[idx] = kNoPosition;
-                was_set[idx] = 1;
-                continue;
+                uint64_t const r = hash_row(v, c_hash_seeds[k], shift, bin_size);
+                if (!((words[r * row_words + (b >> 6)] >> (b & 63u)) & 1u))
+                {
+                    unsigned long long const key = r * tb + b;
+                    uint32_t slot = static_cast<uint32_t>(((key ^ (key >> 32)) * 11400714819323198485ULL) >> 32) & mask;
+                    for (;;)
+                    {
+                        unsigned long long const old = atomicCAS(keys + slot, kFreeEntry, key);
+                        if (old == kFreeEntry || old == key)
+                            break;
+                        slot = (slot + 1u) & mask;
+                    }
+                    atomicMin(lowest + slot, static_cast<unsigned int>(i));
+                    entry = slot;
+                }
             }
-            uint64_t const r = hash_row(v, c_hash_seeds[k], shift, bin_size);
-            keys[idx] = r * tb + b;
-            was_set[idx] = static_cast<uint8_t>((words[r * row_words + (b >> 6)] >> (b & 63u)) & 1u);
+            entries[i * h + k] = entry;
         }
     }
 }
 
-__global__ void k_occ_first(unsigned long long const * __restrict__ keys, unsigned long long const * __restrict__ ids,
-                            uint64_t m, uint32_t h, uint8_t const * __restrict__ was_set,
-                            unsigned int * __restrict__ newly)
+template <bool SYNTH>
+__global__ void k_occ_insert(uint64_t * __restrict__ words, uint64_t bin_size, uint32_t row_words, uint32_t shift,
+                             uint32_t h, uint64_t const * __restrict__ values, uint64_t const * __restrict__ bins,
+                             uint64_t seed, uint64_t vpb, uint64_t first, uint64_t n, uint64_t bin, uint64_t n_bins,
+                             unsigned int const * __restrict__ lowest, uint32_t const * __restrict__ entries,
+                             unsigned long long * __restrict__ occupancy, int * bad_bin)
 {
     uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
-    for (uint64_t j = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; j < m; j += stride)
+    uint64_t const first_i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    int const lane = threadIdx.x & 31;
+    for (uint64_t base = first_i - lane; base < n; base += stride) // whole warps: they add up their counts
     {
-        if (keys[j] == kNoPosition || (j > 0 && keys[j] == keys[j - 1]))
-            continue;
-        uint64_t const idx = ids[j];
-        if (!was_set[idx])
-            newly[idx / h] = 1u;
+        uint64_t const i = base + lane;
+        bool newly = false;
+        uint64_t b = ~0ull;
+        if (i < n)
+        {
+            uint64_t const v = occ_value<SYNTH>(values, bins, seed, vpb, first, i, bin, b);
+            if (b >= n_bins)
+            {
+                *bad_bin = 1; // device-supplied bin index out of range: skipped, reported by hibf_gpu_ibf_status
+            }
+            else
+            {
+                unsigned long long const bit = 1ull << (b & 63u);
+                for (uint32_t k = 0; k < h; ++k)
+                {
+                    uint32_t const entry = entries[i * h + k];
+                    if (entry == kIsSet)
+                        continue;
+                    newly = newly || lowest[entry] == static_cast<unsigned int>(i);
+                    uint64_t const r = hash_row(v, c_hash_seeds[k], shift, bin_size);
+                    atomicOr(reinterpret_cast<unsigned long long *>(words + r * row_words + (b >> 6)), bit);
+                }
+            }
+        }
+        // one addition per bin and warp: a user bin's values usually come together (530,624 values of 64 bins added one
+        // by one took 50 us)
+        unsigned const counted = __ballot_sync(kFullMask, newly);
+        if (newly)
+        {
+            unsigned const same = __match_any_sync(counted, b);
+            if (lane == __ffs(same) - 1)
+                atomicAdd(occupancy + b, static_cast<unsigned long long>(__popc(same)));
+        }
     }
 }
 
-template <bool SYNTH>
-__global__ void k_occ_count(unsigned int const * __restrict__ newly, uint64_t const * __restrict__ bins, uint64_t vpb,
-                            uint64_t first, uint64_t n, uint64_t bin, uint64_t n_bins,
-                            unsigned long long * __restrict__ occupancy)
+// Sets *bad (mapped host memory) when a bin index is out of range.
+__global__ void k_check_bins(uint64_t const * __restrict__ bins, uint64_t n, uint64_t n_bins, int * bad)
 {
     uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
+    bool mine = false;
     for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n; i += stride)
-    {
-        uint64_t const b = SYNTH ? bin : (bins ? bins[i] : bin);
-        if (newly[i] && b < n_bins)
-            atomicAdd(occupancy + b, 1ull);
-    }
+        mine = mine || bins[i] >= n_bins;
+    if (mine)
+        *bad = 1;
 }
 
 // clear(bin) (src/interleaved_bloom_filter.cpp:142-148): clear one bit of every row.
@@ -481,6 +525,8 @@ struct hibf_gpu_ibf
     hbuf h_in, h_out; // small host-pointer calls: values the kernels read in place, results they write
     dbuf io;        // staging for host-pointer calls
     dbuf io2;
+    dbuf occ_scratch; // emplace_exact's table, at most 150 MB, one call at a time
+    std::mutex occ_mu;
     dbuf flag; // device int: an emplace saw a bin index out of range
     cudaStream_t stream{};
     int status{HIBF_GPU_OK};
@@ -533,8 +579,9 @@ cudaStream_t pick(hibf_gpu_ibf * f, void * s)
     return s ? static_cast<cudaStream_t>(s) : f->stream;
 }
 
-// Occupancy in insertion order, chunk by chunk, then each chunk's bits; chunks run one after the other, so each sees
-// the bits of the chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).
+// Occupancy in insertion order and the bits, chunk by chunk; chunks run one after the other, so each sees the bits of the
+// chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).  The scratch belongs to the
+// filter (calls on several streams take turns).
 template <bool SYNTH>
 void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const * d_bins, uint64_t n, uint64_t bin,
                    uint64_t seed, uint64_t vpb, cudaStream_t s)
@@ -543,49 +590,31 @@ void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const *
     unsigned const block = 256;
     uint32_t const h = static_cast<uint32_t>(f->hash_funs);
     uint64_t const m_max = std::min(n, kChunk) * h;
-    dbuf keys, keys2, ids, ids2, was_set, newly, gen, tmp;
-    keys.ensure(m_max * 8);
-    keys2.ensure(m_max * 8);
-    ids.ensure(m_max * 8);
-    ids2.ensure(m_max * 8);
-    was_set.ensure(m_max);
-    newly.ensure(std::min(n, kChunk) * 4);
-    if (SYNTH)
-        gen.ensure(std::min(n, kChunk) * 8);
-    size_t tmp_bytes = 0;
-    HG_CUDA(cub::DeviceRadixSort::SortPairs(nullptr, tmp_bytes, keys.as<unsigned long long>(),
-                                            keys2.as<unsigned long long>(), ids.as<unsigned long long>(),
-                                            ids2.as<unsigned long long>(), static_cast<int>(m_max), 0, 64, s));
-    tmp.ensure(std::max<size_t>(tmp_bytes, 16));
-    uint64_t const tb = f->technical_bins();
+    uint64_t slots = 1024;
+    while (slots < m_max + m_max / 2)
+        slots *= 2;
+    std::lock_guard<std::mutex> lk(f->occ_mu);
+    f->occ_scratch.ensure(slots * 12 + m_max * 4);
+    auto * const keys = f->occ_scratch.as<unsigned long long>();
+    auto * const lowest = reinterpret_cast<unsigned int *>(keys + slots);
+    auto * const entries = lowest + slots;
+    uint32_t const rw = static_cast<uint32_t>(f->row_words);
     for (uint64_t c0 = 0; c0 < n; c0 += kChunk)
     {
         uint64_t const c = std::min(kChunk, n - c0);
-        uint64_t const m = c * h;
-        uint64_t const * vals = SYNTH ? gen.as<uint64_t>() : d_values + c0;
+        uint64_t const * vals = SYNTH ? nullptr : d_values + c0;
         uint64_t const * bins = (SYNTH || !d_bins) ? nullptr : d_bins + c0;
-        k_occ_keys<SYNTH><<<grid_for(c, block), block, 0, s>>>(
-            f->store.as<uint64_t>(), f->bin_size, static_cast<uint32_t>(f->row_words), f->shift, h,
-            SYNTH ? nullptr : vals, bins, seed, vpb, c0, c, bin, f->bins, tb, keys.as<unsigned long long>(),
-            ids.as<unsigned long long>(), was_set.as<uint8_t>(), SYNTH ? gen.as<uint64_t>() : nullptr);
+        HG_CUDA(cudaMemsetAsync(keys, 0xFF, slots * 12, s)); // free entries, no value yet
+        k_occ_enter<SYNTH><<<grid_for(c, block), block, 0, s>>>(
+            f->store.as<uint64_t>(), f->bin_size, rw, f->shift, h, vals, bins, seed, vpb, c0, c, bin, f->bins,
+            f->technical_bins(), keys, lowest, static_cast<uint32_t>(slots - 1), entries);
         HG_CUDA(cudaGetLastError());
-        size_t bytes = tmp_bytes;
-        HG_CUDA(cub::DeviceRadixSort::SortPairs(tmp.p, bytes, keys.as<unsigned long long>(),
-                                                keys2.as<unsigned long long>(), ids.as<unsigned long long>(),
-                                                ids2.as<unsigned long long>(), static_cast<int>(m), 0, 64, s));
-        HG_CUDA(cudaMemsetAsync(newly.p, 0, c * 4, s));
-        k_occ_first<<<grid_for(m, block), block, 0, s>>>(keys2.as<unsigned long long>(), ids2.as<unsigned long long>(),
-                                                         m, h, was_set.as<uint8_t>(), newly.as<unsigned int>());
-        HG_CUDA(cudaGetLastError());
-        k_occ_count<SYNTH><<<grid_for(c, block), block, 0, s>>>(newly.as<unsigned int>(), bins, vpb, c0, c, bin,
-                                                               f->bins, f->occupancy.as<unsigned long long>());
-        HG_CUDA(cudaGetLastError());
-        k_emplace<<<grid_for(c, block), block, 0, s>>>(f->store.as<uint64_t>(), f->bin_size,
-                                                       static_cast<uint32_t>(f->row_words), f->shift, h, vals,
-                                                       SYNTH ? nullptr : bins, c, bin, f->bins, f->flag.as<int>());
+        k_occ_insert<SYNTH><<<grid_for(c, block), block, 0, s>>>(
+            f->store.as<uint64_t>(), f->bin_size, rw, f->shift, h, vals, bins, seed, vpb, c0, c, bin, f->bins, lowest,
+            entries, f->occupancy.as<unsigned long long>(), f->flag.as<int>());
         HG_CUDA(cudaGetLastError());
     }
-    HG_CUDA(cudaStreamSynchronize(s)); // the scratch buffers are freed on return
+    HG_CUDA(cudaStreamSynchronize(s)); // the scratch is free for the next call
 }
 
 void launch_emplace(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const * d_bins, uint64_t n, uint64_t bin,
@@ -675,6 +704,7 @@ void launch_contains(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, ui
     HG_CUDA(cudaGetLastError());
 }
 
+constexpr uint64_t kDeviceCheck = 1u << 14; // host-pointer inserts of this many values have their bins checked on the device
 constexpr uint64_t kSmallBytes = 64u << 10; // host-pointer calls of up to this many bytes in and out need no copies
 
 // bulk_count of host values, finished on return: the counts in page-locked memory of the filter, valid until its next
@@ -922,14 +952,31 @@ extern "C"
             {
                 if (!f || (n && (!values || !bins)))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
-                for (uint64_t i = 0; i < n; ++i)
+                // Nothing is inserted if any bin is out of range.  Many bins are checked on the device, beside the copy of
+                // the values (the host reads 530,624 of them in 0.2 ms, about as long as everything else takes).
+                bool const on_device = n >= kDeviceCheck;
+                for (uint64_t i = 0; i < n && !on_device; ++i)
                     if (bins[i] >= f->bins)
                         fail(HIBF_GPU_ERR_INVALID_ARG, "bin index out of range");
                 std::lock_guard<std::mutex> lk(f->mu);
                 f->io.ensure(n * 8);
                 f->io2.ensure(n * 8);
-                HG_CUDA(cudaMemcpyAsync(f->io.p, values, n * 8, cudaMemcpyHostToDevice, f->stream));
                 HG_CUDA(cudaMemcpyAsync(f->io2.p, bins, n * 8, cudaMemcpyHostToDevice, f->stream));
+                if (on_device)
+                {
+                    f->h_out.ensure(kSmallBytes);
+                    *f->h_out.as<int>() = 0;
+                    k_check_bins<<<grid_for(n, 256), 256, 0, f->stream>>>(f->io2.as<uint64_t>(), n, f->bins,
+                                                                          f->h_out.as<int>());
+                    HG_CUDA(cudaGetLastError());
+                }
+                HG_CUDA(cudaMemcpyAsync(f->io.p, values, n * 8, cudaMemcpyHostToDevice, f->stream));
+                if (on_device)
+                {
+                    HG_CUDA(cudaStreamSynchronize(f->stream));
+                    if (*static_cast<int volatile const *>(f->h_out.p))
+                        fail(HIBF_GPU_ERR_INVALID_ARG, "bin index out of range");
+                }
                 launch_emplace(f, f->io.as<uint64_t>(), f->io2.as<uint64_t>(), n, 0, f->stream);
                 HG_CUDA(cudaStreamSynchronize(f->stream));
             });
@@ -1222,8 +1269,11 @@ extern "C"
                 if (n_words != f->bin_words * f->bin_size)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "word count does not match the filter");
                 std::lock_guard<std::mutex> lk(f->mu);
-                HG_CUDA(cudaMemcpy2DAsync(words, f->bin_words * 8, f->store.p, f->row_words * 8, f->bin_words * 8,
-                                          f->bin_size, cudaMemcpyDeviceToHost, f->stream));
+                if (f->row_words == f->bin_words)
+                    HG_CUDA(cudaMemcpyAsync(words, f->store.p, n_words * 8, cudaMemcpyDeviceToHost, f->stream));
+                else
+                    HG_CUDA(cudaMemcpy2DAsync(words, f->bin_words * 8, f->store.p, f->row_words * 8, f->bin_words * 8,
+                                              f->bin_size, cudaMemcpyDeviceToHost, f->stream));
                 HG_CUDA(cudaStreamSynchronize(f->stream));
             });
     }
