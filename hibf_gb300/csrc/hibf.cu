@@ -860,6 +860,9 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
     {
         query_params p = base_params(a, d_values, d_qoff, d_thr, nq, mask_for(mode, width));
         p.decide = mode == HIBF_GPU_QUERY_MEMBERSHIP;
+        // an in-place host batch: the roots stage the values they read, the lower levels read them from there
+        p.stage = a->stage_values;
+        p.staged = blk ? nullptr : a->stage_counts;
         int const fit = blk ? a->max_blocks_blk : a->max_blocks[a->variant];
         int const per_sm = a->tune.blocks_per_sm ? std::min<int>(fit, static_cast<int>(a->tune.blocks_per_sm)) : fit;
         uint64_t const full = static_cast<uint64_t>(sm_count()) * static_cast<uint64_t>(per_sm);
@@ -874,9 +877,6 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
         HG_CUDA(cudaEventRecordWithFlags(a->ev_k0, s, rec_flags));
         if (levels)
         {
-            // an in-place host batch: the roots stage the values they read, the lower levels read them from there
-            p.stage = a->stage_values;
-            p.staged = a->stage_counts;
             // one launch per level: the roots, then each level's appended tasks grouped by IBF
             // each level counts its work into its own kStats words; read_status sums them
             unsigned long long * const lvl_stats = a->ctrl.as<unsigned long long>() + C_WORDS + kStats;
@@ -1159,6 +1159,21 @@ std::vector<uint64_t> const & traversal_rank(hibf_gpu_hibf * h)
     return h->trav_rank;
 }
 
+// Whether the device reads pageable host memory through the host's page tables (Grace hosts).
+bool host_page_tables()
+{
+    static bool const yes = []
+    {
+        int dev = 0, access = 0, tables = 0;
+        bool const ok = cudaGetDevice(&dev) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&access, cudaDevAttrPageableMemoryAccess, dev) == cudaSuccess &&
+                        cudaDeviceGetAttribute(&tables, cudaDevAttrPageableMemoryAccessUsesHostPageTables, dev) ==
+                            cudaSuccess;
+        return ok && access && tables;
+    }();
+    return yes;
+}
+
 // Events of a host batch's timeline (hibf_gpu_agent_last_timeline) for n copies of values.
 void ensure_timeline(hibf_gpu_agent * a, uint32_t n)
 {
@@ -1296,16 +1311,26 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     check_batch(mode, width, thr, nq, qoff);
     uint64_t const nv = nq ? qoff[nq] : 0;
     // In place: values in mapped page-locked memory are read by the kernel over the host link as it needs them, so
-    // no copy precedes (or paces) the launch; only the offsets and thresholds are copied.
+    // no copy precedes (or paces) the launch; only the offsets and thresholds are copied.  So are pageable values too
+    // few to be streamed where the GPU goes through the host's page tables: 20 MB on the 64-bin workload, 10,000
+    // queries, took 138 us to copy before a kernel of 65, in place the kernel takes 165.
     uint64_t const * in_place = nullptr;
     if (a->host_read && !plain && nv)
     {
         cudaPointerAttributes attr{};
         void * dev = nullptr;
-        if (cudaPointerGetAttributes(&attr, values) == cudaSuccess && attr.type == cudaMemoryTypeHost &&
-            cudaHostGetDevicePointer(&dev, const_cast<uint64_t *>(values), 0) == cudaSuccess)
-            in_place = static_cast<uint64_t const *>(dev);
-        cudaGetLastError(); // pageable memory: the queries above fail, and the values are copied
+        if (cudaPointerGetAttributes(&attr, values) == cudaSuccess)
+        {
+            if (attr.type == cudaMemoryTypeHost)
+            {
+                if (cudaHostGetDevicePointer(&dev, const_cast<uint64_t *>(values), 0) == cudaSuccess)
+                    in_place = static_cast<uint64_t const *>(dev);
+            }
+            else if (attr.type == cudaMemoryTypeUnregistered && nv > kPackValues && nv * 8 < kStreamMinBytes &&
+                     host_page_tables())
+                in_place = values;
+        }
+        cudaGetLastError(); // a query above that failed: the values are copied
     }
     a->last_in_place = in_place != nullptr;
     a->last_chunks = 0;

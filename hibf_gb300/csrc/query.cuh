@@ -134,9 +134,9 @@ struct query_params
     uint32_t level;
     unsigned long long const * in_tasks;
     unsigned long long const * in_count;
-    // in-place host batches under the level schedule: `values` is the host's memory; root tasks store every value
-    // they read at stage[same position] and how many they read (from the query's first value) at staged[query], and
-    // the lower levels read that prefix from stage and only the rest from the host.  k_query_blk's roots read all their
+    // in-place host batches: `values` is the host's memory; root tasks store every value they read at stage[same
+    // position] and how many they read (from the query's first value) at staged[query], and the lower levels read that
+    // prefix from stage and only the rest from the host.  k_query_blk's roots read all their
     // values, so it needs no counts.  Null otherwise.
     uint64_t * stage;
     uint32_t * staged;
@@ -695,10 +695,10 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
     // of the counting code for the stages and the rest: each call site inlines every row width's counting path, and a
     // hierarchy of mixed widths runs them all at once, so a second copy would double the instruction footprint.
     uint64_t done = 0;
-    // in-place host batch under the level schedule: a root stages what it reads; a lower level reads the staged prefix
-    // [0, staged) from device memory and the rest from the host
+    // in-place host batch: a root stages what it reads; a lower level reads the staged prefix [0, staged) from device
+    // memory and the rest from the host
     bool const stage_root = p.staged && depth == 0;
-    uint64_t const staged = p.staged && depth > 0 ? p.staged[q] : 0u;
+    uint64_t const staged = p.staged && depth > 0 ? __ldcg(p.staged + q) : 0u;
     bool const adaptive = p.ee_stages == kEarlyExitAdaptive && n >= p.ee_min;
     uint64_t const most = n * nd.max_seg; // no segment's sum passes this
     bool const narrow = most < kNarrowSums;
@@ -758,7 +758,8 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
     }
     __syncwarp();
     if (stage_root && lane == 0)
-        p.staged[q] = static_cast<uint32_t>(done); // read by the next level's launch
+        p.staged[q] = static_cast<uint32_t>(done); // read by its children, behind emit_bins' fence or in a later launch
+    __syncwarp();
     if (state == kHopeless)
     {
         retire_task(p, q, n, done, lane, n_tasks, n_visits, n_executed); // without results or children
@@ -919,7 +920,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
             else
             {
                 if (lane == 0)
-                    task = wait_for_task(p, slot); // a reserved slot: its writer is storing it
+                    task = wait_for_task(p, slot); // a reserved slot: its writer is storing it (values are on the device)
                 task = __shfl_sync(kFullMask, task, 0);
                 if (task == kEmpty)
                     break;
@@ -989,6 +990,8 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
                 if (lane == 0)
                     task = wait_for_task(p, slot);
                 task = __shfl_sync(kFullMask, task, 0);
+                if (p.staged)
+                    __threadfence(); // another warp's root staged the values this task reads
                 if (task == kEmpty)
                     break;
             }

@@ -381,8 +381,9 @@ int hibf_gpu_agent_level_work(hibf_gpu_agent * a, uint64_t * tasks, uint64_t * v
 /* In place (on by default): host batches (hibf_gpu_agent_query_batch) whose values lie in mapped page-locked memory
  * (cudaHostAlloc, cudaHostRegister) are not copied: the kernel reads the values over the host link as it needs them,
  * and the batch runs its configured schedule from the first root.  in_place == 0 copies them first (a batch of 64 MiB
- * or more is then streamed in chunks and runs the work queue).  Pageable values are always copied.  Results are the
- * same either way; on the 8,192-bin batch (8.1 GB of values) in place took 50.3 ms per call, every call, where the
+ * or more is then streamed in chunks and runs the work queue).  Pageable values of more than 64 KiB and less than 64
+ * MiB are read in place too where the GPU goes through the host's page tables (Grace hosts); others are copied.
+ * Results are the same either way; on the 8,192-bin batch (8.1 GB of values) in place took 50.3 ms per call, every call, where the
  * copy's rate varied with the host link (47-344 ms). */
 int hibf_gpu_agent_set_host_read(hibf_gpu_agent * a, int in_place);
 /* Whether the agent's last host batch was read in place (1) or copied (0). */
@@ -420,8 +421,8 @@ typedef struct hibf_gpu_tuning
     uint32_t early_exit_first;  /* percent of a task's values counted before its first early-exit check */
     uint32_t early_exit_step;   /* percent between later checks (adaptive: the fewest values between checks) */
     uint32_t early_exit_stages; /* number of checks (0: none; first + (stages - 1) * step must stay below 100), or
-                                   HIBF_GPU_EARLY_EXIT_ADAPTIVE: check where the outcome can first change, computed
-                                   from the bin sums at every check (early_exit_first unused) */
+                                   HIBF_GPU_EARLY_EXIT_ADAPTIVE: check where the outcome is expected to be settled,
+                                   projected from the bin sums at every check (early_exit_first unused) */
     uint32_t early_exit_min;    /* tasks with fewer values are counted in one stage */
     uint32_t block_queries;     /* batches of at most this many queries run one task per block of 8 warps (latency
                                    mode: each task's values split over the warps, no early exit); 0: never */
