@@ -398,11 +398,18 @@ void replay_split_history(plan_t const & P, Source const & source, OnSplit const
     };
     auto take = [&](rh_set & k, user_bin_rec const & r)
     {
-        source(r.idx, [&](uint64_t v) { k.insert(v); });
+        rh_feeder feed(k);
+        source(r.idx, [&](uint64_t v) { feed(v); });
+        feed.finish();
         if (r.ntb > 1)
             on_split(r.idx, r.ntb, k);
     };
-    auto add = [](rh_set const & from, rh_set & to) { from.for_each([&](uint64_t v) { to.insert(v); }); };
+    auto add = [](rh_set const & from, rh_set & to)
+    {
+        rh_feeder feed(to);
+        from.for_each([&](uint64_t v) { feed(v); });
+        feed.finish();
+    };
 
     std::function<void(size_t, rh_set *, bool)> run = [&](size_t n, rh_set * parent, bool is_root)
     {

@@ -2,16 +2,17 @@
 //
 // The reference reads every user bin into a hash set (compute_kmers, src/build/compute_kmers.cpp:23-32) and sizes a
 // merged max bin by the distinct count of its subtree's union (src/hierarchical_interleaved_bloom_filter.cpp:39-171,
-// the favourite child's kmers).  Here both are sorts on the device:
-//   distinct_sets_device  every user bin's distinct values in first-appearance order: a segmented radix sort of
-//                         (value, position in the bin) per bin (stable, so equal values keep input order), a flag
-//                         on the first of every run, the flagged positions compacted and sorted back into input
-//                         order, and the values gathered at them;
-//   union_size_device     the distinct count of the union of some user bins' sets: one sort of their
-//                         concatenation and a count of run starts.
+// the favourite child's kmers).  Here both are hash tables on the device:
+//   distinct_sets_device  every user bin's distinct values in first-appearance order: a table entry per (user bin, value)
+//                         keeps the value's first position, the values at such positions are compacted in order;
+//   union_size_device     the distinct count of the union of some user bins' sets: the number of table entries.
+// Bound by the table's random accesses (a 4-byte slot and the value it names, both in L2 for a few million values): the
+// 64-user-bin workload, 1.47e6 values, takes 40 us of kernels; a segmented sort, a selection and a sort back took 2.1 ms,
+// and a dozen buffers were allocated for them.
 // Only the order of split user bins' values depends on the reference's hash set (robin_hood iteration order); the
 // host replays that from the first-appearance order these produce.
 #include <algorithm>
+#include <initializer_list>
 #include <vector>
 
 #include <cub/cub.cuh>
@@ -27,43 +28,76 @@ namespace
 
 constexpr uint64_t kBatchValues = 1ull << 30; // values per device batch (CUB's segmented sort counts items in int)
 
-// Position p of segment s: its index within the segment, and its segment.
-__global__ void k_segment_index(int const * __restrict__ seg_off, uint32_t n_seg, uint32_t * __restrict__ idx,
-                                uint32_t * __restrict__ seg)
+constexpr uint32_t kFreeSlot = ~0u;
+
+// The segment of position i: the last s with seg_off[s] <= i.
+__device__ __forceinline__ uint32_t segment_of(int const * __restrict__ seg_off, uint32_t n_seg, uint32_t i)
 {
-    for (uint32_t s = blockIdx.x; s < n_seg; s += gridDim.x)
+    uint32_t lo = 0, hi = n_seg - 1u;
+    while (lo < hi)
     {
-        int const b = seg_off[s], e = seg_off[s + 1];
-        for (int p = b + static_cast<int>(threadIdx.x); p < e; p += static_cast<int>(blockDim.x))
+        uint32_t const mid = (lo + hi + 1u) >> 1;
+        if (static_cast<uint32_t>(seg_off[mid]) <= i)
+            lo = mid;
+        else
+            hi = mid - 1u;
+    }
+    return lo;
+}
+
+// Enters every position into the table of (segment, value): a slot holds the lowest position of its pair.  mask + 1
+// slots, a power of two and at least 1.5 per position, so a free one is always found.  entry[i]: position i's slot.
+__global__ void k_distinct_enter(uint64_t const * __restrict__ values, uint64_t n, int const * __restrict__ seg_off,
+                                 uint32_t n_seg, uint32_t * slots, uint32_t mask, uint32_t * __restrict__ entry)
+{
+    for (uint64_t p = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; p < n;
+         p += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+    {
+        uint32_t const i = static_cast<uint32_t>(p);
+        uint32_t const s = segment_of(seg_off, n_seg, i);
+        uint32_t const b = static_cast<uint32_t>(seg_off[s]), e = static_cast<uint32_t>(seg_off[s + 1]);
+        uint64_t const v = values[i];
+        uint64_t h = (v ^ (v >> 32) ^ (static_cast<uint64_t>(s) << 17)) * 0x9E3779B97F4A7C15ULL;
+        h ^= h >> 29;
+        uint32_t slot = static_cast<uint32_t>(h >> 16) & mask;
+        for (;;)
         {
-            idx[p] = static_cast<uint32_t>(p - b);
-            seg[p] = s;
+            uint32_t const old = atomicCAS(slots + slot, kFreeSlot, i);
+            if (old == kFreeSlot)
+                break;
+            if (old >= b && old < e && values[old] == v) // a position of this segment: the same pair
+            {
+                atomicMin(slots + slot, i);
+                break;
+            }
+            slot = (slot + 1u) & mask;
+        }
+        entry[i] = slot;
+    }
+}
+
+// flag[i] (optional): position i is its value's first in its segment; count[s]: how many are in segment s.
+__global__ void k_distinct_first(uint32_t const * __restrict__ slots, uint32_t const * __restrict__ entry, uint64_t n,
+                                 int const * __restrict__ seg_off, uint32_t n_seg, unsigned char * __restrict__ flag,
+                                 unsigned long long * __restrict__ count)
+{
+    int const lane = threadIdx.x & 31;
+    uint64_t const at = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
+    for (uint64_t base = at - lane; base < n; base += static_cast<uint64_t>(gridDim.x) * blockDim.x)
+    {
+        uint64_t const i = base + lane; // whole warps: they add up their counts
+        bool const first = i < n && slots[entry[i]] == static_cast<uint32_t>(i);
+        if (flag && i < n)
+            flag[i] = first ? 1 : 0;
+        unsigned const counted = __ballot_sync(0xffffffffu, first);
+        if (first)
+        {
+            uint32_t const s = segment_of(seg_off, n_seg, static_cast<uint32_t>(i));
+            unsigned const same = __match_any_sync(counted, s);
+            if (lane == __ffs(same) - 1)
+                atomicAdd(count + s, static_cast<unsigned long long>(__popc(same)));
         }
     }
-}
-
-// After the segmented sort: flag the first of every run of equal values within a segment and record its position
-// in the batch (segment start + index in the segment).
-__global__ void k_first_of_run(uint64_t const * __restrict__ keys, uint32_t const * __restrict__ idx,
-                               uint32_t const * __restrict__ seg, int const * __restrict__ seg_off, uint64_t n,
-                               uint64_t * __restrict__ pos, unsigned char * __restrict__ flag)
-{
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-    {
-        uint32_t const s = seg[i];
-        bool const first = i == 0 || seg[i - 1] != s || keys[i - 1] != keys[i];
-        flag[i] = first ? 1 : 0;
-        pos[i] = static_cast<uint64_t>(seg_off[s]) + idx[i];
-    }
-}
-
-__global__ void k_gather(uint64_t const * __restrict__ values, uint64_t const * __restrict__ pos, uint64_t n,
-                         uint64_t * __restrict__ out)
-{
-    for (uint64_t i = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x; i < n;
-         i += static_cast<uint64_t>(gridDim.x) * blockDim.x)
-        out[i] = values[pos[i]];
 }
 
 // Number of i with i == 0 or keys[i] != keys[i - 1] (keys sorted).
@@ -83,6 +117,36 @@ unsigned grid_for(uint64_t n)
 {
     return static_cast<unsigned>(std::max<uint64_t>(1, std::min<uint64_t>((n + 255) / 256, sm_count() * 8ull)));
 }
+
+uint64_t table_slots(uint64_t n)
+{
+    uint64_t slots = 1024;
+    while (slots < n + n / 2)
+        slots *= 2;
+    return slots;
+}
+
+// Consecutive pieces of one allocation, each aligned for any type (an allocation and its release cost about 0.1 ms).
+struct arena
+{
+    dbuf buf;
+    size_t used{0};
+    void reserve(std::initializer_list<size_t> pieces)
+    {
+        size_t total = 0;
+        for (size_t p : pieces)
+            total += (p + 255) / 256 * 256;
+        buf.ensure(total);
+        used = 0;
+    }
+    template <typename T>
+    T * take(size_t bytes)
+    {
+        T * const p = reinterpret_cast<T *>(buf.as<char>() + used);
+        used += (bytes + 255) / 256 * 256;
+        return p;
+    }
+};
 
 } // namespace
 
@@ -113,8 +177,9 @@ void distinct_sets_device(uint64_t const * values, std::vector<uint64_t> const &
             cudaStreamDestroy(s);
         }
     } const guard{s};
-    dbuf d_in, d_keys, d_idx_in, d_idx, d_seg, d_off, d_pos, d_flag, d_sel, d_sorted, d_out, d_nsel, d_tmp;
-    hbuf h_out;
+    arena mem;
+    std::vector<uint64_t> distinct;
+    std::vector<unsigned long long> counts;
     for (uint64_t u0 = 0; u0 < nub;)
     {
         // a batch of whole user bins, at most kBatchValues values unless one bin alone is larger
@@ -134,88 +199,60 @@ void distinct_sets_device(uint64_t const * values, std::vector<uint64_t> const &
         std::vector<int> off(nseg + 1);
         for (uint32_t k = 0; k <= nseg; ++k)
             off[k] = static_cast<int>(offsets[u0 + k] - base);
-        d_in.ensure(m * 8);
-        d_keys.ensure(m * 8);
-        d_idx_in.ensure(m * 4);
-        d_idx.ensure(m * 4);
-        d_seg.ensure(m * 4);
-        d_off.ensure((nseg + 1) * sizeof(int));
-        d_pos.ensure(m * 8);
-        d_flag.ensure(m);
-        d_sel.ensure(m * 8);
-        d_sorted.ensure(m * 8);
-        d_out.ensure(m * 8);
-        d_nsel.ensure(8);
-        HG_CUDA(cudaMemcpyAsync(d_in.p, values + base, m * 8, cudaMemcpyHostToDevice, s));
-        HG_CUDA(cudaMemcpyAsync(d_off.p, off.data(), (nseg + 1) * sizeof(int), cudaMemcpyHostToDevice, s));
-        k_segment_index<<<std::min<uint32_t>(nseg, 65535u), 256, 0, s>>>(d_off.as<int>(), nseg, d_idx_in.as<uint32_t>(),
-                                                                       d_seg.as<uint32_t>());
+        uint64_t const slots = table_slots(m);
+        size_t select_bytes = 0;
+        HG_CUDA(cub::DeviceSelect::Flagged(nullptr, select_bytes, static_cast<uint64_t const *>(nullptr),
+                                           static_cast<unsigned char const *>(nullptr), static_cast<uint64_t *>(nullptr),
+                                           static_cast<unsigned long long *>(nullptr), m, s));
+        size_t const off_bytes = (nseg + 1) * sizeof(int), count_bytes = nseg * sizeof(unsigned long long);
+        mem.reserve({m * 8, m * 8, slots * 4, m * 4, m, off_bytes, count_bytes, 8, select_bytes});
+        uint64_t * const d_in = mem.take<uint64_t>(m * 8);
+        uint64_t * const d_out = mem.take<uint64_t>(m * 8);
+        uint32_t * const d_slots = mem.take<uint32_t>(slots * 4);
+        uint32_t * const d_entry = mem.take<uint32_t>(m * 4);
+        unsigned char * const d_flag = mem.take<unsigned char>(m);
+        int * const d_off = mem.take<int>(off_bytes);
+        auto * const d_count = mem.take<unsigned long long>(count_bytes);
+        auto * const d_nsel = mem.take<unsigned long long>(8);
+        void * const d_tmp = mem.take<char>(select_bytes);
+        HG_CUDA(cudaMemcpyAsync(d_in, values + base, m * 8, cudaMemcpyHostToDevice, s));
+        HG_CUDA(cudaMemcpyAsync(d_off, off.data(), off_bytes, cudaMemcpyHostToDevice, s));
+        HG_CUDA(cudaMemsetAsync(d_slots, 0xFF, slots * 4, s));
+        HG_CUDA(cudaMemsetAsync(d_count, 0, count_bytes, s));
+        k_distinct_enter<<<grid_for(m), 256, 0, s>>>(d_in, m, d_off, nseg, d_slots, static_cast<uint32_t>(slots - 1),
+                                                     d_entry);
         HG_CUDA(cudaGetLastError());
-        int const * begin = d_off.as<int>();
-        int const * end = d_off.as<int>() + 1;
-        size_t t1 = 0, t2 = 0, t3 = 0;
-        HG_CUDA(cub::DeviceSegmentedRadixSort::SortPairs(nullptr, t1, d_in.as<uint64_t>(), d_keys.as<uint64_t>(),
-                                                         d_idx_in.as<uint32_t>(), d_idx.as<uint32_t>(),
-                                                         static_cast<int>(m), static_cast<int>(nseg), begin, end, 0,
-                                                         64, s));
-        HG_CUDA(cub::DeviceSelect::Flagged(nullptr, t2, d_pos.as<uint64_t>(), d_flag.as<unsigned char>(),
-                                           d_sel.as<uint64_t>(), d_nsel.as<unsigned long long>(), m, s));
-        HG_CUDA(cub::DeviceRadixSort::SortKeys(nullptr, t3, d_sel.as<uint64_t>(), d_sorted.as<uint64_t>(), m, 0, 64,
-                                               s));
-        d_tmp.ensure(std::max({t1, t2, t3}));
-        HG_CUDA(cub::DeviceSegmentedRadixSort::SortPairs(d_tmp.p, t1, d_in.as<uint64_t>(), d_keys.as<uint64_t>(),
-                                                         d_idx_in.as<uint32_t>(), d_idx.as<uint32_t>(),
-                                                         static_cast<int>(m), static_cast<int>(nseg), begin, end, 0,
-                                                         64, s));
-        k_first_of_run<<<grid_for(m), 256, 0, s>>>(d_keys.as<uint64_t>(), d_idx.as<uint32_t>(), d_seg.as<uint32_t>(),
-                                                   d_off.as<int>(), m, d_pos.as<uint64_t>(),
-                                                   d_flag.as<unsigned char>());
+        k_distinct_first<<<grid_for(m), 256, 0, s>>>(d_slots, d_entry, m, d_off, nseg, d_flag, d_count);
         HG_CUDA(cudaGetLastError());
-        HG_CUDA(cub::DeviceSelect::Flagged(d_tmp.p, t2, d_pos.as<uint64_t>(), d_flag.as<unsigned char>(),
-                                           d_sel.as<uint64_t>(), d_nsel.as<unsigned long long>(), m, s));
-        unsigned long long nsel = 0;
-        HG_CUDA(cudaMemcpyAsync(&nsel, d_nsel.p, 8, cudaMemcpyDeviceToHost, s));
-        HG_CUDA(cudaStreamSynchronize(s));
         // positions ascending = user bins in order, each in first-appearance order
-        HG_CUDA(cub::DeviceRadixSort::SortKeys(d_tmp.p, t3, d_sel.as<uint64_t>(), d_sorted.as<uint64_t>(), nsel, 0, 64,
-                                               s));
-        k_gather<<<grid_for(nsel), 256, 0, s>>>(d_in.as<uint64_t>(), d_sorted.as<uint64_t>(), nsel,
-                                                d_out.as<uint64_t>());
-        HG_CUDA(cudaGetLastError());
-        std::vector<uint64_t> pos(nsel);
-        h_out.ensure(std::max<uint64_t>(nsel, 1) * 8);
-        HG_CUDA(cudaMemcpyAsync(h_out.p, d_out.p, nsel * 8, cudaMemcpyDeviceToHost, s));
-        HG_CUDA(cudaMemcpyAsync(pos.data(), d_sorted.p, nsel * 8, cudaMemcpyDeviceToHost, s));
+        HG_CUDA(cub::DeviceSelect::Flagged(d_tmp, select_bytes, static_cast<uint64_t const *>(d_in),
+                                           static_cast<unsigned char const *>(d_flag), d_out, d_nsel, m, s));
+        counts.resize(nseg);
+        HG_CUDA(cudaMemcpyAsync(counts.data(), d_count, count_bytes, cudaMemcpyDeviceToHost, s));
         HG_CUDA(cudaStreamSynchronize(s));
-        uint64_t const * dist = h_out.as<uint64_t>();
+        uint64_t total = 0;
+        for (unsigned long long c : counts)
+            total += c;
+        distinct.resize(total);
+        HG_CUDA(cudaMemcpyAsync(distinct.data(), d_out, total * 8, cudaMemcpyDeviceToHost, s));
+        HG_CUDA(cudaStreamSynchronize(s));
+        uint64_t at = 0;
         for (uint32_t k = 0; k < nseg; ++k)
         {
-            auto const a = std::lower_bound(pos.begin(), pos.end(), static_cast<uint64_t>(off[k]));
-            auto const b = std::lower_bound(pos.begin(), pos.end(), static_cast<uint64_t>(off[k + 1]));
-            sets[u0 + k].assign(dist + (a - pos.begin()), dist + (b - pos.begin()));
+            sets[u0 + k].assign(distinct.data() + at, distinct.data() + at + counts[k]);
+            at += counts[k];
         }
         u0 = u1;
     }
 }
 
-uint64_t union_size_device(std::vector<std::vector<uint64_t>> const & sets, std::vector<uint64_t> const & members)
+namespace
 {
-    uint64_t n = 0;
-    for (uint64_t u : members)
-        n += sets[u].size();
-    if (n == 0)
-        return 0;
-    cudaStream_t s = nullptr;
-    HG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
-    struct stream_guard
-    {
-        cudaStream_t s;
-        ~stream_guard()
-        {
-            cudaStreamSynchronize(s);
-            cudaStreamDestroy(s);
-        }
-    } const guard{s};
+
+// The union's size by a sort, for more values than the table's 32-bit positions name.
+uint64_t union_size_sorted(std::vector<std::vector<uint64_t>> const & sets, std::vector<uint64_t> const & members,
+                           uint64_t n, cudaStream_t s)
+{
     dbuf d_in, d_sorted, d_tmp, d_count;
     d_in.ensure(n * 8);
     d_sorted.ensure(n * 8);
@@ -237,6 +274,57 @@ uint64_t union_size_device(std::vector<std::vector<uint64_t>> const & sets, std:
     HG_CUDA(cudaGetLastError());
     unsigned long long c = 0;
     HG_CUDA(cudaMemcpyAsync(&c, d_count.p, 8, cudaMemcpyDeviceToHost, s));
+    HG_CUDA(cudaStreamSynchronize(s));
+    return c;
+}
+
+} // namespace
+
+uint64_t union_size_device(std::vector<std::vector<uint64_t>> const & sets, std::vector<uint64_t> const & members)
+{
+    uint64_t n = 0;
+    for (uint64_t u : members)
+        n += sets[u].size();
+    if (n == 0)
+        return 0;
+    cudaStream_t s = nullptr;
+    HG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
+    struct stream_guard
+    {
+        cudaStream_t s;
+        ~stream_guard()
+        {
+            cudaStreamSynchronize(s);
+            cudaStreamDestroy(s);
+        }
+    } const guard{s};
+    if (n >= (1ull << 31))
+        return union_size_sorted(sets, members, n, s);
+    arena mem;
+    uint64_t const slots = table_slots(n);
+    mem.reserve({n * 8, slots * 4, n * 4, 8, 8});
+    uint64_t * const d_in = mem.take<uint64_t>(n * 8);
+    uint32_t * const d_slots = mem.take<uint32_t>(slots * 4);
+    uint32_t * const d_entry = mem.take<uint32_t>(n * 4);
+    int * const d_off = mem.take<int>(8);
+    auto * const d_count = mem.take<unsigned long long>(8);
+    uint64_t at = 0;
+    for (uint64_t u : members)
+    {
+        if (!sets[u].empty())
+            HG_CUDA(cudaMemcpyAsync(d_in + at, sets[u].data(), sets[u].size() * 8, cudaMemcpyHostToDevice, s));
+        at += sets[u].size();
+    }
+    int const off[2] = {0, static_cast<int>(n)};
+    HG_CUDA(cudaMemcpyAsync(d_off, off, 8, cudaMemcpyHostToDevice, s));
+    HG_CUDA(cudaMemsetAsync(d_slots, 0xFF, slots * 4, s));
+    HG_CUDA(cudaMemsetAsync(d_count, 0, 8, s));
+    k_distinct_enter<<<grid_for(n), 256, 0, s>>>(d_in, n, d_off, 1, d_slots, static_cast<uint32_t>(slots - 1), d_entry);
+    HG_CUDA(cudaGetLastError());
+    k_distinct_first<<<grid_for(n), 256, 0, s>>>(d_slots, d_entry, n, d_off, 1, nullptr, d_count);
+    HG_CUDA(cudaGetLastError());
+    unsigned long long c = 0;
+    HG_CUDA(cudaMemcpyAsync(&c, d_count, 8, cudaMemcpyDeviceToHost, s));
     HG_CUDA(cudaStreamSynchronize(s));
     return c;
 }
