@@ -30,6 +30,24 @@ def test_wide_ibf_counts_and_contains(gpu_lib, oracle, bins, h):
     np.testing.assert_array_equal(g.counting_agent(1).bulk_count(q), o.bulk_count(q, 1))
 
 
+@pytest.mark.parametrize("bins", [513, 577, 960, 1024, 1025, 2048, 2100])
+@pytest.mark.parametrize("h", [1, 2])
+def test_counts_by_asynchronous_copies(gpu_lib, oracle, bins, h):
+    """Calls on both sides of the size from which rows of 9 words or more go through shared memory (200,000 pieces of 16
+    words): 9, 10, 15, 16 words, last slabs of 1, 16 and 1 words; a tail of one value and of seven."""
+    rows, slabs = 401, (bins + 1023) // 1024
+    g = hg.interleaved_bloom_filter(hg.bin_count(bins), hg.bin_size(rows), hg.hash_function_count(h))
+    o = oracle.ibf(bins, rows, h)
+    vals = S.stream_range(bins + h, 0, 60_000)
+    to = (np.arange(vals.size, dtype=np.uint64) * np.uint64(7919)) % np.uint64(bins)
+    g.emplace_many(vals, to)
+    o.emplace(vals, to)
+    edge = -(-200_000 // slabs)
+    q = np.concatenate([vals, S.stream_range(6, 0, 400_000)])
+    for n in (edge - 1, edge, edge + 7, 300_001):
+        np.testing.assert_array_equal(g.counting_agent(4).bulk_count(q[:n]), o.bulk_count(q[:n], 4, threads=8))
+
+
 def _one_ibf(oracle, user_bin, rows, h, words):
     bins = user_bin.size
     n_ub = int(user_bin[user_bin < N.BIN_DELETED].max()) + 1
