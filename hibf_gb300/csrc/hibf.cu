@@ -37,15 +37,31 @@ namespace
 
 // One launch readies a batch's workspace: the control and work counters (n_ctrl words, all 0 but the count of
 // unfinished tasks), the queries' result counts, the work queue's empty-slot marks and the levels' histograms.  (A kernel
-// and three or four memsets took about 3 us each of a batch that answers 100 queries in 40.)
+// and three or four memsets took about 3 us each of a batch that answers 100 queries in 40.)  pull.words (optional): the
+// batch's offsets and thresholds are fetched from host memory here too (two copies of 80 KB took 15 us).
+struct pull_inputs
+{
+    uint64_t const * offsets;    // host memory the device reads: words + 1 offsets
+    uint64_t const * thresholds; // and as many thresholds as words
+    uint64_t * to_offsets;
+    uint64_t * to_thresholds;
+    uint64_t words;
+};
 __global__ void k_begin(unsigned long long * __restrict__ ctrl, uint32_t n_ctrl, unsigned long long pending,
                         unsigned int * __restrict__ qcount, uint64_t nq, unsigned long long * __restrict__ tasks,
-                        uint64_t n_marks, unsigned int * __restrict__ hist, uint64_t n_hist)
+                        uint64_t n_marks, unsigned int * __restrict__ hist, uint64_t n_hist, pull_inputs pull)
 {
     uint64_t const first = blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x;
     uint64_t const stride = static_cast<uint64_t>(gridDim.x) * blockDim.x;
     if (first < n_ctrl)
         ctrl[first] = first == C_PENDING ? pending : 0ull;
+    for (uint64_t i = first; i < pull.words; i += stride)
+    {
+        pull.to_offsets[i] = pull.offsets[i];
+        pull.to_thresholds[i] = pull.thresholds[i];
+    }
+    if (first == 0 && pull.words)
+        pull.to_offsets[pull.words] = pull.offsets[pull.words];
     for (uint64_t i = first; i < nq; i += stride)
         qcount[i] = 0;
     for (uint64_t i = first; i < n_hist; i += stride)
@@ -633,6 +649,7 @@ struct hibf_gpu_agent
     // many of each query's values they staged
     uint64_t * stage_values{};
     uint32_t * stage_counts{};
+    pull_inputs pull{}; // set for the duration of a host batch whose offsets and thresholds k_begin fetches
     dbuf staged;
     // host-call staging
     dbuf in_values, in_qoff, in_thr;
@@ -825,7 +842,7 @@ void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t ma
     k_begin<<<grid_cap(most, 256, 8), 256, 0, a->stream>>>(a->ctrl.as<unsigned long long>(), ctrl_words(a->h), pending,
                                                           a->qcount.as<unsigned int>(), nq,
                                                           a->tasks.as<unsigned long long>(), marks,
-                                                          a->lvl_hist.as<unsigned int>(), n_hist);
+                                                          a->lvl_hist.as<unsigned int>(), n_hist, a->pull);
     HG_CUDA(cudaGetLastError());
 }
 
@@ -1285,20 +1302,54 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
     return small_result::kDone;
 }
 
-// The results of a finished batch, whose offsets are in h_roff, into the agent's page-locked buffers.
-void fetch_host_results(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
+// Results copied with a batch's offsets and status, before their number is known: two per query and some, at most 1 MiB
+// of ids (one wait of the host and a copy less, about 10 us of a batch of thousands of queries).
+uint64_t early_results(hibf_gpu_agent const * a, uint64_t nq)
+{
+    return std::min({2 * nq + 64, uint64_t{1} << 17, a->cap_results});
+}
+
+// The host buffers of a batch's offsets and early results; an allocation may wait for the device, so before a launch.
+void ensure_host_results(hibf_gpu_agent * a, uint64_t nq)
+{
+    a->h_roff.ensure((nq + 1) * 8);
+    a->h_ids.ensure(early_results(a, nq) * 8);
+    a->h_cnt.ensure(early_results(a, nq) * 8);
+}
+
+void copy_results(hibf_gpu_agent * a, uint64_t n, int mode, int width)
+{
+    if (!n)
+        return;
+    HG_CUDA(cudaMemcpyAsync(a->h_ids.p, a->out_ids.p, n * 8, cudaMemcpyDeviceToHost, a->stream));
+    if (mode == HIBF_GPU_QUERY_COUNT)
+        HG_CUDA(cudaMemcpyAsync(a->h_cnt.p, width == 8 ? a->out_cnt.p : a->out_cntw.p, n * width,
+                                cudaMemcpyDeviceToHost, a->stream));
+}
+
+// Offsets, early results and status of the batch on the agent's stream; waits for it.  Returns the status, and in
+// `early` how many results were copied (ensure_host_results first).
+int read_results(hibf_gpu_agent * a, uint64_t nq, int mode, int width, uint64_t & early)
+{
+    early = std::min({early_results(a, nq), a->h_ids.bytes / 8, a->h_cnt.bytes / 8});
+    HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
+    copy_results(a, early, mode, width);
+    return read_status(a);
+}
+
+// The results of a finished batch, whose offsets are in h_roff, into the agent's page-locked buffers; the first `early`
+// are there.
+void fetch_host_results(hibf_gpu_agent * a, uint64_t nq, int mode, int width, uint64_t early)
 {
     uint64_t const nr = a->h_roff.as<uint64_t>()[nq];
-    a->h_ids.ensure(nr * 8);
-    a->h_cnt.ensure(nr * 8);
-    if (nr)
+    if (nr > early)
     {
-        HG_CUDA(cudaMemcpyAsync(a->h_ids.p, a->out_ids.p, nr * 8, cudaMemcpyDeviceToHost, a->stream));
-        if (mode == HIBF_GPU_QUERY_COUNT)
-            HG_CUDA(cudaMemcpyAsync(a->h_cnt.p, width == 8 ? a->out_cnt.p : a->out_cntw.p, nr * width,
-                                    cudaMemcpyDeviceToHost, a->stream));
+        a->h_ids.ensure(nr * 8);
+        a->h_cnt.ensure(nr * 8);
+        copy_results(a, nr, mode, width);
     }
-    HG_CUDA(cudaEventRecord(a->tl_done, a->stream));
+    if (a->tl_done)
+        HG_CUDA(cudaEventRecord(a->tl_done, a->stream));
     HG_CUDA(cudaStreamSynchronize(a->stream));
     a->res_off = a->h_roff.as<uint64_t>();
     a->res_ids = a->h_ids.as<uint64_t>();
@@ -1339,14 +1390,14 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         return;
     if (small == small_result::kCounted)
     {
-        a->h_roff.ensure((nq + 1) * 8);
+        ensure_host_results(a, nq);
         ensure_timeline(a, 1);
         launch_postprocess(a, nq, mode, width);
-        HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
-        int const st = read_status(a);
+        uint64_t early = 0;
+        int const st = read_results(a, nq, mode, width, early);
         if (st != HIBF_GPU_OK)
             fail(st, "device-side failure in the last batch");
-        fetch_host_results(a, nq, mode, width);
+        fetch_host_results(a, nq, mode, width, early);
         return;
     }
     a->in_values.ensure(nv * 8); // the copy's destination, or where an in-place batch's roots stage the values
@@ -1359,6 +1410,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         {
             a->stage_values = nullptr;
             a->stage_counts = nullptr;
+            a->pull = pull_inputs{};
         }
     } const stage_guard{a};
     if (in_place)
@@ -1385,14 +1437,21 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     uint64_t tasks = std::max<uint64_t>(a->cap_tasks, nq * 4 + 1024);
     uint64_t results = std::max<uint64_t>(a->cap_results, nq * 4 + 1024);
     ensure_capacity(a, std::max<uint64_t>(nq, 1), tasks, results); // allocations synchronise: before any copy
-    a->h_roff.ensure((nq + 1) * 8);
+    ensure_host_results(a, nq);
     uint32_t const n_tl = streamed ? static_cast<uint32_t>(qb.size() - 1) : 1u;
     ensure_timeline(a, n_tl);
     a->tl_n = 0;
     HG_CUDA(cudaEventRecord(a->tl_t0, a->stream));
-    HG_CUDA(cudaMemcpyAsync(a->in_qoff.p, qoff, (nq + 1) * 8, cudaMemcpyHostToDevice, a->stream));
-    if (nq)
-        HG_CUDA(cudaMemcpyAsync(a->in_thr.p, thr, nq * 8, cudaMemcpyHostToDevice, a->stream));
+    if (!streamed && !plain && nq && host_page_tables())
+    {
+        a->pull = pull_inputs{qoff, thr, a->in_qoff.as<uint64_t>(), a->in_thr.as<uint64_t>(), nq};
+    }
+    else
+    {
+        HG_CUDA(cudaMemcpyAsync(a->in_qoff.p, qoff, (nq + 1) * 8, cudaMemcpyHostToDevice, a->stream));
+        if (nq)
+            HG_CUDA(cudaMemcpyAsync(a->in_thr.p, thr, nq * 8, cudaMemcpyHostToDevice, a->stream));
+    }
     struct arrive_reset
     {
         hibf_gpu_agent * a;
@@ -1460,6 +1519,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         a->tl_n = 1;
     }
     uint64_t const * const d_values = in_place ? in_place : a->in_values.as<uint64_t>();
+    uint64_t early = 0;
     for (int attempt = 0;; ++attempt)
     {
         ensure_capacity(a, std::max<uint64_t>(nq, 1), tasks, results);
@@ -1469,8 +1529,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
             launch_batch(a, mode, d_values, a->in_qoff.as<uint64_t>(), a->in_thr.as<uint64_t>(), nq, width);
         if (streamed && attempt == 0)
             HG_CUDA(cudaStreamWaitEvent(a->stream, a->ev_copied, 0)); // later work on the stream follows the copies
-        HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (nq + 1) * 8, cudaMemcpyDeviceToHost, a->stream));
-        int const st = read_status(a); // waits for the offsets too
+        int const st = read_results(a, nq, mode, width, early);
         if (st == HIBF_GPU_OK)
             break;
         unsigned long long const * c = a->h_ctrl.as<unsigned long long>();
@@ -1486,7 +1545,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
         if (c[C_ERROR] & E_OVERFLOW_REC)
             results = std::max<uint64_t>(results * 4, c[C_NREC] + 1024);
     }
-    fetch_host_results(a, nq, mode, width);
+    fetch_host_results(a, nq, mode, width, early);
 }
 
 // Whether the tuned kernel variants apply: at most 3 hash functions and rows of at most 4 words.
@@ -2713,23 +2772,19 @@ extern "C"
                 if (n_queries > a->cap_queries)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "more queries than the agent's last batch can hold");
                 check_mode(mode, width, nullptr, 0);
-                a->h_roff.ensure((n_queries + 1) * 8);
-                HG_CUDA(cudaMemcpyAsync(a->h_roff.p, a->roff.p, (n_queries + 1) * 8, cudaMemcpyDeviceToHost,
-                                        a->stream));
-                int const st = read_status(a); // waits for the offsets too
+                ensure_host_results(a, n_queries);
+                uint64_t early = 0;
+                int const st = read_results(a, n_queries, mode, width, early);
                 if (st != HIBF_GPU_OK)
                     fail(st, "device-side failure in the last batch");
                 uint64_t const nr = a->h_roff.as<uint64_t>()[n_queries];
-                a->h_ids.ensure(nr * 8);
-                a->h_cnt.ensure(nr * 8);
-                if (nr)
+                if (nr > early)
                 {
-                    HG_CUDA(cudaMemcpyAsync(a->h_ids.p, a->out_ids.p, nr * 8, cudaMemcpyDeviceToHost, a->stream));
-                    if (mode == HIBF_GPU_QUERY_COUNT)
-                        HG_CUDA(cudaMemcpyAsync(a->h_cnt.p, width == 8 ? a->out_cnt.p : a->out_cntw.p, nr * width,
-                                                cudaMemcpyDeviceToHost, a->stream));
+                    a->h_ids.ensure(nr * 8);
+                    a->h_cnt.ensure(nr * 8);
+                    copy_results(a, nr, mode, width);
+                    HG_CUDA(cudaStreamSynchronize(a->stream));
                 }
-                HG_CUDA(cudaStreamSynchronize(a->stream));
                 *result_offsets = a->h_roff.as<uint64_t>();
                 *result_ids = a->h_ids.as<uint64_t>();
                 if (result_counts)
