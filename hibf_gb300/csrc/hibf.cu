@@ -789,6 +789,8 @@ features_kernel_t features_kernel(hibf_gpu_hibf const * h)
     return query_kernels_of(h->hash_count).features(h->wide_rows);
 }
 
+constexpr size_t kBlkSmemMax = 48 * 1024; // counters of a 16-warp block: what a kernel may use without being told
+
 size_t query_smem(hibf_gpu_hibf const * h)
 {
     return static_cast<size_t>(8) * h->counters_per_warp * sizeof(uint32_t);
@@ -1266,7 +1268,11 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
     int const per_sm = a->tune.blocks_per_sm ? std::min<int>(fit, static_cast<int>(a->tune.blocks_per_sm)) : fit;
     unsigned const grid =
         static_cast<unsigned>(std::min<uint64_t>(static_cast<uint64_t>(sm_count()) * per_sm, blk ? nq : 1));
-    (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256, query_smem(h), s>>>(p);
+    // Long queries on a block per SM at most: 16 warps, so that a warp counts 2,000 values' share in one pass.
+    bool const wide_blocks = blk && grid <= static_cast<unsigned>(sm_count()) && nv > 512 * nq &&
+                             2 * query_smem(h) <= kBlkSmemMax;
+    (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, wide_blocks ? kBlkThreadsMax : 256,
+                                                                  query_smem(h) * (wide_blocks ? 2 : 1), s>>>(p);
     HG_CUDA(cudaGetLastError());
     bool const counts = mode == HIBF_GPU_QUERY_COUNT;
     unsigned long long * const host = a->h_small.as<unsigned long long>();

@@ -1006,8 +1006,8 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
     }
 }
 
-// Latency mode: a whole block (eight warps) works on one task.  Warp w counts its eighth of the task's values into
-// its own shared counters, the block adds the eight count arrays, warp 0 scans and emits.  A task then takes about an
+// Latency mode: a whole block (8 or 16 warps) works on one task.  Every warp counts its share of the task's values into
+// its own shared counters, the block adds the count arrays, warp 0 scans and emits.  A task then takes about an
 // eighth of the time, which shortens a batch whose tasks are fewer than the GPU's warps (the chain root -> child ->
 // grandchild of its slowest query bounds it).  No early exit: a slice's counts do not bound the task's.
 //
@@ -1018,8 +1018,10 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
 // host's memory; roots store what they read there, at the same positions, and the other tasks read it.
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
+constexpr unsigned kBlkThreadsMax = 512;
+
 template <int H, typename R>
-__global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query_blk(__grid_constant__ query_params const p)
+__global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant__ query_params const p)
 {
     extern __shared__ uint32_t s_counts[];
     __shared__ unsigned long long s_task, s_keep;

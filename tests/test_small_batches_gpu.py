@@ -116,3 +116,35 @@ def test_small_batch_outgrows_its_capacity(gpu_lib, case):
         _same(a.query_batch(*b), want)
     s = _batch(d, 9, 6)
     _same(a.query_batch(*s), _general(H, s)[0])
+
+
+@pytest.mark.parametrize("nq", [1, 5, 152, 300])
+@pytest.mark.parametrize("where", ["pageable", "pinned", "copied"])
+def test_long_queries_in_small_batches(gpu_lib, case, nq, where):
+    """Queries of hundreds to thousands of values (16 warps per block while an SM has one block at most), their values
+    read in place from ordinary or page-locked memory (the roots leave them on the device for the lower levels) or
+    copied first."""
+    import torch
+
+    d, H = case
+    rng = np.random.default_rng(nq)
+    qv, qo = d["q_values"], d["q_offsets"].astype(np.int64)
+    vals, off, thr = [], [0], []
+    for _ in range(nq):
+        i = rng.integers(0, qo.size - 1)
+        v = np.resize(qv[qo[i]:qo[i + 1]], int(rng.integers(600, 3000)))
+        vals.append(v)
+        off.append(off[-1] + v.size)
+        thr.append(int(0.7 * v.size))
+    b = (np.concatenate(vals), np.array(off, np.uint64), np.array(thr, np.uint64))
+    want, work = _general(H, b)
+    a = H.membership_agent()
+    if where == "pinned":
+        keep = torch.from_numpy(b[0].view(np.int64)).pin_memory()
+        b = (keep.numpy().view(np.uint64), b[1], b[2])
+    if where == "copied":
+        a.set_host_read(False)
+    for _ in range(3):
+        _same(a.query_batch(*b), want)
+        assert a.last_work() == work
+    assert a.last_in_place() or where != "pinned"
