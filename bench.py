@@ -771,9 +771,11 @@ def measure_hibf(args, wl, world, stream, full):
         "batched_vs_plain": value / world / plain_vps,
         "bulk_count": count, "build": build, "autotune": tune, "learned_scheduler": learned,
         "serving": serving, "parity": parity,
-        # per step: control reset, the query kernel (one launch per level, and three grouping kernels between
-        # levels, under the level schedule), six compaction kernels
-        "gpu_launches": steps * (1 + (1 if not level_ms else 1 + 4 * (len(level_ms) - 1)) + 6),
+        # per step: the workspace reset, the query kernel (one launch per level, and three grouping kernels between
+        # levels, under the level schedule), the scan of the result counts (one launch up to 65,536 queries, else
+        # three), the result scatter and the result sort
+        "gpu_launches": steps * (1 + (1 if not level_ms else 1 + 4 * (len(level_ms) - 1))
+                                 + (1 if nq <= 65536 else 3) + 2),
     }
     del agent, hibf, d_v, d_qo, d_thr, d_ub, h_v
     gc.collect()
@@ -1101,7 +1103,7 @@ def run_ibf_ours(args, rank, world, local, own_pg=True):
             "e2e": {"value": world * nq / e2e_s, "unit": "values/s", "h2d_bytes_per_step": 2 * nq * 8,
                     "d2h_bytes_per_step": w["bins"] * 2 + nq * bw * 8, "ms_per_step": e2e_s * 1e3,
                     "call": "hibf_gpu_ibf_bulk_count + hibf_gpu_ibf_bulk_contains (pinned host buffers)"},
-            "gpu_launches": 4 * args.steps,
+            "gpu_launches": 2 * args.steps,
             "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm, "unit": "GB/s", "frac": achieved / hbm,
                          "peak_kind": peak_kind,
                          # both kernels of a step, from the committed ncu capture scaled by the values

@@ -407,8 +407,8 @@ __device__ __forceinline__ void finish_counts(uint32_t const * s_counts, uint32_
 // on 64 bins, h = 5, took 70 us with four, which spill.
 // The grid's first dimension is the slab of a row wider than a warp: a block counts LPV words of every row, a warp one
 // piece of 128 or 256 bytes per value and hash function.  (Rows wider than a warp were counted one value
-// at a time, every set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms, now
-// 0.21.)  One kernel per row width: with all six in one the loop spilled 156 bytes per thread at h = 3.
+// at a time, every set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms; 0.21
+// with this kernel, 0.20 with the asynchronous one below.)  One kernel per row width: with all six in one the loop spilled 156 bytes per thread at h = 3.
 constexpr unsigned count_blocks_per_sm(int h)
 {
     return h <= 3 ? 4 : 3;
