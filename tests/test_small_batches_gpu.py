@@ -148,3 +148,14 @@ def test_long_queries_in_small_batches(gpu_lib, case, nq, where):
         _same(a.query_batch(*b), want)
         assert a.last_work() == work
     assert a.last_in_place() or where != "pinned"
+
+
+@pytest.mark.parametrize("nq,zero", [(255, (254,)), (256, (0, 255)), (257, (256,)), (512, (256, 511))])
+def test_finishing_block_has_a_thread_per_query(gpu_lib, case, nq, zero):
+    """256 threads up to 256 queries, else 1,024; more results than threads in either."""
+    d, H = case
+    b = _batch(d, nq, nq, zero)
+    a = H.membership_agent()
+    want = _general(H, b)[0]
+    for _ in range(2):
+        _same(a.query_batch(*b), want)
