@@ -15,6 +15,18 @@ namespace hibf_gb300
 {
 
 constexpr unsigned kFullMask = 0xFFFFFFFFu;
+
+// For a kernel launched beside the one before it on its stream (launch_beside): waits until that one has ended and its
+// writes are visible; no-op in an ordinary launch.
+__device__ __forceinline__ void wait_for_prerequisites()
+{
+    asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+// Lets the kernel launched beside this one become resident once every block of this one has started.
+__device__ __forceinline__ void launch_dependents()
+{
+    asm volatile("griddepcontrol.launch_dependents;");
+}
 constexpr uint32_t kSlabWords = 32; // words of a row that a warp reads at once, one per lane
 
 // Lanes per value (log2) for a row, or the last slab of a row, of `words` 64-bit words (1 to kSlabWords).

@@ -174,10 +174,12 @@ __global__ void k_level_scatter(unsigned long long const * __restrict__ tasks, u
 }
 
 // ---- exclusive scan of the per-query result counts -> result offsets (n + 1 entries) ----
-// Up to kOneBlockScan queries one block scans them in one launch (four per thread and turn); more take three launches
-// over all SMs.  One block needs about 0.7 us per 4,096 queries, the three launches 10 us before they scale.
+// Up to kOneBlockScan queries one block scans them in one launch; more take three launches over all SMs, 10 us before they
+// scale.  One block is bound by the latency of its turns (loads, two barriers, stores), so a turn takes kScanPieces
+// pieces of 4,096 counts, whose loads are in flight together.
 constexpr uint64_t kOneBlockScan = 65536;
 constexpr int kScanBlock = 1024;
+constexpr int kScanPieces = 4;
 
 __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long x, int lane)
 {
@@ -194,45 +196,65 @@ __device__ __forceinline__ unsigned long long warp_incl_scan(unsigned long long 
 __global__ void __launch_bounds__(kScanBlock) k_scan_one_block(unsigned int const * __restrict__ in, uint64_t n,
                                                               unsigned long long * __restrict__ out)
 {
-    __shared__ unsigned long long warp_sums[32];
+    __shared__ unsigned long long sums[kScanPieces][32];
+    static_assert(kScanPieces <= 32, "a warp scans the sums of a piece");
+    constexpr uint64_t piece = 4u * kScanBlock;
     int const lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    launch_dependents();
     unsigned long long carry = 0;
-    for (uint64_t base = 0; base < n; base += 4u * kScanBlock)
+    for (uint64_t base = 0; base < n; base += kScanPieces * piece)
     {
-        uint64_t const i = base + 4u * threadIdx.x;
-        uint4 v = make_uint4(0u, 0u, 0u, 0u);
-        if (i + 4 <= n)
+        uint4 v[kScanPieces];
+        unsigned long long x[kScanPieces];
+#pragma unroll
+        for (int k = 0; k < kScanPieces; ++k)
         {
-            v = *reinterpret_cast<uint4 const *>(in + i);
+            uint64_t const i = base + k * piece + 4u * threadIdx.x;
+            v[k] = make_uint4(0u, 0u, 0u, 0u);
+            if (i + 4 <= n)
+            {
+                v[k] = *reinterpret_cast<uint4 const *>(in + i);
+            }
+            else
+            {
+                if (i < n)
+                    v[k].x = in[i];
+                if (i + 1 < n)
+                    v[k].y = in[i + 1];
+                if (i + 2 < n)
+                    v[k].z = in[i + 2];
+            }
         }
-        else
+#pragma unroll
+        for (int k = 0; k < kScanPieces; ++k)
         {
+            x[k] = static_cast<unsigned long long>(v[k].x) + v[k].y + v[k].z + v[k].w;
+            if (base + k * piece < n)
+                x[k] = warp_incl_scan(x[k], lane);
+            if (lane == 31)
+                sums[k][w] = x[k];
+        }
+        __syncthreads();
+        if (w < kScanPieces)
+            sums[w][lane] = warp_incl_scan(sums[w][lane], lane);
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kScanPieces; ++k)
+        {
+            uint64_t const i = base + k * piece + 4u * threadIdx.x;
+            unsigned long long const mine = static_cast<unsigned long long>(v[k].x) + v[k].y + v[k].z + v[k].w;
+            unsigned long long const e = x[k] + carry + (w > 0 ? sums[k][w - 1] : 0ull) - mine;
             if (i < n)
-                v.x = in[i];
+                out[i] = e;
             if (i + 1 < n)
-                v.y = in[i + 1];
+                out[i + 1] = e + v[k].x;
             if (i + 2 < n)
-                v.z = in[i + 2];
+                out[i + 2] = e + v[k].x + v[k].y;
+            if (i + 3 < n)
+                out[i + 3] = e + v[k].x + v[k].y + v[k].z;
+            carry += sums[k][31];
         }
-        unsigned long long const mine = static_cast<unsigned long long>(v.x) + v.y + v.z + v.w;
-        unsigned long long x = warp_incl_scan(mine, lane);
-        if (lane == 31)
-            warp_sums[w] = x;
-        __syncthreads();
-        if (w == 0)
-            warp_sums[lane] = warp_incl_scan(warp_sums[lane], lane);
-        __syncthreads();
-        x += carry + (w > 0 ? warp_sums[w - 1] : 0ull) - mine;
-        carry += warp_sums[31];
-        if (i < n)
-            out[i] = x;
-        if (i + 1 < n)
-            out[i + 1] = x + v.x;
-        if (i + 2 < n)
-            out[i + 2] = x + v.x + v.y;
-        if (i + 3 < n)
-            out[i + 3] = x + v.x + v.y + v.z;
-        __syncthreads(); // warp_sums is rewritten
+        __syncthreads(); // sums are rewritten
     }
     if (threadIdx.x == 0)
         out[n] = carry;
@@ -308,12 +330,13 @@ __global__ void k_scan_add(unsigned long long * out, uint64_t n, unsigned long l
 }
 
 // ---- scatter records into per-query segments (each query's count runs down to 0 as its records find their places) ----
-__global__ void k_scatter(unsigned long long const * __restrict__ ctrl, uint32_t const * __restrict__ rec_q,
-                          uint32_t const * __restrict__ rec_ub, unsigned long long const * __restrict__ rec_cnt,
-                          uint64_t rec_cap, unsigned long long const * __restrict__ roff,
-                          unsigned int * __restrict__ qcount, uint64_t * __restrict__ out_ids,
-                          uint64_t * __restrict__ out_cnt)
+// (No __restrict__ on inputs that the kernels before write while this one is resident, here and in k_sort_segments.)
+__global__ void k_scatter(unsigned long long const * ctrl, uint32_t const * rec_q, uint32_t const * rec_ub,
+                          unsigned long long const * rec_cnt, uint64_t rec_cap, unsigned long long const * roff,
+                          unsigned int * qcount, uint64_t * out_ids, uint64_t * out_cnt)
 {
+    launch_dependents();
+    wait_for_prerequisites();
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
         return; // offsets describe records that were not stored; the batch reports OVERFLOW
     uint64_t n = ctrl[C_NREC];
@@ -355,14 +378,14 @@ __device__ __forceinline__ void cmp_asc(uint64_t * kid, uint64_t * kcn, uint64_t
 // the other by rank, one result per lane; the block then takes the longer ones of its warps together.  narrow (count
 // mode, width < 8): the counts in their width.  One launch for what were three (short segments, long ones, counts),
 // each about 3 us of a small batch.
-__global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * __restrict__ roff, uint64_t nq,
-                                                       uint32_t per, unsigned long long const * __restrict__ ctrl,
-                                                       uint64_t * ids, uint64_t * cnt, int width, void * narrow)
+__global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * roff, uint64_t nq, uint32_t per,
+                                                       unsigned long long const * ctrl, uint64_t * ids, uint64_t * cnt, int width, void * narrow)
 {
     __shared__ uint64_t s_ids[kSmemSegment];
     __shared__ uint64_t s_cnt[kSmemSegment];
     __shared__ uint32_t s_long[256]; // the turn's long segments, as offsets from its first query
     __shared__ uint32_t s_n_long;
+    wait_for_prerequisites();
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
         return;
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -496,7 +519,7 @@ __global__ void __launch_bounds__(1024) k_finish_small(unsigned long long * ctrl
     __shared__ uint16_t s_q[kSmallRecords];
     uint32_t const t = threadIdx.x;
     int const lane = t & 31, w = t >> 5;
-    asm volatile("griddepcontrol.wait;" ::: "memory"); // the query kernel has ended, its writes are visible
+    wait_for_prerequisites(); // the query kernel
     if (t == 0)
         host[kSmallBegan] = globaltimer_ns();
     unsigned long long const n_all = __ldcg(ctrl + C_NREC);
@@ -809,6 +832,27 @@ size_t query_smem(hibf_gpu_hibf const * h)
     return static_cast<size_t>(8) * h->counters_per_warp * sizeof(uint32_t);
 }
 
+// Launches a kernel that may become resident while the one before it on the agent's stream still runs, and then waits for
+// that one's end itself (wait_for_prerequisites): its launch costs no gap.  A kernel that calls launch_dependents lets
+// it in early.  `beside` false (in a stream capture): an ordinary launch.
+template <typename... P, typename... A>
+void launch_beside(hibf_gpu_agent * a, bool beside, void (*kernel)(P...), unsigned grid, unsigned block, A... args)
+{
+    cudaLaunchAttribute early{};
+    early.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    early.val.programmaticStreamSerializationAllowed = 1;
+    cudaLaunchConfig_t config{};
+    config.gridDim = dim3(grid);
+    config.blockDim = dim3(block);
+    config.stream = a->stream;
+    config.attrs = &early;
+    config.numAttrs = beside ? 1 : 0;
+    HG_CUDA(cudaLaunchKernelEx(&config, kernel, static_cast<P>(args)...));
+}
+
+// The placing and ordering of a batch's results.  A small batch of resident queries is a chain of short launches: 38
+// queries on 64 user bins, call to results, took 68.7 us and takes 64.5 with two of them launched beside; 8 queries on
+// 8,192 user bins 72.7 and 68.8.
 void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
 {
     cudaStream_t s = a->stream;
@@ -831,20 +875,21 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
     }
     if (!nq)
         return;
-    k_scatter<<<grid_cap(a->cap_results, 256, 8), 256, 0, s>>>(
-        a->ctrl.as<unsigned long long>(), a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(),
-        a->rec_cnt.as<unsigned long long>(), a->cap_results, a->roff.as<unsigned long long>(),
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HG_CUDA(cudaStreamIsCapturing(s, &cap));
+    bool const beside = cap == cudaStreamCaptureStatusNone;
+    launch_beside(
+        a, beside, k_scatter, grid_cap(a->cap_results, 256, 8), 256, a->ctrl.as<unsigned long long>(),
+        a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(), a->rec_cnt.as<unsigned long long>(), a->cap_results, a->roff.as<unsigned long long>(),
         a->qcount.as<unsigned int>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
-    HG_CUDA(cudaGetLastError());
     bool const narrow = mode == HIBF_GPU_QUERY_COUNT && width != 8;
     // few queries: one per warp; from a full wave of warps on, up to 32 per warp (most have no result or one)
     unsigned const sort_grid = grid_cap(nq, 8, 6);
     uint32_t const per =
         static_cast<uint32_t>(std::min<uint64_t>(32, (nq + 8ull * sort_grid - 1) / (8ull * sort_grid)));
-    k_sort_segments<<<sort_grid, 256, 0, s>>>(a->roff.as<unsigned long long>(), nq, per,
-                                              a->ctrl.as<unsigned long long>(), a->out_ids.as<uint64_t>(),
-                                              a->out_cnt.as<uint64_t>(), width, narrow ? a->out_cntw.p : nullptr);
-    HG_CUDA(cudaGetLastError());
+    launch_beside(a, beside, k_sort_segments, sort_grid, 256, a->roff.as<unsigned long long>(), nq, per,
+                  a->ctrl.as<unsigned long long>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>(), width,
+                  narrow ? a->out_cntw.p : static_cast<void *>(nullptr));
 }
 
 // Readies the workspace for a batch of nq queries (k_begin): `marks` empty-slot marks, `levels` histograms.
@@ -1289,21 +1334,13 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
     HG_CUDA(cudaGetLastError());
     bool const counts = mode == HIBF_GPU_QUERY_COUNT;
     unsigned long long * const host = a->h_small.as<unsigned long long>();
-    cudaLaunchAttribute beside{};
-    beside.id = cudaLaunchAttributeProgrammaticStreamSerialization;
-    beside.val.programmaticStreamSerializationAllowed = 1;
-    cudaLaunchConfig_t finish{};
-    finish.gridDim = dim3(1);
-    finish.blockDim = dim3(nq <= 256 ? 256 : 1024); // a thread per query
-    finish.stream = s;
-    finish.attrs = &beside;
-    finish.numAttrs = 1;
-    HG_CUDA(cudaLaunchKernelEx(
-        &finish, k_finish_small, a->ctrl.as<unsigned long long>(), a->qcount.as<unsigned int>(), static_cast<uint32_t>(nq),
+    launch_beside(
+        a, true, k_finish_small, 1, nq <= 256 ? 256 : 1024 /* a thread per query */,
+        a->ctrl.as<unsigned long long>(), a->qcount.as<unsigned int>(), static_cast<uint32_t>(nq),
         a->tasks.as<unsigned long long>(), a->cap_tasks, a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(),
         a->rec_cnt.as<unsigned long long>(), a->roff.as<unsigned long long>(), a->out_ids.as<uint64_t>(),
         a->out_cnt.as<uint64_t>(), width, counts && width != 8 ? a->out_cntw.p : static_cast<void *>(nullptr), counts,
-        host));
+        host);
     HG_CUDA(cudaStreamSynchronize(s));
     a->last_levels = 0;
     a->stamped = true;

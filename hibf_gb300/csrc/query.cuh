@@ -1029,7 +1029,7 @@ __global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant
     int const warp = threadIdx.x >> 5;
     int const nwarps = blockDim.x >> 5;
     uint32_t * counts = s_counts + warp * p.counters_per_warp;
-    asm volatile("griddepcontrol.launch_dependents;"); // a kernel launched beside this one waits for its end itself
+    launch_dependents();
     if (threadIdx.x == 0)
     {
         s_keep = kEmpty;

@@ -159,3 +159,19 @@ def test_finishing_block_has_a_thread_per_query(gpu_lib, case, nq, zero):
     want = _general(H, b)[0]
     for _ in range(2):
         _same(a.query_batch(*b), want)
+
+
+@pytest.mark.parametrize("nq", [1025, 4095, 4096, 4097, 8193, 16383, 16384, 16385, 32769, 65535, 65536, 65537])
+def test_result_offsets_of_many_queries(gpu_lib, case, nq):
+    """Offsets by the one-block scan (pieces of 4,096 counts, four to a turn) and, past 65,536 queries, the three-launch
+    one: a threshold-0 query gives every user bin, one above any possible count none."""
+    d, H = case
+    thr = np.full(nq, 65535, np.uint64)
+    for q in {0, 1, 4094, 4095, 4096, 4097, 8191, 8192, 12287, 12288, 16383, 16384, 16385, 32768, 65535, nq - 1}:
+        if q < nq:
+            thr[q] = 0
+    vals = np.random.default_rng(nq).integers(0, 1 << 63, nq, dtype=np.uint64)
+    want = np.concatenate([[0], np.cumsum(np.where(thr == 0, 600, 0))])
+    off, ids, _ = H.membership_agent().query_batch(vals, np.arange(nq + 1, dtype=np.uint64), thr)
+    np.testing.assert_array_equal(off, want)
+    np.testing.assert_array_equal(ids.reshape(-1, 600), np.tile(np.arange(600), (int(want[-1]) // 600, 1)))
