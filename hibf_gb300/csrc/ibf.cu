@@ -670,6 +670,15 @@ using namespace hibf_gb300;
 // -----------------------------------------------------------------------------------------------------------------
 // Object
 // -----------------------------------------------------------------------------------------------------------------
+// Calls on one stream run one after the other and may share their scratch; those on other streams may run at the same
+// time and have another one.
+struct count_scratch
+{
+    unsigned long long stream{}; // the stream's number, which no later stream gets
+    dbuf buf;
+};
+constexpr uint32_t kCountStreams = 16;
+
 struct hibf_gpu_ibf
 {
     uint64_t bins{};
@@ -681,8 +690,13 @@ struct hibf_gpu_ibf
     bool track_occupancy{};
     dbuf store;     // bin_size * row_words words
     dbuf occupancy; // technical_bins counters
-    dbuf totals;    // technical_bins 64-bit totals and a ticket per slab (bulk_count scratch, cleared by each call)
-    dbuf host_totals; // the same for host-pointer calls, one at a time: left at 0 by each call
+    // bulk_count's scratch, technical_bins 64-bit totals and a ticket per slab: device-pointer calls clear theirs, host-
+    // pointer calls, one at a time, leave host_totals at 0
+    std::mutex count_mu;
+    count_scratch totals[kCountStreams];
+    uint32_t n_totals{};
+    dbuf captured_totals; // of calls in a stream capture
+    dbuf host_totals;
     hbuf h_in, h_out; // small host-pointer calls: values the kernels read in place, results they write
     dbuf io;        // staging for host-pointer calls
     dbuf io2;
@@ -808,9 +822,52 @@ uint64_t count_scratch_bytes(hibf_gpu_ibf const * f)
     return count_counters(f) * sizeof(unsigned long long) + f->slabs(4) * sizeof(unsigned int);
 }
 
+// The scratch of a call on stream s; the caller holds f->count_mu until the call is in the stream.  The first
+// kCountStreams streams have one each, calls on others take and return it in the stream's order (`taken`).  A captured
+// call runs on the stream its graph is launched on, so captured calls have one for themselves, which the first call
+// outside a capture allocates (nothing can be allocated within one); graphs that hold counts on one filter must not
+// overlap.
+struct taken_scratch
+{
+    void * p{};
+    cudaStream_t s{};
+    ~taken_scratch()
+    {
+        if (p)
+            cudaFreeAsync(p, s);
+    }
+};
+unsigned long long * stream_scratch(hibf_gpu_ibf * f, cudaStream_t s, taken_scratch & taken)
+{
+    size_t const bytes = count_scratch_bytes(f);
+    cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+    HG_CUDA(cudaStreamIsCapturing(s, &capture));
+    f->captured_totals.ensure(bytes);
+    if (capture != cudaStreamCaptureStatusNone)
+        return f->captured_totals.as<unsigned long long>();
+    unsigned long long id = 0;
+    HG_CUDA(cudaStreamGetId(s, &id));
+    uint32_t k = 0;
+    while (k < f->n_totals && f->totals[k].stream != id)
+        ++k;
+    if (k == kCountStreams)
+    {
+        taken.s = s;
+        HG_CUDA(cudaMallocAsync(&taken.p, bytes, s));
+        return static_cast<unsigned long long *>(taken.p);
+    }
+    f->totals[k].buf.ensure(bytes);
+    if (k == f->n_totals)
+    {
+        f->totals[k].stream = id;
+        ++f->n_totals;
+    }
+    return f->totals[k].buf.as<unsigned long long>();
+}
+
 // bulk_count of n values into `out` (device memory, or mapped host memory).  `totals` is device scratch of
-// count_scratch_bytes(f); null means the filter's own buffer (grown on demand, the only allocation here).  `reset`: it
-// is at 0 and is left at 0.
+// count_scratch_bytes(f); null means the stream's (grown on demand, the only allocation here).  `reset`: it is at 0 and
+// is left at 0.
 void launch_count(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int width, void * out, cudaStream_t s,
                   unsigned long long * totals = nullptr, bool reset = false)
 {
@@ -819,10 +876,12 @@ void launch_count(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int wid
         HG_CUDA(cudaMemsetAsync(out, 0, f->bins * static_cast<uint64_t>(width), s));
         return;
     }
+    std::unique_lock<std::mutex> lk(f->count_mu, std::defer_lock);
+    taken_scratch taken;
     if (!totals)
     {
-        f->totals.ensure(count_scratch_bytes(f));
-        totals = f->totals.as<unsigned long long>();
+        lk.lock();
+        totals = stream_scratch(f, s, taken);
     }
     auto * const tickets = reinterpret_cast<unsigned int *>(totals + count_counters(f));
     if (uint32_t const slabs = f->slabs(4); async_count_pays(f->hash_funs, f->bin_words, n, slabs))

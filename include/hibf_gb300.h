@@ -95,7 +95,9 @@ int hibf_gpu_ibf_bulk_contains_d(hibf_gpu_ibf * ibf, uint64_t const * d_values, 
                                  void * stream);
 
 /* counting_agent_type<value_t>::bulk_count (include/hibf/interleaved_bloom_filter.hpp:652-665): one counting vector
- * of `bins` counters of `width` bytes over all n values. */
+ * of `bins` counters of `width` bytes over all n values.  Calls of the device form on several streams and threads may
+ * overlap.  In a stream capture it takes a filter on which it was called before; graphs that hold calls on one filter
+ * must not overlap. */
 int hibf_gpu_ibf_bulk_count(hibf_gpu_ibf * ibf, uint64_t const * values, uint64_t n, int width, void * out);
 int hibf_gpu_ibf_bulk_count_d(hibf_gpu_ibf * ibf, uint64_t const * d_values, uint64_t n, int width, void * d_out,
                               void * stream);
