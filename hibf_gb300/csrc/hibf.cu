@@ -16,6 +16,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <utility>
 #include <vector>
 
 #include "../../include/hibf_gb300_synthetic.h"
@@ -729,38 +730,65 @@ uint32_t ctrl_words(hibf_gpu_hibf const * h)
     return C_WORDS + kStats * (2u + h->max_depth);
 }
 
+// Grows the buffers of one capacity.  A buffer that could not be allocated is null, so the capacity is 0 until all of them
+// are there; when they cannot be had, the size before is allocated again and later batches run as before.
+template <typename Allocate>
+void grow(uint64_t & capacity, uint64_t want, Allocate const & allocate)
+{
+    if (want <= capacity)
+        return;
+    constexpr uint64_t most = 1ull << 48; // sizes in bytes stay far below 2^64
+    if (want > most)
+        fail(HIBF_GPU_ERR_OUT_OF_MEMORY, "the workspace is larger than any device's memory");
+    uint64_t const had = std::exchange(capacity, 0);
+    try
+    {
+        allocate(want);
+        capacity = want;
+    }
+    catch (...)
+    {
+        try
+        {
+            if (had)
+                allocate(had);
+            capacity = had;
+        }
+        catch (status_error const &)
+        {
+        }
+        throw;
+    }
+}
+
 void ensure_capacity(hibf_gpu_agent * a, uint64_t nq, uint64_t tasks, uint64_t results)
 {
-    if (nq > a->cap_queries)
-    {
-        a->qcount.ensure(nq * 4);
+    if (nq > a->cap_queries || tasks > a->cap_tasks)
         a->clean = false;
-        a->roff.ensure((nq + 1) * 8);
-        a->bsum.ensure(((nq + kScanBlock - 1) / kScanBlock + 1) * 8);
-        a->cap_queries = nq;
-    }
-    if (tasks > a->cap_tasks)
-    {
-        a->clean = false;
-        a->tasks.ensure(tasks * 8);
-        a->cap_tasks = tasks;
-    }
+    grow(a->cap_queries, nq,
+         [&](uint64_t n)
+         {
+             a->qcount.ensure(n * 4);
+             a->roff.ensure((n + 1) * 8);
+             a->bsum.ensure(((n + kScanBlock - 1) / kScanBlock + 1) * 8);
+         });
+    grow(a->cap_tasks, tasks, [&](uint64_t n) { a->tasks.ensure(n * 8); });
     if (a->tune.schedule == HIBF_GPU_SCHEDULE_LEVELS) // no-ops once large enough
     {
         a->lvl_tasks.ensure(a->cap_tasks * 8);
         a->lvl_hist.ensure(std::max<uint64_t>(a->h->max_depth, 1) * a->h->n_ibfs * 4); // one per level below the root
         a->lvl_count.ensure(8);
     }
-    if (results > a->cap_results)
-    {
-        a->rec_q.ensure(results * 4);
-        a->rec_ub.ensure(results * 4);
-        a->rec_cnt.ensure(results * 8);
-        a->out_ids.ensure(results * 8);
-        a->out_cnt.ensure(results * 8);
-        a->out_cntw.ensure(results * 8);
-        a->cap_results = results;
-    }
+    grow(a->cap_results, results,
+         [&](uint64_t n)
+         {
+             a->rec_q.ensure(n * 4);
+             a->rec_ub.ensure(n * 4);
+             a->rec_cnt.ensure(n * 8);
+             a->out_ids.ensure(n * 8);
+             a->out_cnt.ensure(n * 8);
+             a->out_cntw.ensure(n * 8);
+         });
 }
 
 query_params base_params(hibf_gpu_agent * a, uint64_t const * d_values, uint64_t const * d_qoff,

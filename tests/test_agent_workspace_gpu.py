@@ -1,0 +1,67 @@
+"""An agent's workspace when it cannot grow: a reserve that no device can hold is reported as OUT_OF_MEMORY, and the
+batches after it -- small and general host batches, device batches -- answer as before it."""
+
+import numpy as np
+import pytest
+
+import hibf_gb300 as hg
+from hibf_gb300 import _native as N
+from tests import golden_io as G
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def case():
+    d = G.hibf_case("synth600")
+    t = G.tables(d)
+    H = hg.hierarchical_interleaved_bloom_filter.from_tables(t["n_user_bins"], t["bins"], t["bin_size"], t["hash_funs"],
+                                                             t["next_ibf"], t["user_bin"], words=t["words"])
+    return d, H
+
+
+def _batch(d, nq):
+    """nq of the stored queries, over and over."""
+    qv, qo = d["q_values"], d["q_offsets"].astype(np.int64)
+    pick = np.arange(nq) % (qo.size - 1)
+    vals = np.concatenate([qv[qo[i]:qo[i + 1]] for i in pick])
+    return (vals, np.concatenate([[0], np.cumsum(qo[pick + 1] - qo[pick])]).astype(np.uint64),
+            np.asarray(d["mem_t"])[pick].astype(np.uint64))
+
+
+def _device(a, b):
+    import torch
+
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in b]
+    torch.cuda.synchronize()
+    a.query_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), b[1].size - 1, dev[2].data_ptr())
+    return a.fetch_results(b[1].size - 1)
+
+
+def _same(got, want):
+    np.testing.assert_array_equal(got[0], want[0])
+    np.testing.assert_array_equal(got[1], want[1])
+
+
+@pytest.mark.parametrize("schedule", [N.SCHEDULE_QUEUE, N.SCHEDULE_LEVELS])
+@pytest.mark.parametrize("queries,tasks,results", [(1 << 45, 1, 1), (1, 1 << 45, 1), (1, 1, 1 << 45), (1 << 63, 1, 1),
+                                                   (1, 1 << 61, 1), (1, 1, 1 << 62)])
+def test_batches_after_a_failed_reserve(gpu_lib, case, schedule, queries, tasks, results):
+    """2^45 entries are 140 TB and more; 2^61 and above times an entry's bytes pass 2^64."""
+    d, H = case
+    small, large = _batch(d, 40), _batch(d, 3000)
+    want_small, want_large = H.membership_agent().query_batch(*small), H.membership_agent().query_batch(*large)
+    for first in ("small", "large", "device"):
+        a = H.membership_agent()
+        a.tuning = dict(a.tuning, schedule=schedule)
+        _same(a.query_batch(*large), want_large)
+        _same(a.query_batch(*small), want_small)  # leaves the workspace as the next small batch wants it
+        with pytest.raises((N.HibfGpuError, MemoryError)) as e:
+            a.reserve(queries, 16, tasks, results)
+        assert not isinstance(e.value, hg.InvalidArgument)
+        steps = {"small": lambda: _same(a.query_batch(*small), want_small),
+                 "large": lambda: _same(a.query_batch(*large), want_large),
+                 "device": lambda: _same(_device(a, large), want_large)}
+        steps[first]()
+        for step in steps.values():
+            step()
