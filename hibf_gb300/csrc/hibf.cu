@@ -712,6 +712,7 @@ struct hibf_gpu_agent
     bool stamped{};
     uint64_t stamps[3]{};
     bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: the next one needs no k_begin
+    bool held{}; // the device buffers hold the results of the last batch (false before one, and once they have grown)
     // the last host batch's results: in h_small, or in h_roff / h_ids / h_cnt
     uint64_t const * res_off{};
     uint64_t const * res_ids{};
@@ -728,6 +729,15 @@ namespace
 uint32_t ctrl_words(hibf_gpu_hibf const * h)
 {
     return C_WORDS + kStats * (2u + h->max_depth);
+}
+
+// A captured batch holds the addresses and sizes of the workspace, the schedule, the claim order and the work array of
+// its capture: whoever changes one of them drops it, and a replay then fails.
+void drop_graph(hibf_gpu_agent * a)
+{
+    cudaGraphExec_t const graph = std::exchange(a->graph, nullptr);
+    if (graph)
+        HG_CUDA(cudaGraphExecDestroy(graph));
 }
 
 // Grows the buffers of one capacity.  A buffer that could not be allocated is null, so the capacity is 0 until all of them
@@ -765,6 +775,10 @@ void ensure_capacity(hibf_gpu_agent * a, uint64_t nq, uint64_t tasks, uint64_t r
 {
     if (nq > a->cap_queries || tasks > a->cap_tasks)
         a->clean = false;
+    if (nq > a->cap_queries || results > a->cap_results)
+        a->held = false;
+    if (nq > a->cap_queries || tasks > a->cap_tasks || results > a->cap_results)
+        drop_graph(a);
     grow(a->cap_queries, nq,
          [&](uint64_t n)
          {
@@ -925,6 +939,7 @@ void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t ma
 {
     a->clean = false;
     a->stamped = false;
+    a->held = true;
     uint64_t const n_hist = levels * a->h->n_ibfs;
     uint64_t const most = std::max({static_cast<uint64_t>(ctrl_words(a->h)), nq, marks / 2, n_hist});
     k_begin<<<grid_cap(most, 256, 8), 256, 0, a->stream>>>(a->ctrl.as<unsigned long long>(), ctrl_words(a->h), pending,
@@ -1385,6 +1400,7 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
         return small_result::kRerun;
     }
     a->clean = true;
+    a->held = true;
     a->last_level_stats.clear();
     a->last_tasks = host[C_WORDS];
     a->last_visits = host[C_WORDS + 1];
@@ -1902,15 +1918,11 @@ extern "C"
                 if (!a || !t)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
                 check_tuning(*t, a->h);
+                drop_graph(a);
                 a->tune = *t;
                 a->variant = variant_of(*t);
                 a->child_variant = child_variant_of(*t);
                 ensure_capacity(a, a->cap_queries, a->cap_tasks, a->cap_results); // level buffers, if now needed
-                if (a->graph)
-                {
-                    HG_CUDA(cudaGraphExecDestroy(a->graph));
-                    a->graph = nullptr;
-                }
             });
     }
 
@@ -1923,11 +1935,7 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
                 a->order = n_queries ? d_order : nullptr;
                 a->order_n = a->order ? n_queries : 0;
-                if (a->graph)
-                {
-                    HG_CUDA(cudaGraphExecDestroy(a->graph));
-                    a->graph = nullptr;
-                }
+                drop_graph(a);
             });
     }
 
@@ -1940,11 +1948,7 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
                 a->qwork = n_queries ? reinterpret_cast<unsigned long long *>(d_work) : nullptr;
                 a->qwork_n = a->qwork ? n_queries : 0;
-                if (a->graph)
-                {
-                    HG_CUDA(cudaGraphExecDestroy(a->graph));
-                    a->graph = nullptr;
-                }
+                drop_graph(a);
             });
     }
 
@@ -2006,11 +2010,7 @@ extern "C"
                 check_mode(mode, width, nullptr, n_queries);
                 ensure_capacity(a, n_queries, std::max<uint64_t>(a->cap_tasks, n_queries * 4 + 1024),
                                 std::max<uint64_t>(a->cap_results, n_queries * 4 + 1024));
-                if (a->graph)
-                {
-                    HG_CUDA(cudaGraphExecDestroy(a->graph));
-                    a->graph = nullptr;
-                }
+                drop_graph(a);
                 autotune_ctx c{a, mode, width, reps, d_values, d_query_offsets, d_thresholds, n_queries, {}, {}, {},
                                {}, {}, {}};
                 hibf_gpu_tuning const before = a->tune;
@@ -2864,6 +2864,8 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
                 if (n_queries > a->cap_queries)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "more queries than the agent's last batch can hold");
+                if (!a->held)
+                    fail(HIBF_GPU_ERR_INVALID_ARG, "no batch since the agent's buffers grew");
                 check_mode(mode, width, nullptr, 0);
                 ensure_host_results(a, n_queries);
                 uint64_t early = 0;
@@ -2900,12 +2902,9 @@ extern "C"
                 ensure_capacity(a, std::max<uint64_t>(n_queries, 1), std::max<uint64_t>(a->cap_tasks, 1024),
                                 std::max<uint64_t>(a->cap_results, 1024));
                 HG_CUDA(cudaStreamSynchronize(a->stream));
-                if (a->graph)
-                {
-                    HG_CUDA(cudaGraphExecDestroy(a->graph));
-                    a->graph = nullptr;
-                }
+                drop_graph(a);
                 (void)sm_count();
+                bool const held = a->held; // a capture runs nothing
                 cudaGraph_t g = nullptr;
                 HG_CUDA(cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal));
                 try
@@ -2914,11 +2913,13 @@ extern "C"
                 }
                 catch (...)
                 {
+                    a->held = held;
                     cudaStreamEndCapture(a->stream, &g);
                     if (g)
                         cudaGraphDestroy(g);
                     throw;
                 }
+                a->held = held;
                 HG_CUDA(cudaStreamEndCapture(a->stream, &g));
                 cudaError_t const e = cudaGraphInstantiate(&a->graph, g, 0);
                 cudaGraphDestroy(g);
@@ -2935,6 +2936,7 @@ extern "C"
                     fail(HIBF_GPU_ERR_INVALID_ARG, "no captured batch");
                 a->clean = false;
                 a->stamped = false;
+                a->held = true;
                 HG_CUDA(cudaGraphLaunch(a->graph, a->stream));
             });
     }

@@ -364,7 +364,9 @@ int hibf_gpu_agent_status(hibf_gpu_agent * a);
  * HIBF_GPU_ERR_TIMEOUT through the device status word.  Returns OK when it did; the context stays usable. */
 int hibf_gpu_agent_selftest_wait_limit(hibf_gpu_agent * a, double limit_ms);
 /* Captures one batch's launch sequence (control reset, persistent kernel, compaction) on fixed device buffers into
- * a CUDA graph owned by the agent; hibf_gpu_agent_replay launches it on the agent's stream. */
+ * a CUDA graph owned by the agent; hibf_gpu_agent_replay launches it on the agent's stream.  The graph holds the agent's
+ * workspace: a call that grows it (a larger reserve or batch) or changes its schedule, claim order or work array drops
+ * the graph, and replay then fails with HIBF_GPU_ERR_INVALID_ARG until the next capture. */
 int hibf_gpu_agent_capture_batch_d(hibf_gpu_agent * a, int mode, uint64_t const * d_values,
                                    uint64_t const * d_query_offsets, uint64_t n_queries, uint64_t const * d_thresholds,
                                    int width);

@@ -1,5 +1,6 @@
 """An agent's workspace when it cannot grow: a reserve that no device can hold is reported as OUT_OF_MEMORY, and the
-batches after it -- small and general host batches, device batches -- answer as before it."""
+batches after it -- small and general host batches, device batches -- answer as before it.  And when it grows: a captured
+batch and the last batch's results, which lie in the buffers before, are gone and say so."""
 
 import numpy as np
 import pytest
@@ -65,3 +66,50 @@ def test_batches_after_a_failed_reserve(gpu_lib, case, schedule, queries, tasks,
         steps[first]()
         for step in steps.values():
             step()
+
+
+@pytest.mark.parametrize("grow", ["queries", "tasks", "results", "host batch", "small batch", "device batch"])
+def test_a_captured_batch_ends_with_its_workspace(gpu_lib, case, grow):
+    import torch
+
+    d, H = case
+    b = _batch(d, 2000)
+    want = H.membership_agent().query_batch(*b)
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in b]
+    torch.cuda.synchronize()
+    nq = b[1].size - 1
+    a = H.membership_agent()
+    a.reserve(nq, 16, 20_000, int(want[0][-1]) + 1)
+    for _ in range(2):
+        with pytest.raises(hg.InvalidArgument):
+            a.fetch_results(nq)  # no batch has run
+        a.capture_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), nq, dev[2].data_ptr())
+        with pytest.raises(hg.InvalidArgument):
+            a.fetch_results(nq)  # a capture runs nothing
+        for _ in range(2):
+            a.replay()
+            _same(a.fetch_results(nq), want)
+        if grow == "host batch":
+            a.query_batch(*_batch(d, 9000))
+        elif grow == "small batch":  # 100 queries that report every user bin outgrow the results
+            s = _batch(d, 100)
+            a.query_batch(s[0], s[1], np.zeros(100, np.uint64))
+        elif grow == "device batch":  # its queries outgrow the agent's; the results it makes room for may not do
+            big = [torch.from_numpy(x.view(np.int64)).cuda() for x in _batch(d, 9000)]
+            torch.cuda.synchronize()
+            a.query_batch_device(big[0].data_ptr(), big[1].data_ptr(), 9000, big[2].data_ptr())
+            torch.cuda.synchronize()
+        else:
+            a.reserve(*[(1 << 17 if k == grow else 1) for k in ("queries", "values", "tasks", "results")])
+        with pytest.raises(hg.InvalidArgument):
+            a.replay()
+        if grow in ("queries", "results"):
+            with pytest.raises(hg.InvalidArgument):
+                a.fetch_results(nq)
+        elif grow == "tasks":  # the results stayed where they were
+            _same(a.fetch_results(nq), want)
+        a.capture_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), nq, dev[2].data_ptr())
+        a.replay()
+        _same(a.fetch_results(nq), want)
+        a = H.membership_agent()
+        a.reserve(nq, 16, 20_000, int(want[0][-1]) + 1)
