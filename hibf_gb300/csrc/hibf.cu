@@ -869,6 +869,10 @@ features_kernel_t features_kernel(hibf_gpu_hibf const * h)
 
 constexpr size_t kBlkSmemMax = 48 * 1024; // counters of a 16-warp block: what a kernel may use without being told
 
+// Shared counters of a hierarchy's query kernels at most; a wider IBF is refused.  Every kernel is given this limit: it
+// belongs to the kernel, which all hierarchies of a process share.
+constexpr size_t kQuerySmemMax = 200 * 1024;
+
 size_t query_smem(hibf_gpu_hibf const * h)
 {
     return static_cast<size_t>(8) * h->counters_per_warp * sizeof(uint32_t);
@@ -2209,7 +2213,7 @@ extern "C"
                     }
                     h->counters_per_warp = cpw;
                     h->hash_count = static_cast<uint32_t>(hash_funs[0]);
-                    if (static_cast<size_t>(8) * cpw * 4 > 200 * 1024)
+                    if (query_smem(h) > kQuerySmemMax)
                         fail(HIBF_GPU_ERR_INVALID_ARG, "an IBF is too wide for the query kernel's shared counters");
                     h->d_nodes.ensure(n_ibfs * sizeof(dev_node));
                     HG_CUDA(cudaMemcpyAsync(h->d_nodes.p, h->nodes.data(), n_ibfs * sizeof(dev_node),
@@ -2218,17 +2222,15 @@ extern "C"
                     HG_CUDA(cudaMemcpyAsync(h->d_descs.p, descs.data(), descs.size() * sizeof(uint2),
                                             cudaMemcpyHostToDevice, h->stream));
                     HG_CUDA(cudaStreamSynchronize(h->stream));
-                    size_t const smem = query_smem(h);
+                    auto raise_limit = [](auto kernel)
+                    {
+                        HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                                     static_cast<int>(kQuerySmemMax)));
+                    };
                     for (int v = 0; v < kQueryVariants; ++v)
-                        HG_CUDA(cudaFuncSetAttribute(query_kernel(h, v),
-                                                     cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                     static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
-                    HG_CUDA(cudaFuncSetAttribute(features_kernel(h),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
-                    HG_CUDA(cudaFuncSetAttribute(query_block_kernel(h),
-                                                 cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                                 static_cast<int>(std::max<size_t>(smem, 48 * 1024))));
+                        raise_limit(query_kernel(h, v));
+                    raise_limit(features_kernel(h));
+                    raise_limit(query_block_kernel(h));
                 }
                 catch (...)
                 {
