@@ -16,6 +16,7 @@
 #include <mutex>
 #include <string>
 #include <thread>
+#include <tuple>
 #include <utility>
 #include <vector>
 
@@ -657,6 +658,7 @@ struct hibf_gpu_agent
     cudaStream_t stream{};
     cudaEvent_t ev_k0{}, ev_k1{}; // around the persistent query kernel of the last batch
     cudaGraphExec_t graph{};      // captured launch sequence of one batch (hibf_gpu_agent_capture_batch_d)
+    uint32_t graph_levels{};      // its last_levels
     int status{HIBF_GPU_OK};
     uint64_t last_tasks{}, last_visits{}, last_executed{};
     uint64_t cap_queries{}, cap_tasks{}, cap_results{};
@@ -712,6 +714,10 @@ struct hibf_gpu_agent
     bool stamped{};
     uint64_t stamps[3]{};
     bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: the next one needs no k_begin
+    bool counted{true}; // the last batch's status (OK) and work counters are on the host: a small batch, or none yet
+    // the last host batch was a small one: its timeline is in `stamps`, and if its results took the general passes, their
+    // time is between tl_t0 and tl_done
+    bool tl_stamped{}, tl_passes{};
     bool held{}; // the device buffers hold the results of the last batch (false before one, and once they have grown)
     // the last host batch's results: in h_small, or in h_roff / h_ids / h_cnt
     uint64_t const * res_off{};
@@ -943,6 +949,7 @@ void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t ma
 {
     a->clean = false;
     a->stamped = false;
+    a->counted = false;
     a->held = true;
     uint64_t const n_hist = levels * a->h->n_ibfs;
     uint64_t const most = std::max({static_cast<uint64_t>(ctrl_words(a->h)), nq, marks / 2, n_hist});
@@ -1107,7 +1114,7 @@ int status_of(unsigned long long e)
 
 int read_status(hibf_gpu_agent * a)
 {
-    if (a->clean) // the last batch was a small one that succeeded: its counters are read, the device's reset
+    if (a->counted) // its counters are read, and the device's may be reset
     {
         HG_CUDA(cudaStreamSynchronize(a->stream));
         return HIBF_GPU_OK;
@@ -1351,7 +1358,7 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
         std::memcpy(hp + 2 * nq + 1, values, nv * 8);
     if (!a->clean)
         launch_begin(a, 0, a->cap_queries, a->cap_tasks, 0);
-    a->clean = false; // until k_finish_small has run
+    a->clean = a->counted = false; // until k_finish_small has run
     a->tl_n = 1;
     uint64_t const * inputs = hp;
     uint64_t const * dv = in_place ? in_place : hp + 2 * nq + 1;
@@ -1390,7 +1397,8 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
         host);
     HG_CUDA(cudaStreamSynchronize(s));
     a->last_levels = 0;
-    a->stamped = true;
+    a->stamped = a->tl_stamped = true;
+    a->tl_passes = false;
     a->stamps[0] = host[C_STAMP];
     a->stamps[1] = host[kSmallBegan];
     a->stamps[2] = host[kSmallEnded];
@@ -1403,7 +1411,7 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
                                                        : a->cap_results);
         return small_result::kRerun;
     }
-    a->clean = true;
+    a->clean = a->counted = true;
     a->held = true;
     a->last_level_stats.clear();
     a->last_tasks = host[C_WORDS];
@@ -1505,6 +1513,8 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     {
         ensure_host_results(a, nq);
         ensure_timeline(a, 1);
+        a->tl_passes = true;
+        HG_CUDA(cudaEventRecord(a->tl_t0, a->stream));
         launch_postprocess(a, nq, mode, width);
         uint64_t early = 0;
         int const st = read_results(a, nq, mode, width, early);
@@ -1554,6 +1564,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     uint32_t const n_tl = streamed ? static_cast<uint32_t>(qb.size() - 1) : 1u;
     ensure_timeline(a, n_tl);
     a->tl_n = 0;
+    a->tl_stamped = false;
     HG_CUDA(cudaEventRecord(a->tl_t0, a->stream));
     if (!streamed && !plain && nq && host_page_tables())
     {
@@ -2906,7 +2917,9 @@ extern "C"
                 HG_CUDA(cudaStreamSynchronize(a->stream));
                 drop_graph(a);
                 (void)sm_count();
-                bool const held = a->held; // a capture runs nothing
+                // a capture runs nothing: what is known of the last batch and its workspace stays
+                auto const ran = std::make_tuple(a->held, a->counted, a->clean, a->stamped, a->last_levels);
+                auto restore = [&] { std::tie(a->held, a->counted, a->clean, a->stamped, a->last_levels) = ran; };
                 cudaGraph_t g = nullptr;
                 HG_CUDA(cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal));
                 try
@@ -2915,13 +2928,14 @@ extern "C"
                 }
                 catch (...)
                 {
-                    a->held = held;
+                    restore();
                     cudaStreamEndCapture(a->stream, &g);
                     if (g)
                         cudaGraphDestroy(g);
                     throw;
                 }
-                a->held = held;
+                a->graph_levels = a->last_levels;
+                restore();
                 HG_CUDA(cudaStreamEndCapture(a->stream, &g));
                 cudaError_t const e = cudaGraphInstantiate(&a->graph, g, 0);
                 cudaGraphDestroy(g);
@@ -2936,9 +2950,9 @@ extern "C"
             {
                 if (!a || !a->graph)
                     fail(HIBF_GPU_ERR_INVALID_ARG, "no captured batch");
-                a->clean = false;
-                a->stamped = false;
+                a->clean = a->stamped = a->counted = false;
                 a->held = true;
+                a->last_levels = a->graph_levels;
                 HG_CUDA(cudaGraphLaunch(a->graph, a->stream));
             });
     }
@@ -3045,13 +3059,19 @@ extern "C"
             {
                 if (!a || !n || (cap && !out_ms))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
-                if (a->tl_n == 0 || (!a->stamped && !a->tl_t0))
+                if (a->tl_n == 0 || (!a->tl_stamped && !a->tl_t0))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "the agent has not answered a host batch");
                 *n = a->tl_n + 3;
-                if (a->stamped) // a small batch: from its kernel's start, before which its inputs were in place
+                if (a->tl_stamped) // a small batch: from its kernel's start, before which its inputs were in place
                 {
+                    float passes = 0;
+                    if (a->tl_passes)
+                    {
+                        HG_CUDA(cudaEventSynchronize(a->tl_done));
+                        HG_CUDA(cudaEventElapsedTime(&passes, a->tl_t0, a->tl_done));
+                    }
                     double const t[4] = {0.0, 0.0, static_cast<double>(a->stamps[1] - a->stamps[0]) * 1e-6,
-                                         static_cast<double>(a->stamps[2] - a->stamps[0]) * 1e-6};
+                                         static_cast<double>(a->stamps[2] - a->stamps[0]) * 1e-6 + passes};
                     std::copy_n(t, std::min<uint32_t>(cap, 4), out_ms);
                     return;
                 }

@@ -1,6 +1,7 @@
 """An agent's workspace when it cannot grow: a reserve that no device can hold is reported as OUT_OF_MEMORY, and the
 batches after it -- small and general host batches, device batches -- answer as before it.  And when it grows: a captured
-batch and the last batch's results, which lie in the buffers before, are gone and say so."""
+batch and the last batch's results, which lie in the buffers before, are gone and say so; its work counters and times
+stay, as they do when a batch is captured, which runs nothing."""
 
 import numpy as np
 import pytest
@@ -113,3 +114,76 @@ def test_a_captured_batch_ends_with_its_workspace(gpu_lib, case, grow):
         _same(a.fetch_results(nq), want)
         a = H.membership_agent()
         a.reserve(nq, 16, 20_000, int(want[0][-1]) + 1)
+
+
+@pytest.mark.parametrize("schedule", [N.SCHEDULE_QUEUE, N.SCHEDULE_LEVELS])
+def test_last_work_outlives_growth_and_captures(gpu_lib, case, schedule):
+    import torch
+
+    d, H = case
+    sizes = {"small": 40, "large": 3000}
+    b = {k: _batch(d, n) for k, n in sizes.items()}
+    dev = {k: [torch.from_numpy(x.view(np.int64)).cuda() for x in v] for k, v in b.items()}
+    torch.cuda.synchronize()
+
+    def agent():
+        a = H.membership_agent()
+        a.tuning = dict(a.tuning, schedule=schedule, block_queries=1024)
+        a.reserve(3000, 16, 20_000, 200_000)
+        return a
+
+    def seen(a):
+        return a.last_work(), a.last_work_executed(), a.level_work()
+
+    def capture(a, k):
+        a.capture_batch_device(dev[k][0].data_ptr(), dev[k][1].data_ptr(), sizes[k], dev[k][2].data_ptr())
+
+    def timed(a):
+        return a.kernel_ms(), a.level_ms(), a.last_timeline()
+
+    fresh = agent()
+    assert fresh.last_work() == (0, 0) and fresh.last_work_executed() == 0 and fresh.level_work() == []
+    fresh.status()
+    want = {}
+    for k in sizes:
+        a = agent()
+        a.query_batch(*b[k])
+        want[k] = seen(a)
+        assert want[k][0][0] >= sizes[k]
+    assert bool(want["large"][2]) == (schedule == N.SCHEDULE_LEVELS) and want["small"][2] == []
+    for k in sizes:
+        for other in sizes:
+            a = agent()
+            a.query_batch(*b[k])
+            times = timed(a)
+            a.reserve(5000, 16, 30_000, 300_000)  # before the counters were asked for
+            assert seen(a) == want[k]
+            capture(a, other)
+            assert seen(a) == want[k] and timed(a) == times
+            a.replay()
+            assert seen(a) == want[other]
+            a.query_batch(*b[k])
+            assert seen(a) == want[k]
+            a.replay()
+            a.status()
+            assert seen(a) == want[other]
+
+
+def test_timeline_is_of_the_last_host_batch(gpu_lib, case):
+    import torch
+
+    d, H = case
+    small, large = _batch(d, 40), _batch(d, 3000)
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in large]
+    torch.cuda.synchronize()
+    for many in (False, True):  # 40 queries that report all 600 user bins take the general result passes
+        a = H.membership_agent()
+        a.reserve(3000, 16, 20_000, 200_000)
+        thr = np.zeros(40, np.uint64) if many else small[2]
+        a.query_batch(*large)
+        a.query_batch(small[0], small[1], thr)
+        t = a.last_timeline()
+        assert len(t) == 4 and t[0] == t[1] == 0.0 and 0.0 < t[2] <= t[3]
+        a.query_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), 3000, dev[2].data_ptr())
+        a.status()
+        assert a.last_timeline() == t
