@@ -376,34 +376,39 @@ __device__ __forceinline__ void cmp_asc(uint64_t * kid, uint64_t * kcn, uint64_t
     }
 }
 
-// A warp takes `per` queries a turn (at most 32, one per lane): it sorts their segments of 2 to 32 results one after
-// the other by rank, one result per lane; the block then takes the longer ones of its warps together.  narrow (count
-// mode, width < 8): the counts in their width.  One launch for what were three (short segments, long ones, counts),
-// each about 3 us of a small batch.
+// A warp takes `per` neighbouring queries a turn (at most 32, one per lane) and sorts their segments of 2 to 32 results
+// one after the other by rank, one result per lane.  A longer segment takes a whole block; these are dealt out query by
+// query, gridDim.x apart, so that neighbours with many results each (reads of one sample) fall to as many blocks: 256 of
+// them among 300,000 queries, 8,100 results each, took 378 ms in the one block whose turn held them and take 2.6 ms.  (The
+// short ones dealt out like that as well cost 4 of 194 us: neighbours share cache lines.)  narrow (count mode, width <
+// 8): the counts in their width.  One launch for what were three (short segments, long ones, counts), each about 3 us of
+// a small batch.
 __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * roff, uint64_t nq, uint32_t per,
                                                        unsigned long long const * ctrl, uint64_t * ids, uint64_t * cnt, int width, void * narrow)
 {
     __shared__ uint64_t s_ids[kSmemSegment];
     __shared__ uint64_t s_cnt[kSmemSegment];
-    __shared__ uint32_t s_long[256]; // the turn's long segments, as offsets from its first query
+    __shared__ uint32_t s_long[256]; // the turn's long segments, by their number in the deal
     __shared__ uint32_t s_n_long;
     wait_for_prerequisites();
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
         return;
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-    uint64_t const turn = 8ull * per;
-    for (uint64_t base = blockIdx.x * turn; base < nq; base += gridDim.x * turn)
+    uint64_t const turn = 8ull * per * gridDim.x;
+    for (uint64_t base = 0; base < nq; base += turn)
     {
         if (threadIdx.x == 0)
             s_n_long = 0;
         __syncthreads();
         uint32_t const k = warp * per + lane;
-        bool const has = static_cast<uint32_t>(lane) < per && base + k < nq;
-        uint64_t const b = has ? roff[base + k] : 0u;
-        uint64_t const len = has ? roff[base + k + 1] - b : 0u;
-        if (len > 32)
+        bool const mine = static_cast<uint32_t>(lane) < per;
+        uint64_t const q = base + 8ull * per * blockIdx.x + k;
+        uint64_t const b = mine && q < nq ? roff[q] : 0u;
+        uint64_t const len = mine && q < nq ? roff[q + 1] - b : 0u;
+        uint64_t const dealt = base + static_cast<uint64_t>(k) * gridDim.x + blockIdx.x;
+        if (mine && dealt < nq && roff[dealt + 1] - roff[dealt] > 32)
             s_long[atomicAdd(&s_n_long, 1u)] = k;
-        else if (len == 1 && narrow)
+        if (len == 1 && narrow)
             store_count(narrow, width, b, cnt[b]);
         for (unsigned todo = __ballot_sync(kFullMask, len > 1 && len <= 32); todo; todo &= todo - 1)
         {
@@ -430,8 +435,9 @@ __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const 
         __syncthreads();
         for (uint32_t l = 0; l < s_n_long; ++l)
         {
-            uint64_t const lb = roff[base + s_long[l]];
-            uint64_t const llen = roff[base + s_long[l] + 1] - lb;
+            uint64_t const lq = base + static_cast<uint64_t>(s_long[l]) * gridDim.x + blockIdx.x;
+            uint64_t const lb = roff[lq];
+            uint64_t const llen = roff[lq + 1] - lb;
             uint64_t P = 1;
             while (P < llen)
                 P <<= 1;
@@ -935,8 +941,9 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
         a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(), a->rec_cnt.as<unsigned long long>(), a->cap_results, a->roff.as<unsigned long long>(),
         a->qcount.as<unsigned int>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
     bool const narrow = mode == HIBF_GPU_QUERY_COUNT && width != 8;
-    // few queries: one per warp; from a full wave of warps on, up to 32 per warp (most have no result or one)
-    unsigned const sort_grid = grid_cap(nq, 8, 6);
+    // few queries: one per block, which a long segment takes whole; from a full wave of warps on, up to 32 per warp (most
+    // have no result or one)
+    unsigned const sort_grid = grid_cap(nq, 1, 6);
     uint32_t const per =
         static_cast<uint32_t>(std::min<uint64_t>(32, (nq + 8ull * sort_grid - 1) / (8ull * sort_grid)));
     launch_beside(a, beside, k_sort_segments, sort_grid, 256, a->roff.as<unsigned long long>(), nq, per,
