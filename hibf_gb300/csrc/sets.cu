@@ -7,7 +7,7 @@
 //                         keeps the value's first position, the values at such positions are compacted in order;
 //   union_size_device     the distinct count of the union of some user bins' sets: the number of table entries.
 // Bound by the table's random accesses (a 4-byte slot and the value it names, both in L2 for a few million values): the
-// 64-user-bin workload, 1.47e6 values, takes 40 us of kernels; a segmented sort, a selection and a sort back took 2.1 ms,
+// 64-user-bin workload, 1.47e6 values, takes 50 us of kernels; a segmented sort, a selection and a sort back took 2.1 ms,
 // and a dozen buffers were allocated for them.
 // Only the order of split user bins' values depends on the reference's hash set (robin_hood iteration order); the
 // host replays that from the first-appearance order these produce.
@@ -45,8 +45,23 @@ __device__ __forceinline__ uint32_t segment_of(int const * __restrict__ seg_off,
     return lo;
 }
 
+// The first slot of (segment, value).  Each enters through a multiplication of its own: with the segment's number only
+// added or xored to the value's bits, user bins of dense values (short k-mers, ids) or of ranges of ids share their
+// hashes, and 1,024 bins that hold (bin << 17) + 0..2^14 took 926 probes per value.
+__device__ __forceinline__ uint32_t first_slot(uint64_t v, uint32_t segment, uint32_t mask)
+{
+    uint64_t h = v * 0x9E3779B97F4A7C15ULL;
+    h = (h ^ (h >> 32)) + segment * 0xD6E8FEB86659FD93ULL;
+    return static_cast<uint32_t>((h * 0xC2B2AE3D27D4EB4FULL) >> 32) & mask;
+}
+
 // Enters every position into the table of (segment, value): a slot holds the lowest position of its pair.  mask + 1
 // slots, a power of two and at least 1.5 per position, so a free one is always found.  entry[i]: position i's slot.
+// Bound by random accesses to slots and values.  A slot is looked at before it is claimed, and a pair's position is
+// lowered only where it is lower, so that values repeated many times read one address instead of queueing for it: 2^22
+// positions of one value 8,096 -> 137 us, of 16 values 996 -> 47.  Distinct values (us, one claim and no look before
+// -> now): 32 bins of 2^20 random ones 1,865 -> 1,624, 64 bins of 23,000 37 -> 47; 32 bins of all 22-bit values
+// 126,179 -> 10,144, (bin << 17) + 0..2^14 145,041 -> 543.
 __global__ void k_distinct_enter(uint64_t const * __restrict__ values, uint64_t n, int const * __restrict__ seg_off,
                                  uint32_t n_seg, uint32_t * slots, uint32_t mask, uint32_t * __restrict__ entry)
 {
@@ -57,17 +72,18 @@ __global__ void k_distinct_enter(uint64_t const * __restrict__ values, uint64_t 
         uint32_t const s = segment_of(seg_off, n_seg, i);
         uint32_t const b = static_cast<uint32_t>(seg_off[s]), e = static_cast<uint32_t>(seg_off[s + 1]);
         uint64_t const v = values[i];
-        uint64_t h = (v ^ (v >> 32) ^ (static_cast<uint64_t>(s) << 17)) * 0x9E3779B97F4A7C15ULL;
-        h ^= h >> 29;
-        uint32_t slot = static_cast<uint32_t>(h >> 16) & mask;
+        uint32_t slot = first_slot(v, s, mask);
         for (;;)
         {
-            uint32_t const old = atomicCAS(slots + slot, kFreeSlot, i);
+            uint32_t old = __ldcg(slots + slot);
+            if (old == kFreeSlot)
+                old = atomicCAS(slots + slot, kFreeSlot, i);
             if (old == kFreeSlot)
                 break;
             if (old >= b && old < e && values[old] == v) // a position of this segment: the same pair
             {
-                atomicMin(slots + slot, i);
+                if (i < old)
+                    atomicMin(slots + slot, i);
                 break;
             }
             slot = (slot + 1u) & mask;

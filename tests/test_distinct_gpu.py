@@ -30,3 +30,38 @@ def test_distinct_values_in_first_appearance_order(gpu_lib, seed):
     for u, v in enumerate(inputs):
         _, first = np.unique(v, return_index=True)
         np.testing.assert_array_equal(vals[int(offs[u]):int(offs[u + 1])], v[np.sort(first)], err_msg=f"user bin {u}")
+
+
+def _took(inputs):
+    """Seconds of build_inputs, the fastest of three, and its last results."""
+    import time
+
+    cfg = B.config(input_fn=lambda u, it: it.push(inputs[u]), number_of_user_bins=len(inputs))
+    layout, times = _layout(len(inputs)), []
+    for _ in range(3):
+        t = time.perf_counter()
+        got = B.build_inputs(cfg, layout)
+        times.append(time.perf_counter() - t)
+    return min(times), got
+
+
+@pytest.mark.parametrize("values", ["dense", "ranges", "one"])
+def test_dense_and_repeated_values_take_no_longer(gpu_lib, values):
+    """User bins of the same small values, of neighbouring ranges of ids and of one value each against random ones: 2^24
+    values in 4,096 bins.  Hashed alike, the ranges took a second and more on the device."""
+    rng = np.random.default_rng(3)
+    bins, n = 4096, 4096
+    random = [rng.integers(0, 1 << 64, n, dtype=np.uint64) for _ in range(bins)]
+    make = {"dense": lambda u: rng.permutation(n).astype(np.uint64) << np.uint64(14),
+            "ranges": lambda u: rng.permutation(n).astype(np.uint64) + np.uint64(u << 17),
+            "one": lambda u: np.full(n, u >> 6, np.uint64)}[values]
+    inputs = [make(u) for u in range(bins)]
+    base, _ = _took(random)
+    took, (offs, vals) = _took(inputs)
+    assert took < 2 * base + 0.1, (took, base)
+    if values == "one":
+        np.testing.assert_array_equal(offs, np.arange(bins + 1))
+        np.testing.assert_array_equal(vals, np.arange(bins) >> 6)
+    else:
+        np.testing.assert_array_equal(offs, np.arange(bins + 1) * n)
+        np.testing.assert_array_equal(vals, np.concatenate(inputs))
