@@ -6,6 +6,8 @@
 
 #include <algorithm>
 #include <cstring>
+#include <map>
+#include <memory>
 #include <mutex>
 #include <string>
 #include <vector>
@@ -670,6 +672,63 @@ using namespace hibf_gb300;
 // -----------------------------------------------------------------------------------------------------------------
 // Object
 // -----------------------------------------------------------------------------------------------------------------
+// The tables of inserts with exact occupancy, up to 122 MB each: an allocation and its release take longer than the
+// insert, so the filters of a device share what is kept, which is given back with the last of them.  Every call has a
+// buffer of its own while it runs; two are kept.  (With one kept by every filter a thousand filters held 122 GB.)
+class scratch_pool
+{
+public:
+    std::unique_ptr<dbuf> take(size_t bytes)
+    {
+        std::unique_ptr<dbuf> buf;
+        {
+            std::lock_guard<std::mutex> lk(mu_);
+            auto better = [bytes](size_t x, size_t y) // the smallest that is large enough, else the largest
+            {
+                if ((x >= bytes) != (y >= bytes))
+                    return x >= bytes;
+                return x >= bytes ? x < y : x > y;
+            };
+            auto best = kept_.begin();
+            for (auto it = kept_.begin(); it != kept_.end(); ++it)
+                if (better((*it)->bytes, (*best)->bytes))
+                    best = it;
+            if (best != kept_.end())
+            {
+                buf = std::move(*best);
+                kept_.erase(best);
+            }
+        }
+        if (!buf)
+            buf = std::make_unique<dbuf>();
+        buf->ensure(bytes);
+        return buf;
+    }
+    void give(std::unique_ptr<dbuf> buf) // nothing on the device uses it any more
+    {
+        std::lock_guard<std::mutex> lk(mu_);
+        if (kept_.size() < 2)
+            kept_.push_back(std::move(buf));
+    }
+    // The current device's.
+    static std::shared_ptr<scratch_pool> of_device()
+    {
+        static std::mutex mu;
+        static std::map<int, std::weak_ptr<scratch_pool>> pools;
+        int dev = 0;
+        HG_CUDA(cudaGetDevice(&dev));
+        std::lock_guard<std::mutex> lk(mu);
+        std::shared_ptr<scratch_pool> p = pools[dev].lock();
+        if (!p)
+            pools[dev] = p = std::make_shared<scratch_pool>();
+        return p;
+    }
+
+private:
+    std::mutex mu_;
+    std::vector<std::unique_ptr<dbuf>> kept_;
+};
+
 // Calls on one stream run one after the other and may share their scratch; those on other streams may run at the same
 // time and have another one.
 struct count_scratch
@@ -700,8 +759,8 @@ struct hibf_gpu_ibf
     hbuf h_in, h_out; // small host-pointer calls: values the kernels read in place, results they write
     dbuf io;        // staging for host-pointer calls
     dbuf io2;
-    dbuf occ_scratch; // emplace_exact's table, at most 150 MB, one call at a time
-    std::mutex occ_mu;
+    std::mutex occ_mu; // one insert with exact occupancy at a time
+    std::shared_ptr<scratch_pool> occ_pool;
     dbuf flag; // device int: an emplace saw a bin index out of range
     cudaStream_t stream{};
     int status{HIBF_GPU_OK};
@@ -755,8 +814,8 @@ cudaStream_t pick(hibf_gpu_ibf * f, void * s)
 }
 
 // Occupancy in insertion order and the bits, chunk by chunk; chunks run one after the other, so each sees the bits of the
-// chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).  The scratch belongs to the
-// filter (calls on several streams take turns).
+// chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).  Calls on several streams take
+// turns.
 template <bool SYNTH>
 void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const * d_bins, uint64_t n, uint64_t bin,
                    uint64_t seed, uint64_t vpb, cudaStream_t s)
@@ -769,8 +828,10 @@ void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const *
     while (slots < m_max + m_max / 2)
         slots *= 2;
     std::lock_guard<std::mutex> lk(f->occ_mu);
-    f->occ_scratch.ensure(slots * 12 + m_max * 4);
-    auto * const keys = f->occ_scratch.as<unsigned long long>();
+    if (!f->occ_pool)
+        f->occ_pool = scratch_pool::of_device();
+    std::unique_ptr<dbuf> scratch = f->occ_pool->take(slots * 12 + m_max * 4);
+    auto * const keys = scratch->as<unsigned long long>();
     auto * const lowest = reinterpret_cast<unsigned int *>(keys + slots);
     auto * const entries = lowest + slots;
     uint32_t const rw = static_cast<uint32_t>(f->row_words);
@@ -789,7 +850,8 @@ void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const *
             entries, f->occupancy.as<unsigned long long>(), f->flag.as<int>());
         HG_CUDA(cudaGetLastError());
     }
-    HG_CUDA(cudaStreamSynchronize(s)); // the scratch is free for the next call
+    HG_CUDA(cudaStreamSynchronize(s));
+    f->occ_pool->give(std::move(scratch));
 }
 
 void launch_emplace(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const * d_bins, uint64_t n, uint64_t bin,
