@@ -1119,6 +1119,16 @@ int status_of(unsigned long long e)
     return HIBF_GPU_OK;
 }
 
+[[noreturn]] void fail_batch(int st)
+{
+    fail(st, st == HIBF_GPU_ERR_TIMEOUT     ? "device wait limit expired" :
+             st == HIBF_GPU_ERR_CYCLE       ? "merged bins form a cycle (descent deeper than the hierarchy)" :
+             st == HIBF_GPU_ERR_INVALID_ARG ? "a claim-order entry is not a query index of the batch" :
+             st == HIBF_GPU_ERR_LOGIC       ? "a tuned kernel variant met an IBF it does not handle, or a task named a "
+                                              "query or IBF out of range" :
+                                              "batch capacity exceeded");
+}
+
 int read_status(hibf_gpu_agent * a)
 {
     if (a->counted) // its counters are read, and the device's may be reset
@@ -1330,7 +1340,7 @@ void ensure_timeline(hibf_gpu_agent * a, uint32_t n)
 
 // A host batch of at most kSmallBatch queries that runs a task per block (or is one plain query): one copy in (two when
 // the values do not fit the packed buffer), the query kernel, k_finish_small, one wait.  kRerun: not a small batch, or a
-// capacity was exceeded (now larger) or an error occurred: the general path starts over; kCounted: more results than
+// capacity was exceeded (now larger): the general path starts over; kCounted: more results than
 // k_finish_small takes, they wait in the workspace for the general passes.  One plain query of 250 values on 8,192 user
 // bins took 105 us through the general path: three waits, a dozen launches, memsets and copies.
 enum class small_result
@@ -1413,6 +1423,8 @@ small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, 
     {
         if (host[C_ERROR] == 0)
             return small_result::kCounted;
+        if (int const st = status_of(host[C_ERROR]); st != HIBF_GPU_ERR_OVERFLOW)
+            fail_batch(st); // larger buffers would not help
         ensure_capacity(a, nq, host[C_ERROR] & E_OVERFLOW_TASK ? a->cap_tasks * 4 : a->cap_tasks,
                         host[C_ERROR] & E_OVERFLOW_REC ? std::max<uint64_t>(a->cap_results * 4, host[C_NREC] + 1024)
                                                        : a->cap_results);
@@ -1665,12 +1677,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
             break;
         unsigned long long const * c = a->h_ctrl.as<unsigned long long>();
         if (st != HIBF_GPU_ERR_OVERFLOW || attempt > 8)
-            fail(st, st == HIBF_GPU_ERR_TIMEOUT     ? "device wait limit expired" :
-                     st == HIBF_GPU_ERR_CYCLE       ? "merged bins form a cycle (descent deeper than the hierarchy)" :
-                     st == HIBF_GPU_ERR_INVALID_ARG ? "a claim-order entry is not a query index of the batch" :
-                     st == HIBF_GPU_ERR_LOGIC       ? "a tuned kernel variant met an IBF it does not handle, or a "
-                                                      "task named a query or IBF out of range" :
-                                                      "batch capacity exceeded");
+            fail_batch(st);
         if (c[C_ERROR] & E_OVERFLOW_TASK)
             tasks *= 4;
         if (c[C_ERROR] & E_OVERFLOW_REC)

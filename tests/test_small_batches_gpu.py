@@ -175,3 +175,32 @@ def test_result_offsets_of_many_queries(gpu_lib, case, nq):
     off, ids, _ = H.membership_agent().query_batch(vals, np.arange(nq + 1, dtype=np.uint64), thr)
     np.testing.assert_array_equal(off, want)
     np.testing.assert_array_equal(ids.reshape(-1, 600), np.tile(np.arange(600), (int(want[-1]) // 600, 1)))
+
+
+def test_a_failed_small_batch_runs_once(gpu_lib):
+    """Two IBFs that are each other's child: the descent ends at the hierarchy's depth and reports the cycle.  The times are
+    those of the small batch (its start and its inputs at 0), not of a second run through the general path."""
+    user_bin = np.arange(128, dtype=np.uint64)
+    user_bin[[0, 64]] = N.BIN_MERGED
+    user_bin = np.where(user_bin == N.BIN_MERGED, user_bin, np.arange(128, dtype=np.uint64) - 1)
+    user_bin[65:] -= np.uint64(1)
+    next_ibf = np.concatenate([np.zeros(64, np.uint64), np.ones(64, np.uint64)])
+    next_ibf[[0, 64]] = (1, 0)
+    ones = np.full(101, ~np.uint64(0), np.uint64)
+    H = hg.hierarchical_interleaved_bloom_filter.from_tables(126, np.array([64, 64], np.uint64),
+                                                             np.array([101, 101], np.uint64),
+                                                             np.array([2, 2], np.uint64), next_ibf, user_bin,
+                                                             words=[ones, ones])
+    a = H.membership_agent()
+    b = (np.arange(30, dtype=np.uint64), np.array([0, 10, 30], np.uint64), np.array([1, 1], np.uint64))
+    for _ in range(2):
+        with pytest.raises(hg.HibfGpuError) as e:
+            a.query_batch(*b)
+        assert e.value.status == N.ERR_CYCLE
+        t = a.last_timeline()
+        assert t[0] == t[1] == 0.0 and 0.0 < t[2] <= t[3]
+        with pytest.raises(hg.HibfGpuError):
+            a.status()
+        high = (b[0], b[1], np.array([11, 21], np.uint64))  # more than a query has values: nothing to descend to
+        assert a.query_batch(*high)[1].size == 0
+        a.status()
