@@ -107,6 +107,7 @@ struct query_params
     // words at 0
     uint64_t pending_bias;
     int stamp;     // the kernel notes its start in ctrl[C_STAMP]
+    int keep;      // k_query: a worker goes on with the first child of its task
     int self_init; // single-block launch that resets its own control words first
     // early exit: after counting first + s * step percent of a task's values (s < stages), stop when no segment can
     // reach the threshold any more; tasks shorter than ee_min values are counted in one stage
@@ -846,11 +847,11 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
             process_task<H, V, R>(p, task, counts, lane, n_tasks, n_visits, n_executed, nullptr);
         }
     }
-    // With a claim order (longest query first) a worker goes on with the first child of its task instead of queueing it
-    // behind the roots: a query's work then runs in one piece, in the order given, and the batch ends with the shortest
-    // queries.  (Children behind all roots ended it with the descents of long ones: 20,000 queries of 8,192 user bins at
-    // a hundredth of their size, 0.242 ms in the learned order against 0.249 in query order.)
-    bool const chain = p.order && !p.arrived;
+    // With `keep` a worker goes on with the first child of its task instead of queueing it behind the roots: in a claim
+    // order (longest query first) a query's work then runs in one piece and the batch ends with the shortest queries.
+    // Children behind all roots end it with the descents of long ones, but leave L2 to one level at a time, so this is
+    // for hierarchies that L2 holds (keeps_first_child).
+    bool const chain = p.keep && !p.arrived;
     for (; !p.level;)
     {
         unsigned long long task = kEmpty;
