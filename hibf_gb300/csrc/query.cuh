@@ -1019,6 +1019,19 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
 // host's memory; roots store what they read there, at the same positions, and the other tasks read it.
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
+// Whether a task of n values keeps its first child: what that saves is a queue's latency, and what it costs is that other
+// blocks cannot share a long descent and that the levels do not have L2 to themselves one by one.  So long tasks keep
+// theirs only while there is a block per query, short ones also when there are several queries per block, and in between
+// those of the roots that the blocks claim first (500 queries of 1,000 values on 65,536 user bins: 100 us with all kept, 83
+// so, 90 before any was).  2,000 queries on 8,192 user bins, us with the child queued and kept: 500 values 144 / 131,
+// 1,000 216 / 221, 1,500 305 / 324, 3,000 576 / 616, 10,000 1,866 / 2,014; on 65,536: 500 values 216 / 198, 1,000 275 / 259,
+// 1,500 324 / 308, 3,000 485 / 478, 10,000 1,189 / 1,204.
+constexpr uint64_t kKeepValues = 1536;
+__device__ __forceinline__ bool keeps_child(uint64_t n, bool first, uint64_t n_queries)
+{
+    return n <= kKeepValues ? first || n_queries >= 4u * gridDim.x : n_queries <= gridDim.x;
+}
+
 constexpr unsigned kBlkThreadsMax = 512;
 
 template <int H, typename R>
@@ -1026,6 +1039,7 @@ __global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant
 {
     extern __shared__ uint32_t s_counts[];
     __shared__ unsigned long long s_task, s_keep;
+    __shared__ bool s_first; // the task at hand descends from one of the first roots claimed, a block each
     int const lane = threadIdx.x & 31;
     int const warp = threadIdx.x >> 5;
     int const nwarps = blockDim.x >> 5;
@@ -1062,6 +1076,7 @@ __global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant
             else if (task == kEmpty)
             {
                 unsigned long long const idx = atomicAdd(p.ctrl + C_HEAD, 1ull);
+                s_first = idx < gridDim.x;
                 ++claims;
                 if (idx < p.n_queries)
                 {
@@ -1141,7 +1156,8 @@ __global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant
         }
         __syncthreads();
         if (warp == 0)
-            emit_task(p, nd, s_counts, q, depth, n, n, thr, lane, n_tasks, n_visits, n_executed, &s_keep);
+            emit_task(p, nd, s_counts, q, depth, n, n, thr, lane, n_tasks, n_visits, n_executed,
+                      keeps_child(n, s_first, p.n_queries) ? &s_keep : nullptr);
         __syncthreads(); // the counters, s_task and s_keep are used by the next task
     }
     if (threadIdx.x == 0 && n_tasks)

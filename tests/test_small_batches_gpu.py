@@ -204,3 +204,32 @@ def test_a_failed_small_batch_runs_once(gpu_lib):
         high = (b[0], b[1], np.array([11, 21], np.uint64))  # more than a query has values: nothing to descend to
         assert a.query_batch(*high)[1].size == 0
         a.status()
+
+
+@pytest.mark.parametrize("nq", [60, 700, 1023, 1300, 3000])
+@pytest.mark.parametrize("n", [1535, 1536, 1537])
+def test_descents_kept_and_queued(gpu_lib, case, nq, n):
+    """Blocks that keep a task's first child or queue it (1,536 values; a block per query, several queries per block, and
+    in between), with short queries between the long ones, as host and device batches."""
+    import torch
+
+    d, H = case
+    rng = np.random.default_rng(nq + n)
+    qv, qo = d["q_values"], d["q_offsets"].astype(np.int64)
+    vals = []
+    for k in range(nq):
+        i = rng.integers(0, qo.size - 1)
+        v = qv[qo[i]:qo[i + 1]]
+        vals.append(v if k % 3 else np.resize(v, n))
+    off = np.concatenate([[0], np.cumsum([v.size for v in vals])]).astype(np.uint64)
+    b = (np.concatenate(vals), off, np.array([max(1, int(0.6 * v.size)) for v in vals], np.uint64))
+    want, work = _general(H, b)
+    a = H.membership_agent()
+    dev = [torch.from_numpy(x.view(np.int64)).cuda() for x in b]
+    torch.cuda.synchronize()
+    a.reserve(nq, 16, nq * 16 + 4096, nq * 64 + 4096)
+    for _ in range(2):
+        _same(a.query_batch(*b), want)
+        assert a.last_work() == work
+        a.query_batch_device(dev[0].data_ptr(), dev[1].data_ptr(), nq, dev[2].data_ptr())
+        _same(a.fetch_results(nq), want)
