@@ -1320,6 +1320,12 @@ std::vector<uint64_t> const & traversal_rank(hibf_gpu_hibf * h)
     return h->trav_rank;
 }
 
+// Whether the device can read these words where they are: its loads need their alignment, which the host's copies do not.
+bool aligned(uint64_t const * p)
+{
+    return reinterpret_cast<uintptr_t>(p) % alignof(uint64_t) == 0;
+}
+
 // Whether the device reads pageable host memory through the host's page tables (Grace hosts).
 bool host_page_tables()
 {
@@ -1517,9 +1523,10 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     // In place: values in mapped page-locked memory are read by the kernel over the host link as it needs them, so
     // no copy precedes (or paces) the launch; only the offsets and thresholds are copied.  So are pageable values too
     // few to be streamed where the GPU goes through the host's page tables: 20 MB on the 64-bin workload, 10,000
-    // queries, took 138 us to copy before a kernel of 65, in place the kernel takes 165.
+    // queries, took 138 us to copy before a kernel of 65, in place the kernel takes 165.  Values that do not start at a
+    // multiple of eight bytes (a view into a file's buffer) are copied.
     uint64_t const * in_place = nullptr;
-    if (a->host_read && !plain && nv)
+    if (a->host_read && !plain && nv && aligned(values))
     {
         cudaPointerAttributes attr{};
         void * dev = nullptr;
@@ -1598,7 +1605,7 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
     a->tl_n = 0;
     a->tl_stamped = false;
     HG_CUDA(cudaEventRecord(a->tl_t0, a->stream));
-    if (!streamed && !plain && nq && host_page_tables())
+    if (!streamed && !plain && nq && aligned(qoff) && aligned(thr) && host_page_tables())
     {
         a->pull = pull_inputs{qoff, thr, a->in_qoff.as<uint64_t>(), a->in_thr.as<uint64_t>(), nq};
     }
