@@ -332,8 +332,9 @@ __global__ void k_scan_add(unsigned long long * out, uint64_t n, unsigned long l
 }
 
 // ---- scatter records into per-query segments (each query's count runs down to 0 as its records find their places) ----
+constexpr uint32_t kWarpSegment = 32; // results of a query that one warp sorts, one per lane
 // (No __restrict__ on inputs that the kernels before write while this one is resident, here and in k_sort_segments.)
-__global__ void k_scatter(unsigned long long const * ctrl, uint32_t const * rec_q, uint32_t const * rec_ub,
+__global__ void k_scatter(unsigned long long * ctrl, uint32_t const * rec_q, uint32_t const * rec_ub,
                           unsigned long long const * rec_cnt, uint64_t rec_cap, unsigned long long const * roff,
                           unsigned int * qcount, uint64_t * out_ids, uint64_t * out_cnt)
 {
@@ -348,7 +349,10 @@ __global__ void k_scatter(unsigned long long const * ctrl, uint32_t const * rec_
          r += static_cast<uint64_t>(gridDim.x) * blockDim.x)
     {
         uint32_t const q = rec_q[r];
-        uint64_t const pos = roff[q] + (atomicSub(qcount + q, 1u) - 1u);
+        uint32_t const left = atomicSub(qcount + q, 1u);
+        if (left > kWarpSegment)
+            ctrl[C_LONG] = 1;
+        uint64_t const pos = roff[q] + (left - 1u);
         out_ids[pos] = rec_ub[r];
         out_cnt[pos] = rec_cnt[r];
     }
@@ -380,7 +384,8 @@ __device__ __forceinline__ void cmp_asc(uint64_t * kid, uint64_t * kcn, uint64_t
 // one after the other by rank, one result per lane.  A longer segment takes a whole block; these are dealt out query by
 // query, gridDim.x apart, so that neighbours with many results each (reads of one sample) fall to as many blocks: 256 of
 // them among 300,000 queries, 8,100 results each, took 378 ms in the one block whose turn held them and take 2.6 ms.  (The
-// short ones dealt out like that as well cost 4 of 194 us: neighbours share cache lines.)  narrow (count mode, width <
+// short ones dealt out like that as well cost 4 of 194 us: neighbours share cache lines; and looking for long ones where
+// there are none 13 us of a million queries' 20, hence C_LONG.)  narrow (count mode, width <
 // 8): the counts in their width.  One launch for what were three (short segments, long ones, counts), each about 3 us of
 // a small batch.
 __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * roff, uint64_t nq, uint32_t per,
@@ -393,6 +398,7 @@ __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const 
     wait_for_prerequisites();
     if (ctrl[C_ERROR] & (E_OVERFLOW_REC | E_OVERFLOW_TASK))
         return;
+    bool const any_long = ctrl[C_LONG] != 0;
     int const lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
     uint64_t const turn = 8ull * per * gridDim.x;
     for (uint64_t base = 0; base < nq; base += turn)
@@ -406,11 +412,11 @@ __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const 
         uint64_t const b = mine && q < nq ? roff[q] : 0u;
         uint64_t const len = mine && q < nq ? roff[q + 1] - b : 0u;
         uint64_t const dealt = base + static_cast<uint64_t>(k) * gridDim.x + blockIdx.x;
-        if (mine && dealt < nq && roff[dealt + 1] - roff[dealt] > 32)
+        if (any_long && mine && dealt < nq && roff[dealt + 1] - roff[dealt] > kWarpSegment)
             s_long[atomicAdd(&s_n_long, 1u)] = k;
         if (len == 1 && narrow)
             store_count(narrow, width, b, cnt[b]);
-        for (unsigned todo = __ballot_sync(kFullMask, len > 1 && len <= 32); todo; todo &= todo - 1)
+        for (unsigned todo = __ballot_sync(kFullMask, len > 1 && len <= kWarpSegment); todo; todo &= todo - 1)
         {
             int const src = __ffs(todo) - 1;
             uint64_t const sb = __shfl_sync(kFullMask, b, src);

@@ -53,6 +53,7 @@ enum : int
     C_ERROR = 4,
     C_STAMP = 5, // when the query kernel began (query_params::stamp), on the GPU's clock
     C_CHILD = 6, // streamed inputs: claims of child slots (roots and children are then claimed separately)
+    C_LONG = 7,  // some query has more than 32 results (k_scatter)
     C_WORDS = 8
 };
 // error bits
