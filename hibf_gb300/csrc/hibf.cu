@@ -671,6 +671,9 @@ struct hibf_gpu_agent
     cudaEvent_t ev_k0{}, ev_k1{}; // around the persistent query kernel of the last batch
     cudaGraphExec_t graph{};      // captured launch sequence of one batch (hibf_gpu_agent_capture_batch_d)
     uint32_t graph_levels{};      // its last_levels
+    bool capturing{};             // hibf_gpu_agent_capture_batch_d is at work
+    // a batch was captured by its caller, who may replay it at any time: nothing is known of the workspace from then on
+    bool caller_replays{};
     int status{HIBF_GPU_OK};
     uint64_t last_tasks{}, last_visits{}, last_executed{};
     uint64_t cap_queries{}, cap_tasks{}, cap_results{};
@@ -960,6 +963,10 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
 // Readies the workspace for a batch of nq queries (k_begin): `marks` empty-slot marks, `levels` histograms.
 void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t marks, uint64_t levels)
 {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    HG_CUDA(cudaStreamIsCapturing(a->stream, &cap));
+    if (cap != cudaStreamCaptureStatusNone && !a->capturing)
+        a->caller_replays = true;
     a->clean = false;
     a->stamped = false;
     a->counted = false;
@@ -1377,7 +1384,8 @@ enum class small_result
 small_result small_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t const * qoff, uint64_t nq,
                          uint64_t const * thr, int width, bool plain, uint64_t const * in_place)
 {
-    if (nq == 0 || nq > kSmallBatch || (!plain && nq > a->tune.block_queries) || a->order || a->qwork)
+    if (nq == 0 || nq > kSmallBatch || (!plain && nq > a->tune.block_queries) || a->order || a->qwork ||
+        a->caller_replays)
         return small_result::kRerun;
     hibf_gpu_hibf * h = a->h;
     cudaStream_t s = a->stream;
@@ -2959,9 +2967,14 @@ extern "C"
                 (void)sm_count();
                 // a capture runs nothing: what is known of the last batch and its workspace stays
                 auto const ran = std::make_tuple(a->held, a->counted, a->clean, a->stamped, a->last_levels);
-                auto restore = [&] { std::tie(a->held, a->counted, a->clean, a->stamped, a->last_levels) = ran; };
+                auto restore = [&]
+                {
+                    a->capturing = false;
+                    std::tie(a->held, a->counted, a->clean, a->stamped, a->last_levels) = ran;
+                };
                 cudaGraph_t g = nullptr;
                 HG_CUDA(cudaStreamBeginCapture(a->stream, cudaStreamCaptureModeThreadLocal));
+                a->capturing = true;
                 try
                 {
                     launch_batch(a, mode, d_values, d_query_offsets, d_thresholds, n_queries, width);

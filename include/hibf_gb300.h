@@ -345,7 +345,9 @@ int hibf_gpu_agent_query_batch(hibf_gpu_agent * a, int mode, uint64_t const * va
                                int width, uint64_t const ** result_offsets, uint64_t const ** result_ids,
                                void const ** result_counts);
 /* Device form: inputs already in HBM; results stay in the agent's device buffers (returned as device pointers).
- * Asynchronous on the agent's stream; hibf_gpu_agent_status() after synchronising gives OVERFLOW / TIMEOUT. */
+ * Asynchronous on the agent's stream; hibf_gpu_agent_status() after synchronising gives OVERFLOW / TIMEOUT.  A caller may
+ * capture it into a graph of its own and replay that between the agent's other calls; such a graph holds the workspace's
+ * addresses, so the agent must have room for its largest batch (hibf_gpu_agent_reserve) before the capture. */
 int hibf_gpu_agent_query_batch_d(hibf_gpu_agent * a, int mode, uint64_t const * d_values,
                                  uint64_t const * d_query_offsets, uint64_t n_queries, uint64_t const * d_thresholds,
                                  int width, uint64_t const ** d_result_offsets, uint64_t const ** d_result_ids,
