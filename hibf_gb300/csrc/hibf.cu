@@ -1333,12 +1333,6 @@ std::vector<uint64_t> const & traversal_rank(hibf_gpu_hibf * h)
     return h->trav_rank;
 }
 
-// Whether the device can read these words where they are: its loads need their alignment, which the host's copies do not.
-bool aligned(uint64_t const * p)
-{
-    return reinterpret_cast<uintptr_t>(p) % alignof(uint64_t) == 0;
-}
-
 // Whether the device reads pageable host memory through the host's page tables (Grace hosts).
 bool host_page_tables()
 {

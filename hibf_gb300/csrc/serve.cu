@@ -196,7 +196,7 @@ std::vector<request *> run_batch(hibf_gpu_server * S, slot & sl)
     for (size_t k = 0; zc && k < sl.reqs.size(); ++k)
     {
         request const * r = sl.reqs[k];
-        zc = r->pinned && r->dev_values &&
+        zc = r->pinned && r->dev_values && aligned(r->dev_values) &&
              (k == 0 || (r->values == sl.reqs[k - 1]->values + sl.reqs[k - 1]->nv &&
                          r->dev_values == sl.reqs[k - 1]->dev_values + sl.reqs[k - 1]->nv));
     }

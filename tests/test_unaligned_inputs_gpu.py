@@ -1,6 +1,7 @@
 """Host batches whose arrays do not start at a multiple of eight bytes (views into a buffer that was read from a file), in
 ordinary and page-locked memory, at sizes where aligned ones are packed, read in place, and fetched by the first kernel:
-they are copied, and answer like aligned ones.  The single-level filter's host calls copy theirs as well."""
+they are copied, and answer like aligned ones.  The single-level filter's host calls copy theirs as well, and the server
+copies the values of requests that lie like that in a registered range."""
 
 import numpy as np
 import pytest
@@ -72,3 +73,33 @@ def test_unaligned_ibf_calls(gpu_lib, n):
     np.testing.assert_array_equal(g.membership_agent().membership_for(u, 3), f.membership_agent().membership_for(v, 3))
     np.testing.assert_array_equal(g.containment_agent().bulk_contains_words(u),
                                   f.containment_agent().bulk_contains_words(v))
+
+
+def test_unaligned_served_requests(gpu_lib):
+    import torch
+
+    from hibf_gb300.serve import server
+
+    d = G.hibf_case("synth600")
+    t = G.tables(d)
+    H = hg.hierarchical_interleaved_bloom_filter.from_tables(t["n_user_bins"], t["bins"], t["bin_size"], t["hash_funs"],
+                                                             t["next_ibf"], t["user_bin"], words=t["words"])
+    agent = H.membership_agent()
+    qv, qo, thr = d["q_values"], d["q_offsets"].astype(np.int64), np.asarray(d["mem_t"]).astype(np.uint64)
+    raw = torch.empty(qv.nbytes + 16, dtype=torch.uint8, pin_memory=True).numpy()
+    for shift in (0, 4):
+        start = -raw.ctypes.data % 8 + shift
+        raw[start:start + qv.nbytes] = qv.view(np.uint8)
+        base = raw.ctypes.data + start
+        srv = server(H, slots=1, max_batch_queries=4096, max_batch_values=1 << 20, admission_bytes=1 << 30)
+        srv.register_host(raw.ctypes.data, raw.nbytes, already_pinned=True)
+        reqs = [(qo[k], (qo[k:k + 8] - qo[k]).astype(np.uint64), thr[k:k + 7].copy()) for k in range(0, qo.size - 8, 7)]
+        ids = [srv.submit_borrowed(base + 8 * int(first), o, th) for first, o, th in reqs]
+        for rid, (first, o, th) in zip(ids, reqs):
+            st, offs, res, _ = srv.wait_result(rid, 7)
+            want = agent.query_batch(qv[first:first + int(o[-1])], o, th)
+            assert st == 0
+            np.testing.assert_array_equal(offs, want[0])
+            np.testing.assert_array_equal(res, want[1])
+        assert bool(srv.batch_log()[:, 11].any()) == (shift == 0)  # the aligned ones ran zero copy
+        srv.close()
