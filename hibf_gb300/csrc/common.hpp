@@ -86,7 +86,8 @@ inline uint64_t padded_row_words(uint64_t bin_words)
     return (bin_words + 3) / 4 * 4;
 }
 
-// Whether the device can read a caller's words where they are: its loads need their alignment, the host's copies do not.
+// Whether the device can read a caller's words where they are: its loads need their alignment, the host's copies do
+// not.
 inline bool aligned(uint64_t const * p)
 {
     return reinterpret_cast<uintptr_t>(p) % alignof(uint64_t) == 0;

@@ -6,8 +6,8 @@
 // Work mapping.  A row of bin_words 64-bit words is read by LPV = next_pow2(bin_words) lanes (capped at 32), lane
 // j of a group reading word j, so a row is one coalesced access of ceil(bytes/32) sectors.  Each lane first hashes
 // a different value (32 values per warp per pass), then the groups take turns on those values, receiving the row
-// indices (of type R) by shuffle.  Each lane accumulates its word's 64 bins in K bit-sliced planes (planes_add4) and flushes
-// them through a warp transpose into 32-bit counters in shared memory before they can overflow (2^K - 1 masks).
+// indices (of type R) by shuffle.  Each lane accumulates its word's 64 bins in K bit-sliced planes (planes_add4) and
+// flushes them through a warp transpose into 32-bit counters in shared memory before they can overflow (2^K - 1 masks).
 // Counts are exact; the caller reduces them modulo the counter width, which equals the reference's wraparound.
 #pragma once
 
@@ -23,7 +23,6 @@ struct row_params
     uint32_t row_words;
     uint32_t bin_words;
     uint32_t hash_shift;
-    uint32_t hash_funs;
 };
 
 // `added` (warp-uniform) masks went into the planes since the last flush, so planes k with 2^k > added are zero and
@@ -102,9 +101,9 @@ __device__ __forceinline__ void load_row_words(uint64_t const * p, uint64_t (&w)
 // loads must not come from a non-coherent cache.  Each task reads its values once, so L1 gives them nothing.
 //
 // One warp counts vals[0, n) into counts[0, 64 * LPV * W) with H hash functions.  A row is read by LPV lanes, each
-// loading W consecutive words (W = 2: one 16-byte load; the row stride must then be even).  Each lane hashes U values per pass and keeps their H row indices; the row words of
-// GS = 4 * UM masks per lane are loaded together, so GS * H * W loads per lane are in flight.  K planes count up to
-// 2^K - 1 masks between flushes.
+// loading W consecutive words (W = 2: one 16-byte load; the row stride must then be even).  Each lane hashes U values
+// per pass and keeps their H row indices; the row words of GS = 4 * UM masks per lane are loaded together, so GS * H *
+// W loads per lane are in flight.  K planes count up to 2^K - 1 masks between flushes.
 //
 // stage (optional): every value read is also stored at stage[i], so that later reads of the same values (the lower
 // levels of an in-place host batch) come from device memory instead of the host link.
@@ -241,8 +240,8 @@ __device__ __forceinline__ void warp_count(row_params const & rp, uint64_t const
     }
 }
 
-// Rows wider than a warp (more than kSlabWords words) are counted in slabs of as many words as lanes read them; the last
-// slab may have fewer.
+// Rows wider than a warp (more than kSlabWords words) are counted in slabs of as many words as lanes read them; the
+// last slab may have fewer.
 __device__ __forceinline__ row_params row_slab(row_params const & rp, uint32_t first_word, uint32_t slab_words)
 {
     row_params sp = rp;

@@ -38,9 +38,10 @@ namespace
 
 
 // One launch readies a batch's workspace: the control and work counters (n_ctrl words, all 0 but the count of
-// unfinished tasks), the queries' result counts, the work queue's empty-slot marks and the levels' histograms.  (A kernel
-// and three or four memsets took about 3 us each of a batch that answers 100 queries in 40.)  pull.words (optional): the
-// batch's offsets and thresholds are fetched from host memory here too (two copies of 80 KB took 15 us).
+// unfinished tasks), the queries' result counts, the work queue's empty-slot marks and the levels' histograms.  (A
+// kernel and three or four memsets took about 3 us each of a batch that answers 100 queries in 40.)  pull.words
+// (optional): the batch's offsets and thresholds are fetched from host memory here too (two copies of 80 KB took 15
+// us).
 struct pull_inputs
 {
     uint64_t const * offsets;    // host memory the device reads: words + 1 offsets
@@ -176,9 +177,9 @@ __global__ void k_level_scatter(unsigned long long const * __restrict__ tasks, u
 }
 
 // ---- exclusive scan of the per-query result counts -> result offsets (n + 1 entries) ----
-// Up to kOneBlockScan queries one block scans them in one launch; more take three launches over all SMs, 10 us before they
-// scale.  One block is bound by the latency of its turns (loads, two barriers, stores), so a turn takes kScanPieces
-// pieces of 4,096 counts, whose loads are in flight together.
+// Up to kOneBlockScan queries one block scans them in one launch; more take three launches over all SMs, 10 us before
+// they scale.  One block is bound by the latency of its turns (loads, two barriers, stores), so a turn takes
+// kScanPieces pieces of 4,096 counts, whose loads are in flight together.
 constexpr uint64_t kOneBlockScan = 65536;
 constexpr int kScanBlock = 1024;
 constexpr int kScanPieces = 4;
@@ -331,7 +332,7 @@ __global__ void k_scan_add(unsigned long long * out, uint64_t n, unsigned long l
         out[n] = sums[nb];
 }
 
-// ---- scatter records into per-query segments (each query's count runs down to 0 as its records find their places) ----
+// ---- scatter records into per-query segments (a query's count runs down to 0 as its records find their places) ----
 constexpr uint32_t kWarpSegment = 32; // results of a query that one warp sorts, one per lane
 // (No __restrict__ on inputs that the kernels before write while this one is resident, here and in k_sort_segments.)
 __global__ void k_scatter(unsigned long long * ctrl, uint32_t const * rec_q, uint32_t const * rec_ub,
@@ -382,14 +383,15 @@ __device__ __forceinline__ void cmp_asc(uint64_t * kid, uint64_t * kcn, uint64_t
 
 // A warp takes `per` neighbouring queries a turn (at most 32, one per lane) and sorts their segments of 2 to 32 results
 // one after the other by rank, one result per lane.  A longer segment takes a whole block; these are dealt out query by
-// query, gridDim.x apart, so that neighbours with many results each (reads of one sample) fall to as many blocks: 256 of
-// them among 300,000 queries, 8,100 results each, took 378 ms in the one block whose turn held them and take 2.6 ms.  (The
-// short ones dealt out like that as well cost 4 of 194 us: neighbours share cache lines; and looking for long ones where
-// there are none 13 us of a million queries' 20, hence C_LONG.)  narrow (count mode, width <
-// 8): the counts in their width.  One launch for what were three (short segments, long ones, counts), each about 3 us of
-// a small batch.
+// query, gridDim.x apart, so that neighbours with many results each (reads of one sample) fall to as many blocks: 256
+// of them among 300,000 queries, 8,100 results each, took 378 ms in the one block whose turn held them and take 2.6 ms.
+// (The short ones dealt out like that as well cost 4 of 194 us: neighbours share cache lines; and looking for long ones
+// where there are none took 13 of 20 us at a million queries, hence C_LONG.)  narrow (count mode, width <
+// 8): the counts in their width.  One launch for what were three (short segments, long ones, counts), each about 3 us
+// of a small batch.
 __global__ void __launch_bounds__(256) k_sort_segments(unsigned long long const * roff, uint64_t nq, uint32_t per,
-                                                       unsigned long long const * ctrl, uint64_t * ids, uint64_t * cnt, int width, void * narrow)
+                                                       unsigned long long const * ctrl, uint64_t * ids,
+                                                       uint64_t * cnt, int width, void * narrow)
 {
     __shared__ uint64_t s_ids[kSmemSegment];
     __shared__ uint64_t s_cnt[kSmemSegment];
@@ -515,9 +517,9 @@ constexpr uint32_t kSmallWords = kSmallCounts + kSmallRecords;
 // leaves the workspace as the next batch wants it (control words, counts and used task slots reset), so that nothing
 // precedes the next query kernel.  Bound by latency: one block, a handful of dependent steps, about 4 us, for seven
 // launches and three copies before (17 us of kernels alone).  So everything it reads is asked for at once, the first
-// record of each thread (the record arrays hold more than 1,024) before their number is known; and it is launched beside
-// the query kernel, which it waits for here: no launch gap.  (One query of 250 values on 8,192 user bins, call to return:
-// 35.5 -> 32.7 us; 100 queries 59.7 -> 56.8.)  Its inputs change while it is resident, hence __ldcg.
+// record of each thread (the record arrays hold more than 1,024) before their number is known; and it is launched
+// beside the query kernel, which it waits for here: no launch gap.  (One query of 250 values on 8,192 user bins, call
+// to return: 35.5 -> 32.7 us; 100 queries 59.7 -> 56.8.)  Its inputs change while it is resident, hence __ldcg.
 __global__ void __launch_bounds__(1024) k_finish_small(unsigned long long * ctrl, unsigned int * qcount, uint32_t nq,
                                                        unsigned long long * tasks, uint64_t task_cap,
                                                        uint32_t const * rec_q, uint32_t const * rec_ub,
@@ -728,10 +730,10 @@ struct hibf_gpu_agent
     // batches record no events (each costs the stream about 1.8 us)
     bool stamped{};
     uint64_t stamps[3]{};
-    bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: the next one needs no k_begin
+    bool clean{}; // control words, counts and task slots are as k_finish_small leaves them: no k_begin for the next one
     bool counted{true}; // the last batch's status (OK) and work counters are on the host: a small batch, or none yet
-    // the last host batch was a small one: its timeline is in `stamps`, and if its results took the general passes, their
-    // time is between tl_t0 and tl_done
+    // the last host batch was a small one: its timeline is in `stamps`, and if its results took the general passes,
+    // their time is between tl_t0 and tl_done
     bool tl_stamped{}, tl_passes{};
     bool held{}; // the device buffers hold the results of the last batch (false before one, and once they have grown)
     // the last host batch's results: in h_small, or in h_roff / h_ids / h_cnt
@@ -761,8 +763,8 @@ void drop_graph(hibf_gpu_agent * a)
         HG_CUDA(cudaGraphExecDestroy(graph));
 }
 
-// Grows the buffers of one capacity.  A buffer that could not be allocated is null, so the capacity is 0 until all of them
-// are there; when they cannot be had, the size before is allocated again and later batches run as before.
+// Grows the buffers of one capacity.  A buffer that could not be allocated is null, so the capacity is 0 until all of
+// them are there; when they cannot be had, the size before is allocated again and later batches run as before.
 template <typename Allocate>
 void grow(uint64_t & capacity, uint64_t want, Allocate const & allocate)
 {
@@ -899,9 +901,9 @@ size_t query_smem(hibf_gpu_hibf const * h)
     return static_cast<size_t>(8) * h->counters_per_warp * sizeof(uint32_t);
 }
 
-// Launches a kernel that may become resident while the one before it on the agent's stream still runs, and then waits for
-// that one's end itself (wait_for_prerequisites): its launch costs no gap.  A kernel that calls launch_dependents lets
-// it in early.  `beside` false (in a stream capture): an ordinary launch.
+// Launches a kernel that may become resident while the one before it on the agent's stream still runs, and then waits
+// for that one's end itself (wait_for_prerequisites): its launch costs no gap.  A kernel that calls launch_dependents
+// lets it in early.  `beside` false (in a stream capture): an ordinary launch.
 template <typename... P, typename... A>
 void launch_beside(hibf_gpu_agent * a, bool beside, void (*kernel)(P...), unsigned grid, unsigned block, A... args)
 {
@@ -947,11 +949,12 @@ void launch_postprocess(hibf_gpu_agent * a, uint64_t nq, int mode, int width)
     bool const beside = cap == cudaStreamCaptureStatusNone;
     launch_beside(
         a, beside, k_scatter, grid_cap(a->cap_results, 256, 8), 256, a->ctrl.as<unsigned long long>(),
-        a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(), a->rec_cnt.as<unsigned long long>(), a->cap_results, a->roff.as<unsigned long long>(),
-        a->qcount.as<unsigned int>(), a->out_ids.as<uint64_t>(), a->out_cnt.as<uint64_t>());
+        a->rec_q.as<uint32_t>(), a->rec_ub.as<uint32_t>(), a->rec_cnt.as<unsigned long long>(), a->cap_results,
+        a->roff.as<unsigned long long>(), a->qcount.as<unsigned int>(), a->out_ids.as<uint64_t>(),
+        a->out_cnt.as<uint64_t>());
     bool const narrow = mode == HIBF_GPU_QUERY_COUNT && width != 8;
-    // few queries: one per block, which a long segment takes whole; from a full wave of warps on, up to 32 per warp (most
-    // have no result or one)
+    // few queries: one per block, which a long segment takes whole; from a full wave of warps on, up to 32 per warp
+    // (most have no result or one)
     unsigned const sort_grid = grid_cap(nq, 1, 6);
     uint32_t const per =
         static_cast<uint32_t>(std::min<uint64_t>(32, (nq + 8ull * sort_grid - 1) / (8ull * sort_grid)));
@@ -981,9 +984,9 @@ void launch_begin(hibf_gpu_agent * a, uint64_t pending, uint64_t nq, uint64_t ma
 }
 
 // Whether the workers of an ordered batch keep their tasks' first children (query.cuh): where L2 holds (most of) the
-// hierarchy, the line lying between 127 and 255 MB with 129 MB of L2.  20,000 queries of 8,192 user bins, longest first, us with children kept and
-// queued: 63 MB 227 / 234, 127 MB 235 / 242, 255 MB 254 / 251, 637 MB 423 / 323, 3.8 GB 814 / 719; 60,000 of them 601 /
-// 622, 624 / 637, 675 / 659, 1,219 / 861, 2,361 / 2,033.
+// hierarchy, the line lying between 127 and 255 MB with 129 MB of L2.  20,000 queries of 8,192 user bins, longest
+// first, us with children kept and queued: 63 MB 227 / 234, 127 MB 235 / 242, 255 MB 254 / 251, 637 MB 423 / 323, 3.8
+// GB 814 / 719; 60,000 of them 601 / 622, 624 / 637, 675 / 659, 1,219 / 861, 2,361 / 2,033.
 bool keeps_first_child(hibf_gpu_hibf const * h)
 {
     int dev = 0, l2 = 0;
@@ -1089,8 +1092,7 @@ void launch_batch(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
         }
         else
         {
-            (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256,
-                                                                                               query_smem(h), s>>>(p);
+            (blk ? query_block_kernel(h) : query_kernel(h, a->variant))<<<grid, 256, query_smem(h), s>>>(p);
             HG_CUDA(cudaGetLastError());
         }
         HG_CUDA(cudaEventRecordWithFlags(a->ev_k1, s, rec_flags));
@@ -1120,8 +1122,7 @@ void launch_plain(hibf_gpu_agent * a, int mode, uint64_t const * d_values, uint6
         p.self_init = 1;
         HG_CUDA(cudaMemsetAsync(a->tasks.p, 0xFF, std::min<uint64_t>(a->cap_tasks, 64u * h->n_ibfs + 64u) * 8, s));
         p.task_cap = std::min<uint64_t>(a->cap_tasks, 64u * h->n_ibfs + 64u);
-        (a->tune.block_queries ? query_block_kernel(h) : query_kernel(h, a->variant))<<<
-            1, 256, query_smem(h), s>>>(p);
+        (a->tune.block_queries ? query_block_kernel(h) : query_kernel(h, a->variant))<<<1, 256, query_smem(h), s>>>(p);
         HG_CUDA(cudaGetLastError());
     }
     launch_postprocess(a, nq, mode, width);
@@ -1365,8 +1366,8 @@ void ensure_timeline(hibf_gpu_agent * a, uint32_t n)
 }
 
 // A host batch of at most kSmallBatch queries that runs a task per block (or is one plain query): one copy in (two when
-// the values do not fit the packed buffer), the query kernel, k_finish_small, one wait.  kRerun: not a small batch, or a
-// capacity was exceeded (now larger): the general path starts over; kCounted: more results than
+// the values do not fit the packed buffer), the query kernel, k_finish_small, one wait.  kRerun: not a small batch, or
+// a capacity was exceeded (now larger): the general path starts over; kCounted: more results than
 // k_finish_small takes, they wait in the workspace for the general passes.  One plain query of 250 values on 8,192 user
 // bins took 105 us through the general path: three waits, a dozen launches, memsets and copies.
 enum class small_result

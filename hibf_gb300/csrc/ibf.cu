@@ -88,8 +88,8 @@ __global__ void k_synth_emplace(uint64_t * __restrict__ words, uint64_t bin_size
 // IBF that tracks occupancy inserts in chunks, in two passes.  The first enters every position (row * tb + bin) that is
 // still unset into a hash table and lowers the position's entry to the chunk's first value there; the second counts a
 // value that is first at one of its positions and sets its bits.  Both are bound by random accesses that L2 serves (the
-// table of a chunk is at most 100 MB): 530,624 values with h = 2 take 41 us; sorting the positions took 14 launches, 260
-// us, and as much again in allocations.
+// table of a chunk is at most 100 MB): 530,624 values with h = 2 take 41 us; sorting the positions took 14 launches,
+// 260 us, and as much again in allocations.
 // ---------------------------------------------------------------------------------------------------------------
 constexpr unsigned long long kFreeEntry = ~0ull;
 constexpr uint32_t kIsSet = ~0u; // the entry of a position whose bit was set before the chunk, or of no position
@@ -106,10 +106,10 @@ __device__ __forceinline__ uint64_t occ_value(uint64_t const * values, uint64_t 
         return values[i];
 }
 
-// The table has mask + 1 slots (a power of two, at least 1.5 per position, so that a free one is always found): keys and
-// the lowest value index per key.  entries[i * h + k]: the slot of value i's position k.  A value that repeats the one
-// before it in its bin is not entered: that one has its positions and comes first.  (2^20 times one value, h = 2: every
-// position queued for two addresses, 1,715 us a call, now 85.)
+// The table has mask + 1 slots (a power of two, at least 1.5 per position, so that a free one is always found): keys
+// and the lowest value index per key.  entries[i * h + k]: the slot of value i's position k.  A value that repeats the
+// one before it in its bin is not entered: that one has its positions and comes first.  (2^20 times one value, h = 2:
+// every position queued for two addresses, 1,715 us a call, now 85.)
 template <bool SYNTH>
 __global__ void k_occ_enter(uint64_t const * __restrict__ words, uint64_t bin_size, uint32_t row_words, uint32_t shift,
                             uint32_t h, uint64_t const * __restrict__ values, uint64_t const * __restrict__ bins,
@@ -250,12 +250,12 @@ __global__ void k_widen(uint64_t * __restrict__ dst, uint32_t dst_row_words, uin
     }
 }
 
-// bulk_contains (src/interleaved_bloom_filter.cpp:204-291) for many values with H hash functions: out[v * bin_words + j]
-// = AND of word j of the h rows.  The same work mapping as the counting loop (count.cuh) -- LPV lanes per row, lanes
+// bulk_contains (src/interleaved_bloom_filter.cpp:204-291) for many values with H hash functions: out[v * bin_words +
+// j] = AND of word j of the h rows.  The same work mapping as the counting loop (count.cuh) -- LPV lanes per row, lanes
 // hash U values each, the H row words of four sub-steps are loaded together (4 * H loads per lane in flight) -- and
-// each lane stores its word of the AND.  The grid's first dimension is the slab (LPV words) of a row wider than a warp, so
-// that blocks which start together read the pieces of the same rows.  A warp takes all values that it hashes at once, or
-// (FEW, rows of four words and more) only those whose words it loads together.
+// each lane stores its word of the AND.  The grid's first dimension is the slab (LPV words) of a row wider than a warp,
+// so that blocks which start together read the pieces of the same rows.  A warp takes all values that it hashes at
+// once, or (FEW, rows of four words and more) only those whose words it loads together.
 template <int LPV, int H, typename R, bool FEW>
 __global__ void __launch_bounds__(256) k_bulk_contains_h(row_params row, uint64_t const * __restrict__ values,
                                                          uint64_t n, uint64_t * __restrict__ out)
@@ -365,8 +365,8 @@ contains_kernel_t contains_kernel(uint64_t h, uint32_t lpv_log2, bool few)
 }
 
 // The end of a counting block: the sum of its warps' counters, in the caller's width.  A block on its own in its slab
-// writes its sums, else the slab's last block (by ticket) writes the totals, and with `reset` leaves totals and ticket at
-// 0 for the next call.  (Clearing before and a storing kernel after cost a read of 250 values on 64 bins 5 of its 36
+// writes its sums, else the slab's last block (by ticket) writes the totals, and with `reset` leaves totals and ticket
+// at 0 for the next call.  (Clearing before and a storing kernel after cost a read of 250 values on 64 bins 5 of its 36
 // us.)
 __device__ __forceinline__ void finish_counts(uint32_t const * s_counts, uint32_t n_counters, uint32_t w0,
                                               uint32_t slab_words, unsigned long long * totals, unsigned int * ticket,
@@ -413,13 +413,14 @@ __device__ __forceinline__ void finish_counts(uint32_t const * s_counts, uint32_
 
 // bulk_count over n values into one counting vector: every warp counts a contiguous chunk into shared counters of its
 // own (planes_flush_to, no shared-memory atomics), the block adds them up and to the 64-bit global totals.
-// Four blocks per SM (64 registers) measured faster than two (1.53 vs 2.16 ms for 2^24 values on 1,024 bins, h = 3): more
-// warps keep more row loads in flight.  For h of 4 and 5, whose rows fill more registers, three blocks: a million values
-// on 64 bins, h = 5, took 70 us with four, which spill.
+// Four blocks per SM (64 registers) measured faster than two (1.53 vs 2.16 ms for 2^24 values on 1,024 bins, h = 3):
+// more warps keep more row loads in flight.  For h of 4 and 5, whose rows fill more registers, three blocks: a million
+// values on 64 bins, h = 5, took 70 us with four, which spill.
 // The grid's first dimension is the slab of a row wider than a warp: a block counts LPV words of every row, a warp one
 // piece of 128 or 256 bytes per value and hash function.  (Rows wider than a warp were counted one value
 // at a time, every set bit by an atomic: 200,003 values on 8,192 bins, h = 2, counted and looked up took 9.43 ms; 0.21
-// with this kernel, 0.20 with the asynchronous one below.)  One kernel per row width: with all six in one the loop spilled 156 bytes per thread at h = 3.
+// with this kernel, 0.20 with the asynchronous one below.)  One kernel per row width: with all six in one the loop
+// spilled 156 bytes per thread at h = 3.
 constexpr unsigned count_blocks_per_sm(int h)
 {
     return h <= 3 ? 4 : 3;
@@ -452,13 +453,13 @@ __global__ void __launch_bounds__(256, count_blocks_per_sm(H))
     finish_counts(s_counts, n_counters, w0, rp.bin_words, totals, tickets + blockIdx.x, reset, bins, width, out);
 }
 
-// The same count with one or two hash functions for rows, or slabs of rows, of 9 to 16 words (128-byte pieces) and calls
-// that fill the GPU: the pieces go to shared memory by asynchronous copies, three stages of eight values ahead of their
-// use, so that reads are in flight all the time and hold no registers; the loop above issues a group, waits for it and
-// adds it up.  Eight lanes copy a piece (16 bytes each), 16 lanes add it up (one word each).  8,192 bins, a million
-// values, h = 1: 331 -> 229 us; 2,048 bins, h = 2: 133 -> 89; 600 bins, h = 1: 69 -> 53.  With three hash functions and
-// more the loop above has enough reads in flight (1,000 bins, h = 3, four million values: 254 us against 271 here), so
-// they have no asynchronous form.
+// The same count with one or two hash functions for rows, or slabs of rows, of 9 to 16 words (128-byte pieces) and
+// calls that fill the GPU: the pieces go to shared memory by asynchronous copies, three stages of eight values ahead of
+// their use, so that reads are in flight all the time and hold no registers; the loop above issues a group, waits for
+// it and adds it up.  Eight lanes copy a piece (16 bytes each), 16 lanes add it up (one word each).  8,192 bins, a
+// million values, h = 1: 331 -> 229 us; 2,048 bins, h = 2: 133 -> 89; 600 bins, h = 1: 69 -> 53.  With three hash
+// functions and more the loop above has enough reads in flight (1,000 bins, h = 3, four million values: 254 us against
+// 271 here), so they have no asynchronous form.
 constexpr int kAsyncStages = 4;      // stages in the ring of a warp
 constexpr int kAsyncValues = 8;      // values per stage
 constexpr int kAsyncWarps = 4;       // warps per block
@@ -590,8 +591,8 @@ __global__ void __launch_bounds__(32 * kAsyncWarps, async_blocks_per_sm<H>())
     finish_counts(s_counts, n_counters, w0, rp.bin_words, totals, tickets + blockIdx.x, reset, bins, width, out);
 }
 
-using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *, unsigned int *,
-                                     bool, uint64_t, int, void *);
+using bulk_count_kernel_t = void (*)(row_params, uint64_t const *, uint64_t, uint64_t, unsigned long long *,
+                                     unsigned int *, bool, uint64_t, int, void *);
 
 template <int H, typename R>
 bulk_count_kernel_t bulk_count_kernel_h(uint32_t lpv_log2)
@@ -646,9 +647,9 @@ async_count async_count_h(bool wide)
                        async_blocks_per_sm<H>()};
 }
 
-// Whether a call of n values over `slabs` pieces per row is large enough for the asynchronous kernel: its warps then have
-// some 100 values each.  (1,000 bins, h = 2: 100,000 values 25 us against 26, 300,000 34 against 33; 2,048 bins, 100,000
-// values 31 against 27; 8,192 bins, h = 1, 10,000 values 22.3 against 21.7, 30,000 30 against 26.)
+// Whether a call of n values over `slabs` pieces per row is large enough for the asynchronous kernel: its warps then
+// have some 100 values each.  (1,000 bins, h = 2: 100,000 values 25 us against 26, 300,000 34 against 33; 2,048 bins,
+// 100,000 values 31 against 27; 8,192 bins, h = 1, 10,000 values 22.3 against 21.7, 30,000 30 against 26.)
 bool async_count_pays(uint64_t h, uint64_t bin_words, uint64_t n, uint32_t slabs)
 {
     return h <= 2 && bin_words > kAsyncWords / 2 && n * slabs >= 200000;
@@ -758,8 +759,8 @@ struct hibf_gpu_ibf
     bool track_occupancy{};
     dbuf store;     // bin_size * row_words words
     dbuf occupancy; // technical_bins counters
-    // bulk_count's scratch, technical_bins 64-bit totals and a ticket per slab: device-pointer calls clear theirs, host-
-    // pointer calls, one at a time, leave host_totals at 0
+    // bulk_count's scratch, technical_bins 64-bit totals and a ticket per slab: device-pointer calls clear theirs,
+    // host-pointer calls, one at a time, leave host_totals at 0
     std::mutex count_mu;
     count_scratch totals[kCountStreams];
     uint32_t n_totals{};
@@ -778,25 +779,25 @@ struct hibf_gpu_ibf
     row_params rp() const
     {
         return row_params{store.as<uint64_t>(), bin_size, static_cast<uint32_t>(row_words),
-                          static_cast<uint32_t>(bin_words), shift, static_cast<uint32_t>(hash_funs)};
+                          static_cast<uint32_t>(bin_words), shift};
     }
     bool wide_rows() const // the kernels take 64-bit row indices
     {
         return bin_size > UINT32_MAX;
     }
-    // Lanes (log2) that read a row, or a slab of a row, for n values.  Rows of up to 16 words are read whole.  Wider ones
-    // are counted in slabs of 16 words: with 32, whose counters leave room for three blocks per SM, 8,192 bins (h = 1, a
-    // million values) took 421 us against 336, 3,000 values 24 against 18.  Only long calls on rows of 17 to 31 words
-    // take one slab of 32 (1,500 bins, h = 4, 300,000 values: 64 us against 71).
+    // Lanes (log2) that read a row, or a slab of a row, for n values.  Rows of up to 16 words are read whole.  Wider
+    // ones are counted in slabs of 16 words: with 32, whose counters leave room for three blocks per SM, 8,192 bins (h
+    // = 1, a million values) took 421 us against 336, 3,000 values 24 against 18.  Only long calls on rows of 17 to 31
+    // words take one slab of 32 (1,500 bins, h = 4, 300,000 values: 64 us against 71).
     uint32_t count_lanes_log2(uint64_t n) const
     {
         if (bin_words <= 16)
             return lanes_log2(static_cast<uint32_t>(bin_words));
         return bin_words < kSlabWords && n > (1u << 17) ? 5 : 4;
     }
-    // bulk_contains keeps no counters, so long calls read slabs of 32 words where those leave at most half a slab idle at
-    // the row's end (2,048 bins, h = 2, a million values: 119 us against 123 with slabs of 16; 3,000 values 10.3 against
-    // 8.4; 2,500 bins, 40 words, 238 us with slabs of 16 and 251 with 32).
+    // bulk_contains keeps no counters, so long calls read slabs of 32 words where those leave at most half a slab idle
+    // at the row's end (2,048 bins, h = 2, a million values: 119 us against 123 with slabs of 16; 3,000 values 10.3
+    // against 8.4; 2,500 bins, 40 words, 238 us with slabs of 16 and 251 with 32).
     uint32_t contains_lanes_log2(uint64_t n) const
     {
         if (bin_words <= 16)
@@ -822,9 +823,9 @@ cudaStream_t pick(hibf_gpu_ibf * f, void * s)
     return s ? static_cast<cudaStream_t>(s) : f->stream;
 }
 
-// Occupancy in insertion order and the bits, chunk by chunk; chunks run one after the other, so each sees the bits of the
-// chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).  Calls on several streams take
-// turns.
+// Occupancy in insertion order and the bits, chunk by chunk; chunks run one after the other, so each sees the bits of
+// the chunks before it.  SYNTH: the n values are the generated values of bin `bin` (vpb per bin).  Calls on several
+// streams take turns.
 template <bool SYNTH>
 void emplace_exact(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t const * d_bins, uint64_t n, uint64_t bin,
                    uint64_t seed, uint64_t vpb, cudaStream_t s)
@@ -973,10 +974,10 @@ void launch_count(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int wid
     }
     unsigned const block = 256;
     // One contiguous chunk per warp of a full wave, over all slabs: as many blocks of 8 warps per SM as the kernel is
-    // built for, or the 3 whose 64 KiB of counters fit where a slab is 32 words.  A chunk is at least 32 values, one per
-    // lane: a call of 250 values then runs on eight warps of one block instead of one warp, one of 10,000 on 40 SMs
-    // (with chunks of 512: 1,000 bins, h = 3, 10,000 values 92 us, now 18).  From 128 values on, narrow rows round it to
-    // whole passes of four values per lane.
+    // built for, or the 3 whose 64 KiB of counters fit where a slab is 32 words.  A chunk is at least 32 values, one
+    // per lane: a call of 250 values then runs on eight warps of one block instead of one warp, one of 10,000 on 40 SMs
+    // (with chunks of 512: 1,000 bins, h = 3, 10,000 values 92 us, now 18).  From 128 values on, narrow rows round it
+    // to whole passes of four values per lane.
     uint32_t const lanes = f->count_lanes_log2(n);
     uint32_t const slabs = f->slabs(lanes);
     bool const full_slabs = lanes == 5;
@@ -995,7 +996,8 @@ void launch_count(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int wid
                                                       : bulk_count_kernel<uint32_t>(f->hash_funs, lanes);
     if (smem > 48 * 1024)
         HG_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-    kernel<<<dim3(slabs, grid), block, smem, s>>>(f->rp(), values, n, chunk, totals, tickets, reset, f->bins, width, out);
+    kernel<<<dim3(slabs, grid), block, smem, s>>>(f->rp(), values, n, chunk, totals, tickets, reset, f->bins, width,
+                                                  out);
     HG_CUDA(cudaGetLastError());
 }
 
@@ -1015,12 +1017,12 @@ void launch_contains(hibf_gpu_ibf * f, uint64_t const * d_values, uint64_t n, ui
     HG_CUDA(cudaGetLastError());
 }
 
-constexpr uint64_t kDeviceCheck = 1u << 14; // host-pointer inserts of this many values have their bins checked on the device
+constexpr uint64_t kDeviceCheck = 1u << 14; // host-pointer inserts of as many values check their bins on the device
 constexpr uint64_t kSmallBytes = 64u << 10; // host-pointer calls of up to this many bytes in and out need no copies
 
 // bulk_count of host values, finished on return: the counts in page-locked memory of the filter, valid until its next
-// host-pointer call (the caller holds f->mu).  Few values are read in place by the kernel, others are copied; the kernel
-// writes the counts to the host.
+// host-pointer call (the caller holds f->mu).  Few values are read in place by the kernel, others are copied; the
+// kernel writes the counts to the host.
 void const * count_host(hibf_gpu_ibf * f, uint64_t const * values, uint64_t n, int width)
 {
     if (!f->host_totals.p || f->host_totals.bytes < count_scratch_bytes(f))
@@ -1263,8 +1265,8 @@ extern "C"
             {
                 if (!f || (n && (!values || !bins)))
                     fail(HIBF_GPU_ERR_INVALID_ARG, "null argument");
-                // Nothing is inserted if any bin is out of range.  Many bins are checked on the device, beside the copy of
-                // the values (the host reads 530,624 of them in 0.2 ms, about as long as everything else takes).
+                // Nothing is inserted if any bin is out of range.  Many bins are checked on the device, beside the copy
+                // of the values (the host reads 530,624 of them in 0.2 ms, about as long as everything else takes).
                 bool const on_device = n >= kDeviceCheck;
                 for (uint64_t i = 0; i < n && !on_device; ++i)
                     if (bins[i] >= f->bins)

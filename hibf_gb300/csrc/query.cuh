@@ -4,10 +4,10 @@
 // Query semantics (membership_for_impl HIBF.hpp:322-355, bulk_count_impl HIBF.hpp:463-496): for a query and an IBF,
 // count every value per technical bin, then scan the bins in order adding each bin's count to a running sum in the
 // counter type: deleted -> no report, no reset;   merged -> descend if sum >= t, reset;   last bin of a user bin ->
-// report if sum >= t, reset.  Per bin the host precomputes MERGED, DELETED, RUN_END (last bin of a user bin's run) and HEAD (first bin
-// of a summation segment: bin 0 or the bin after a MERGED / RUN_END bin), which turns the scan into a segmented
-// prefix sum, done 32 bins at a time by a warp.  Counter wraparound: exact sums reduced modulo 2^(8*width) before
-// the comparison equal the reference's wrapping value_t sums.
+// report if sum >= t, reset.  Per bin the host precomputes MERGED, DELETED, RUN_END (last bin of a user bin's run) and
+// HEAD (first bin of a summation segment: bin 0 or the bin after a MERGED / RUN_END bin), which turns the scan into a
+// segmented prefix sum, done 32 bins at a time by a warp.  Counter wraparound: exact sums reduced modulo 2^(8*width)
+// before the comparison equal the reference's wrapping value_t sums.
 //
 // Work queue: task = (query, depth, IBF).  Claim indices below n_queries are the implicit root tasks; children are
 // appended behind them.  A worker that claims an index whose task is not written yet waits (bounded by a time
@@ -468,7 +468,8 @@ __device__ __forceinline__ void count_variant(row_params const & rp, uint32_t lp
         if constexpr (V == 0)
 #pragma unroll 1
             for (uint32_t w0 = 0; w0 < rp.bin_words; w0 += kSlabWords) // one slab unless the row is wider than a warp
-                warp_count<R, 32, H, Q::K>(row_slab(rp, w0, kSlabWords), vals, n, counts + 64u * w0, lane, w0 ? nullptr : stage);
+                warp_count<R, 32, H, Q::K>(row_slab(rp, w0, kSlabWords), vals, n, counts + 64u * w0, lane,
+                                           w0 ? nullptr : stage);
     }
 }
 
@@ -692,7 +693,7 @@ __device__ void process_task(query_params const & p, unsigned long long task, ui
     for (uint32_t i = lane; i < ncount; i += 32)
         counts[i] = 0;
     __syncwarp();
-    row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift, nd.hash_funs};
+    row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift};
     // Count in stages; after each stage stop if the outcome is already fixed (segment_state: exact).  One call site
     // of the counting code for the stages and the rest: each call site inlines every row width's counting path, and a
     // hierarchy of mixed widths runs them all at once, so a second copy would double the instruction footprint.
@@ -922,7 +923,7 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
             else
             {
                 if (lane == 0)
-                    task = wait_for_task(p, slot); // a reserved slot: its writer is storing it (values are on the device)
+                    task = wait_for_task(p, slot); // a reserved slot: its writer is storing it (its values are here)
                 task = __shfl_sync(kFullMask, task, 0);
                 if (task == kEmpty)
                     break;
@@ -1015,18 +1016,18 @@ __global__ void __launch_bounds__(256, HIBF_QUERY_MIN_BLOCKS) k_query(__grid_con
 //
 // A task is a chain of dependent accesses (claim, task, IBF, values, rows, bin tables, results), about 10 us of which
 // little is work, so the chain is kept short: the block goes on with its task's first child (no queue, no claim, the
-// query's bounds at hand), the bin tables are on their way while the values are counted, and a block on its own looks at
-// the count of unfinished tasks before it claims a slot nobody will fill.  p.stage (optional): the values are the
+// query's bounds at hand), the bin tables are on their way while the values are counted, and a block on its own looks
+// at the count of unfinished tasks before it claims a slot nobody will fill.  p.stage (optional): the values are the
 // host's memory; roots store what they read there, at the same positions, and the other tasks read it.
 constexpr unsigned long long kSkipTask = kEmpty - 1u; // an order entry that was not a query index
 
-// Whether a task of n values keeps its first child: what that saves is a queue's latency, and what it costs is that other
-// blocks cannot share a long descent and that the levels do not have L2 to themselves one by one.  So long tasks keep
-// theirs only while there is a block per query, short ones also when there are several queries per block, and in between
-// those of the roots that the blocks claim first (500 queries of 1,000 values on 65,536 user bins: 100 us with all kept, 83
-// so, 90 before any was).  2,000 queries on 8,192 user bins, us with the child queued and kept: 500 values 144 / 131,
-// 1,000 216 / 221, 1,500 305 / 324, 3,000 576 / 616, 10,000 1,866 / 2,014; on 65,536: 500 values 216 / 198, 1,000 275 / 259,
-// 1,500 324 / 308, 3,000 485 / 478, 10,000 1,189 / 1,204.
+// Whether a task of n values keeps its first child: what that saves is a queue's latency, and what it costs is that
+// other blocks cannot share a long descent and that the levels do not have L2 to themselves one by one.  So long tasks
+// keep theirs only while there is a block per query, short ones also when there are several queries per block, and in
+// between those of the roots that the blocks claim first (500 queries of 1,000 values on 65,536 user bins: 100 us with
+// all kept, 83 so, 90 before any was).  2,000 queries on 8,192 user bins, us with the child queued and kept: 500 values
+// 144 / 131, 1,000 216 / 221, 1,500 305 / 324, 3,000 576 / 616, 10,000 1,866 / 2,014; on 65,536: 500 values 216 / 198,
+// 1,000 275 / 259, 1,500 324 / 308, 3,000 485 / 478, 10,000 1,189 / 1,204.
 constexpr uint64_t kKeepValues = 1536;
 __device__ __forceinline__ bool keeps_child(uint64_t n, bool first, uint64_t n_queries)
 {
@@ -1140,7 +1141,7 @@ __global__ void __launch_bounds__(kBlkThreadsMax, 1) k_query_blk(__grid_constant
             for (uint32_t i = 16u * lane; i < nd.bins; i += 512u)
                 asm volatile("prefetch.global.L1 [%0];" ::"l"(p.descs + nd.desc_offset + i));
         __syncwarp();
-        row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift, nd.hash_funs};
+        row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift};
         uint64_t const per = (n + nwarps - 1) / nwarps;
         uint64_t const lo = min(n, static_cast<uint64_t>(warp) * per);
         uint64_t const hi = min(n, lo + per);
@@ -1180,7 +1181,8 @@ constexpr int kCostFeatures = 6;
 using features_kernel_t = void (*)(query_params, uint32_t, float *);
 
 template <int H, typename R>
-__global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_params const p, uint32_t probe, float * __restrict__ out)
+__global__ void __launch_bounds__(256)
+    k_query_features(__grid_constant__ query_params const p, uint32_t probe, float * __restrict__ out)
 {
     extern __shared__ uint32_t s_counts[];
     int const lane = threadIdx.x & 31;
@@ -1188,7 +1190,7 @@ __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_
     uint64_t const warp = (blockIdx.x * static_cast<uint64_t>(blockDim.x) + threadIdx.x) >> 5;
     uint64_t const nwarps = (static_cast<uint64_t>(gridDim.x) * blockDim.x) >> 5;
     dev_node const nd = p.nodes[0];
-    row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift, nd.hash_funs};
+    row_params const rp{nd.words, nd.bin_size, nd.row_words, nd.bin_words, nd.hash_shift};
     uint32_t const ncount = row_counters(nd.bin_words);
     uint2 const * d = p.descs + nd.desc_offset;
     for (uint64_t q = warp; q < p.n_queries; q += nwarps)
@@ -1258,8 +1260,8 @@ __global__ void __launch_bounds__(256) k_query_features(__grid_constant__ query_
     }
 }
 
-// The kernel of variant v (0 <= v < kQueryVariants; H > 3 has the default variant only).  `wide`: some IBF has 2^32 rows
-// or more, so row indices are 64 bits wide (the default variant only; a schedule does not change results).
+// The kernel of variant v (0 <= v < kQueryVariants; H > 3 has the default variant only).  `wide`: some IBF has 2^32
+// rows or more, so row indices are 64 bits wide (the default variant only; a schedule does not change results).
 template <int H>
 query_kernel_t query_kernel_variant(int v, bool wide)
 {

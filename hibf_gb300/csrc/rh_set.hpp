@@ -108,8 +108,9 @@ public:
         if (num_ == 0)
             return;
         size_t const n = with_buffer(mask_ + 1);
-        // Eight info bytes at a time (info_ has n + 8), the occupied ones by their bits: a branch per slot is mispredicted
-        // every other time in a half-full table, and a set cleared after a large user bin is mostly empty slots.
+        // Eight info bytes at a time (info_ has n + 8), the occupied ones by their bits: a branch per slot is
+        // mispredicted every other time in a half-full table, and a set cleared after a large user bin is mostly empty
+        // slots.
         constexpr uint64_t low = 0x7F7F7F7F7F7F7F7FULL;
         for (size_t i = 0; i < n; i += 8)
         {
@@ -282,8 +283,8 @@ private:
     std::vector<uint8_t> info_;
 };
 
-// Inserts keys in the order given, each a few keys after its cache lines were asked for: the inserts of a large set wait
-// for memory (two lines per key), and each depends on the table the one before left.
+// Inserts keys in the order given, each a few keys after its cache lines were asked for: the inserts of a large set
+// wait for memory (two lines per key), and each depends on the table the one before left.
 class rh_feeder
 {
 public:

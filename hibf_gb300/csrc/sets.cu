@@ -3,12 +3,12 @@
 // The reference reads every user bin into a hash set (compute_kmers, src/build/compute_kmers.cpp:23-32) and sizes a
 // merged max bin by the distinct count of its subtree's union (src/hierarchical_interleaved_bloom_filter.cpp:39-171,
 // the favourite child's kmers).  Here both are hash tables on the device:
-//   distinct_sets_device  every user bin's distinct values in first-appearance order: a table entry per (user bin, value)
+//   distinct_sets_device  every user bin's distinct values in first-appearance order: an entry per (user bin, value)
 //                         keeps the value's first position, the values at such positions are compacted in order;
 //   union_size_device     the distinct count of the union of some user bins' sets: the number of table entries.
 // Bound by the table's random accesses (a 4-byte slot and the value it names, both in L2 for a few million values): the
-// 64-user-bin workload, 1.47e6 values, takes 50 us of kernels; a segmented sort, a selection and a sort back took 2.1 ms,
-// and a dozen buffers were allocated for them.
+// 64-user-bin workload, 1.47e6 values, takes 50 us of kernels; a segmented sort, a selection and a sort back took 2.1
+// ms, and a dozen buffers were allocated for them.
 // Only the order of split user bins' values depends on the reference's hash set (robin_hood iteration order); the
 // host replays that from the first-appearance order these produce.
 #include <algorithm>
@@ -26,7 +26,7 @@ int sm_count();
 namespace
 {
 
-constexpr uint64_t kBatchValues = 1ull << 30; // values per device batch (CUB's segmented sort counts items in int)
+constexpr uint64_t kBatchValues = 1ull << 30; // values per device batch (positions and user bin bounds are ints)
 
 constexpr uint32_t kFreeSlot = ~0u;
 

@@ -267,9 +267,10 @@ class _agent_base:
         """All queries in one persistent launch.  Returns (offsets, ids, counts); ids ascending per query; counts
         (mode COUNT) are the non-zero entries of each dense counting vector.  Values in page-locked memory are read
         in place by the kernel (and pageable ones of up to 64 MiB where the GPU goes through the host's page tables);
-        batches of at least 64 MiB of pageable values are copied in chunks while the kernel answers the chunks already copied (input_chunks() reports how many).  The arrays are copies, or with
-        copy=False views of the agent's page-locked result buffers, valid until the agent's next call (as the
-        reference's agents hand out their own result buffers)."""
+        batches of at least 64 MiB of pageable values are copied in chunks while the kernel answers the chunks already
+        copied (input_chunks() reports how many).  The arrays are copies, or with copy=False views of the agent's
+        page-locked result buffers, valid until the agent's next call (as the reference's agents hand out their own
+        result buffers)."""
         v, qo = _u64(values), _u64(query_offsets)
         nq = qo.size - 1
         t = _u64(thresholds)
@@ -329,8 +330,8 @@ class _agent_base:
         return [float(out[i]) for i in range(min(n.value, 16))]
 
     def set_host_read(self, in_place: bool) -> None:
-        """Host batches in mapped page-locked memory (and smaller pageable ones, where the GPU goes through the host's page
-        tables) are read in place by the kernel (the default) or copied first."""
+        """Host batches in mapped page-locked memory (and smaller pageable ones, where the GPU goes through the host's
+        page tables) are read in place by the kernel (the default) or copied first."""
         N.call("hibf_gpu_agent_set_host_read", self._a, int(in_place))
 
     def last_in_place(self) -> bool:

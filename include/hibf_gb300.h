@@ -345,9 +345,9 @@ int hibf_gpu_agent_query_batch(hibf_gpu_agent * a, int mode, uint64_t const * va
                                int width, uint64_t const ** result_offsets, uint64_t const ** result_ids,
                                void const ** result_counts);
 /* Device form: inputs already in HBM; results stay in the agent's device buffers (returned as device pointers).
- * Asynchronous on the agent's stream; hibf_gpu_agent_status() after synchronising gives OVERFLOW / TIMEOUT.  A caller may
- * capture it into a graph of its own and replay that between the agent's other calls; such a graph holds the workspace's
- * addresses, so the agent must have room for its largest batch (hibf_gpu_agent_reserve) before the capture. */
+ * Asynchronous on the agent's stream; hibf_gpu_agent_status() after synchronising gives OVERFLOW / TIMEOUT.  A caller
+ * may capture it into a graph of its own and replay that between the agent's other calls; such a graph holds the
+ * workspace's addresses, so the agent must have room for its largest batch before (hibf_gpu_agent_reserve). */
 int hibf_gpu_agent_query_batch_d(hibf_gpu_agent * a, int mode, uint64_t const * d_values,
                                  uint64_t const * d_query_offsets, uint64_t n_queries, uint64_t const * d_thresholds,
                                  int width, uint64_t const ** d_result_offsets, uint64_t const ** d_result_ids,
@@ -366,9 +366,9 @@ int hibf_gpu_agent_status(hibf_gpu_agent * a);
  * HIBF_GPU_ERR_TIMEOUT through the device status word.  Returns OK when it did; the context stays usable. */
 int hibf_gpu_agent_selftest_wait_limit(hibf_gpu_agent * a, double limit_ms);
 /* Captures one batch's launch sequence (control reset, persistent kernel, compaction) on fixed device buffers into
- * a CUDA graph owned by the agent; hibf_gpu_agent_replay launches it on the agent's stream.  The graph holds the agent's
- * workspace: a call that grows it (a larger reserve or batch) or changes its schedule, claim order or work array drops
- * the graph, and replay then fails with HIBF_GPU_ERR_INVALID_ARG until the next capture. */
+ * a CUDA graph owned by the agent; hibf_gpu_agent_replay launches it on the agent's stream.  The graph holds the
+ * agent's workspace: a call that grows it (a larger reserve or batch) or changes its schedule, claim order or work
+ * array drops the graph, and replay then fails with HIBF_GPU_ERR_INVALID_ARG until the next capture. */
 int hibf_gpu_agent_capture_batch_d(hibf_gpu_agent * a, int mode, uint64_t const * d_values,
                                    uint64_t const * d_query_offsets, uint64_t n_queries, uint64_t const * d_thresholds,
                                    int width);
@@ -389,8 +389,8 @@ int hibf_gpu_agent_level_work(hibf_gpu_agent * a, uint64_t * tasks, uint64_t * v
  * and the batch runs its configured schedule from the first root.  in_place == 0 copies them first (a batch of 64 MiB
  * or more is then streamed in chunks and runs the work queue).  Pageable values of more than 64 KiB and less than 64
  * MiB are read in place too where the GPU goes through the host's page tables (Grace hosts); others are copied.
- * Results are the same either way; on the 8,192-bin batch (8.1 GB of values) in place took 50.3 ms per call, every call, where the
- * copy's rate varied with the host link (47-344 ms). */
+ * Results are the same either way; on the 8,192-bin batch (8.1 GB of values) in place took 50.3 ms per call, every
+ * call, where the copy's rate varied with the host link (47-344 ms). */
 int hibf_gpu_agent_set_host_read(hibf_gpu_agent * a, int in_place);
 /* Whether the agent's last host batch was read in place (1) or copied (0). */
 int hibf_gpu_agent_last_in_place(hibf_gpu_agent const * a, int * in_place);
