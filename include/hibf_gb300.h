@@ -356,7 +356,8 @@ int hibf_gpu_agent_query_batch_d(hibf_gpu_agent * a, int mode, uint64_t const * 
 int hibf_gpu_agent_query_plain_d(hibf_gpu_agent * a, int mode, uint64_t const * d_values,
                                  uint64_t const * h_query_offsets, uint64_t n_queries, uint64_t const * h_thresholds,
                                  int width);
-/* Copies the results of the agent's last batch (_d or plain) into agent-owned host memory; synchronises. */
+/* Copies the results of the agent's last batch (_d or plain) into agent-owned host memory; synchronises.
+ * HIBF_GPU_ERR_INVALID_ARG when no batch has run since the agent's result buffers last grew. */
 int hibf_gpu_agent_fetch_results(hibf_gpu_agent * a, uint64_t n_queries, int mode, int width,
                                  uint64_t const ** result_offsets, uint64_t const ** result_ids,
                                  void const ** result_counts);
