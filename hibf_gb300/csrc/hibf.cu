@@ -1528,6 +1528,22 @@ void host_batch(hibf_gpu_agent * a, int mode, uint64_t const * values, uint64_t 
                 uint64_t const * thr, int width, bool plain)
 {
     check_batch(mode, width, thr, nq, qoff);
+    // The caller may free its arrays on return, also from an error (a failed launch or allocation) behind a kernel or a
+    // copy that reads them.
+    struct reader_guard
+    {
+        hibf_gpu_agent * a;
+        int before{std::uncaught_exceptions()};
+        ~reader_guard()
+        {
+            if (std::uncaught_exceptions() == before)
+                return;
+            cudaStreamSynchronize(a->stream);
+            if (a->copy_stream)
+                cudaStreamSynchronize(a->copy_stream);
+            (void)cudaGetLastError();
+        }
+    } const readers{a};
     uint64_t const nv = nq ? qoff[nq] : 0;
     // In place: values in mapped page-locked memory are read by the kernel over the host link as it needs them, so
     // no copy precedes (or paces) the launch; only the offsets and thresholds are copied.  So are pageable values too
